@@ -315,11 +315,10 @@ int nv_set_normal_fluid_noise(nv_handle *h, int32_t sys, const double *noise, in
 int nv_set_normal_fluid_grid(nv_handle *h, int32_t sys, const double *u, int32_t nx, int32_t ny, int32_t nz,
                              const double *yp);
 /* Split of the plain FP64 direct sum's work.  64: one thread per target, each summing its
- * terms as it computes them.  1, 2, 4 or 8: a block of 128 threads per that many targets;
- * three warps compute the terms tile by tile and one lane per (target, component) adds them
- * in the reference's order, so a small system still fills the GPU (the result is the same
- * bit for bit).  0 (the default) takes 64 when the direct-sum systems' slots give at least
- * two blocks of 64 per SM, else the largest split with about four blocks per SM. */
+ * terms as it computes them.  1, 2, 4 or 8: a block per that many targets, eight of its warps
+ * computing the terms tile by tile and one lane per (target, component) adding them in the
+ * reference's order, so a small system still fills the GPU (the result is the same bit for
+ * bit).  0 (the default) takes 2, 8 or 64 by the direct-sum systems' slots. */
 int nv_set_direct_split(nv_handle *h, int32_t targets_per_block);
 /* How pclose (systems with tree_theta 0, src/line.f90:135-160) finds each point's nearest
  * live non-neighbour: 0 (the default) from a cell list of the live points, rebuilt on every

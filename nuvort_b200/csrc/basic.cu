@@ -56,9 +56,10 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
   store3(GB, T, (int)g, gb);
   double d[3] = {e_sub(gi[0], x[0]), e_sub(gi[1], x[1]), e_sub(gi[2], x[2])};
   const double c = e_add(e_add(e_sq(d[0]), e_sq(d[1])), e_sq(d[2]));
-  // a segment pinned in front goes into the wall: no Biot-Savart source (timestep.f90:161,187)
+  // a segment pinned in front goes into the wall: no Biot-Savart source (timestep.f90:161,187);
+  // with a zero segment vector its terms drop out by 4ac - b^2 = 0, like an empty slot's
   seg[2 * g] = make_double4(x[0], x[1], x[2], pin_i(pin) ? 0.0 : 1.0);
-  seg[2 * g + 1] = make_double4(d[0], d[1], d[2], c);
+  seg[2 * g + 1] = pin_i(pin) ? make_double4(0, 0, 0, 0) : make_double4(d[0], d[1], d[2], c);
   if (seg32) {  // FP32 record: position split hi + lo (x = hi + lo to ~1e-16), segment vector
     const float h0 = (float)x[0], h1 = (float)x[1], h2 = (float)x[2];
     seg32[3 * g] = make_float4(h0, h1, h2, 1.0f);

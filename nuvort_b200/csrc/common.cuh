@@ -192,6 +192,11 @@ __device__ __forceinline__ void cross3(const double a[3], const double b[3], dou
   c[2] = e_sub(e_mul(a[0], b[1]), e_mul(a[1], b[0]));
 }
 
+__device__ __forceinline__ double4 ldg4(const double4 *p) {
+  const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+  const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
 __device__ __forceinline__ void load3(const double *__restrict__ a, long long T, int g, double v[3]) {
   v[0] = a[g];
   v[1] = a[T + g];
@@ -468,25 +473,4 @@ __device__ __forceinline__ bool mirror_skips_own(const SysConst &sc, int pin_g, 
     w += pin_w(pin_g, c);
   }
   return d == 0 && w < 2;
-}
-
-// One term of biot_savart_mirror (timestep.f90:201-234): segment j (x_j to ghosti_j) reflected
-// in mirror m, its orientation reversed (from the reflected ghost to the reflected point), at
-// target g (position xi, pinned record pin_g, behind pi); false when the reference skips it.
-__device__ __forceinline__ bool mirror_term(const SysConst &sc, int m, const double *__restrict__ X,
-                                            const double *__restrict__ GI, const int *__restrict__ nxt, long long T,
-                                            int j, int g, int pi, int pin_g, bool skip_own, const double xi[3],
-                                            double out[3]) {
-  if (nxt[j] == 0 || pin_i(sc.pin[j])) return false;
-  if (skip_own && ((pin_b(pin_g) && j == g) || (pin_i(pin_g) && j == pi))) return false;
-  double sgi[3], s[3];
-  for (int c = 0; c < 3; ++c) {
-    sgi[c] = reflect1(X[c * T + j], sc.mirror[m][c], sc.box[c]);
-    s[c] = reflect1(GI[c * T + j], sc.mirror[m][c], sc.box[c]);
-  }
-  const double a = e_add(e_add(e_sq(e_sub(xi[0], s[0])), e_sq(e_sub(xi[1], s[1]))), e_sq(e_sub(xi[2], s[2])));
-  const double r[3] = {e_sub(s[0], xi[0]), e_sub(s[1], xi[1]), e_sub(s[2], xi[2])};
-  const double d[3] = {e_sub(sgi[0], s[0]), e_sub(sgi[1], s[1]), e_sub(sgi[2], s[2])};
-  const double c = e_add(e_add(e_sq(e_sub(s[0], sgi[0])), e_sq(e_sub(s[1], sgi[1]))), e_sq(e_sub(s[2], sgi[2])));
-  return bs_term_exact(r, d, a, c, sc.quant_circ, sc.two_pi, out);
 }

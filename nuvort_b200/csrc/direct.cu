@@ -11,6 +11,7 @@
 // re-streams the tiles (from L2; the kernel is FP64-pipe bound, not memory bound).
 #include <vector>
 
+#include "fp64.cuh"
 #include "handle.cuh"
 #include "tma.cuh"
 
@@ -96,40 +97,27 @@ __global__ void __launch_bounds__(64) k_direct_fp64(
     const int j0 = base + 1 + t * TJ;
     const double4 *tl = tiles + buf * 2 * TJ;
     if (active) {
-      if (m == 0) {
+      // the unshifted image as a shift of +0.0, which leaves the positions as they are; a
+      // skipped term adds +0.0, which leaves a sum that starts at +0.0 as it is (so do empty
+      // slots, whose records are zero, and the target's own segment, r = 0)
+      const double s0 = m ? sc.shift[m - 1][0] : 0.0, s1 = m ? sc.shift[m - 1][1] : 0.0,
+                   s2 = m ? sc.shift[m - 1][2] : 0.0;
+      double ub[3] = {m ? ubs[0] : ub0[0], m ? ubs[1] : ub0[1], m ? ubs[2] : ub0[2]};
 #pragma unroll 2
-        for (int jj = 0; jj < n; ++jj) {
-          const double4 A = tl[2 * jj], B = tl[2 * jj + 1];
-          const int gj = j0 + jj;
-          if (A.w == 0.0 || gj == g || gj == pi) continue;
-          const double r[3] = {e_sub(A.x, xi[0]), e_sub(A.y, xi[1]), e_sub(A.z, xi[2])};
-          const double d[3] = {B.x, B.y, B.z};
-          const double a = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
-          double tm[3];
-          if (bs_term_exact(r, d, a, B.w, qc, two_pi, tm)) {
-            ub0[0] = e_add(ub0[0], tm[0]);
-            ub0[1] = e_add(ub0[1], tm[1]);
-            ub0[2] = e_add(ub0[2], tm[2]);
-          }
-        }
-      } else {
-        const double s0 = sc.shift[m - 1][0], s1 = sc.shift[m - 1][1], s2 = sc.shift[m - 1][2];
-#pragma unroll 2
-        for (int jj = 0; jj < n; ++jj) {
-          const double4 A = tl[2 * jj], B = tl[2 * jj + 1];
-          const int gj = j0 + jj;
-          if (A.w == 0.0 || gj == pi) continue;
-          const double r[3] = {e_sub(e_add(A.x, s0), xi[0]), e_sub(e_add(A.y, s1), xi[1]), e_sub(e_add(A.z, s2), xi[2])};
-          const double d[3] = {B.x, B.y, B.z};
-          const double a = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
-          double tm[3];
-          if (bs_term_exact(r, d, a, B.w, qc, two_pi, tm)) {
-            ubs[0] = e_add(ubs[0], tm[0]);
-            ubs[1] = e_add(ubs[1], tm[1]);
-            ubs[2] = e_add(ubs[2], tm[2]);
-          }
-        }
+      for (int jj = 0; jj < n; ++jj) {
+        const double4 A = tl[2 * jj], B = tl[2 * jj + 1];
+        const int gj = j0 + jj;
+        const double r[3] = {e_sub(e_add(A.x, s0), xi[0]), e_sub(e_add(A.y, s1), xi[1]), e_sub(e_add(A.z, s2), xi[2])};
+        const double d[3] = {B.x, B.y, B.z};
+        const double a = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
+        double tm[3];
+        bs_term(gj != pi, r, d, a, B.w, qc, two_pi, tm);
+        ub[0] = e_add(ub[0], tm[0]);
+        ub[1] = e_add(ub[1], tm[1]);
+        ub[2] = e_add(ub[2], tm[2]);
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) (m ? ubs[c] : ub0[c]) = ub[c];
     }
     __syncthreads();
     if (q + 2 < Q) {
@@ -151,8 +139,8 @@ __global__ void __launch_bounds__(64) k_direct_fp64(
       const bool own = mirror_skips_own(sc, pin_g, m);
       for (int j = base + 1; j <= base + pc; ++j) {
         double tm[3];
-        if (mirror_term(sc, m, X, GI, nxt, T, j, g, pi, pin_g, own, xi, tm))
-          for (int c = 0; c < 3; ++c) um[c] = e_add(um[c], tm[c]);
+        mirror_term_sum(sc, m, X, GI, nxt, T, j, g, pi, pin_g, own, xi, tm);
+        for (int c = 0; c < 3; ++c) um[c] = e_add(um[c], tm[c]);
       }
     }
   }
@@ -177,27 +165,81 @@ __global__ void __launch_bounds__(64) k_direct_fp64(
   store3(U, T, g, u);
 }
 
-// Few targets (a small system, or a short list of targets): the same sums with the work of
-// each target spread over a block.  A block takes G targets; three warps compute the terms
-// of a step -- one tile of segments of one image, 192 terms -- into shared memory while warp
-// 0 adds the previous step's terms, one lane per (target, component), in slot order: the
+// The same sums with the work of a target spread over a block, one summing warp and eight
+// computing warps to G targets.  The computing warps take the terms of a step -- TJ consecutive
+// segments for each target, of the sequence unshifted image, shifted images, mirror images,
+// each over j ascending -- into shared memory while the summing
+// warp adds the previous step's, one lane per (target, component), in sequence order: the
 // additions are the reference's, in the reference's order, only the terms are computed
-// elsewhere.  A skipped term (empty slot, excluded neighbour, 4ac-b^2 == 0) is stored as
-// +0.0: the accumulators start at +0.0 and a round-to-nearest sum is never -0.0 unless both
-// operands are, so adding +0.0 leaves them bit for bit unchanged, exactly as skipping does.
-constexpr int kSplitTerms = 192;  // terms per step: two per computing thread
+// elsewhere.  Skipped terms are stored as +0.0: the accumulators start at +0.0 and a
+// round-to-nearest sum is never -0.0 unless both operands are, so adding +0.0 leaves them bit
+// for bit unchanged, exactly as skipping does.
+//
+// Bound: the FP64 pipe (84 FP64 instructions a term, see fp64.cuh) where the blocks fill the
+// GPU: 12,289 points 31.4 ms (102 ms with the IEEE operations one by one, three computing warps
+// and a barrier every 192 terms), 18.4 ms at the pipe's full rate.  With few targets the
+// summing lanes' chain, one addition of 8 cycles per segment and image, which is why they only
+// load (ahead of the chain) and add: 600 points 183 us, before 357 us.  A step is one tile of
+// one image, so that the image and its shift are uniform; four terms a thread and step with
+// G = 8 share the cost of the barrier and of the staging (two: 32.6 ms).  The lanes of a warp
+// take G targets x 32/G segments, and a step's segment records are staged in shared memory a
+// step ahead, each read from global memory once for the block's G targets.
+constexpr int kSplitWarps = 8;
+constexpr int kSplitComp = 32 * kSplitWarps;       // computing threads
+constexpr int kSplitThreads = 32 + kSplitComp;
+constexpr int kSegPad = 5;  // 16-byte units per staged record (4 used): no bank conflicts at any G
+
+constexpr int split_per(int G) { return G == 8 ? 4 : G == 4 ? 2 : 1; }
+constexpr size_t split_smem(int G) {  // the terms and segments of two steps
+  const int terms = kSplitComp * split_per(G);
+  return 2 * (3 * (terms + (G == 8 ? 8 : 4)) * sizeof(double) + terms / G * kSegPad * sizeof(double2));
+}
+
+// acc + p[0] + p[stride] + ... in order, n terms and +0.0s up to a multiple of 16: two sets of
+// 8 in turn, one loading while the other is added, without a branch between (the last set
+// loaded, from past the end but inside the block's shared memory, is not used).  9.2 cycles per addition alone on its SM; 12.4 as a plain
+// loop unrolled by 8, whose loads wait for the chain; 13.5 with the last loads left out.
+template <int kStride>
+__device__ __forceinline__ double add_in_order(double acc, const double *p, int n) {
+  constexpr int kU = 8;
+  double a[kU], b[kU];
+#pragma unroll
+  for (int u = 0; u < kU; ++u) a[u] = p[u * kStride];
+  for (int k = 0; k < n; k += 2 * kU) {
+#pragma unroll
+    for (int u = 0; u < kU; ++u) b[u] = p[(kU + u) * kStride];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) acc = e_add(acc, a[u]);
+    p += 2 * kU * kStride;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) a[u] = p[u * kStride];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) acc = e_add(acc, b[u]);
+  }
+  return acc;
+}
 
 template <int G>
-__global__ void __launch_bounds__(128) k_direct_fp64_split(
+__global__ void __launch_bounds__(kSplitThreads, G == 8 ? 2 : 3) k_direct_fp64_split(
     const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn, const int2 *__restrict__ work,
     const double *__restrict__ X, const double *__restrict__ GI, const double *__restrict__ GB,
     const int *__restrict__ nxt, const int *__restrict__ prv, const double4 *__restrict__ seg,
     double *__restrict__ U, long long T, const unsigned *err, const int *__restrict__ targets, int ntargets,
     double *__restrict__ Uout) {
-  constexpr int TJ = kSplitTerms / G;  // segments per step
-  constexpr int LD = TJ + 1;           // padded row: the adding lanes read different banks
-  __shared__ double s_terms[2][3 * G][LD];
-  __shared__ double s_x[G][3];
+  constexpr int kPer = split_per(G);               // terms per computing thread and step
+  constexpr int kTerms = kSplitComp * kPer;        // terms per step
+  constexpr int TJ = kTerms / G;                   // segments per step
+  constexpr int kStep = kSplitComp / G;            // segments between a thread's terms
+  constexpr int kLoads = 4 * TJ / kSplitComp;      // 16-byte loads per thread that stage a step
+  static_assert(4 * TJ % kSplitComp == 0 && TJ % 16 == 0, "whole loads per thread, whole sets of additions");
+  // component rows of a step's terms, [segment][target]; padded so that the summing lanes of
+  // the components read different banks
+  constexpr int LD = kTerms + (G == 8 ? 8 : 4);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto s_terms = reinterpret_cast<double(*)[3][LD]>(smem_raw);  // [2][3][LD]
+  auto s_seg = reinterpret_cast<double2(*)[TJ * kSegPad]>(smem_raw + sizeof(double) * 2 * 3 * LD);  // [2]
+  static_assert(split_smem(G) == sizeof(double) * 2 * 3 * LD + sizeof(double2) * 2 * TJ * kSegPad, "layout");
+  __shared__ double s_x[G][3], s_shift[27][3];
   __shared__ double s_sum[G][3][3];
   __shared__ int s_g[G], s_p[G], s_act[G], s_pin[G];
   __shared__ int s_abort;
@@ -209,6 +251,7 @@ __global__ void __launch_bounds__(128) k_direct_fp64_split(
   const int tid = threadIdx.x;
   if (!targets && w.y - base > pc) return;  // block-uniform: every target beyond pcount
   if (tid == 0) s_abort = (*err != 0);
+  for (int k = tid; k < 81; k += kSplitThreads) s_shift[k / 3][k % 3] = k < 3 ? 0.0 : sc.shift[k / 3 - 1][k % 3];
   if (tid < G) {
     int g;
     bool act;
@@ -231,74 +274,103 @@ __global__ void __launch_bounds__(128) k_direct_fp64_split(
   __syncthreads();
   if (s_abort) return;
 
-  const int nt = (pc + TJ - 1) / TJ;
-  const int Q = (1 + sc.n_shift + sc.n_mirror) * nt;  // unshifted, shifted, then mirror images
   const double qc = sc.quant_circ, two_pi = sc.two_pi;
-  double acc0 = 0.0, accs = 0.0, accm = 0.0;  // adding lanes: unshifted, shifted, mirror sums
-  for (int q = 0; q <= Q; ++q) {
-    if (tid >= 32) {
-      if (q < Q) {  // terms of step q
-        const int m = q / nt, t = q % nt;
-        const int n = min(TJ, pc - t * TJ);
-        double(*out)[LD] = s_terms[q & 1];
-        double s0 = 0, s1 = 0, s2 = 0;
-        if (m > 0) {
-          s0 = sc.shift[m - 1][0];
-          s1 = sc.shift[m - 1][1];
-          s2 = sc.shift[m - 1][2];
-        }
+  double acc0 = 0.0, accs = 0.0, accm = 0.0;  // summing lanes: unshifted, shifted, mirror sums
+  const bool comp = tid >= 32;
+  const int e0 = comp ? tid - 32 : 0;
+  const int tq = e0 % G;  // computing threads: their target
+  const bool act = s_act[tq];  // used by the mirror images; other inactive targets' sums go nowhere
+  {  // the unshifted and the shifted images; a step is one tile of one image
+    const double2 *rec = reinterpret_cast<const double2 *>(seg + 2 * (long long)(base + 1));
+    const int nt = (pc + TJ - 1) / TJ, Q = (1 + sc.n_shift) * nt;
+    const double x0 = s_x[tq][0], x1 = s_x[tq][1], x2 = s_x[tq][2];
+    const int behind = s_p[tq] - base - 1;  // as a segment counted from 0
+    int m = 0, t = 0;                       // image and tile of the step, of the summing warp's step
+    int tl = 0;                             // tile staged next
+    double2 ld[kLoads];
+    auto fetch = [&]() {
 #pragma unroll
-        for (int r = 0; r < kSplitTerms / 96; ++r) {
-          const int e = (tid - 32) + 96 * r;
-          const int tq = e / TJ, jj = e % TJ;
-          if (jj >= n) continue;
-          const int gj = base + 1 + t * TJ + jj;
-          double tm[3] = {0.0, 0.0, 0.0};
-          if (m > sc.n_shift) {  // mirror image m - 1 - n_shift
-            const int mm = m - 1 - sc.n_shift;
-            if (!s_act[tq] || !mirror_term(sc, mm, X, GI, nxt, T, gj, s_g[tq], s_p[tq], s_pin[tq],
-                                           mirror_skips_own(sc, s_pin[tq], mm), s_x[tq], tm))
-              tm[0] = tm[1] = tm[2] = 0.0;
-          } else if (s_act[tq] && gj != s_p[tq] && (m > 0 || gj != s_g[tq])) {
-            const double4 A = seg[2 * (long long)gj], B = seg[2 * (long long)gj + 1];
-            if (A.w != 0.0) {
-              double rr[3];
-              if (m == 0) {
-                rr[0] = e_sub(A.x, s_x[tq][0]);
-                rr[1] = e_sub(A.y, s_x[tq][1]);
-                rr[2] = e_sub(A.z, s_x[tq][2]);
-              } else {
-                rr[0] = e_sub(e_add(A.x, s0), s_x[tq][0]);
-                rr[1] = e_sub(e_add(A.y, s1), s_x[tq][1]);
-                rr[2] = e_sub(e_add(A.z, s2), s_x[tq][2]);
-              }
-              const double d[3] = {B.x, B.y, B.z};
-              const double a = e_add(e_add(e_sq(rr[0]), e_sq(rr[1])), e_sq(rr[2]));
-              if (!bs_term_exact(rr, d, a, B.w, qc, two_pi, tm)) tm[0] = tm[1] = tm[2] = 0.0;
-            }
-          }
-          out[3 * tq + 0][jj] = tm[0];
-          out[3 * tq + 1][jj] = tm[1];
-          out[3 * tq + 2][jj] = tm[2];
-        }
+      for (int k = 0; k < kLoads; ++k) {
+        const int jl = tl * TJ + e0 / 4 + k * (kSplitComp / 4);
+        ld[k] = jl < pc ? __ldg(rec + 4 * (long long)jl + (e0 & 3)) : make_double2(0., 0.);
       }
-    } else if (q >= 1 && tid < 3 * G) {  // add the terms of step q-1, in slot order
-      const int m = (q - 1) / nt, t = (q - 1) % nt;
-      const int n = min(TJ, pc - t * TJ);
-      const double *row = s_terms[(q - 1) & 1][tid];
-      double acc = m == 0 ? acc0 : m <= sc.n_shift ? accs : accm;
-#pragma unroll 8
-      for (int jj = 0; jj < n; ++jj) acc = e_add(acc, row[jj]);
-      if (m == 0) acc0 = acc;
-      else if (m <= sc.n_shift) accs = acc;
-      else accm = acc;
+      if (++tl == nt) tl = 0;
+    };
+    auto stage = [&](int b) {
+#pragma unroll
+      for (int k = 0; k < kLoads; ++k) s_seg[b][(e0 / 4 + k * (kSplitComp / 4)) * kSegPad + (e0 & 3)] = ld[k];
+    };
+    if (comp) {
+      fetch();
+      stage(0);
     }
     __syncthreads();
+    for (int q = 0; q <= Q; ++q) {
+      const int b = q & 1;
+      if (comp) {
+        if (q < Q) {
+          fetch();  // the next step's tile, stored once this step's terms are done
+          const double sh0 = s_shift[m][0], sh1 = s_shift[m][1], sh2 = s_shift[m][2];
+          // records past the end of the list and empty slots are zero, and the target's own
+          // segment has r = 0: all have 4ac - b^2 = 0 and drop out like the reference's
+#pragma unroll 2
+          for (int r = 0; r < kPer; ++r) {
+            const double2 *sp = &s_seg[b][(e0 / G + r * kStep) * kSegPad];
+            const double2 A0 = sp[0], A1 = sp[1], B0 = sp[2], B1 = sp[3];
+            const double rr[3] = {e_sub(e_add(A0.x, sh0), x0), e_sub(e_add(A0.y, sh1), x1), e_sub(e_add(A1.x, sh2), x2)};
+            const double d[3] = {B0.x, B0.y, B1.x};
+            const double a = e_add(e_add(e_sq(rr[0]), e_sq(rr[1])), e_sq(rr[2]));
+            double tm[3];
+            bs_term(t * TJ + e0 / G + r * kStep != behind, rr, d, a, B1.y, qc, two_pi, tm);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s_terms[b][c][e0 + r * kSplitComp] = tm[c];
+          }
+          stage(b ^ 1);
+          if (++t == nt) {
+            t = 0;
+            ++m;
+          }
+        }
+      } else if (q >= 1 && tid < 3 * G) {  // add the terms of step q-1, in slot order
+        const double *row = &s_terms[b ^ 1][tid / G][tid % G];
+        const int n = min(TJ, pc - t * TJ);
+        if (m == 0) acc0 = add_in_order<G>(acc0, row, n);
+        else accs = add_in_order<G>(accs, row, n);
+        if (++t == nt) {
+          t = 0;
+          ++m;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (sc.n_mirror) {  // solid walls: the mirror images, in mirror order
+    const long long F = (long long)sc.n_mirror * pc;
+    const int Q = (int)((F + TJ - 1) / TJ);
+    for (int q = 0; q <= Q; ++q) {
+      if (comp) {
+        for (int r = 0; r < kPer; ++r) {
+          const long long f = (long long)q * TJ + e0 / G + r * kStep;
+          double tm[3] = {0.0, 0.0, 0.0};
+          if (act && f < F) {
+            const int mm = (int)(f / pc), jj = (int)(f - (long long)mm * pc);
+            mirror_term_sum(sc, mm, X, GI, nxt, T, base + 1 + jj, s_g[tq], s_p[tq], s_pin[tq],
+                            mirror_skips_own(sc, s_pin[tq], mm), s_x[tq], tm);
+          }
+#pragma unroll
+          for (int c = 0; c < 3; ++c) s_terms[q & 1][c][e0 + r * kSplitComp] = tm[c];
+        }
+      } else if (q >= 1 && tid < 3 * G) {
+        const int n = (int)min((long long)TJ, F - (long long)(q - 1) * TJ);
+        accm = add_in_order<G>(accm, &s_terms[(q - 1) & 1][tid / G][tid % G], n);
+      }
+      __syncthreads();
+    }
   }
   if (tid < 3 * G) {
-    s_sum[tid / 3][tid % 3][0] = acc0;
-    s_sum[tid / 3][tid % 3][1] = accs;
-    s_sum[tid / 3][tid % 3][2] = accm;
+    s_sum[tid % G][tid / G][0] = acc0;
+    s_sum[tid % G][tid / G][1] = accs;
+    s_sum[tid % G][tid / G][2] = accm;
   }
   __syncthreads();
   if (tid >= G || !s_act[tid]) return;
@@ -327,7 +399,10 @@ __global__ void __launch_bounds__(128) k_direct_fp64_split(
 template <int G>
 void launch_split(cudaStream_t st, const nv_handle *h, const int2 *work, int nwork, const int *targets, int ntargets,
                   double *Uout) {
-  k_direct_fp64_split<G><<<nwork, 128, 0, st>>>(h->d_sc, h->d_dyn, work, h->x, h->gi, h->gb, h->nxt, h->prv,
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_direct_fp64_split<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem(G));
+  (void)attr;
+  k_direct_fp64_split<G><<<nwork, kSplitThreads, split_smem(G), st>>>(h->d_sc, h->d_dyn, work, h->x, h->gi, h->gb, h->nxt, h->prv,
                                                    h->seg, h->u, h->T, h->d_err, targets, ntargets, Uout);
 }
 
@@ -343,22 +418,19 @@ void launch_split_g(int G, cudaStream_t st, const nv_handle *h, const int2 *work
 
 }  // namespace
 
-// Targets per block of the split direct sum for n target slots: the largest of 8, 4, 2, 1
-// that still gives about four blocks per SM (1 when even that is not reached).
-int direct_split_g(long long n) {
-  const long long want = 4LL * n_sms_host();
-  int G = 8;
-  while (G > 1 && n / G < want) G /= 2;
-  return G;
-}
-
-// Direct-sum targets per block in use: 64 (one thread per target, k_direct_fp64) when the
-// direct systems' slots fill the GPU with at least two blocks of 64 per SM, else the split
-// kernel's G.  direct_split (nv_set_direct_split) overrides the choice.
+// Direct-sum targets per block in use for this many target slots (direct_split, set by
+// nv_set_direct_split, overrides the choice): 8 per block of the split kernel, except
+//   * 2 while the blocks of 2 (three to an SM) about fit the GPU at once, counting two thirds
+//     of the slots as live: the summing chain sets the time then, and it is the shorter the
+//     fewer terms an SM computes beside it (600 points: 183 us, 206 with 8; but 1000 points,
+//     a second wave of blocks: 452 us, 327 with 8; 4 per block is nowhere ahead by 3 %);
+//   * one thread per target (64 to a block) from 80,000 slots on, four warps to each
+//     scheduler, which need no exchange (50,000 points: 623 ms, 488 with 8; 80,000: 1.22 s,
+//     1.23 s).
 int direct_targets_per_block(const nv_handle *h, long long slots) {
   if (h->direct_split > 0) return h->direct_split;
-  if (slots >= 2LL * 64 * n_sms_host()) return 64;
-  return direct_split_g(slots);
+  if (slots >= 80000) return 64;
+  return slots <= 9LL * n_sms_host() ? 2 : 8;
 }
 
 void launch_direct(nv_handle *h) {

@@ -210,12 +210,6 @@ __device__ __forceinline__ int octant(const double x[3], const double4 P, double
   return in ? (4 * up[1] + 2 * up[2] + up[0]) : 8;
 }
 
-__device__ __forceinline__ double4 ldg4(const double4 *p) {
-  const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-  const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-  return make_double4(a.x, a.y, b.x, b.y);
-}
-
 __device__ __forceinline__ void load_x(const double *__restrict__ X, long long T, int g, double x[3]) {
   x[0] = __ldg(X + g);
   x[1] = __ldg(X + T + g);
