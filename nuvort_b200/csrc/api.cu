@@ -373,7 +373,7 @@ int rebuild_worklists(nv_handle *h) {
   int rc;
   if (h->precision == NV_PREC_MIXED) {
     std::vector<int4> w4;
-    build_image_worklist(h, 1, 128, w4);
+    build_image_worklist(h, 1, 32, w4);
     if ((rc = upload_worklist4(&h->d_work_img, &h->n_work_img, w4)) != NV_OK) return rc;
     h->walk_parts_used = h->walk_parts > 0 ? h->walk_parts : auto_walk_parts(h);
     build_image_worklist(h, 2, 128, w4, h->walk_parts_used);
@@ -712,7 +712,9 @@ int nv_create(const nv_params *params, int32_t nsys, const int32_t *capacity, in
     if ((rc = dalloc(&h->stage, 3 * ((size_t)maxcap + 1)))) return bail(rc);
   }
   if (h->precision == NV_PREC_MIXED) {
-    if ((rc = dalloc(&h->seg32, 3 * T))) return bail(rc);
+    bool direct = false;
+    for (auto &c : h->sc) direct |= c.velocity == NV_VEL_BS;
+    if (direct && (rc = dalloc(&h->seg32, 12 * ((size_t)T + 1)))) return bail(rc);
     const int nimg = 27 + kMaxWalkParts - 1;  // the images, then the central image's extra parts
     if ((rc = dalloc(&h->partial, (size_t)nimg * 3 * T))) return bail(rc);
   }

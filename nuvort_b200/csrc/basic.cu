@@ -21,14 +21,39 @@ __global__ void k_begin_step(SysDyn *dyn, int nsys, const unsigned *err) {
   dyn[s].itime += 1;
 }
 
+// The FP32 record of system slot k (mixed precision): position split hi + lo (x = hi + lo to
+// ~1e-16), segment vector; zero for an empty slot (no contribution).  The last slot of an odd
+// capacity also clears the other half of its pair.
+__device__ __forceinline__ void put_seg32(float *seg32, const SysConst &sc, int k, const double x[3],
+                                          const double d[3], double c, double near_factor) {
+  if (k < 1 || k > sc.cap) return;
+  float *p = seg32 + seg32_at(sc.base, k) + ((k - 1) & 1);
+  float v[12];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    v[a] = (float)x[a];
+    v[3 + a] = (float)(x[a] - (double)v[a]);
+    v[6 + a] = (float)d[a];
+  }
+  const double nr = near_factor * sc.delta;
+  v[9] = fmaxf(kFarRatio * (float)c, (float)(nr * nr));
+  v[10] = -v[6];
+  v[11] = -v[7];
+#pragma unroll
+  for (int a = 0; a < 12; ++a) p[2 * a] = v[a];
+  if (k == sc.cap && (k & 1))
+#pragma unroll
+    for (int a = 0; a < 12; ++a) p[2 * a + 1] = 0.f;
+}
+
 // ghostp (boundary.f90:10-19) + get_ghost_p (:26-84); also packs the segment records
-// (x_j, gi_j - x_j, c_j) that the direct sums stage in shared memory: FP64 (2 x 32 B)
-// and, for mixed precision, FP32 (3 x 16 B: position hi, position lo, segment).
+// (x_j, gi_j - x_j, c_j) that the direct sums stage in shared memory: FP64 (2 x 32 B) and, for
+// mixed precision with direct-sum systems, FP32 pairs.
 __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
                         const int *__restrict__ sys_of, const double *__restrict__ X,
                         const int *__restrict__ nxt, const int *__restrict__ prv,
                         double *__restrict__ GI, double *__restrict__ GB, double4 *__restrict__ seg,
-                        float4 *__restrict__ seg32, long long T, const unsigned *err) {
+                        float *__restrict__ seg32, double near_factor, long long T, const unsigned *err) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= T || *err) return;
   int s;
@@ -37,11 +62,8 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
   if (n == 0) {
     seg[2 * g] = make_double4(0, 0, 0, 0);
     seg[2 * g + 1] = make_double4(0, 0, 0, 0);
-    if (seg32) {
-      seg32[3 * g] = make_float4(0, 0, 0, 0);
-      seg32[3 * g + 1] = make_float4(0, 0, 0, 0);
-      seg32[3 * g + 2] = make_float4(0, 0, 0, 0);
-    }
+    const double zero[3] = {0, 0, 0};
+    if (seg32) put_seg32(seg32, scs[s], (int)(g - scs[s].base), zero, zero, 0.0, near_factor);
     return;
   }
   const SysConst &sc = scs[s];
@@ -60,12 +82,7 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
   // with a zero segment vector its terms drop out by 4ac - b^2 = 0, like an empty slot's
   seg[2 * g] = make_double4(x[0], x[1], x[2], pin_i(pin) ? 0.0 : 1.0);
   seg[2 * g + 1] = pin_i(pin) ? make_double4(0, 0, 0, 0) : make_double4(d[0], d[1], d[2], c);
-  if (seg32) {  // FP32 record: position split hi + lo (x = hi + lo to ~1e-16), segment vector
-    const float h0 = (float)x[0], h1 = (float)x[1], h2 = (float)x[2];
-    seg32[3 * g] = make_float4(h0, h1, h2, 1.0f);
-    seg32[3 * g + 1] = make_float4((float)(x[0] - (double)h0), (float)(x[1] - (double)h1), (float)(x[2] - (double)h2), 0.0f);
-    seg32[3 * g + 2] = make_float4((float)d[0], (float)d[1], (float)d[2], (float)c);
-  }
+  if (seg32) put_seg32(seg32, sc, (int)(g - sc.base), x, d, c, near_factor);
 }
 
 // calc_velocity with velocity 'LIA' (timestep.f90:60-73): local term + MF only.
@@ -185,7 +202,7 @@ void launch_begin_step(nv_handle *h) {
 
 void launch_ghost(nv_handle *h) {
   k_ghost<<<grid_for(h->T, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, h->prv,
-                                                     h->gi, h->gb, h->seg, h->seg32, h->T, h->d_err);
+                                                     h->gi, h->gb, h->seg, h->seg32, h->near_factor, h->T, h->d_err);
 }
 
 void launch_velocity(nv_handle *h) {
@@ -235,5 +252,5 @@ void launch_end_step(nv_handle *h) {
 void launch_ghost_raw(cudaStream_t st, const SysConst *sc, const SysDyn *dyn, const int *sys_of, const double *x,
                       const int *nxt, const int *prv, double *gi, double *gb, double4 *seg, long long T,
                       unsigned *err) {
-  k_ghost<<<grid_for(T, TB), TB, 0, st>>>(sc, dyn, sys_of, x, nxt, prv, gi, gb, seg, nullptr, T, err);
+  k_ghost<<<grid_for(T, TB), TB, 0, st>>>(sc, dyn, sys_of, x, nxt, prv, gi, gb, seg, nullptr, 0.0, T, err);
 }

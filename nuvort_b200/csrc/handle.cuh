@@ -34,7 +34,7 @@ struct nv_handle {
   double *gi = nullptr, *gb = nullptr, *closestd = nullptr;
   int *nxt = nullptr, *prv = nullptr, *closest = nullptr, *sys_of = nullptr;
   double4 *seg = nullptr;   // FP64 segment records, 2 per slot
-  float4 *seg32 = nullptr;  // FP32 segment records, 3 per slot (mixed precision)
+  float *seg32 = nullptr;   // FP32 segment records, pairs (seg32_at), mixed precision with direct-sum systems
   double *partial = nullptr; // per-image partial sums [image][component][slot] (mixed precision)
   std::vector<void *> nf_buffers;  // normal-fluid noise and grid data (nv_set_normal_fluid_*)
   double *usm = nullptr;     // f(:)%u_sup, f(:)%u_mf of the last velocity pass [6][T]
@@ -48,7 +48,7 @@ struct nv_handle {
   int4 *d_btab = nullptr;    // their per-system table (base, rows, n, offset), nsys entries
   int *d_bcheck = nullptr;   // their link checks, two ints per system
   int *d_upck = nullptr;     // nv_upload checks: [0] link errors (1 out of range, 2 empty-slot mismatch), [1] live slots
-  int4 *d_work_img = nullptr;  // (system, image, first slot) items of the mixed direct sum
+  int4 *d_work_img = nullptr;  // (system, image, first slot) items of 32 slots of the mixed direct sum
   int n_work_img = 0;
   int4 *d_work_timg = nullptr; // same for the mixed tree walk
   int n_work_timg = 0;

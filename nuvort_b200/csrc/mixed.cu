@@ -1,32 +1,147 @@
 // mixed.cu -- mixed-precision direct sum and the FP64 epilogue shared with the mixed tree walk.
 //
-// k_direct_mixed: one thread per (target, periodic image); the target's system's segments
-// stream through shared memory in tiles by 1-D bulk copies (48-byte FP32 records: position
-// hi, position lo, segment vector).  r = x_j - x_i is formed from the hi/lo split, so it is
-// exact to ~1e-16 before rounding to FP32.  Each tile is summed in FP32 and the tile sums are
-// added with Kahan compensation; pairs closer than near_radius are evaluated in FP64 with the
-// reference expression from the FP64 segment records.  Per-image partial sums go to a buffer;
-// k_mixed_combine adds them per target in FP64, in image order, to the FP64 local term and
-// mutual friction (timestep.f90:79-140).
+// k_direct_mixed: a block per 32 targets and periodic image, each of its eight warps (a lane per
+// target) over an eighth of every tile of the target system's segments.  The tiles stream
+// through shared memory by 1-D bulk copies (pairs of segments side by side, 96 bytes a pair:
+// position hi, position lo, segment vector).  r = x_j - x_i is formed from the hi/lo split, so
+// it is exact to ~1e-16 before rounding to FP32.  Every 32 terms are summed in FP32 and those
+// sums are added with Kahan compensation; pairs closer than near_radius are evaluated in FP64
+// with the reference expression from the FP64 segment records.  The warps' sums are added in
+// FP64, in warp order; per-image partial sums go to a buffer; k_mixed_combine adds them per
+// target in FP64, in image order, to the FP64 local term and mutual friction
+// (timestep.f90:79-140).
 #include "handle.cuh"
 #include "mixed.cuh"
 #include "tma.cuh"
 
 namespace {
 
-constexpr int kTJ = 128;  // segments per staged tile (48 B each)
-constexpr int kTB = 128;  // targets per block
+constexpr int kPairs = 128;                // segment pairs per staged tile (96 B each)
+constexpr int kWarps = 8;                  // warps of a block, sharing its 32 targets
+constexpr int kTB = 32 * kWarps;
+constexpr int kWarpPairs = kPairs / kWarps;  // pairs of a tile per warp: one FP32 sub-sum
+constexpr int kStages = 4;
+constexpr size_t kMixedSmem = kStages * kPairs * 96;
 
-template <int TJ>
-__global__ void __launch_bounds__(kTB) k_direct_mixed(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
-                                                      const int4 *__restrict__ work, const double *__restrict__ X,
-                                                      const int *__restrict__ nxt, const int *__restrict__ prv,
-                                                      const float4 *__restrict__ seg32, const double4 *__restrict__ seg64,
-                                                      double *__restrict__ partial, long long T, double near_factor, Fp32Guards gd,
-                                                      unsigned *err) {
+// One term in FP64 from the FP64 segment records, for near and ill-conditioned pairs: the
+// reference's skip decision (4ac - b^2 == 0, timestep.f90:166,192) in its own arithmetic, the
+// value from the cancellation-free form.
+__device__ __noinline__ double3 direct_term64(const double4 *__restrict__ rec, double s0, double s1, double s2,
+                                              double x0, double x1, double x2, double gq) {
+  const double4 A = rec[0], B = rec[1];
+  const double r[3] = {e_sub(e_add(A.x, s0), x0), e_sub(e_add(A.y, s1), x1), e_sub(e_add(A.z, s2), x2)};
+  const double d[3] = {B.x, B.y, B.z};
+  const double a = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
+  const double b = e_mul(2.0, dot3(r, d));
+  if (e_sub(e_mul(e_mul(4.0, a), B.w), e_mul(b, b)) == 0.0) return make_double3(0., 0., 0.);
+  double t[3];
+  term64_stable(r, d, a, gq, t);
+  return make_double3(t[0], t[1], t[2]);
+}
+
+// What the lanes of a warp hold of their targets.
+struct MixedTarget {
+  double x[3], s[3];     // position, image shift
+  f32x2 h[3], l[3];      // shift - position, FP32 high and low parts
+  int behind, own;       // segments (from 0) that are skipped
+  bool active;
+};
+
+// Two segments (pair p of the system, its record at q) for a lane: r from the target, its
+// square; then the term f (r x d).
+struct PairVec {
+  f32x2 rx, ry, rz, a;
+};
+__device__ __forceinline__ PairVec pair_vec(const ulonglong2 *q, const MixedTarget &t) {
+  const ulonglong2 v0 = q[0], v1 = q[1], v2 = q[2];
+  PairVec r;
+  r.rx = add2(add2({v0.x}, t.h[0]), add2({v1.y}, t.l[0]));
+  r.ry = add2(add2({v0.y}, t.h[1]), add2({v2.x}, t.l[1]));
+  r.rz = add2(add2({v1.x}, t.h[2]), add2({v2.y}, t.l[2]));
+  r.a = fma2(r.rx, r.rx, fma2(r.ry, r.ry, mul2(r.rz, r.rz)));
+  return r;
+}
+struct PairSeg {
+  f32x2 dx, dy, dz, ndx, ndy;
+};
+struct PairGeo {
+  f32x2 cx, cy, cz;      // r x d
+  f32x2 ee, re, pp, num; // |e|^2, r.e, |r||e|, 1/|r| + 1/|e| with e = r + d
+};
+__device__ __forceinline__ PairGeo pair_geo(const PairVec &r, const PairSeg &d) {
+  const f32x2 kMinus = pack2(-1.f, -1.f);
+  PairGeo g;
+  const f32x2 ex = add2(r.rx, d.dx), ey = add2(r.ry, d.dy), ez = add2(r.rz, d.dz);
+  g.ee = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
+  g.re = fma2(r.rx, ex, fma2(r.ry, ey, mul2(r.rz, ez)));
+  g.cx = fma2(r.ry, d.dz, mul2(r.rz, d.ndy));
+  g.cy = fma2(r.rz, d.dx, mul2(mul2(r.rx, kMinus), d.dz));
+  g.cz = fma2(r.rx, d.dy, mul2(r.ry, d.ndx));
+  const f32x2 ia = pack2(rsqrt_fast(lo2(r.a)), rsqrt_fast(hi2(r.a)));
+  const f32x2 ib = pack2(rsqrt_fast(lo2(g.ee)), rsqrt_fast(hi2(g.ee)));
+  g.pp = mul2(mul2(r.a, ia), mul2(g.ee, ib));
+  g.num = add2(ia, ib);
+  return g;
+}
+
+// A pair that some lane of the warp is not far from: every lane's own guards decide between
+// FP32 and FP64 (into n).
+__device__ __forceinline__ void pair_guarded(const PairVec &r, const PairSeg &d, const MixedTarget &t, int p,
+                                             float near2, const Fp32Guards &gd, const double4 *__restrict__ seg64,
+                                             double gq64, f32x2 u[3], double n[3]) {
+  const PairGeo g = pair_geo(r, d);
+  const f32x2 c = fma2(d.dx, d.dx, fma2(d.dy, d.dy, mul2(d.dz, d.dz)));
+  const f32x2 cr2 = fma2(g.cx, g.cx, fma2(g.cy, g.cy, mul2(g.cz, g.cz)));
+  float f[2];
+  bool bad[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    auto of = [&](f32x2 v) { return h ? hi2(v) : lo2(v); };
+    const float a = of(r.a), ee = of(g.ee), re = of(g.re), pp = of(g.pp), cc = of(c), k2 = of(cr2);
+    const int j = 2 * p + h;
+    bad[h] = j == t.behind || j == t.own || a < near2 || !(a > 0.f) || k2 < gd.line * cc * fminf(a, ee) ||
+             ee < gd.end * fmaxf(a, cc) || pp + re < gd.angle * pp;
+    // pp + r.e = |r x d|^2 / (pp - r.e) when r.e < 0: no cancellation either way
+    const bool obtuse = re < 0.f;
+    f[h] = bad[h] ? 0.f : of(g.num) * (obtuse ? pp - re : 1.f) * rcp_fast(obtuse ? k2 : pp + re);
+  }
+  const f32x2 ff = pack2(f[0], f[1]);
+  u[0] = fma2(ff, g.cx, u[0]);
+  u[1] = fma2(ff, g.cy, u[1]);
+  u[2] = fma2(ff, g.cz, u[2]);
+  if (t.active && (bad[0] || bad[1])) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int j = 2 * p + h;
+      if (!(h ? bad[1] : bad[0]) || j == t.behind || j == t.own) continue;
+      const double3 v = direct_term64(seg64 + 2 * (long long)j, t.s[0], t.s[1], t.s[2], t.x[0], t.x[1], t.x[2], gq64);
+      n[0] += v.x;
+      n[1] += v.y;
+      n[2] += v.z;
+    }
+  }
+}
+
+// Bound: the FP32 pipe (about 35 lane operations a far term, the adds, multiplies and FMAs of
+// two segments packed into one instruction).  A pair of segments that every lane's target is
+// far from needs none of the conditioning guards, nearly all pairs of a tangle; the other
+// pairs take them lane by lane.  The tiles pass through a ring of kStages buffers with an
+// mbarrier for full and one for empty each, so that no warp waits for the block's others.
+// 30,011 points: 39.4 ms; 1,500 points: 147 us (a lane per target and image with scalar
+// arithmetic and all guards, 113 issue slots a term: 74.1 ms and 409 us; packed, but all guards
+// and a barrier per tile: 55.4 ms and 236 us).
+__global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restrict__ scs,
+                                                         const SysDyn *__restrict__ dyn,
+                                                         const int4 *__restrict__ work, const double *__restrict__ X,
+                                                         const int *__restrict__ nxt, const int *__restrict__ prv,
+                                                         const float *__restrict__ seg32,
+                                                         const double4 *__restrict__ seg64,
+                                                         double *__restrict__ partial, long long T,
+                                                         double near_factor, Fp32Guards gd, unsigned *err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  float4 *tiles = reinterpret_cast<float4 *>(smem_raw);  // [2][3*TJ]
-  __shared__ __align__(8) uint64_t bar[2];
+  ulonglong2 *tiles = reinterpret_cast<ulonglong2 *>(smem_raw);  // [kStages][6 * kPairs]
+  __shared__ double s_red[3][kWarps][32];
+  __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
   __shared__ int s_abort;
 
   const int4 w = work[blockIdx.x];  // system, image, first slot
@@ -34,142 +149,111 @@ __global__ void __launch_bounds__(kTB) k_direct_mixed(const SysConst *__restrict
   const int base = sc.base, m = w.y;
   const int pc = dyn[w.x].pcount;
   if (w.z - base > pc) return;  // block-uniform
-  const int tid = threadIdx.x;
-  const int g = w.z + tid;
-  const bool active = (g - base <= pc) && (g - base <= sc.cap) && nxt[g] != 0;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int g = w.z + lane;
+  MixedTarget t;
+  t.active = (g - base <= pc) && (g - base <= sc.cap) && nxt[g] != 0;
   if (tid == 0) {
     s_abort = (*err != 0);
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    for (int k = 0; k < kStages; ++k) {
+      mbar_init(&full[k], 1);
+      mbar_init(&empty[k], kWarps);
+    }
     mbar_fence_init();
   }
   __syncthreads();
   if (s_abort) return;
 
-  // target, moved by minus the image shift: r = (x_j + s) - x_i = x_j - (x_i - s)
-  double xi[3] = {0, 0, 0}, s[3] = {0, 0, 0};
-  if (m > 0)
-    for (int c = 0; c < 3; ++c) s[c] = sc.shift[m - 1][c];
-  int pi_ = -1;
-  if (active) {
-    load3(X, T, g, xi);
-    pi_ = prv[g];
-  }
-  float th[3], tl[3];
+  // target, moved by minus the image shift: r = (x_j + s) - x_i = x_j - (x_i - s); a lane
+  // without one is far from everything.  The behind segment is skipped in every image, the
+  // target's own in the central one (their pairs take the guarded path, which skips them).
+  t.behind = t.own = -1;
   for (int c = 0; c < 3; ++c) {
-    const double t = xi[c] - s[c];
-    th[c] = (float)t;
-    tl[c] = (float)(t - (double)th[c]);
+    t.s[c] = m > 0 ? sc.shift[m - 1][c] : 0.0;
+    t.x[c] = -1e9;
   }
+  if (t.active) {
+    load3(X, T, g, t.x);
+    t.behind = prv[g] - base - 1;
+    if (m == 0) t.own = g - base - 1;
+  }
+  for (int c = 0; c < 3; ++c) {
+    const double v = t.s[c] - t.x[c];
+    const float h = (float)v, l = (float)(v - (double)h);
+    t.h[c] = pack2(h, h);
+    t.l[c] = pack2(l, l);
+  }
+  const int behind_p = t.behind >= 0 ? t.behind >> 1 : -1;
   const double gq64 = sc.quant_circ / (4.0 * NV_PI);
-  const float gq = (float)gq64;
   const double nr = near_factor * sc.delta;
   const float near2 = (float)(nr * nr);
+  const double4 *rec64 = seg64 + 2 * (long long)(base + 1);
 
-  const int nt = (pc + TJ - 1) / TJ;
-  auto issue = [&](int t) {
-    const int n = min(TJ, pc - t * TJ);
-    const int buf = t & 1;
-    mbar_expect_tx(&bar[buf], (unsigned)(n * 48));
-    bulk_g2s(tiles + buf * 3 * TJ, seg32 + 3 * (long long)(base + 1 + t * TJ), (unsigned)(n * 48), &bar[buf]);
+  const int np = (pc + 1) / 2;  // pairs of the system (an odd last one is half empty)
+  const int nt = (np + kPairs - 1) / kPairs;
+  const float *src = seg32 + seg32_at(base, 1);
+  auto issue = [&](int k) {
+    const unsigned bytes = (unsigned)min(kPairs, np - k * kPairs) * 96u;
+    mbar_expect_tx(&full[k % kStages], bytes);
+    bulk_g2s(tiles + (k % kStages) * 6 * kPairs, src + 24ll * k * kPairs, bytes, &full[k % kStages]);
   };
-  if (tid == 0) {
-    if (nt > 0) issue(0);
-    if (nt > 1) issue(1);
-  }
-  int issued = nt < 2 ? nt : 2, consumed = 0;
-  float hx = 0, hy = 0, hz = 0, cx = 0, cy = 0, cz = 0;  // Kahan sums over tiles
-  double nx = 0, ny = 0, nz = 0;                          // FP64 near field
-  for (int t = 0; t < nt; ++t) {
-    const int buf = t & 1;
-    const bool ok = mbar_wait(&bar[buf], (unsigned)((t >> 1) & 1));
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicOr(err, DERR_TIMEOUT);
+  int issued = 0;
+  if (tid == 0)
+    for (; issued < nt && issued < kStages - 1; ++issued) issue(issued);
+  float hs[3] = {0, 0, 0}, hc[3] = {0, 0, 0};  // Kahan sums
+  double n[3] = {0, 0, 0};                     // FP64 terms
+  for (int k = 0; k < nt; ++k) {
+    bool ok = true;
+    if (tid == 0 && issued < nt) {  // the next tile, once every warp has left its buffer
+      if (issued >= kStages) ok = mbar_wait(&empty[issued % kStages], (unsigned)((issued / kStages - 1) & 1));
+      if (ok) issue(issued++);
+    }
+    ok = ok && mbar_wait(&full[k % kStages], (unsigned)((k / kStages) & 1));
+    if (!__all_sync(0xffffffffu, ok)) {  // gave up: the other warps give up at their own waits
+      if (lane == 0) atomicOr(err, DERR_TIMEOUT);
       break;
     }
-    consumed = t + 1;
-    const int n = min(TJ, pc - t * TJ);
-    const int j0 = base + 1 + t * TJ;
-    const float4 *tl4 = tiles + buf * 3 * TJ;
-    if (active) {
-      // FP32 partial sums over sub-tiles of 32 segments, each added with Kahan compensation
-      for (int q0 = 0; q0 < n; q0 += 32) {
-        const int q1 = min(n, q0 + 32);
-        float ux = 0, uy = 0, uz = 0;
-#pragma unroll 4
-        for (int jj = q0; jj < q1; ++jj) {
-          const float4 H = tl4[3 * jj], L = tl4[3 * jj + 1], D = tl4[3 * jj + 2];
-          const int gj = j0 + jj;
-          if (H.w == 0.f || gj == pi_ || (m == 0 && gj == g)) continue;
-          const float rx = (H.x - th[0]) + (L.x - tl[0]);
-          const float ry = (H.y - th[1]) + (L.y - tl[1]);
-          const float rz = (H.z - th[2]) + (L.z - tl[2]);
-          const float a = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-          if (a >= near2) {
-            // FP32 unless the pair is ill-conditioned in FP32: the segment subtends more than
-            // 120 degrees, the target lies near its line (typically the next-but-one segment
-            // along the target's own filament), or near its far end
-            const float ex = rx + D.x, ey = ry + D.y, ez = rz + D.z;
-            const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-            const float crx = fmaf(ry, D.z, -rz * D.y), cry = fmaf(rz, D.x, -rx * D.z), crz = fmaf(rx, D.y, -ry * D.x);
-            const float cr2 = fmaf(crx, crx, fmaf(cry, cry, crz * crz));
-            const float re = fmaf(rx, ex, fmaf(ry, ey, rz * ez));
-            const float r1 = a * rsqrtf(a), r2 = ee * rsqrtf(ee);
-            const float pp = r1 * r2;
-            if (!(cr2 < gd.line * D.w * fminf(a, ee) || ee < gd.end * fmaxf(a, D.w) || pp + re < gd.angle * pp)) {
-              // pp + r.e = |r x d|^2 / (pp - r.e) when r.e < 0: no cancellation either way
-              const bool obtuse = re < 0.f;
-              const float num = gq * (r1 + r2) * (obtuse ? pp - re : 1.f);
-              const float f = __fdividef(num, pp * (obtuse ? cr2 : pp + re));  // MUFU reciprocal
-              ux = fmaf(f, crx, ux);
-              uy = fmaf(f, cry, uy);
-              uz = fmaf(f, crz, uz);
-              continue;
-            }
-          }
-          {
-            // near field and ill-conditioned pairs in FP64 from the FP64 segment records: the
-            // reference's skip decision (4ac - b^2 == 0, timestep.f90:166,192) in its own
-            // arithmetic, the value from the cancellation-free form
-            const double4 A = seg64[2 * (long long)gj], B = seg64[2 * (long long)gj + 1];
-            double r[3];
-            if (m == 0) {
-              r[0] = e_sub(A.x, xi[0]); r[1] = e_sub(A.y, xi[1]); r[2] = e_sub(A.z, xi[2]);
-            } else {
-              r[0] = e_sub(e_add(A.x, s[0]), xi[0]);
-              r[1] = e_sub(e_add(A.y, s[1]), xi[1]);
-              r[2] = e_sub(e_add(A.z, s[2]), xi[2]);
-            }
-            const double d[3] = {B.x, B.y, B.z};
-            const double aa = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
-            const double bb = e_mul(2.0, dot3(r, d));
-            if (e_sub(e_mul(e_mul(4.0, aa), B.w), e_mul(bb, bb)) != 0.0) {
-              double tm[3];
-              term64_stable(r, d, aa, gq64, tm);
-              nx += tm[0];
-              ny += tm[1];
-              nz += tm[2];
-            }
-          }
+    const ulonglong2 *tile = tiles + (k % kStages) * 6 * kPairs;
+    const int p0 = wid * kWarpPairs, p1 = min(min(kPairs, np - k * kPairs), p0 + kWarpPairs);
+    if (p0 < p1) {
+      const int bp = behind_p - k * kPairs;
+      f32x2 u[3] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
+#pragma unroll 2
+      for (int p = p0; p < p1; ++p) {
+        const ulonglong2 *q = tile + 6 * p;
+        const PairVec r = pair_vec(q, t);
+        const ulonglong2 v3 = q[3], v4 = q[4], v5 = q[5];
+        const PairSeg d = {{v3.x}, {v3.y}, {v4.x}, {v5.x}, {v5.y}};
+        const f32x2 far = {v4.y};
+        if (__all_sync(0xffffffffu, lo2(r.a) > lo2(far) && hi2(r.a) > hi2(far) && p != bp)) {
+          const PairGeo g2 = pair_geo(r, d);
+          const f32x2 sum = add2(g2.pp, g2.re);
+          const f32x2 f = mul2(g2.num, pack2(rcp_fast(lo2(sum)), rcp_fast(hi2(sum))));
+          u[0] = fma2(f, g2.cx, u[0]);
+          u[1] = fma2(f, g2.cy, u[1]);
+          u[2] = fma2(f, g2.cz, u[2]);
+        } else {
+          pair_guarded(r, d, t, k * kPairs + p, near2, gd, rec64, gq64, u, n);
         }
-        kahan_add(hx, cx, ux);
-        kahan_add(hy, cy, uy);
-        kahan_add(hz, cz, uz);
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) kahan_add(hs[c], hc[c], lo2(u[c]) + hi2(u[c]));
     }
-    __syncthreads();
-    if (t + 2 < nt) {
-      if (tid == 0) issue(t + 2);
-      issued = t + 3;
-    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[k % kStages]);
   }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) s_red[c][wid][lane] = gq64 * ((double)hs[c] - (double)hc[c]) + n[c];
+  __syncthreads();
+  // A give-up leaves copies in flight: wait for them (bounded) before shared memory is released.
   if (tid == 0)
-    for (int q = consumed; q < issued; ++q) mbar_wait(&bar[q & 1], (unsigned)((q >> 1) & 1));
-  if (!active) return;
-  const long long o = (long long)m * 3 * T + g;
-  partial[o] = ((double)hx - (double)cx) + nx;
-  partial[o + T] = ((double)hy - (double)cy) + ny;
-  partial[o + 2 * T] = ((double)hz - (double)cz) + nz;
+    for (int k = max(0, issued - kStages); k < issued; ++k) mbar_wait(&full[k % kStages], (unsigned)((k / kStages) & 1));
+  if (wid < 3 && t.active) {
+    double v = 0.;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) v += s_red[wid][k][lane];
+    partial[((long long)m * 3 + wid) * T + g] = v;
+  }
 }
 
 // Per target: u = local + partial[image 0] + sum_{images 1..n} partial[image], then MF and
@@ -210,8 +294,10 @@ __global__ void k_mixed_combine(const SysConst *__restrict__ scs, const SysDyn *
 
 void launch_direct_mixed(nv_handle *h) {
   if (h->n_work_img == 0) return;
-  const size_t smem = 2 * 3 * kTJ * sizeof(float4);
-  k_direct_mixed<kTJ><<<h->n_work_img, kTB, smem, h->stream>>>(
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(k_direct_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMixedSmem);
+  (void)attr;
+  k_direct_mixed<<<h->n_work_img, kTB, kMixedSmem, h->stream>>>(
       h->d_sc, h->d_dyn, h->d_work_img, h->x, h->nxt, h->prv, h->seg32, h->seg, h->partial, h->T, h->near_factor, h->guards,
       h->d_err);
 }
@@ -226,5 +312,3 @@ void launch_mixed_combine(nv_handle *h, int which) {
                                                      h->u, h->T, extra, which == 2 ? tree_iperm(h) : nullptr,
                                                      h->d_err);
 }
-
-int mixed_tiles_per_block() { return kTB; }

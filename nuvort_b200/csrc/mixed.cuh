@@ -78,6 +78,66 @@ __device__ __forceinline__ void term64_stable(const double r[3], const double d[
   out[2] = f * cr[2];
 }
 
+// ---- two FP32 values in one 64-bit register (packed FADD, FMUL, FFMA of sm_100) --------------
+// The packed instructions do two operations at the FP32 pipe's rate for one issue slot; each
+// half is rounded as the scalar operation rounds it.
+struct f32x2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float lo2(f32x2 x) {
+  return __uint_as_float((unsigned)x.v);
+}
+__device__ __forceinline__ float hi2(f32x2 x) {
+  return __uint_as_float((unsigned)(x.v >> 32));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+// Hardware 1/sqrt and 1/x without the scaling that denormal operands would need: the callers'
+// operands are squared distances and their products, far inside the normal range, or belong
+// to a term whose FP32 value is not used.
+__device__ __forceinline__ float rsqrt_fast(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The FP32 segment records of the direct sum, two segments side by side: 24 floats a pair,
+// {xh yh}{zh xl}{yl zl}{dx dy}{dz far}{-dx -dy}, each name the pair's two values; far is the
+// squared distance beyond which a target takes the segment's term without any guard
+// (kFarRatio |d|^2, and at least the near radius).  System slot k (from 1) is half (k-1) & 1
+// of the pair at seg32_at(base, k).
+//
+// Beyond 4|d| the segment subtends less than 30 degrees, r.e > 0 and |e| > 3/4 |r|: nothing in
+// the FP32 term cancels but r x d for a target near the segment's line, whose error stays
+// 2^-24 |r||d|, that of a term off the line.
+constexpr float kFarRatio = 16.f;
+__host__ __device__ __forceinline__ long long seg32_at(long long base, int k) {
+  return 12 * (base + 1) + 24 * (long long)((k - 1) >> 1);
+}
+
 // One node as the mixed walk reads it: 64 bytes, four 16-byte loads.
 struct __align__(16) WalkNode {
   float4 a;  // centre (FP32 high part), accept threshold t1^2 rounded to FP32
