@@ -266,9 +266,8 @@ int nv_set_insert_iterations(nv_handle *h, int32_t n);
  * through the exact path, for testing. */
 int nv_set_root_band(nv_handle *h, double scale);
 /* Split of the tree walks' work, so that a small system still fills the GPU.  Mixed
- * precision: the central image's walks (the deepest) are split over `parts` groups of the
- * root's children (1, 2, 4 or 8), each a work item of its own; the groups' sums are added in
- * group order.  Plain FP64: parts > 1 gives each target two threads, one summing the
+ * precision: `parts` warps (1, 2, 4 or 8) share the walk of 32 neighbouring targets; their sums
+ * are added in warp order.  Plain FP64: parts > 1 gives each target two threads, one summing the
  * unshifted image and one the 26 shifted ones, added in the reference's order (the result
  * is the same bit for bit); 1 keeps one thread per target.  0 (the default) picks the split
  * from the number of work items and the SM count. */
@@ -290,8 +289,8 @@ int nv_event_margins_get(nv_handle *h, int32_t sys, double *out);
  * nv_step(1).  With nv_set_walk_range a tree-walk system's velocity pass computes only the
  * targets at walk positions lo <= q < hi (the walk order: the live points in Morton order at
  * positions 1 .. live, then the empty slots).  The ends fall on warp boundaries: lo - 1 a
- * multiple of 32, and hi - 1 one too or hi = cap + 1 (the mixed walk's 32 targets of a warp
- * share their FP32 partial sums' flush points, which a warp cut in two would change); other
+ * multiple of 32, and hi - 1 one too or hi = cap + 1 (the mixed walk's 32 targets of a group
+ * share the order of their terms, which a group cut in two would change); other
  * ends are refused with NV_ERR_ARG.  nv_velocity_pack copies the velocities of
  * positions lo .. lo+count-1 into a device buffer [count][3] and nv_velocity_unpack writes
  * them back, so that ranks split the positions, exchange their parts between the two halves

@@ -430,7 +430,7 @@ class Handle:
         _check(lib().nv_set_root_band(self.h, float(scale)))
 
     def set_walk_parts(self, parts: int):
-        """Split of the tree walks' work (mixed: central image over groups of root children;
+        """Split of the tree walks' work (mixed: warps per group of 32 targets;
         FP64: unshifted / shifted images on two threads per target); 0: automatic."""
         _check(lib().nv_set_walk_parts(self.h, int(parts)))
 

@@ -115,8 +115,8 @@ def tune_launch_shapes(handle, repeats: int = 3) -> Dict:
     """Block shapes of the velocity pass, measured on `handle`'s own systems, the fastest kept
     (set on the handle):
 
-    * walk_parts (nv_set_walk_parts) for tree-walk systems: the mixed walk's central image over
-      1, 2, 4 or 8 groups of root children (more, shorter blocks for small systems); the
+    * walk_parts (nv_set_walk_parts) for tree-walk systems: the mixed walk's groups of 32
+      targets on 1, 2, 4 or 8 warps each (more for small systems); the
       plain FP64 walk's unshifted and shifted images on one or two threads per target;
     * direct split (nv_set_direct_split) for plain FP64 direct-sum systems: one thread per
       target (64) or 8, 4, 2, 1 targets per block, each target's terms spread over the block.

@@ -307,9 +307,8 @@ int dalloc(T **p, size_t n) {
   return NV_OK;
 }
 
-void build_worklist(nv_handle *h, int which, std::vector<int2> &w) {
+void build_worklist(nv_handle *h, int which, std::vector<int2> &w, int tb) {
   w.clear();
-  const int tb = h->direct_tb;
   for (int s = 0; s < h->nsys; ++s) {
     const SysConst &sc = h->sc[s];
     int kind = sc.velocity == NV_VEL_LIA ? 0 : (sc.sched_tree ? 2 : 1);
@@ -338,34 +337,27 @@ int upload_worklist4(int4 **dptr, int *n, const std::vector<int4> &w) {
   return NV_OK;
 }
 
-// (system, image, first slot, part) items over every image of every system of one kind.
-// With parts > 1 the central image (the deepest walks) is listed once per part, each part
-// walking a group of the root's children; all central items come first.
-void build_image_worklist(nv_handle *h, int which, int tb, std::vector<int4> &w, int parts = 1) {
+// (system, image, first slot) items over every image of every direct-sum system.
+void build_image_worklist(nv_handle *h, int tb, std::vector<int4> &w) {
   w.clear();
-  for (int pass = 0; pass < 2; ++pass)
-    for (int s = 0; s < h->nsys; ++s) {
-      const SysConst &sc = h->sc[s];
-      int kind = sc.velocity == NV_VEL_LIA ? 0 : (sc.sched_tree ? 2 : 1);
-      if (kind != which) continue;
-      for (int m = pass == 0 ? 0 : 1; m <= (pass == 0 ? 0 : sc.n_shift); ++m)
-        for (int part = 0; part < (m == 0 ? parts : 1); ++part)
-          for (int k = 1; k <= h->cap[s]; k += tb) w.push_back(make_int4(s, m, sc.base + k, part));
-    }
+  for (int s = 0; s < h->nsys; ++s) {
+    const SysConst &sc = h->sc[s];
+    if (sc.velocity == NV_VEL_LIA || sc.sched_tree) continue;
+    for (int m = 0; m <= sc.n_shift; ++m)
+      for (int k = 1; k <= h->cap[s]; k += tb) w.push_back(make_int4(s, m, sc.base + k, 0));
+  }
 }
 
-// Central-image split of the mixed tree walk: enough central blocks to fill the GPU about
-// four times over (the central walks are the longest, and a few hundred of them leave most
-// SMs idle), at most one part per root child.
+// Warps per group of 32 targets of the mixed tree walk: 8 while the groups' blocks are all
+// resident at once (three of 256 threads to an SM), where a group's own time counts (8,000
+// points: 164 us, 217 with 4), 4 up to 40 groups an SM (100,000 points: 1.41 ms; 1.67 with 8,
+// 1.54 with 2), and 2 beyond, where the groups fill the GPU anyway and a round's barriers
+// cost more than its parallelism gives (1M points: 9.8 ms, 10.3 with 4, 10.2 with 1).
 int auto_walk_parts(const nv_handle *h) {
-  long long central = 0;
+  long long groups = 0;
   for (int s = 0; s < h->nsys; ++s)
-    if (h->sc[s].sched_tree && h->sc[s].velocity != NV_VEL_LIA) central += (h->cap[s] + 127) / 128;
-  if (central == 0) return 1;
-  const long long resident = 8LL * n_sms_host();
-  int p = 1;
-  while (p < kMaxWalkParts && central * p < 4 * resident) p *= 2;
-  return p;
+    if (h->sc[s].sched_tree && h->sc[s].velocity != NV_VEL_LIA) groups += (h->cap[s] + 31) / 32;
+  return groups <= 3LL * n_sms_host() ? 8 : groups <= 40LL * n_sms_host() ? 4 : 2;
 }
 
 int rebuild_worklists(nv_handle *h) {
@@ -373,21 +365,21 @@ int rebuild_worklists(nv_handle *h) {
   int rc;
   if (h->precision == NV_PREC_MIXED) {
     std::vector<int4> w4;
-    build_image_worklist(h, 1, 32, w4);
+    build_image_worklist(h, 32, w4);
     if ((rc = upload_worklist4(&h->d_work_img, &h->n_work_img, w4)) != NV_OK) return rc;
     h->walk_parts_used = h->walk_parts > 0 ? h->walk_parts : auto_walk_parts(h);
-    build_image_worklist(h, 2, 128, w4, h->walk_parts_used);
-    if ((rc = upload_worklist4(&h->d_work_timg, &h->n_work_timg, w4)) != NV_OK) return rc;
+    build_worklist(h, 2, w, 32);
+    if ((rc = upload_worklist(&h->d_work_grp, &h->n_work_grp, w)) != NV_OK) return rc;
   }
   for (int s = 0; s < h->nsys; ++s)
     if (h->sc[s].sched_tree) {
       h->tree_sys0 = s;
       break;
     }
-  build_worklist(h, 0, w);
+  build_worklist(h, 0, w, h->direct_tb);
   if ((rc = upload_worklist(&h->d_work_lia, &h->n_work_lia, w)) != NV_OK) return rc;
   h->any_lia = !w.empty();
-  build_worklist(h, 1, w);
+  build_worklist(h, 1, w, h->direct_tb);
   if ((rc = upload_worklist(&h->d_work_direct, &h->n_work_direct, w)) != NV_OK) return rc;
   h->any_direct = !w.empty();
   {  // the split direct sum for few targets: items of direct_g slots
@@ -402,7 +394,7 @@ int rebuild_worklists(nv_handle *h) {
           for (int k = 1; k <= h->cap[s]; k += h->direct_g) w.push_back(make_int2(s, h->sc[s].base + k));
     if ((rc = upload_worklist(&h->d_work_split, &h->n_work_split, w)) != NV_OK) return rc;
   }
-  build_worklist(h, 2, w);
+  build_worklist(h, 2, w, h->direct_tb);
   if ((rc = upload_worklist(&h->d_work_tree, &h->n_work_tree, w)) != NV_OK) return rc;
   h->any_tree = !w.empty();
   return NV_OK;
@@ -715,8 +707,8 @@ int nv_create(const nv_params *params, int32_t nsys, const int32_t *capacity, in
     bool direct = false;
     for (auto &c : h->sc) direct |= c.velocity == NV_VEL_BS;
     if (direct && (rc = dalloc(&h->seg32, 12 * ((size_t)T + 1)))) return bail(rc);
-    const int nimg = 27 + kMaxWalkParts - 1;  // the images, then the central image's extra parts
-    if ((rc = dalloc(&h->partial, (size_t)nimg * 3 * T))) return bail(rc);
+    // the direct sum's images one by one; the tree walk's targets take the first for all
+    if ((rc = dalloc(&h->partial, (size_t)(direct ? 27 : 1) * 3 * T))) return bail(rc);
   }
   h->event_cap = (int)std::min<long long>(std::max<long long>(1 << 16, T), 1 << 24);
   if ((rc = dalloc(&h->d_events, h->event_cap))) return bail(rc);
@@ -754,7 +746,7 @@ int nv_destroy(nv_handle *h) {
   for (void *p : h->nf_buffers) cudaFree(p);
   void *ptrs[] = {h->bstage, h->d_btab, h->d_bcheck, h->pin, h->umir, h->usm, h->cs, h->d_drec, h->partial, h->stage, h->d_upck, h->d_sc, h->d_dyn, h->x, h->u, h->u1, h->u2, h->gi, h->gb, h->closestd, h->nxt, h->prv,
                   h->closest, h->sys_of, h->seg, h->seg32, h->d_err, h->d_events, h->d_event_count,
-                  h->d_work_direct, h->d_work_tree, h->d_work_lia, h->d_work_img, h->d_work_timg, h->d_work_split};
+                  h->d_work_direct, h->d_work_tree, h->d_work_lia, h->d_work_img, h->d_work_grp, h->d_work_split};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : h->ev)

@@ -25,7 +25,7 @@ __global__ void k_begin_step(SysDyn *dyn, int nsys, const unsigned *err) {
 // ~1e-16), segment vector; zero for an empty slot (no contribution).  The last slot of an odd
 // capacity also clears the other half of its pair.
 __device__ __forceinline__ void put_seg32(float *seg32, const SysConst &sc, int k, const double x[3],
-                                          const double d[3], double c, double near_factor) {
+                                          const double d[3], double c, double near_factor, float far_ratio) {
   if (k < 1 || k > sc.cap) return;
   float *p = seg32 + seg32_at(sc.base, k) + ((k - 1) & 1);
   float v[12];
@@ -36,7 +36,7 @@ __device__ __forceinline__ void put_seg32(float *seg32, const SysConst &sc, int 
     v[6 + a] = (float)d[a];
   }
   const double nr = near_factor * sc.delta;
-  v[9] = fmaxf(kFarRatio * (float)c, (float)(nr * nr));
+  v[9] = fmaxf(far_ratio * (float)c, (float)(nr * nr));
   v[10] = -v[6];
   v[11] = -v[7];
 #pragma unroll
@@ -53,7 +53,8 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
                         const int *__restrict__ sys_of, const double *__restrict__ X,
                         const int *__restrict__ nxt, const int *__restrict__ prv,
                         double *__restrict__ GI, double *__restrict__ GB, double4 *__restrict__ seg,
-                        float *__restrict__ seg32, double near_factor, long long T, const unsigned *err) {
+                        float *__restrict__ seg32, double near_factor, float far_ratio, long long T,
+                        const unsigned *err) {
   const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= T || *err) return;
   int s;
@@ -63,7 +64,7 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
     seg[2 * g] = make_double4(0, 0, 0, 0);
     seg[2 * g + 1] = make_double4(0, 0, 0, 0);
     const double zero[3] = {0, 0, 0};
-    if (seg32) put_seg32(seg32, scs[s], (int)(g - scs[s].base), zero, zero, 0.0, near_factor);
+    if (seg32) put_seg32(seg32, scs[s], (int)(g - scs[s].base), zero, zero, 0.0, near_factor, far_ratio);
     return;
   }
   const SysConst &sc = scs[s];
@@ -82,7 +83,7 @@ __global__ void k_ghost(const SysConst *__restrict__ scs, const SysDyn *__restri
   // with a zero segment vector its terms drop out by 4ac - b^2 = 0, like an empty slot's
   seg[2 * g] = make_double4(x[0], x[1], x[2], pin_i(pin) ? 0.0 : 1.0);
   seg[2 * g + 1] = pin_i(pin) ? make_double4(0, 0, 0, 0) : make_double4(d[0], d[1], d[2], c);
-  if (seg32) put_seg32(seg32, sc, (int)(g - sc.base), x, d, c, near_factor);
+  if (seg32) put_seg32(seg32, sc, (int)(g - sc.base), x, d, c, near_factor, far_ratio);
 }
 
 // calc_velocity with velocity 'LIA' (timestep.f90:60-73): local term + MF only.
@@ -202,7 +203,8 @@ void launch_begin_step(nv_handle *h) {
 
 void launch_ghost(nv_handle *h) {
   k_ghost<<<grid_for(h->T, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, h->prv,
-                                                     h->gi, h->gb, h->seg, h->seg32, h->near_factor, h->T, h->d_err);
+                                                     h->gi, h->gb, h->seg, h->seg32, h->near_factor, far_ratio(h->guards), h->T,
+                                                     h->d_err);
 }
 
 void launch_velocity(nv_handle *h) {
@@ -252,5 +254,5 @@ void launch_end_step(nv_handle *h) {
 void launch_ghost_raw(cudaStream_t st, const SysConst *sc, const SysDyn *dyn, const int *sys_of, const double *x,
                       const int *nxt, const int *prv, double *gi, double *gb, double4 *seg, long long T,
                       unsigned *err) {
-  k_ghost<<<grid_for(T, TB), TB, 0, st>>>(sc, dyn, sys_of, x, nxt, prv, gi, gb, seg, nullptr, 0.0, T, err);
+  k_ghost<<<grid_for(T, TB), TB, 0, st>>>(sc, dyn, sys_of, x, nxt, prv, gi, gb, seg, nullptr, 0.0, 0.f, T, err);
 }

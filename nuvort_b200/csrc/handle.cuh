@@ -50,15 +50,15 @@ struct nv_handle {
   int *d_upck = nullptr;     // nv_upload checks: [0] link errors (1 out of range, 2 empty-slot mismatch), [1] live slots
   int4 *d_work_img = nullptr;  // (system, image, first slot) items of 32 slots of the mixed direct sum
   int n_work_img = 0;
-  int4 *d_work_timg = nullptr; // same for the mixed tree walk
-  int n_work_timg = 0;
+  int2 *d_work_grp = nullptr;  // (system, first walk position) items of 32 targets of the mixed tree walk
+  int n_work_grp = 0;
   double near_factor = 2.0;    // near field: pairs closer than near_factor*delta run in FP64
   Fp32Guards guards;
   double root_band_scale = 1.0;  // scale of the root centre estimate's error bound
   int ins_iters = 6;  // fixed-point iterations of the parallel pinsert; 0: serial sweep only
   int tree_sys0 = 0;           // first system that walks the tree (its theta0 builds the mixed nodes)
-  int walk_parts = 0;          // central image of the mixed tree walk split over this many root-child groups (0: automatic)
-  int walk_parts_used = 1;     // the split the work list was built with
+  int walk_parts = 0;          // warps per group of 32 targets of the mixed tree walk (0: automatic)
+  int walk_parts_used = 1;     // the number in use
   unsigned links_epoch = 0;    // bumped by every stage that relinks points (pinsert, precon, premove, upload)
   unsigned *d_err = nullptr;
   DevEvent *d_events = nullptr;
@@ -117,7 +117,7 @@ void launch_tree_walk_mixed(nv_handle *h);
 const int *tree_iperm(nv_handle *h);  // slot -> walk position of the last tree build (or null)
 const int *tree_perm(nv_handle *h);   // walk position (global: base + q) -> slot
 // tree (tree.cu)
-constexpr int kMaxWalkParts = 8;  // the central image's walk splits over at most the root's 8 children
+constexpr int kMaxWalkParts = 8;
 int n_sms_host();                  // SMs of the current device
 void tree_alloc(nv_handle *h);
 void tree_free(nv_handle *h);

@@ -40,49 +40,11 @@ __device__ __noinline__ double3 direct_term64(const double4 *__restrict__ rec, d
 }
 
 // What the lanes of a warp hold of their targets.
-struct MixedTarget {
-  double x[3], s[3];     // position, image shift
-  f32x2 h[3], l[3];      // shift - position, FP32 high and low parts
-  int behind, own;       // segments (from 0) that are skipped
+struct MixedTarget : LaneTarget {
+  double x[3], s[3];  // position, image shift
+  int behind, own;    // segments (from 0) that are skipped
   bool active;
 };
-
-// Two segments (pair p of the system, its record at q) for a lane: r from the target, its
-// square; then the term f (r x d).
-struct PairVec {
-  f32x2 rx, ry, rz, a;
-};
-__device__ __forceinline__ PairVec pair_vec(const ulonglong2 *q, const MixedTarget &t) {
-  const ulonglong2 v0 = q[0], v1 = q[1], v2 = q[2];
-  PairVec r;
-  r.rx = add2(add2({v0.x}, t.h[0]), add2({v1.y}, t.l[0]));
-  r.ry = add2(add2({v0.y}, t.h[1]), add2({v2.x}, t.l[1]));
-  r.rz = add2(add2({v1.x}, t.h[2]), add2({v2.y}, t.l[2]));
-  r.a = fma2(r.rx, r.rx, fma2(r.ry, r.ry, mul2(r.rz, r.rz)));
-  return r;
-}
-struct PairSeg {
-  f32x2 dx, dy, dz, ndx, ndy;
-};
-struct PairGeo {
-  f32x2 cx, cy, cz;      // r x d
-  f32x2 ee, re, pp, num; // |e|^2, r.e, |r||e|, 1/|r| + 1/|e| with e = r + d
-};
-__device__ __forceinline__ PairGeo pair_geo(const PairVec &r, const PairSeg &d) {
-  const f32x2 kMinus = pack2(-1.f, -1.f);
-  PairGeo g;
-  const f32x2 ex = add2(r.rx, d.dx), ey = add2(r.ry, d.dy), ez = add2(r.rz, d.dz);
-  g.ee = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
-  g.re = fma2(r.rx, ex, fma2(r.ry, ey, mul2(r.rz, ez)));
-  g.cx = fma2(r.ry, d.dz, mul2(r.rz, d.ndy));
-  g.cy = fma2(r.rz, d.dx, mul2(mul2(r.rx, kMinus), d.dz));
-  g.cz = fma2(r.rx, d.dy, mul2(r.ry, d.ndx));
-  const f32x2 ia = pack2(rsqrt_fast(lo2(r.a)), rsqrt_fast(hi2(r.a)));
-  const f32x2 ib = pack2(rsqrt_fast(lo2(g.ee)), rsqrt_fast(hi2(g.ee)));
-  g.pp = mul2(mul2(r.a, ia), mul2(g.ee, ib));
-  g.num = add2(ia, ib);
-  return g;
-}
 
 // A pair that some lane of the warp is not far from: every lane's own guards decide between
 // FP32 and FP64 (into n).
@@ -90,8 +52,7 @@ __device__ __forceinline__ void pair_guarded(const PairVec &r, const PairSeg &d,
                                              float near2, const Fp32Guards &gd, const double4 *__restrict__ seg64,
                                              double gq64, f32x2 u[3], double n[3]) {
   const PairGeo g = pair_geo(r, d);
-  const f32x2 c = fma2(d.dx, d.dx, fma2(d.dy, d.dy, mul2(d.dz, d.dz)));
-  const f32x2 cr2 = fma2(g.cx, g.cx, fma2(g.cy, g.cy, mul2(g.cz, g.cz)));
+  const f32x2 c = square2(d.dx, d.dy, d.dz), cr2 = square2(g.cx, g.cy, g.cz);
   float f[2];
   bool bad[2];
 #pragma unroll
@@ -222,10 +183,8 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
       for (int p = p0; p < p1; ++p) {
         const ulonglong2 *q = tile + 6 * p;
         const PairVec r = pair_vec(q, t);
-        const ulonglong2 v3 = q[3], v4 = q[4], v5 = q[5];
-        const PairSeg d = {{v3.x}, {v3.y}, {v4.x}, {v5.x}, {v5.y}};
-        const f32x2 far = {v4.y};
-        if (__all_sync(0xffffffffu, lo2(r.a) > lo2(far) && hi2(r.a) > hi2(far) && p != bp)) {
+        const PairSeg d = pair_seg(q);
+        if (__all_sync(0xffffffffu, lo2(r.a) > lo2(d.far) && hi2(r.a) > hi2(d.far) && p != bp)) {
           const PairGeo g2 = pair_geo(r, d);
           const f32x2 sum = add2(g2.pp, g2.re);
           const f32x2 f = mul2(g2.num, pack2(rcp_fast(lo2(sum)), rcp_fast(hi2(sum))));
@@ -262,7 +221,7 @@ __global__ void k_mixed_combine(const SysConst *__restrict__ scs, const SysDyn *
                                 const int2 *__restrict__ work, const double *__restrict__ X,
                                 const double *__restrict__ GI, const double *__restrict__ GB,
                                 const int *__restrict__ nxt, const double *__restrict__ partial,
-                                double *__restrict__ U, long long T, int extra, const int *__restrict__ iperm,
+                                double *__restrict__ U, long long T, bool per_image, const int *__restrict__ iperm,
                                 const unsigned *err) {
   if (*err) return;
   const int2 w = work[blockIdx.x];
@@ -281,10 +240,9 @@ __global__ void k_mixed_combine(const SysConst *__restrict__ scs, const SysDyn *
   local_velocity(sc, xi, gi, gb, u, fdot);
   double b0[3], bs[3] = {0, 0, 0};
   for (int c = 0; c < 3; ++c) b0[c] = partial[(long long)c * T + g];
-  for (int e = 1; e <= extra; ++e)  // the central image's other parts, in part order
-    for (int c = 0; c < 3; ++c) b0[c] += partial[((long long)(26 + e) * 3 + c) * T + g];
-  for (int m = 1; m <= sc.n_shift; ++m)
-    for (int c = 0; c < 3; ++c) bs[c] += partial[((long long)m * 3 + c) * T + g];
+  if (per_image)  // the direct sum's images; the tree walk's one sum holds them all
+    for (int m = 1; m <= sc.n_shift; ++m)
+      for (int c = 0; c < 3; ++c) bs[c] += partial[((long long)m * 3 + c) * T + g];
   for (int c = 0; c < 3; ++c) u[c] = e_add(e_add(u[c], b0[c]), bs[c]);
   mf_epilogue(sc, dyn[w.x], xi, fdot, u, g);
   store3(U, T, g, u);
@@ -307,8 +265,7 @@ void launch_mixed_combine(nv_handle *h, int which) {
   const int2 *wl = which == 1 ? h->d_work_direct : h->d_work_tree;
   const int n = which == 1 ? h->n_work_direct : h->n_work_tree;
   if (n == 0) return;
-  const int extra = which == 2 ? h->walk_parts_used - 1 : 0;
   k_mixed_combine<<<n, h->direct_tb, 0, h->stream>>>(h->d_sc, h->d_dyn, wl, h->x, h->gi, h->gb, h->nxt, h->partial,
-                                                     h->u, h->T, extra, which == 2 ? tree_iperm(h) : nullptr,
+                                                     h->u, h->T, which == 1, which == 2 ? tree_iperm(h) : nullptr,
                                                      h->d_err);
 }

@@ -127,23 +127,74 @@ __device__ __forceinline__ float rcp_fast(float x) {
 // The FP32 segment records of the direct sum, two segments side by side: 24 floats a pair,
 // {xh yh}{zh xl}{yl zl}{dx dy}{dz far}{-dx -dy}, each name the pair's two values; far is the
 // squared distance beyond which a target takes the segment's term without any guard
-// (kFarRatio |d|^2, and at least the near radius).  System slot k (from 1) is half (k-1) & 1
+// (far_ratio |d|^2, and at least the near radius).  System slot k (from 1) is half (k-1) & 1
 // of the pair at seg32_at(base, k).
-//
-// Beyond 4|d| the segment subtends less than 30 degrees, r.e > 0 and |e| > 3/4 |r|: nothing in
-// the FP32 term cancels but r x d for a target near the segment's line, whose error stays
-// 2^-24 |r||d|, that of a term off the line.
-constexpr float kFarRatio = 16.f;
 __host__ __device__ __forceinline__ long long seg32_at(long long base, int k) {
   return 12 * (base + 1) + 24 * (long long)((k - 1) >> 1);
+}
+
+// Terms beyond far_ratio |d|^2 are taken without the guards: there, beyond 4|d|, the segment
+// subtends less than 30 degrees, r.e > 0 and |e| > 3/4 |r|, so that nothing cancels in FP32 but
+// r x d for a target near the segment's line, whose error stays 2^-24 |r||d|, that of a term
+// off the line.  Guards that a caller widened past these bounds apply to every term.
+inline float far_ratio(const Fp32Guards &g) {
+  return g.angle <= 1.9f && g.end <= 0.5f && g.line <= 1e-3f ? 16.f : 3e38f;
+}
+
+// What a lane holds of its target for the packed terms, and a pair of segments (or accepted
+// tree nodes) as a 24-float record q (see seg32_at): r from the target, its square, the term's
+// parts.
+struct LaneTarget {
+  f32x2 h[3], l[3];  // minus the target (direct sum: image shift - target), FP32 high and low
+};
+struct PairVec {
+  f32x2 rx, ry, rz, a;
+};
+__device__ __forceinline__ PairVec pair_vec(const ulonglong2 *q, const LaneTarget &t) {
+  const ulonglong2 v0 = q[0], v1 = q[1], v2 = q[2];
+  PairVec r;
+  r.rx = add2(add2({v0.x}, t.h[0]), add2({v1.y}, t.l[0]));
+  r.ry = add2(add2({v0.y}, t.h[1]), add2({v2.x}, t.l[1]));
+  r.rz = add2(add2({v1.x}, t.h[2]), add2({v2.y}, t.l[2]));
+  r.a = fma2(r.rx, r.rx, fma2(r.ry, r.ry, mul2(r.rz, r.rz)));
+  return r;
+}
+struct PairSeg {
+  f32x2 dx, dy, dz, ndx, ndy, far;  // d, -dx, -dy, the far bound (direct sum)
+};
+__device__ __forceinline__ PairSeg pair_seg(const ulonglong2 *q) {
+  const ulonglong2 v3 = q[3], v4 = q[4], v5 = q[5];
+  return {{v3.x}, {v3.y}, {v4.x}, {v5.x}, {v5.y}, {v4.y}};
+}
+struct PairGeo {
+  f32x2 cx, cy, cz;      // r x d
+  f32x2 ee, re, pp, num; // |e|^2, r.e, |r||e|, 1/|r| + 1/|e| with e = r + d
+};
+__device__ __forceinline__ PairGeo pair_geo(const PairVec &r, const PairSeg &d) {
+  const f32x2 kMinus = pack2(-1.f, -1.f);
+  PairGeo g;
+  const f32x2 ex = add2(r.rx, d.dx), ey = add2(r.ry, d.dy), ez = add2(r.rz, d.dz);
+  g.ee = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
+  g.re = fma2(r.rx, ex, fma2(r.ry, ey, mul2(r.rz, ez)));
+  g.cx = fma2(r.ry, d.dz, mul2(r.rz, d.ndy));
+  g.cy = fma2(r.rz, d.dx, mul2(mul2(r.rx, kMinus), d.dz));
+  g.cz = fma2(r.rx, d.dy, mul2(r.ry, d.ndx));
+  const f32x2 ia = pack2(rsqrt_fast(lo2(r.a)), rsqrt_fast(hi2(r.a)));
+  const f32x2 ib = pack2(rsqrt_fast(lo2(g.ee)), rsqrt_fast(hi2(g.ee)));
+  g.pp = mul2(mul2(r.a, ia), mul2(g.ee, ib));
+  g.num = add2(ia, ib);
+  return g;
+}
+__device__ __forceinline__ f32x2 square2(f32x2 x, f32x2 y, f32x2 z) {
+  return fma2(x, x, fma2(y, y, mul2(z, z)));
 }
 
 // One node as the mixed walk reads it: 64 bytes, four 16-byte loads.
 struct __align__(16) WalkNode {
   float4 a;  // centre (FP32 high part), accept threshold t1^2 rounded to FP32
   float4 b;  // centre (FP32 low part: centre - high part), |circ|^2 in FP32
-  float4 c;  // circulation in FP32, the line guard's threshold (Fp32Guards::line x |circ|^2)
-  int4 d;    // pcount, first child, next sibling, first member's infront
+  float4 c;  // circulation in FP32, unused
+  int4 d;    // pcount, first child, number of children, first member's infront (a leaf's: prv of it)
 };
 
 struct MixedNodes {  // per tree node, built after the FP64 node sums

@@ -34,9 +34,7 @@ constexpr int kSnapLevel = 1;  // the early block sums: the big nodes of depth 1
 // [+0..+2] nodes above kBigNode members (split by a block), [+3..+5] the others with >= 2
 constexpr int kCtrSplit = kMaxLevels + 8;
 constexpr int kCtrSize = kMaxLevels + 16;
-constexpr int kDeferCap = 1 << 20;  // deferred root tests listed per velocity pass
-constexpr int kFlush = 16;      // FP32 far-field terms summed before promotion to FP64
-static_assert((kFlush & (kFlush - 1)) == 0, "the walk tests the flush by a mask");
+constexpr int kDeferCap = 1 << 20;  // targets with a deferred root test listed per velocity pass
 
 struct TreeBuffers {
   int max_nodes = 0;
@@ -48,7 +46,7 @@ struct TreeBuffers {
   int2 *nR = nullptr;     // member range start, member count
   int *nDepth = nullptr;
   int *nLeaf = nullptr;
-  int *nSib = nullptr;    // next sibling, or kEnd for a last child (and roots)
+  int *nKids = nullptr;   // number of children (contiguous from first_child)
   int *members = nullptr;
   // roots: a parallel estimate of the centre with a bound on its distance to the exact
   // (sequential) one, so the walks need not wait for the exact sum; (target, image) pairs
@@ -64,7 +62,7 @@ struct TreeBuffers {
   double4 *root_apx = nullptr;  // per system: centre estimate, bound
   double *root_part = nullptr;  // per system and part: partial sums of x, y, z, |x|, |y|, |z|
   int root_parts = 1;
-  int2 *defer = nullptr;        // (slot, image) pairs, image -1: the whole target (FP64 walk)
+  int *defer = nullptr;         // slots of the deferred targets
   int *defer_n = nullptr;
   int *bigl = nullptr;    // non-root nodes with more than kBlockSumNode members
   int max_big = 0;
@@ -137,7 +135,7 @@ __global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
   tb.nI[s] = make_int4(pc, kEnd, kEnd, pc >= 1 ? nxt[sc.base + 1] : 0);
   tb.nR[s] = make_int2(pos[sc.base], pos[sc.base + sc.cap + 1] - pos[sc.base]);
   tb.nDepth[s] = 0;
-  tb.nSib[s] = kEnd;
+  tb.nKids[s] = 0;
   for (int d = 0; d < 8; ++d) tb.root_cnt[8 * s + d] = 0;
   tb.nLeaf[s] = pc == 1 ? sc.base + 1 : 0;
   dyn[s].tree_eval = 0;
@@ -266,7 +264,7 @@ __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const S
     tb.nI[id] = make_int4(cnt[d], kEnd, last ? Ip.z : id + 1, 0);
     tb.nR[id] = make_int2(mb0 + off, cnt[d]);
     tb.nDepth[id] = depth;
-    tb.nSib[id] = last ? kEnd : id + 1;
+    tb.nKids[id] = 0;
     if (cnt[d] >= 2) {  // the child's level list of nodes still to split
       if (cnt[d] > kBigNode) tb.split_blk[lb][qb + kb++] = id;
       else tb.split_wrp[lb][qw + kw++] = id;
@@ -276,6 +274,7 @@ __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const S
     ++k;
   }
   tb.nI[p].y = id0;
+  tb.nKids[p] = n.nchild;
   return true;
 }
 
@@ -334,7 +333,7 @@ __device__ void make_children(TreeBuffers &tb, int p, const int cnt[8], int *id0
     tb.nI[id] = make_int4(cnt[d], kEnd, last ? Ip.z : id + 1, 0);
     tb.nR[id] = make_int2(mb0 + off, cnt[d]);
     tb.nDepth[id] = depth;
-    tb.nSib[id] = last ? kEnd : id + 1;
+    tb.nKids[id] = 0;
     if (cnt[d] >= 2) {  // the child's level list of nodes still to split
       if (cnt[d] > kBigNode) tb.split_blk[lb][qb + kb++] = id;
       else tb.split_wrp[lb][qw + kw++] = id;
@@ -344,6 +343,7 @@ __device__ void make_children(TreeBuffers &tb, int p, const int cnt[8], int *id0
     ++k;
   }
   tb.nI[p].y = id0;
+  tb.nKids[p] = nchild;
   *id0_out = id0;
   *mb0_out = mb0;
 }
@@ -1070,9 +1070,9 @@ __device__ __forceinline__ int root_decision(const TreeBuffers &tb, const SysCon
   return 2;
 }
 
-__device__ __forceinline__ void defer_push(const TreeBuffers &tb, int g, int m, unsigned *err) {
+__device__ __forceinline__ void defer_push(const TreeBuffers &tb, int g, unsigned *err) {
   const int q = atomicAdd(tb.defer_n, 1);
-  if (q < kDeferCap) tb.defer[q] = make_int2(g, m);
+  if (q < kDeferCap) tb.defer[q] = g;
   else atomicOr(err, DERR_QUEUE);
 }
 
@@ -1253,7 +1253,8 @@ __global__ void k_tree_walk_mirror(const SysConst *__restrict__ scs, SysDyn *dyn
 
 // The tree sums of target g (timestep.f90:49-141 with tree_walk): over the unshifted image
 // into ub0, then over the 26 shifts in order into ubs.  part 0 does both and the epilogue;
-// part 1 only ub0, part 2 only ubs (the epilogue then runs where both are known) -- each
+// part 1 only ub0, part 2 only ubs (the epilogue then runs where both are known), part 3 both
+// without the epilogue -- each
 // sum is the same chain of additions either way.  With `decided` the root's tests come from
 // the centre estimate: a target for which any of them is too close to call is deferred
 // whole (nothing counted; part 2 leaves the push to part 1), to be redone exactly.  Returns
@@ -1274,7 +1275,7 @@ __device__ bool fp64_target(const SysConst &sc, const SysDyn &dy, int sys, int g
     if (!decided) continue;
     const int d = root_decision(tb, sc, sys, xi, m == 0 ? zero : sc.shift[m - 1]);
     if (d == 2) {
-      if (part != 2) defer_push(tb, g, -1, err);
+      if (part != 2) defer_push(tb, g, err);
       return false;
     }
     start[m] = d == 1 ? kEnd : first;  // accepted: adds nothing; opened: walk the children
@@ -1335,36 +1336,21 @@ __global__ void __launch_bounds__(128) k_tree_walk_fp64(const SysConst *__restri
   if ((threadIdx.x & 31) == 0 && tt) atomicAdd(&dyn[w.x].tree_tests, tt);
 }
 
-// The deferred root tests, after the exact root sums: FP64 targets again whole (image -1),
-// mixed (target, image) pairs as that image's partial sum from the exact FP64 walk.
+// The targets with a deferred root test, after the exact root sums: again whole, by the exact
+// FP64 walk (with `partial`, the mixed path, their sums go there).
 __global__ void k_walk_fixup(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of,
                              const double *__restrict__ X, const double *__restrict__ GI,
                              const double *__restrict__ GB, const int *__restrict__ prv, double *__restrict__ U,
                              double *__restrict__ partial, long long T, TreeBuffers tb, unsigned *err) {
   const int n = min(*tb.defer_n, kDeferCap);
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const int2 d = tb.defer[e];
-    const int g = d.x, s = sys_of[g];
+    const int g = tb.defer[e], s = sys_of[g];
     const SysConst &sc = scs[s];
     unsigned long long evals = 0, tests = 0;
-    if (d.y < 0) {
-      double ub0[3], ubs[3];
-      fp64_target(sc, dyn[s], s, g, X, GI, GB, prv, U, T, tb, false, 0, ub0, ubs, evals, tests, err);
-    } else {
-      const int m = d.y;
-      double xi[3], acc[3] = {0, 0, 0};
-      const double zero[3] = {0, 0, 0};
-      load3(X, T, g, xi);
-      bool singular = false, overrun = false;
-      walk_fp64(tb, s, sc, xi, g, prv[g], prv, m == 0 ? zero : sc.shift[m - 1], m == 0, acc, evals, tests,
-                singular, overrun);
-      if (singular) atomicOr(err, DERR_SINGULAR);
-      if (overrun) atomicOr(err, DERR_WALK);
-      const long long o = (long long)m * 3 * T + g;
-      partial[o] = acc[0];
-      partial[o + T] = acc[1];
-      partial[o + 2 * T] = acc[2];
-    }
+    double ub0[3], ubs[3];
+    fp64_target(sc, dyn[s], s, g, X, GI, GB, prv, U, T, tb, false, partial ? 3 : 0, ub0, ubs, evals, tests, err);
+    if (partial)
+      for (int c = 0; c < 3; ++c) partial[c * T + g] = ub0[c] + ubs[c];
     if (evals) atomicAdd(&dyn[s].tree_eval, evals);
     if (tests) atomicAdd(&dyn[s].tree_tests, tests);
   }
@@ -1577,8 +1563,7 @@ __global__ void k_closest_tree(const SysConst *__restrict__ scs, const SysDyn *_
 // walk's FP32 test defers to the FP64 one (the FP32 |r|^2 is within ~1e-6 of its value).
 constexpr float kTestBand = 1e-5f;
 
-__global__ void k_node_prep(TreeBuffers tb, int nsys, double theta0, int corr, float line_guard,
-                            const int *__restrict__ prv) {
+__global__ void k_node_prep(TreeBuffers tb, int nsys, double theta0, int corr, const int *__restrict__ prv) {
   const int n = tb.ctr[0];
   for (int id = nsys + blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const double4 A = tb.nA[id], B = tb.nB[id];
@@ -1593,8 +1578,8 @@ __global__ void k_node_prep(TreeBuffers tb, int nsys, double theta0, int corr, f
     wn.a = make_float4(hx, hy, hz, (float)(t1 * t1));
     const float q2 = qx * qx + qy * qy + qz * qz;
     wn.b = make_float4((float)(A.x - hx), (float)(A.y - hy), (float)(A.z - hz), q2);
-    wn.c = make_float4(qx, qy, qz, line_guard * q2);
-    wn.d = make_int4(I.x, I.y, tb.nSib[id], I.x == 1 ? prv[I.w] : I.w);
+    wn.c = make_float4(qx, qy, qz, 0.f);
+    wn.d = make_int4(I.x, I.y, tb.nKids[id], I.x == 1 ? prv[I.w] : I.w);
     tb.mx.W[id] = wn;
   }
 }
@@ -1609,283 +1594,482 @@ __global__ void k_leaf_links(TreeBuffers tb, int nsys, const int *__restrict__ p
   }
 }
 
-// Mixed tree walk: one lane per (target, image), a warp walking together.  A warp holds 32
-// targets that are close in space (consecutive in the Morton walk order) against one image
-// and traverses the union of their walks: a stack of (node, lane mask) entries, where an
-// entry stands for a node and its following siblings and the mask holds the lanes whose
-// walk reaches them.  The stack lives in registers, entry d in lane d % 32.  Each node's
-// 64-byte record is read once per warp (broadcast); each lane takes the reference's opening
-// decision for itself, so a lane accepts exactly the nodes its own walk (tree.f90:250-316)
-// accepts, in the same preorder.
+// Mixed tree walk: a block of W warps per group of 32 targets that are close in space
+// (consecutive in the walk order), lane k of every warp holding target k, for all images
+// at once.  An entry of the work list is (node, image, mask of the lanes whose walk reaches the
+// node); the block takes up to 32 W entries a round, one per lane, and
+//   1. each lane tests its entry's node against the box around the group's targets: most nodes
+//      are accepted by every target or opened by every target, which settles 32 entries in one
+//      pass over the lanes;
+//   2. the entries in between are tested target by target, the lanes taking the reference's
+//      opening decision each for its own target;
+//   3. accepted nodes go to the term list with their lanes, the children of opened ones back
+//      to the work list (a prefix sum over the block gives every entry its place, so that the
+//      order, and with it every rounding, is the same in every run);
+//   4. a full term list is summed: each warp takes 32 of its nodes, loads them (a lane a node)
+//      into shared memory, two nodes side by side, and every lane adds its target's terms, two
+//      in one packed instruction.
+// So a node's record is loaded once per group, by lanes in parallel, and neither the loop over
+// the nodes nor the tests diverge.  Which nodes a target accepts is the reference's choice
+// (tree.f90:250-316), node by node; only the order of the additions is not.
 //
-// The opening test compares |r|^2 with t1^2.  r is formed in FP32 from the high and low
-// parts of the centre and of the image-shifted target (|r_FP32 - r| <~ 2^-23 |r|), so
-// |r|^2 in FP32 is within 1e-6 of its value; outside a 1e-5 band around t1^2 the FP32
-// comparison gives the FP64 answer, inside it the FP64 test runs.  Far interactions in FP32;
-// accepted leaves within the near radius and ill-conditioned far terms in FP64.  Writes
-// the image's partial sum.
-constexpr int kWalkStack = 64;  // two register entries per lane; the build stops at depth 42
+// The opening test compares |r|^2 with t1^2.  r is formed in FP32 from the high and low parts
+// of the image-shifted centre and of the target (|r_FP32 - r| <~ 2^-23 |r|), so |r|^2 in FP32
+// is within 1e-6 of its value; outside a 1e-5 band around t1^2 the FP32 comparison gives the
+// FP64 answer, inside it the FP64 test runs.  The box's distances are widened by 1e-6 of
+// themselves and of the box, so that a verdict for the box holds for every target in it.
+// FP32 terms are summed over one term list (at most 16 to a partial sum) and promoted to FP64;
+// leaves within the near radius and ill-conditioned terms are evaluated in FP64.  Writes the
+// target's sum over all images.
+//
+// Bound: instruction issue, three quarters of it in the terms (61 issue slots a term of two
+// packed ones, of which the conditioning guards that the long summed circulations need take
+// about 20), with 58 % of the lanes in an average term's mask; a fifth of the nodes need the
+// target-by-target test.  100,000 points: 1.54 ms; 1M: 10.6 ms (2.27 and 14.1 ms for a warp
+// stepping through the union of its targets' walks node by node, 148 issue slots a node).
+// FP64 terms where they occur instead of from the queue: 1.59 ms at 100,000 points in place of
+// 1.54.
+constexpr int walk_cap(int W) { return W == 8 ? 4096 : W == 4 ? 2048 : 1024; }  // work-list entries
+// Entries kept free: taking one entry at a time (depth first), a list grows by at most this.
+constexpr int kWalkReserve = 8 * kMaxLevels;
 
-// Large systems (kSplit false, the GPU full of long walks): the FP64 accumulators live in
-// shared memory and 9 blocks fit on an SM; small ones (split central image, a short tail):
-// accumulators in registers, 8 blocks (both measured faster than the other choice).
-template <bool kSplit>
-__global__ void __launch_bounds__(128, kSplit ? 8 : 9) k_tree_walk_mixed(const SysConst *__restrict__ scs, SysDyn *dyn,
-                                                            const int4 *__restrict__ work,
-                                                            const double *__restrict__ X,
-                                                            const int *__restrict__ nxt, const int *__restrict__ prv,
-                                                            double *__restrict__ partial, long long T, TreeBuffers tb,
-                                                            double near_factor, Fp32Guards gd, int parts,
-                                                            unsigned *err) {
-  const int lane = threadIdx.x & 31;
-  const int4 w = work[blockIdx.x];  // system, image, first position, part of a split central image
+template <int W>
+struct WalkShared {
+  int node[walk_cap(W)];
+  unsigned mask[walk_cap(W)];
+  unsigned char image[walk_cap(W)];
+  // the term list: at most 32 W - 1 entries left over and 32 W of a round
+  int tnode[64 * W];
+  unsigned tmask[64 * W];
+  unsigned char timage[64 * W];
+  // per warp: its round's centres (hi, threshold; lo, lanes), later its 32 terms' records
+  union Warp {
+    float4 centre[32][2];
+    float pair[16 * 28];
+  } warp[W];
+  unsigned tlanes[W][32];  // per term: its lanes
+  int2 info[W][32];        // per term: node, image << 5
+  unsigned own[32];        // filter of the targets' own segments: bit (slot mod 1024)
+  int2 queue[W][96];       // per warp: FP64 terms (node, image << 5 | lane), at most 31 + 64
+  double result[W][3][32];
+  double target[3][32];
+  double shift[27][3];
+  unsigned open[27], undecided[W];
+  int wterms[W], wkids[W];
+  double red[3][W][32];
+};
+
+template <int W>
+__global__ void __launch_bounds__(32 * W, 24 / W) k_tree_walk_mixed(
+    const SysConst *__restrict__ scs, SysDyn *dyn, const int2 *__restrict__ work, const double *__restrict__ X,
+    const int *__restrict__ nxt, const int *__restrict__ prv, double *__restrict__ partial, long long T,
+    TreeBuffers tb, double near_factor, Fp32Guards gd, unsigned *err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WalkShared<W> &S = *reinterpret_cast<WalkShared<W> *>(smem_raw);
+  constexpr unsigned kAll = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int2 w = work[blockIdx.x];  // system, first position
   const SysConst &sc = scs[w.x];
-  const int m = w.y, part = w.w;
-  const int q = w.z + threadIdx.x - sc.base;  // position in the system's walk order
+  const int q = w.y + lane - sc.base;  // position in the system's walk order
   const int g = q >= 1 && q <= sc.cap ? tb.perm[sc.base + q] : sc.base;
   const int k = g - sc.base;
-  unsigned evals = 0, tests = 0, n64 = 0, nband = 0;
-  // A walk range's ends fall on warp boundaries (nv_set_walk_range): a warp walks all its
-  // targets or none, and the warp's visits (the union of its lanes' walks), which set where
-  // the FP32 partials are flushed, are the same as without a range.
+  // A walk range's ends fall on group boundaries (nv_set_walk_range): a group walks all its
+  // targets or none, so its rounds and partial sums are the same as without a range.
   const bool valid = !*err && k >= 1 && k <= dyn[w.x].pcount && nxt[g] != 0 && q >= sc.walk_lo && q < sc.walk_hi;
-  const unsigned live = __ballot_sync(0xffffffffu, valid);
-  float xh[3] = {0, 0, 0}, xl[3] = {0, 0, 0};  // target - shift, FP32 high and low parts
+  unsigned evals = 0, tests = 0, n64 = 0, nband = 0;
+  double xi[3] = {0, 0, 0};
   int pi_ = 0;
   if (valid) {
-    double xs[3];
-    load3(X, T, g, xs);
-    if (m > 0)
-      for (int c = 0; c < 3; ++c) xs[c] -= sc.shift[m - 1][c];
-    for (int c = 0; c < 3; ++c) {
-      xh[c] = (float)xs[c];
-      xl[c] = (float)(xs[c] - (double)xh[c]);
-    }
+    load3(X, T, g, xi);
     pi_ = prv[g];
+  }
+  const int n_img = 1 + sc.n_shift;
+  if (wid == 0) {
+    for (int c = 0; c < 3; ++c) S.target[c][lane] = xi[c];
+    S.own[lane] = 0;
+    __syncwarp();
+    if (valid) {
+      atomicOr(&S.own[(g >> 5) & 31], 1u << (g & 31));
+      atomicOr(&S.own[(pi_ >> 5) & 31], 1u << (pi_ & 31));
+    }
+  }
+  for (int i = tid; i < 3 * n_img; i += 32 * W) S.shift[i / 3][i % 3] = i < 3 ? 0.0 : sc.shift[i / 3 - 1][i % 3];
+  __syncthreads();
+  // the root's test in every image from the centre estimate: accepted (nothing to add), opened
+  // (the walk starts at its children) or undecided: the target is redone whole once the exact
+  // centre is known
+  {
+    unsigned undec = 0;
+    for (int m = wid; m < n_img; m += W) {
+      const int rd = valid ? root_decision(tb, sc, w.x, xi, S.shift[m]) : 1;
+      const unsigned open = __ballot_sync(kAll, rd == 0);
+      undec |= __ballot_sync(kAll, rd == 2);
+      if (lane == 0) S.open[m] = open;
+    }
+    if (lane == 0) S.undecided[wid] = undec;
+  }
+  __syncthreads();
+  unsigned undec = 0;
+#pragma unroll
+  for (int v = 0; v < W; ++v) undec |= S.undecided[v];
+  const unsigned live = __ballot_sync(kAll, valid) & ~undec;
+  const bool mine = (live >> lane) & 1u;
+  if (wid == 0) {
+    if (valid && !mine) defer_push(tb, g, err);
+    if (mine) tests += n_img;
+  }
+  const int first = tb.nI[w.x].y, n_kids = tb.nKids[w.x];
+  int top = 0, nterm = 0;  // entries of the work list, of the term list (block-uniform)
+  if (live) {  // the root's children in every image that some target opens
+    for (int m = 0; m < n_img; ++m) {
+      const unsigned open = S.open[m] & live;
+      if (!open) continue;
+      if (tid < n_kids) {
+        S.node[top + tid] = first + tid;
+        S.mask[top + tid] = open;
+        S.image[top + tid] = (unsigned char)m;
+      }
+      top += n_kids;
+    }
+  }
+  // the box around the live targets
+  float bh[3], bl[3], bw[3];  // centre high and low, half width
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    double lo = mine ? xi[c] : 1e300, hi = mine ? xi[c] : -1e300;
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(kAll, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(kAll, hi, o));
+    }
+    const double mid = 0.5 * (lo + hi);
+    bh[c] = (float)mid;
+    bl[c] = (float)(mid - (double)bh[c]);
+    bw[c] = (float)(0.5 * (hi - lo)) * 1.000002f;
+  }
+  LaneTarget t;
+  float xh[3], xl[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    xh[c] = (float)xi[c];
+    xl[c] = (float)(xi[c] - (double)xh[c]);
+    t.h[c] = pack2(-xh[c], -xh[c]);
+    t.l[c] = pack2(-xl[c], -xl[c]);
   }
   const float near2 = (float)(near_factor * sc.delta * near_factor * sc.delta);
   const double gq64 = sc.quant_circ / (4.0 * NV_PI);
-  const float gq = (float)gq64;
   const bool second = sc.tree_extra_correction && sc.tree_theta > 1.1547;
-  // FP32 partial over at most kFlush far interactions: a lane adds at most one term per
-  // node visit and the warp promotes every lane's partial to FP64 after kFlush visits
-  float fx = 0, fy = 0, fz = 0;
-  int since_flush = 0;  // warp-uniform
-  // FP64: near field plus the flushed FP32 partials (touched only at a flush or an FP64 term)
-  __shared__ double s_acc[kSplit ? 1 : 3][128];
-  double r_acc0 = 0., r_acc1 = 0., r_acc2 = 0.;
-  double &nx = kSplit ? r_acc0 : s_acc[0][threadIdx.x];
-  double &ny = kSplit ? r_acc1 : s_acc[kSplit ? 0 : 1][threadIdx.x];
-  double &nz = kSplit ? r_acc2 : s_acc[kSplit ? 0 : 2][threadIdx.x];
-  nx = ny = nz = 0.;
+  double nx = 0., ny = 0., nz = 0.;  // FP64 terms and the promoted FP32 sums
   bool singular = false;
   // r and |r|^2 in FP64 as the FP64 walk forms them: (centre + shift) - target
-  auto exact_r = [&](int cur, double r[3]) -> double {
+  auto exact_r = [&](int cur, int m, double r[3]) -> double {
     const double4 C = ldg4(&tb.mx.C[cur]);
-    double xi[3];
-    load3(X, T, g, xi);
-    const double s0 = m > 0 ? sc.shift[m - 1][0] : 0., s1 = m > 0 ? sc.shift[m - 1][1] : 0.,
-                 s2 = m > 0 ? sc.shift[m - 1][2] : 0.;
-    r[0] = e_sub(e_add(C.x, s0), xi[0]);
-    r[1] = e_sub(e_add(C.y, s1), xi[1]);
-    r[2] = e_sub(e_add(C.z, s2), xi[2]);
+    r[0] = e_sub(e_add(C.x, S.shift[m][0]), xi[0]);
+    r[1] = e_sub(e_add(C.y, S.shift[m][1]), xi[1]);
+    r[2] = e_sub(e_add(C.z, S.shift[m][2]), xi[2]);
     return e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
   };
-  // FP64 evaluation of an accepted node: the reference's singularity check and skip decision
-  // in its own arithmetic (tree.f90:289-303), the value from the cancellation-free form
-  auto exact_term = [&](int cur) {
-    double r[3];
-    const double d2 = exact_r(cur, r);
-    const double dist = e_sqrt(d2);
-    if (dist < NV_EPS) {
-      singular = true;
-      return;
+  // The terms that go to FP64 wait in a queue of the warp until there are 32, then a lane takes
+  // one each, whoever's target it is for, and the targets' lanes add the results in queue order.
+  int nq = 0;  // warp-uniform
+  auto flush64 = [&]() {
+    const int n = min(nq, 32);
+    __syncwarp();
+    double tm[3] = {0., 0., 0.};
+    int to = -1;
+    if (lane < n) {
+      const int2 item = S.queue[wid][lane];
+      to = item.y & 31;
+      const int m = item.y >> 5;
+      const double4 C = ldg4(&tb.mx.C[item.x]), B = ldg4(&tb.nB[item.x]);
+      const double r[3] = {e_sub(e_add(C.x, S.shift[m][0]), S.target[0][to]),
+                           e_sub(e_add(C.y, S.shift[m][1]), S.target[1][to]),
+                           e_sub(e_add(C.z, S.shift[m][2]), S.target[2][to])};
+      const double circ[3] = {B.x, B.y, B.z};
+      // the reference's singularity check and skip decision in its own arithmetic
+      // (tree.f90:289-303), the value from the cancellation-free form
+      const double d2 = e_add(e_add(e_sq(r[0]), e_sq(r[1])), e_sq(r[2]));
+      const double dist = e_sqrt(d2);
+      const double a = e_mul(dist, dist);
+      const double b = e_mul(2.0, dot3(r, circ));
+      const double c = dot3(circ, circ);
+      if (dist < NV_EPS) {
+        singular = true;
+        --evals;
+      } else if (e_sub(e_mul(e_mul(4.0, a), c), e_mul(b, b)) < NV_EPS) {
+        --evals;
+      } else {
+        term64_stable(r, circ, d2, gq64, tm);
+        ++n64;
+      }
     }
-    const double4 B = ldg4(&tb.nB[cur]);
-    const double circ[3] = {B.x, B.y, B.z};
-    const double a = e_mul(dist, dist);
-    const double b = e_mul(2.0, dot3(r, circ));
-    const double c = dot3(circ, circ);
-    const double D = e_sub(e_mul(e_mul(4.0, a), c), e_mul(b, b));
-    if (D < NV_EPS) return;
-    double tm[3];
-    term64_stable(r, circ, d2, gq64, tm);
-    nx += tm[0];
-    ny += tm[1];
-    nz += tm[2];
-    ++evals;
-    ++n64;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) S.result[wid][c][lane] = tm[c];
+    const int2 left = lane < nq - 32 ? S.queue[wid][32 + lane] : make_int2(0, 0);
+    const int2 left2 = lane < nq - 64 ? S.queue[wid][64 + lane] : make_int2(0, 0);
+    __syncwarp();
+    for (int i = 0; i < n; ++i) {
+      const int l = __shfl_sync(kAll, to, i);
+      if (l == lane) {
+        nx += S.result[wid][0][i];
+        ny += S.result[wid][1][i];
+        nz += S.result[wid][2][i];
+      }
+    }
+    if (lane < nq - 32) S.queue[wid][lane] = left;
+    if (lane < nq - 64) S.queue[wid][32 + lane] = left2;
+    nq -= n;
+    __syncwarp();
   };
-  // the root's test from the centre estimate: accepted (nothing to add), opened (the walk
-  // starts at its children) or deferred until the exact centre is known
-  int rd = 1;
-  if (valid) {
-    double xi[3];
-    const double zero[3] = {0, 0, 0};
-    load3(X, T, g, xi);
-    rd = root_decision(tb, sc, w.x, xi, m > 0 ? sc.shift[m - 1] : zero);
-    if (part == 0) {  // the parts of a split central image share one root test
-      if (rd == 2) defer_push(tb, g, m, err);
-      else ++tests;
+  // lanes of term (entry k of the warp's 32) into the queue
+  auto push64 = [&](bool bad, int k) {
+    const unsigned b = __ballot_sync(kAll, bad);
+    if (bad) {
+      const int2 inf = S.info[wid][k];
+      S.queue[wid][nq + __popc(b & ((1u << lane) - 1u))] = make_int2(inf.x, inf.y | lane);
     }
-  }
-  const unsigned open0 = __ballot_sync(0xffffffffu, valid && rd == 0);
-  const int first = tb.nI[w.x].y;
-  // The root's children are nodes first .. first+nc-1.  A part of a split central image
-  // walks children lo .. hi-1 of them (ids below lim); every other item walks them all.
-  int start = first, lim = INT_MAX;
-  if (kSplit && m == 0 && first != kEnd) {
-    int nc = 0;
-    for (int d = 0; d < 8; ++d) nc += tb.root_cnt[8 * w.x + d] != 0;
-    const int lo = part * 8 / parts, hi = min((part + 1) * 8 / parts, nc);
-    start = lo < nc ? first + lo : kEnd;
-    lim = first + hi;
-  }
-  (void)live;
-  // (cur, mask): the node the warp is at and the lanes whose walk reaches it, warp-uniform.
-  // The stack holds the pending next siblings of the nodes opened on the way down: entry d
-  // (node, mask) in lane d % 32, register pair 0 for d < 32, 1 above.
-  int sn0 = 0, sn1 = 0;
-  unsigned sm0 = 0, sm1 = 0;
-  int top = -1;
-  int cur = start;
-  unsigned mask = open0;
-  bool more = open0 && start != kEnd;
-  // (no visit budget here, unlike the FP64 walks: even a check per flush cost 3% of the
-  // walk; the warp visits each node of the tree the build makes at most once)
-  while (more) {
-    const WalkNode *wn = tb.mx.W + cur;
-    // the whole 64-byte record at once: one load latency per node instead of a chain
-    const int4 D = __ldg(&wn->d);
-    const float4 A = __ldg(&wn->a), B = __ldg(&wn->b), Q = __ldg(&wn->c);
-    // the next sibling, none past the last root child of this item's group (the root's
-    // children are the only nodes with ids in [first, lim))
-    const int sib = kSplit && D.z >= lim && cur >= first && cur < lim ? kEnd : D.z;
-    bool open = false;
-    if ((mask >> lane) & 1u) {  // (every node below a root has members)
-      ++tests;
-      const float rx = (A.x - xh[0]) + (B.x - xl[0]);
-      const float ry = (A.y - xh[1]) + (B.y - xl[1]);
-      const float rz = (A.z - xh[2]) + (B.z - xl[2]);
-      const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-      bool acc;
+    nq += __popc(b);
+  };
+  // a node's centre moved by the image's shift, FP32 high and low parts
+  auto shifted = [&](const float4 &hi, const float4 &lo, int m, float h[3], float l[3]) {
+    const float ch[3] = {hi.x, hi.y, hi.z}, cl[3] = {lo.x, lo.y, lo.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double v = (double)ch[c] + (double)cl[c] + S.shift[m][c];
+      h[c] = (float)v;
+      l[c] = (float)(v - (double)h[c]);
+    }
+  };
+  // The terms of list entries [t0, t1): 32 to a warp, a partial FP32 sum of at most 16 each.
+  const f32x2 kMinus = pack2(-1.f, -1.f), kAngle = pack2(gd.angle, gd.angle), kEndG = pack2(gd.end, gd.end);
+  auto sum_terms = [&](int t0, int t1) {
+    const int e = t0 + 32 * wid + lane;
+    const int n = min(32, t1 - (t0 + 32 * wid));
+    if (n <= 0) return;  // warp-uniform
+    float *pr = S.warp[wid].pair;
+    __syncwarp();
+    {
+      unsigned lanes = 0;
+      int id = 0, m = 0, leaf = -1;
+      float h[3] = {0, 0, 0}, l[3] = {0, 0, 0}, qx = 0, qy = 0, qz = 0, q2 = 0, near = 0;
+      if (lane < n) {
+        lanes = S.tmask[e];
+        id = S.tnode[e];
+        m = S.timage[e];
+        const WalkNode *wn = tb.mx.W + id;
+        const float4 A = __ldg(&wn->a), B = __ldg(&wn->b), Q = __ldg(&wn->c);
+        const int4 D = __ldg(&wn->d);
+        shifted(A, B, m, h, l);
+        qx = Q.x;
+        qy = Q.y;
+        qz = Q.z;
+        q2 = B.w;
+        if (D.x == 1) {
+          near = near2;  // near leaves in FP64
+          if (m == 0 && ((S.own[(D.w >> 5) & 31] >> (D.w & 31)) & 1u)) leaf = D.w;
+        }
+      }
+      // the targets' own segments are skipped in the central image: a leaf that the filter
+      // lets through is compared with every target's two
+      for (unsigned hit = __ballot_sync(kAll, leaf >= 0); hit; hit &= hit - 1) {
+        const int j = __ffs(hit) - 1, sl = __shfl_sync(kAll, leaf, j);
+        const unsigned own = __ballot_sync(kAll, sl == g || sl == pi_);
+        if (lane == j) {
+          evals -= __popc(lanes & own);
+          lanes &= ~own;
+        }
+      }
+      const float v[14] = {h[0], h[1], h[2], l[0], l[1], l[2], qx, qy, qz, -qx, -qy, near, gd.line * q2, gd.end * q2};
+      float *rec = pr + 28 * (lane >> 1) + (lane & 1);
+#pragma unroll
+      for (int c = 0; c < 14; ++c) rec[2 * c] = v[c];
+      S.tlanes[wid][lane] = lanes;
+      S.info[wid][lane] = make_int2(id, m << 5);
+    }
+    __syncwarp();
+    f32x2 ux = pack2(0.f, 0.f), uy = ux, uz = ux;
+    const int np = (n + 1) / 2;
+    for (int p = 0; p < np; ++p) {
+      const ulonglong2 *rec = reinterpret_cast<const ulonglong2 *>(pr + 28 * p);
+      const PairVec r = pair_vec(rec, t);
+      const ulonglong2 v3 = rec[3], v4 = rec[4], v5 = rec[5], v6 = rec[6];
+      const PairSeg d = {{v3.x}, {v3.y}, {v4.x}, {v4.y}, {v5.x}, {v5.y}};
+      const f32x2 near = {v5.y}, line = {v6.x}, end = {v6.y};
+      const uint2 lanes = *reinterpret_cast<const uint2 *>(&S.tlanes[wid][2 * p]);
+      const PairGeo geo = pair_geo(r, d);
+      const f32x2 cr2 = square2(geo.cx, geo.cy, geo.cz);
+      const f32x2 sum = add2(geo.pp, geo.re), dif = fma2(geo.re, kMinus, geo.pp);
+      // FP64 for a near leaf, a term the reference skips (4ac-b^2 = 4|r x circ|^2 < epsilon,
+      // tree.f90:303) and where FP32 would cancel digits: the target near the segment's line,
+      // near its far end, or under a wide angle (Fp32Guards)
+      const f32x2 wide = mul2(geo.pp, kAngle), ea = mul2(r.a, kEndG);
+      const f32x2 ln = mul2(line, pack2(fminf(lo2(r.a), lo2(geo.ee)), fminf(hi2(r.a), hi2(geo.ee))));
+      constexpr float kSkip = 0.25f * (float)NV_EPS;
+      const bool in0 = (lanes.x >> lane) & 1u, in1 = (lanes.y >> lane) & 1u;
+      const bool bad0 = lo2(r.a) < lo2(near) || lo2(cr2) < lo2(ln) || lo2(cr2) < kSkip || lo2(geo.ee) < lo2(ea) ||
+                        lo2(geo.ee) < lo2(end) || lo2(sum) < lo2(wide);
+      const bool bad1 = hi2(r.a) < hi2(near) || hi2(cr2) < hi2(ln) || hi2(cr2) < kSkip || hi2(geo.ee) < hi2(ea) ||
+                        hi2(geo.ee) < hi2(end) || hi2(sum) < hi2(wide);
+      // pp + r.e = |r x circ|^2 / (pp - r.e) when r.e < 0 (no cancellation either way)
+      const bool ob0 = lo2(geo.re) < 0.f, ob1 = hi2(geo.re) < 0.f;
+      const f32x2 topf = mul2(geo.num, pack2(ob0 ? lo2(dif) : 1.f, ob1 ? hi2(dif) : 1.f));
+      const f32x2 f = mul2(topf, pack2(rcp_fast(ob0 ? lo2(cr2) : lo2(sum)), rcp_fast(ob1 ? hi2(cr2) : hi2(sum))));
+      const f32x2 fk = pack2(in0 && !bad0 ? lo2(f) : 0.f, in1 && !bad1 ? hi2(f) : 0.f);
+      ux = fma2(fk, geo.cx, ux);
+      uy = fma2(fk, geo.cy, uy);
+      uz = fma2(fk, geo.cz, uz);
+      if (__any_sync(kAll, (in0 && bad0) || (in1 && bad1))) {
+        push64(in0 && bad0, 2 * p);
+        push64(in1 && bad1, 2 * p + 1);
+        while (nq >= 32) flush64();
+      }
+    }
+    nx += gq64 * ((double)lo2(ux) + (double)hi2(ux));
+    ny += gq64 * ((double)lo2(uy) + (double)hi2(uy));
+    nz += gq64 * ((double)lo2(uz) + (double)hi2(uz));
+    __syncwarp();
+  };
+  __syncthreads();
+  // (no visit budget here, unlike the FP64 walks: an image's entries are distinct nodes, and the
+  // build makes a tree)
+  while (top > 0) {
+    const int n = min(min(top, 32 * W), max(1, (walk_cap(W) - kWalkReserve - top) / 8));
+    const int base = top - n;
+    const int e = base + 32 * wid + lane;
+    const bool have = 32 * wid + lane < n;
+    int id = 0, m = 0, kids = 0, first_kid = 0;
+    unsigned mask = 0, acc_lanes = 0, open_lanes = 0;
+    bool split = false;
+    if (have) {
+      id = S.node[e];
+      mask = S.mask[e];
+      m = S.image[e];
+      const WalkNode *wn = tb.mx.W + id;
+      const int4 D = __ldg(&wn->d);
+      const float4 A = __ldg(&wn->a), B = __ldg(&wn->b);
+      kids = D.z;
+      first_kid = D.y;
+      tests += __popc(mask);  // (every node below a root has members)
       if (D.x == 1) {
-        acc = true;
-      } else if (!second && d2 > A.w * (1.f + kTestBand)) {
-        acc = true;
-      } else if (!second && d2 < A.w * (1.f - kTestBand)) {
-        acc = false;
-      } else {  // near the threshold (or the second criterion): the FP64 test
+        acc_lanes = mask;
+      } else {
+        float h[3], l[3];
+        shifted(A, B, m, h, l);
+        float dmin2 = 0.f, dmax2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float d = fabsf((h[c] - bh[c]) + (l[c] - bl[c]));
+          const float lo = fmaxf(fmaf(d, 0.999999f, -bw[c]), 0.f), hi = fmaf(d, 1.000001f, bw[c]);
+          dmin2 = fmaf(lo, lo, dmin2);
+          dmax2 = fmaf(hi, hi, dmax2);
+        }
+        if (!second && dmin2 > A.w * (1.f + kTestBand)) {
+          acc_lanes = mask;
+        } else if (!second && dmax2 < A.w * (1.f - kTestBand)) {
+          open_lanes = mask;
+        } else {
+          split = true;
+          S.warp[wid].centre[lane][0] = make_float4(h[0], h[1], h[2], A.w);
+          S.warp[wid].centre[lane][1] = make_float4(l[0], l[1], l[2], __uint_as_float(mask));
+        }
+      }
+    }
+    const unsigned todo = __ballot_sync(kAll, split);
+    __syncwarp();
+    for (unsigned rest = todo; rest; rest &= rest - 1) {
+      const int j = __ffs(rest) - 1;
+      const float4 H = S.warp[wid].centre[j][0], L = S.warp[wid].centre[j][1];
+      const float rx = (H.x - xh[0]) + (L.x - xl[0]);
+      const float ry = (H.y - xh[1]) + (L.y - xl[1]);
+      const float rz = (H.z - xh[2]) + (L.z - xl[2]);
+      const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+      const unsigned lanes = __float_as_uint(L.w);
+      bool acc = d2 > H.w * (1.f + kTestBand);
+      // near the threshold (or the second criterion): the FP64 test
+      if (((lanes >> lane) & 1u) && (second || (!acc && !(d2 < H.w * (1.f - kTestBand))))) {
         ++nband;
+        const int cur = S.node[base + 32 * wid + j];
         double r[3];
-        const double d2e = exact_r(cur, r);
+        const double d2e = exact_r(cur, S.image[base + 32 * wid + j], r);
         acc = d2e > tb.mx.C[cur].w;
         if (!acc && second) {
           const double2 G = tb.mx.G[cur];
           acc = d2e <= G.x && d2e > G.y;
         }
       }
-      if (!acc) {
-        open = true;
-      } else {
-        bool done = false;
-        if (D.x == 1) {
-          if (m == 0)  // the target's own segments are skipped in the central image
-            done = D.w == g || D.w == pi_;  // D.w: prv of the leaf's member
-          if (!done && d2 < near2) {
-            exact_term(cur);  // near leaf: the reference arithmetic in FP64
-            done = true;
-          }
-        }
-        if (!done) {
-          // the reference skips 4ac-b^2 < epsilon (tree.f90:303); 4ac-b^2 = 4|r x circ|^2
-          const float cx = fmaf(ry, Q.z, -rz * Q.y), cy = fmaf(rz, Q.x, -rx * Q.z), cz = fmaf(rx, Q.y, -ry * Q.x);
-          const float cr2 = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
-          if (!(4.f * cr2 < (float)NV_EPS)) {
-            const float ex = rx + Q.x, ey = ry + Q.y, ez = rz + Q.z;
-            const float ee = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-            const float re = fmaf(rx, ex, fmaf(ry, ey, rz * ez));
-            // ia = 1/|r|, ib = 1/|r + circ|; pp = |r||r + circ|
-            const float ia = rsqrtf(d2), ib = rsqrtf(ee);
-            const float pp = (d2 * ia) * (ee * ib);
-            if (cr2 < Q.w * fminf(d2, ee) || ee < gd.end * fmaxf(d2, B.w) || pp + re < gd.angle * pp) {
-              // the target lies near the segment's line or near its far end (or the optional
-              // angle guard): FP32 would cancel digits there
-              exact_term(cur);
-            } else {
-              // (|r| + |e|) / (pp (pp + r.e)) = (ia + ib) / (pp + r.e), e = r + circ, with
-              // pp + r.e = |r x circ|^2 / (pp - r.e) when r.e < 0 (no cancellation either way)
-              const bool obtuse = re < 0.f;
-              const float num = gq * (ia + ib) * (obtuse ? pp - re : 1.f);
-              const float f = __fdividef(num, obtuse ? cr2 : pp + re);  // MUFU reciprocal
-              fx = fmaf(f, cx, fx);
-              fy = fmaf(f, cy, fy);
-              fz = fmaf(f, cz, fz);
-              ++evals;
-            }
-          }
-        }
+      const unsigned al = __ballot_sync(kAll, acc) & lanes;
+      if (lane == j) {
+        acc_lanes = al;
+        open_lanes = lanes & ~al;
       }
     }
-    const unsigned omask = __ballot_sync(0xffffffffu, open);
-    if (omask && D.y != kEnd) {  // the lanes that open cur walk its children first
-      if (sib != kEnd) {         // and come back to cur's next sibling afterwards
-        ++top;
-        if (top >= kWalkStack) {  // deeper than any tree the build makes; guard only
-          if (lane == 0) atomicOr(err, DERR_TREE_DEPTH);
-          break;
-        }
-        if (lane == (top & 31)) {
-          if (top >= 32) {
-            sn1 = sib;
-            sm1 = mask;
-          } else {
-            sn0 = sib;
-            sm0 = mask;
-          }
-        }
-      }
-      cur = D.y;
-      mask = omask;
-    } else if (sib != kEnd) {
-      cur = sib;
-    } else if (top >= 0) {
-      const int src = top & 31;
-      const bool hi = top >= 32;
-      cur = __shfl_sync(0xffffffffu, hi ? sn1 : sn0, src);
-      mask = __shfl_sync(0xffffffffu, hi ? sm1 : sm0, src);
-      --top;
-    } else {
-      more = false;
+    // places: accepted nodes behind the term list, opened nodes' children on the work list
+    if (!open_lanes) kids = 0;
+    evals += __popc(acc_lanes);
+    const unsigned accb = __ballot_sync(kAll, acc_lanes != 0);
+    int scan = kids;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(kAll, scan, o);
+      if (lane >= o) scan += v;
     }
-    if (++since_flush == kFlush) {  // at most kFlush FP32 terms per partial
-      nx += (double)fx;
-      ny += (double)fy;
-      nz += (double)fz;
-      fx = fy = fz = 0.f;
-      since_flush = 0;
+    if (lane == 31) {
+      S.wkids[wid] = scan;
+      S.wterms[wid] = __popc(accb);
+    }
+    __syncthreads();
+    int koff = base + scan - kids, toff = nterm + __popc(accb & ((1u << lane) - 1u)), ktot = 0, ttot = 0;
+#pragma unroll
+    for (int v = 0; v < W; ++v) {
+      if (v < wid) {
+        koff += S.wkids[v];
+        toff += S.wterms[v];
+      }
+      ktot += S.wkids[v];
+      ttot += S.wterms[v];
+    }
+    if (acc_lanes) {
+      S.tnode[toff] = id;
+      S.tmask[toff] = acc_lanes;
+      S.timage[toff] = (unsigned char)m;
+    }
+    for (int c = 0; c < kids; ++c) {
+      S.node[koff + c] = first_kid + c;
+      S.mask[koff + c] = open_lanes;
+      S.image[koff + c] = (unsigned char)m;
+    }
+    top = base + ktot;
+    nterm += ttot;
+    __syncthreads();
+    if (nterm >= 32 * W) {
+      nterm -= 32 * W;
+      sum_terms(nterm, nterm + 32 * W);
+      // (the next round's barrier comes before its writes to the term list)
     }
   }
+  sum_terms(0, nterm);
+  if (nq) flush64();
+  S.red[0][wid][lane] = nx;
+  S.red[1][wid][lane] = ny;
+  S.red[2][wid][lane] = nz;
   if (singular) atomicOr(err, DERR_SINGULAR);
-  if (valid) {
-    const int slot = m == 0 && part > 0 ? 26 + part : m;  // extra parts after the 27 images
-    const long long o = (long long)slot * 3 * T + g;
-    partial[o] = (double)fx + nx;
-    partial[o + T] = (double)fy + ny;
-    partial[o + 2 * T] = (double)fz + nz;
+  __syncthreads();
+  for (int c = wid; c < 3; c += W) {
+    double v = 0.;
+#pragma unroll
+    for (int u = 0; u < W; ++u) v += S.red[c][u][lane];
+    if (mine) partial[c * T + g] = v;
   }
-  unsigned long long tot = evals, tt = tests, t64 = n64, tb_ = nband;
-  for (int o = 16; o > 0; o >>= 1) {
-    tot += __shfl_down_sync(0xffffffffu, tot, o);
-    tt += __shfl_down_sync(0xffffffffu, tt, o);
-    t64 += __shfl_down_sync(0xffffffffu, t64, o);
-    tb_ += __shfl_down_sync(0xffffffffu, tb_, o);
+  int v[4] = {(int)evals, (int)tests, (int)n64, (int)nband};  // (a lane's evals can be below zero)
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(kAll, v[c], o);
+  if (lane == 0) {
+    if (v[0]) atomicAdd(&dyn[w.x].tree_eval, (unsigned long long)(long long)v[0]);
+    if (v[1]) atomicAdd(&dyn[w.x].tree_tests, (unsigned long long)(long long)v[1]);
+    if (v[2]) atomicAdd((unsigned long long *)&dyn[w.x].diag[8], (unsigned long long)(long long)v[2]);
+    if (v[3]) atomicAdd((unsigned long long *)&dyn[w.x].diag[9], (unsigned long long)(long long)v[3]);
+    if (v[0] != v[2]) atomicAdd((unsigned long long *)&dyn[w.x].diag[10], (unsigned long long)(long long)(v[0] - v[2]));
   }
-  if (lane == 0 && tot) atomicAdd(&dyn[w.x].tree_eval, tot);
-  if (lane == 0 && tt) atomicAdd(&dyn[w.x].tree_tests, tt);
-  if (lane == 0 && t64) atomicAdd((unsigned long long *)&dyn[w.x].diag[8], t64);
-  if (lane == 0 && tb_) atomicAdd((unsigned long long *)&dyn[w.x].diag[9], tb_);
-  if (lane == 0 && tot > t64) atomicAdd((unsigned long long *)&dyn[w.x].diag[10], tot - t64);
 }
 
 int n_sms() {
@@ -1919,7 +2103,7 @@ void tree_alloc(nv_handle *h) {
   cudaMalloc(&tb->nI, (size_t)tb->max_nodes * sizeof(int4));
   cudaMalloc(&tb->nR, (size_t)tb->max_nodes * sizeof(int2));
   cudaMalloc(&tb->nDepth, (size_t)tb->max_nodes * sizeof(int));
-  cudaMalloc(&tb->nSib, (size_t)tb->max_nodes * sizeof(int));
+  cudaMalloc(&tb->nKids, (size_t)tb->max_nodes * sizeof(int));
   cudaMalloc(&tb->nLeaf, (size_t)tb->max_nodes * sizeof(int));
   cudaMalloc(&tb->members, (size_t)tb->max_members * sizeof(int));
   // each level holds at most T / (kBlockSumNode + 1) nodes above the block threshold
@@ -1942,7 +2126,7 @@ void tree_alloc(nv_handle *h) {
   }
   tb->root_parts = std::max(1, std::min(64, 4096 / h->nsys));
   cudaMalloc(&tb->root_part, (size_t)h->nsys * tb->root_parts * 6 * sizeof(double));
-  cudaMalloc(&tb->defer, (size_t)kDeferCap * sizeof(int2));
+  cudaMalloc(&tb->defer, (size_t)kDeferCap * sizeof(int));
   cudaMalloc(&tb->defer_n, sizeof(int));
   cudaMemset(tb->defer_n, 0, sizeof(int));
   cudaFuncSetAttribute(k_root_sums, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSumSmem);
@@ -1983,7 +2167,7 @@ void tree_alloc(nv_handle *h) {
 void tree_free(nv_handle *h) {
   TreeBuffers *tb = h->tree;
   if (!tb) return;
-  void *ptrs[] = {tb->nA, tb->nB, tb->nP, tb->nI, tb->nR, tb->nDepth, tb->nLeaf, tb->nSib, tb->members, tb->bigl, tb->root_apx, tb->root_part, tb->defer, tb->defer_n,
+  void *ptrs[] = {tb->nA, tb->nB, tb->nP, tb->nI, tb->nR, tb->nDepth, tb->nLeaf, tb->nKids, tb->members, tb->bigl, tb->root_apx, tb->root_part, tb->defer, tb->defer_n,
                   tb->rkey[0], tb->rkey[1], tb->rval[0], tb->rval[1], tb->root_cnt, tb->root_mb, tb->rsort_tmp, tb->ctr,
                   tb->flag, tb->pos, tb->cub_tmp, tb->mx.C, tb->mx.W, tb->mx.G, tb->okey[0], tb->okey[1],
                   tb->oval[0], tb->oval[1], tb->iperm, tb->sort_tmp, tb->split_blk[0], tb->split_blk[1],
@@ -2049,7 +2233,7 @@ void launch_tree_build(nv_handle *h) {
     // theta0 and the correction flag are per system; a handle's systems share them when
     // any of them walks the tree (checked at creation)
     k_node_prep<<<sms * 4, 256, 0, h->stream>>>(*tb, h->nsys, h->sc[h->tree_sys0].tree_theta,
-                                                h->sc[h->tree_sys0].tree_extra_correction, h->guards.line, h->prv);
+                                                h->sc[h->tree_sys0].tree_extra_correction, h->prv);
     tb->prep_epoch = h->links_epoch;
   }
   tb->built = true;
@@ -2083,17 +2267,32 @@ void launch_tree_walk(nv_handle *h) {
       h->d_sc, h->d_dyn, h->d_work_tree, h->x, h->gi, h->gb, h->nxt, h->prv, h->u, h->T, *tb, split, h->d_err);
 }
 
+namespace {
+template <int W>
+void launch_walk(nv_handle *h) {
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      k_tree_walk_mixed<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared<W>));
+  (void)attr;
+  k_tree_walk_mixed<W><<<h->n_work_grp, 32 * W, sizeof(WalkShared<W>), h->stream>>>(
+      h->d_sc, h->d_dyn, h->d_work_grp, h->x, h->nxt, h->prv, h->partial, h->T, *h->tree, h->near_factor, h->guards,
+      h->d_err);
+}
+}  // namespace
+
 void launch_tree_walk_mixed(nv_handle *h) {
   TreeBuffers *tb = h->tree;
-  if (!tb || h->n_work_timg == 0) return;
+  if (!tb || h->n_work_grp == 0) return;
   if (tb->prep_epoch != h->links_epoch) {  // relinked since the build
     k_leaf_links<<<n_sms() * 4, 256, 0, h->stream>>>(*tb, h->nsys, h->prv);
     tb->prep_epoch = h->links_epoch;
   }
   cudaMemsetAsync(tb->defer_n, 0, sizeof(int), h->stream);
-  auto walk = h->walk_parts_used > 1 ? k_tree_walk_mixed<true> : k_tree_walk_mixed<false>;
-  walk<<<h->n_work_timg, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->d_work_timg, h->x, h->nxt, h->prv, h->partial,
-                                              h->T, *tb, h->near_factor, h->guards, h->walk_parts_used, h->d_err);
+  switch (h->walk_parts_used) {
+    case 1: launch_walk<1>(h); break;
+    case 2: launch_walk<2>(h); break;
+    case 4: launch_walk<4>(h); break;
+    default: launch_walk<8>(h); break;
+  }
 }
 
 void launch_closest_tree(nv_handle *h) {
