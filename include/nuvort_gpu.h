@@ -287,7 +287,7 @@ int nv_event_margins_get(nv_handle *h, int32_t sys, double *out);
  * state): nv_step_velocity runs a step up to and including the velocity pass,
  * nv_step_finish the rest (AB3 update, topology, wrap, clock), the two together exactly
  * nv_step(1).  With nv_set_walk_range a tree-walk system's velocity pass computes only the
- * targets at walk positions lo <= q < hi (the walk order: the live points in Morton order at
+ * targets at walk positions lo <= q < hi (the walk order: the live points along a Hilbert curve at
  * positions 1 .. live, then the empty slots).  The ends fall on warp boundaries: lo - 1 a
  * multiple of 32, and hi - 1 one too or hi = cap + 1 (the mixed walk's 32 targets of a group
  * share the order of their terms, which a group cut in two would change); other

@@ -78,7 +78,7 @@ struct SysConst {
   int mirror[26][3];
   int solid[3];
   // the tree walks compute targets at walk positions walk_lo <= q < walk_hi only (the walk
-  // order: the system's dummy slot, its live points in Morton order, its empty slots); all
+  // order: the system's dummy slot, its live points along a Hilbert curve, its empty slots); all
   // by default, a range when one tangle's velocity is split over several GPUs
   int walk_lo, walk_hi;
 };

@@ -73,7 +73,7 @@ struct TreeBuffers {
   int *flag = nullptr, *pos = nullptr;
   void *cub_tmp = nullptr;
   size_t cub_bytes = 0;
-  // walk order: each system's slots sorted by Morton code of the position (live slots first)
+  // walk order: each system's slots sorted along a Hilbert curve (live slots first)
   unsigned long long *okey[2] = {nullptr, nullptr};
   int *oval[2] = {nullptr, nullptr};
   int *perm = nullptr;  // = oval[1]: position base+q of system s -> slot
@@ -143,9 +143,12 @@ __global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
   dyn[s].diag[8] = dyn[s].diag[9] = dyn[s].diag[10] = 0;
 }
 
-// Sort keys of the walk order: (system, class, Morton code of the position on a 1024^3 grid
-// of the box); class 0 is the dummy slot, 1 live slots, 2 the rest.  The order only decides
-// which lanes walk together; every target's result is independent of it.
+// Sort keys of the walk order: (system, class, place of the position on a Hilbert curve through a
+// 1024^3 grid of the box); class 0 is the dummy slot, 1 live slots, 2 the rest.  The order only
+// decides which lanes walk together; every target's accepted nodes are independent of it.
+// Neighbours on the Hilbert curve stay closer together than on the Morton curve (no jumps):
+// the mixed walk of 100,000 points visits 5 % fewer nodes and tests 23 % fewer target by target
+// (1.54 -> 1.41 ms), the plain walk of 32,768 points takes 2.49 instead of 3.13 ms.
 __device__ __forceinline__ unsigned spread3(unsigned v) {
   v &= 0x3ffu;
   v = (v | (v << 16)) & 0x030000ffu;
@@ -153,6 +156,32 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {
   v = (v | (v << 4)) & 0x030c30c3u;
   v = (v | (v << 2)) & 0x09249249u;
   return v;
+}
+// Grid coordinates (10 bits) to the transposed Hilbert index (J. Skilling, AIP Conf. Proc. 707,
+// 381, 2004): interleaving the three words' bits, q[0] first, gives the place on the curve.
+__device__ __forceinline__ void hilbert3(unsigned q[3]) {
+#pragma unroll
+  for (unsigned b = 512; b > 1; b >>= 1) {
+    const unsigned low = b - 1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const unsigned t = (q[0] ^ q[i]) & low;
+      if (q[i] & b) {
+        q[0] ^= low;
+      } else {
+        q[0] ^= t;
+        q[i] ^= t;
+      }
+    }
+  }
+  q[1] ^= q[0];
+  q[2] ^= q[1];
+  unsigned t = 0;
+#pragma unroll
+  for (unsigned b = 512; b > 1; b >>= 1)
+    if (q[2] & b) t ^= b - 1;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) q[i] ^= t;
 }
 __global__ void k_order_keys(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
                              const int *__restrict__ sys_of, const double *__restrict__ X,
@@ -171,7 +200,8 @@ __global__ void k_order_keys(const SysConst *__restrict__ scs, const SysDyn *__r
       const double f = (X[c * T + g] / sc.bsize + 0.5) * 1024.0;
       q[c] = f <= 0. ? 0u : f >= 1023. ? 1023u : (unsigned)f;
     }
-    inner = (1ull << 32) | (spread3(q[0]) | (spread3(q[1]) << 1) | (spread3(q[2]) << 2));
+    hilbert3(q);
+    inner = (1ull << 32) | (spread3(q[2]) | (spread3(q[1]) << 1) | (spread3(q[0]) << 2));
   } else {
     inner = (2ull << 32) | (unsigned)k;
   }
@@ -1625,10 +1655,10 @@ __global__ void k_leaf_links(TreeBuffers tb, int nsys, const int *__restrict__ p
 // Bound: instruction issue, three quarters of it in the terms (61 issue slots a term of two
 // packed ones, of which the conditioning guards that the long summed circulations need take
 // about 20), with 58 % of the lanes in an average term's mask; a fifth of the nodes need the
-// target-by-target test.  100,000 points: 1.54 ms; 1M: 10.6 ms (2.27 and 14.1 ms for a warp
+// target-by-target test.  100,000 points: 1.41 ms; 1M: 9.8 ms (2.27 and 14.1 ms for a warp
 // stepping through the union of its targets' walks node by node, 148 issue slots a node).
 // FP64 terms where they occur instead of from the queue: 1.59 ms at 100,000 points in place of
-// 1.54.
+// 1.54 (both on the Morton order).
 constexpr int walk_cap(int W) { return W == 8 ? 4096 : W == 4 ? 2048 : 1024; }  // work-list entries
 // Entries kept free: taking one entry at a time (depth first), a list grows by at most this.
 constexpr int kWalkReserve = 8 * kMaxLevels;
