@@ -85,7 +85,7 @@ __device__ __forceinline__ void term_value(const double r[3], const double d[3],
 
 // bs_term_exact out of line: for the rare term outside the ranges above, kept apart so that it
 // costs the loops neither registers nor instruction cache.
-__device__ __noinline__ double3 bs_term_rare(double r0, double r1, double r2, double d0, double d1, double d2,
+[[maybe_unused]] static __device__ __noinline__ double3 bs_term_rare(double r0, double r1, double r2, double d0, double d1, double d2,
                                              double a, double c, double qc, double two_pi) {
   const double r[3] = {r0, r1, r2}, d[3] = {d0, d1, d2};
   double out[3];

@@ -20,6 +20,7 @@
 // :206-244) in the same order, so the accumulated velocity is the reference's bit for bit.
 #include <cub/cub.cuh>
 
+#include "fp64.cuh"
 #include "handle.cuh"
 #include "mixed.cuh"
 
@@ -1106,67 +1107,130 @@ __device__ __forceinline__ void defer_push(const TreeBuffers &tb, int g, unsigne
   else atomicOr(err, DERR_QUEUE);
 }
 
+// The opening test of a node (tree.f90:264-278) and the term of an accepted one (:289-308) in
+// the reference's own operations, for the rare node whose squared distance lies within 1e-12 of
+// the threshold's square, or whose operands lie outside the range of fp64.cuh's seeds.
+__device__ __noinline__ bool accept_exact(double d2, double w, double geo, double theta0, bool corr) {
+  const double dist = e_sqrt(d2);
+  const double dg = corr ? e_sub(dist, geo) : dist;
+  return (dg > 0. ? e_div(w, dg) : e_div(w, dist)) < theta0;
+}
+__device__ __noinline__ double3 node_term_exact(double v0, double v1, double v2, double c0, double c1, double c2,
+                                                double dist, double qc, double two_pi) {
+  const double vect[3] = {v0, v1, v2}, circ[3] = {c0, c1, c2};
+  const double a = e_mul(dist, dist), b = e_mul(2.0, dot3(vect, circ)), c = dot3(circ, circ);
+  const double D = term_d(a, b, c);
+  double cr[3];
+  cross3(vect, circ, cr);
+  const double den = e_mul(two_pi, D);
+  const double fac = e_sub(e_div(e_add(e_mul(2.0, c), b), e_sqrt(e_add(e_add(a, b), c))), e_div(b, e_sqrt(a)));
+  return make_double3(e_mul(e_div(e_mul(cr[0], qc), den), fac), e_mul(e_div(e_mul(cr[1], qc), den), fac),
+                      e_mul(e_div(e_mul(cr[2], qc), den), fac));
+}
+
 // tree_walk (tree.f90:250-316) for one image; accumulates into acc in preorder.
 // `start` is the root, or the root's first child when the root is already known to be
 // opened (its test then counted by the caller).
+//
+// Six of seven nodes visited are accepted, so the walk is a chain of loads, one distance and a
+// term: the record of the node after this one's subtree is requested before this node is
+// tested, and the test compares squares (no root, no quotient for an opened node; a band of
+// 1e-12, far above the rounding of either form, goes to the reference's own test).  The
+// distance's root serves the term too: sqrt(a) with a = dist*dist rounded is dist itself.
+// 100,000 points: 4.40 ms, 32,768: 1.52 ms (6.95 and 2.48 ms with the IEEE operations one by one
+// and no request ahead).  A lane per (target, sum) in blocks of their own, so that no sum waits
+// for the other: 4.87 and 1.82 ms (the two sums of a block share their nodes in L1).
 __device__ __forceinline__ void walk_fp64(const TreeBuffers &tb, int start, const SysConst &sc, const double xi[3],
                                           int gi_, int pi_, const int *__restrict__ prv, const double s[3], bool unshifted,
                                           double acc[3], unsigned long long &evals, unsigned long long &tests,
                                           bool &singular, bool &overrun) {
-  const double qc = sc.quant_circ, two_pi = sc.two_pi, theta0 = sc.tree_theta;
+  if (start == kEnd) return;
+  const double qc = sc.quant_circ, two_pi = sc.two_pi, theta0 = sc.tree_theta, inv_theta = 1.0 / sc.tree_theta;
   const bool corr = sc.tree_extra_correction;
+  // (theta above 2/sqrt(3) with the correction: a node closer than its centre's offset can be
+  // accepted, which no single threshold tells)
+  const bool square = !(corr && theta0 > 1.1547);
   int node = start;
   int left = tb.ctr[0];  // a walk of a well-formed tree visits each node at most once
-  while (node != kEnd) {
+  unsigned ev = 0, te = 0;
+  double4 A = ldg4(&tb.nA[node]), B = ldg4(&tb.nB[node]);
+  int4 I = __ldg(&tb.nI[node]);
+  for (;;) {
     if (--left < 0) {
       overrun = true;
       break;
     }
-    const double4 A = ldg4(&tb.nA[node]);
-    const int4 I = __ldg(&tb.nI[node]);
-    if (I.x == 0) {
-      node = I.z;
-      continue;
+    const int nz = I.z;
+    double4 An = make_double4(0, 0, 0, 0), Bn = An;
+    int4 In = make_int4(0, kEnd, kEnd, 0);
+    if (nz != kEnd) {
+      An = ldg4(&tb.nA[nz]);
+      Bn = ldg4(&tb.nB[nz]);
+      In = __ldg(&tb.nI[nz]);
     }
-    ++tests;
-    const double cs[3] = {e_add(A.x, s[0]), e_add(A.y, s[1]), e_add(A.z, s[2])};
-    const double dist = e_sqrt(e_add(e_add(e_sq(e_sub(xi[0], cs[0])), e_sq(e_sub(xi[1], cs[1]))), e_sq(e_sub(xi[2], cs[2]))));
-    const double4 B = ldg4(&tb.nB[node]);
-    double theta;
-    if (corr) {
-      const double dg = e_sub(dist, B.w);
-      theta = dg > 0. ? e_div(A.w, dg) : e_div(A.w, dist);
-    } else {
-      theta = e_div(A.w, dist);
-    }
-    if (I.x == 1 || theta < theta0) {
-      node = I.z;
-      if (I.x == 1) {
-        const int j = __ldg(prv + I.w);
-        if (unshifted && (j == gi_ || j == pi_)) continue;
-        if (dist < NV_EPS) {
-          singular = true;
-          continue;
+    int next = nz;
+    if (I.x != 0) {
+      ++te;
+      const double vect[3] = {e_sub(e_add(A.x, s[0]), xi[0]), e_sub(e_add(A.y, s[1]), xi[1]),
+                              e_sub(e_add(A.z, s[2]), xi[2])};
+      const double d2 = e_add(e_add(e_sq(vect[0]), e_sq(vect[1])), e_sq(vect[2]));
+      bool take = I.x == 1;
+      if (!take) {
+        const double t1 = corr ? fma(A.w, inv_theta, B.w) : A.w * inv_theta;
+        const double gap = fma(-t1, t1, d2);
+        take = gap > 0.;
+        if (!(fabs(gap) > 1e-12 * d2) || !square) take = accept_exact(d2, A.w, B.w, theta0, corr);
+      }
+      if (!take) {
+        if (I.y != kEnd) next = I.y;
+      } else {
+        bool use = true;
+        if (unshifted && I.x == 1) {  // the target's own segments are skipped
+          const int j = __ldg(prv + I.w);
+          use = !(j == gi_ || j == pi_);
+        }
+        if (use) {
+          const double circ[3] = {B.x, B.y, B.z};
+          const double b = e_mul(2.0, dot3(vect, circ));
+          const double c = dot3(circ, circ);
+          double ya;
+          double dist = near_sqrt(d2, ya);
+          const bool far = mid_range<true>(d2);
+          if (!far) dist = e_sqrt(d2);
+          const double a = e_mul(dist, dist);
+          const double D = term_d(a, b, c);
+          const double abc = e_add(e_add(a, b), c);
+          if (I.x == 1 && dist < NV_EPS) {
+            singular = true;
+          } else if (!(D < NV_EPS)) {
+            double tm[3];
+            term_value(vect, circ, b, c, D, abc, dist, ya, qc, two_pi, tm);
+            if (!(far && mid_range<false>(D) && mid_range<true>(abc))) {
+              const double3 t = node_term_exact(vect[0], vect[1], vect[2], circ[0], circ[1], circ[2], dist, qc, two_pi);
+              tm[0] = t.x;
+              tm[1] = t.y;
+              tm[2] = t.z;
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[k] = e_add(acc[k], tm[k]);
+            ++ev;
+          }
         }
       }
-      const double vect[3] = {e_sub(cs[0], xi[0]), e_sub(cs[1], xi[1]), e_sub(cs[2], xi[2])};
-      const double circ[3] = {B.x, B.y, B.z};
-      const double a = e_mul(dist, dist);
-      const double b = e_mul(2.0, dot3(vect, circ));
-      const double c = dot3(circ, circ);
-      const double D = e_sub(e_mul(e_mul(4.0, a), c), e_mul(b, b));
-      if (D < NV_EPS) continue;
-      double cr[3];
-      cross3(vect, circ, cr);
-      const double den = e_mul(two_pi, D);
-      const double fac = e_sub(e_div(e_add(e_mul(2.0, c), b), e_sqrt(e_add(e_add(a, b), c))), e_div(b, e_sqrt(a)));
-#pragma unroll
-      for (int k = 0; k < 3; ++k) acc[k] = e_add(acc[k], e_mul(e_div(e_mul(cr[k], qc), den), fac));
-      ++evals;
+    }
+    if (next == kEnd) break;
+    if (next == nz) {
+      A = An;
+      B = Bn;
+      I = In;
     } else {
-      node = I.y != kEnd ? I.y : I.z;
+      A = ldg4(&tb.nA[next]);
+      B = ldg4(&tb.nB[next]);
+      I = __ldg(&tb.nI[next]);
     }
   }
+  evals += ev;
+  tests += te;
 }
 
 // Local term, the unshifted image's tree sum ub0, the shifted images' sum ubs, mutual
@@ -2290,9 +2354,9 @@ void launch_tree_walk(nv_handle *h) {
                                                              h->T, *tb, h->d_err);
   }
   cudaMemsetAsync(tb->defer_n, 0, sizeof(int), h->stream);
-  // two threads per target while the one-thread blocks would fill the GPU less than ~4
-  // times (automatic), or as nv_set_walk_parts asks
-  const int split = h->walk_parts == 0 ? h->n_work_tree < 32 * n_sms() : h->walk_parts > 1;
+  // two threads per target up to 20 blocks of targets an SM (automatic), or as
+  // nv_set_walk_parts asks: 100,000 points 4.37 ms (4.58 with one), 262,144 points 5.85 ms (5.37)
+  const int split = h->walk_parts == 0 ? h->n_work_tree < 20 * n_sms() : h->walk_parts > 1;
   k_tree_walk_fp64<<<h->n_work_tree, split ? 128 : 64, 0, h->stream>>>(
       h->d_sc, h->d_dyn, h->d_work_tree, h->x, h->gi, h->gb, h->nxt, h->prv, h->u, h->T, *tb, split, h->d_err);
 }

@@ -65,3 +65,22 @@ def test_terms_outside_the_shared_seeds_range(scale):
         with Handle(p, [96], states=[st]) as h:
             h.set_direct_split(split)
             assert np.array_equal(h.calc_velocity(), uo, equal_nan=True)
+
+
+# one leaf level and less, several levels, rings across the box; the tree's own accepted nodes,
+# single points among them, with the opening test by squares and by quotients (theta > 2/sqrt(3))
+@pytest.mark.parametrize("n", [7, 129, 650])
+@pytest.mark.parametrize("theta", [0.4, 0.9, 1.3])
+@pytest.mark.parametrize("corr", [True, False])
+def test_tree_walk_bit_identical_to_the_reference_order(n, theta, corr):
+    from nuvort_b200.api import Handle
+    st = _lines(n, n)
+    p = config0_params(box_size=L, delta=0.02, velocity="Tree", tree_theta=theta, tree_extra_correction=corr)
+    o = Oracle(p, st)
+    uo = o.calc_velocity()
+    with Handle(p, [n + 3], states=[st]) as h:
+        for parts in (1, 2):
+            h.set_walk_parts(parts)
+            assert np.array_equal(h.calc_velocity(), uo)
+            c = h.counters()
+            assert (c.tree_eval, c.tree_tests) == (o.counters().tree_eval, o.counters().tree_tests)
