@@ -307,6 +307,14 @@ int dalloc(T **p, size_t n) {
   return NV_OK;
 }
 
+// Waits for the clearing of the buffers allocated so far: cudaMemset runs on the null stream,
+// which the handle's non-blocking streams do not wait for, and returns before it is done; a
+// copy or kernel of theirs into such a buffer could otherwise be cleared again.
+int cleared() {
+  NV_CUDA(cudaStreamSynchronize(nullptr));
+  return NV_OK;
+}
+
 void build_worklist(nv_handle *h, int which, std::vector<int2> &w, int tb) {
   w.clear();
   for (int s = 0; s < h->nsys; ++s) {
@@ -539,7 +547,7 @@ int ensure_batch(nv_handle *h) {
   if ((rc = dalloc(&h->bstage, 3 * (size_t)h->T)) || (rc = dalloc(&h->d_btab, (size_t)h->nsys)) ||
       (rc = dalloc(&h->d_bcheck, 2 * (size_t)h->nsys)))
     return rc;
-  return NV_OK;
+  return cleared();
 }
 // every listed state gives the optional array or none does
 template <class F>
@@ -732,6 +740,7 @@ int nv_create(const nv_params *params, int32_t nsys, const int32_t *capacity, in
   tree_alloc(h);
   topo_alloc(h);
   if (cudaGetLastError() != cudaSuccess) return bail(set_error(NV_ERR_CUDA, "allocation failed"));
+  if ((rc = cleared())) return bail(rc);
   *out = h;
   return NV_OK;
 }
@@ -1702,7 +1711,7 @@ int nv_calc_velocity_direct_at(nv_handle *h, int32_t sys, const int32_t *targets
   NV_CUDA(cudaMalloc(&dt, std::max(n, 1) * sizeof(int)));
   NV_CUDA(cudaMalloc(&du, std::max(n, 1) * 3 * sizeof(double)));
   cudaMemcpy(dt, g.data(), n * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemset(du, 0, std::max(n, 1) * 3 * sizeof(double));
+  cudaMemsetAsync(du, 0, std::max(n, 1) * 3 * sizeof(double), h->stream);
   launch_ghost(h);
   launch_direct_targets(h, sys, dt, n, du);
   rc = finish(h);
