@@ -106,12 +106,11 @@ struct SysDyn {
   unsigned long long tree_tests;
   int event_seq;
   unsigned long long ev_hash;  // sum of event_digest over this system's events
-  int live;          // pinsert: the system has a live point (src/line.f90:25-27)
   int nlive;         // live slots: set by nv_upload, kept by the topology stages' events
   int old_pcount;
   int ins_fallback;  // pinsert needs the serial sweep this step
   int ins_conv;      // pinsert's fixed-point iteration has converged
-  int ins_mismatch;  // positions where the iteration's H and H' differ
+  int ins_high, ins_high2;  // elements of its H, of the last walk's H'
   int noise_counter; // noisey_xflow: 1-based sample in use (xflow_noise_counter)
   int wall_recon_count;  // wall_recon cuts (reconnection.f90:91)
   long long diag[12];  // see nv_diagnostics

@@ -25,21 +25,23 @@
 
 struct TopoBuffers {
   int *flag_a = nullptr, *pos_a = nullptr, *list_a = nullptr;
-  int *flag_b = nullptr, *pos_b = nullptr, *list_b = nullptr;
-  int *flag_c = nullptr, *pos_c = nullptr, *list_c = nullptr;
+  int *pos_b = nullptr, *list_b = nullptr;
+  int *pos_c = nullptr, *list_c = nullptr;
+  unsigned long long *pass_state = nullptr;  // ordered_pass: per list and block
+  unsigned *pass_ctl = nullptr;              // its block ticket, finished blocks, epoch
   int *dec = nullptr;       // per slot: bit0 stale test, bit1 fresh test, bit2 inserts, bit3 case A
   int *newslot = nullptr;   // per slot: the slot its insertion fills
   double *xnew = nullptr;   // per insertion position: new point position [3][T]
   double *unew = nullptr;   // per insertion position: new point velocity [3][T]
   int *segnx = nullptr;     // per insertion position: infront of the original slot
-  int *fh[2] = {nullptr, nullptr};  // higher-order insertion positions, H and H'
-  int *pos_h = nullptr;     // exclusive prefix sum of H
+  int *high = nullptr, *high2 = nullptr;  // per system, from its first slot: higher-order insertion positions
   unsigned *l0 = nullptr, *l1 = nullptr;  // sweep bitmaps
-  // pinsert's measured segment lengths (total_length, line.f90:39): per slot the stale and
-  // the fresh distance, the one the sweep used, and per inserting slot the distance its new
-  // point measured when the sweep reached it (-1: not reached)
-  double *len_st = nullptr, *len_fr = nullptr, *seglen = nullptr, *dn_new = nullptr;
+  // pinsert's measured segment lengths (total_length, line.f90:39): per slot the distance the
+  // sweep used, and per inserting slot the distance its new point measured when the sweep
+  // reached it (-1: not reached)
+  double *seglen = nullptr, *dn_new = nullptr;
   int total_parts = 1;                          // blocks per system summing the lengths
+  int *part_done = nullptr;                     // per system: parts summed
   double *psum = nullptr, *pnear = nullptr;     // per (system, part): their sum and nearest to delta
   void *cub_tmp = nullptr;
   size_t cub_bytes = 0;
@@ -51,6 +53,7 @@ struct TopoBuffers {
   int *cell_start = nullptr;        // per cell: first entry in cell_items (exclusive sum, n_cells + 1)
   int *cell_items = nullptr;        // slots grouped by cell
   bool any_cells = false;
+  bool small_pclose = false;  // the tree-less systems' slots are few: a warp per target scans them
 };
 
 // A system's cell grid over its box [-L/2, L/2)^3 (points outside are clamped to the edge
@@ -108,26 +111,129 @@ struct Sweep {
   }
 };
 
-// l0/l1 from a 0/1 flag per slot (one thread per l0 word, then one per l1 word).
-__global__ void k_bits_l0(const int *__restrict__ flag, unsigned *l0, long long T) {
-  const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w * 32 >= T + 32) return;
-  unsigned b = 0;
-  for (int k = 0; k < 32; ++k) {
-    const long long g = w * 32 + k;
-    if (g < T && flag[g]) b |= 1u << k;
+// Clears the bitmaps' words of slot g (a pass over 0 <= g <= T clears them all).
+__device__ __forceinline__ void clear_bits(unsigned *l0, unsigned *l1, long long g, long long T) {
+  if ((g & 31) == 0) l0[g >> 5] = 0;
+  if ((g & 1023) == 0) l1[g >> 10] = 0;
+  if (g == T) {
+    l0[(T >> 5) + 1] = 0;
+    l1[(T >> 10) + 1] = 0;
   }
-  l0[w] = b;
 }
-__global__ void k_bits_l1(const unsigned *__restrict__ l0, unsigned *l1, long long nw0) {
-  const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w * 32 >= nw0 + 32) return;
-  unsigned b = 0;
-  for (int k = 0; k < 32; ++k) {
-    const long long q = w * 32 + k;
-    if (q < nw0 && l0[q]) b |= 1u << k;
+
+// ---- ordered lists in one pass ---------------------------------------------------------------
+// flags(g), for 0 <= g <= n in ascending order over the grid, gives K bits per slot; list[k]
+// receives the slots with bit k in ascending order and pos[k][g] the number of such slots below
+// g.  A block takes 1,024 consecutive slots (a ticket, so that the blocks before it have
+// started), counts its bits, and finds the blocks' sum before it by looking back: every block
+// publishes its own sum and, once known, its inclusive sum, each in one 64-bit word with the
+// launch's epoch, so that nothing is cleared between launches (the last block to finish sets up
+// the next).  One launch for what a flag kernel, a two-kernel scan and a scatter did in four
+// (per list): of the 158 launches of a tree system's step, 28 compactions' worth.
+constexpr int kPassThreads = 256, kPassItems = 4, kPassSlots = kPassThreads * kPassItems;
+constexpr int kPassPolls = 1 << 22;  // polls of a predecessor before giving up
+
+template <int K>
+struct Lists {
+  int *pos[K], *list[K];
+  unsigned long long *state;  // [K][blocks]
+  unsigned *ctl;              // ticket, finished blocks, epoch
+};
+
+template <int K, class F>
+__device__ void ordered_pass(const Lists<K> &L, long long n, unsigned *err, F flags) {
+  constexpr int kWarps = kPassThreads / 32;
+  static_assert(K <= kWarps, "a warp looks back for each list");
+  __shared__ int s_block, s_sum[K][kWarps], s_base[K];
+  __shared__ unsigned s_epoch;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid == 0) {
+    s_epoch = *(volatile unsigned *)&L.ctl[2];
+    s_block = (int)atomicAdd(&L.ctl[0], 1u);
   }
-  l1[w] = b;
+  __syncthreads();
+  const int b = s_block, nb = gridDim.x;
+  const unsigned epoch = s_epoch;
+  const long long g0 = (long long)b * kPassSlots + wid * (32 * kPassItems) + lane;
+  unsigned m[K][kPassItems];
+#pragma unroll
+  for (int it = 0; it < kPassItems; ++it) {
+    const long long g = g0 + 32 * it;
+    const unsigned f = g <= n ? flags(g) : 0u;
+#pragma unroll
+    for (int k = 0; k < K; ++k) m[k][it] = __ballot_sync(0xffffffffu, (f >> k) & 1u);
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      int v = 0;
+#pragma unroll
+      for (int it = 0; it < kPassItems; ++it) v += __popc(m[k][it]);
+      s_sum[k][wid] = v;
+    }
+  __syncthreads();
+  if (wid < K) {  // warp k: the sum of list k's bits before this block
+    volatile unsigned long long *st = L.state + (long long)wid * nb;
+    auto word = [&](unsigned flag, int v) {
+      return (unsigned long long)((epoch << 2) | flag) << 32 | (unsigned long long)(unsigned)v;
+    };
+    int own = 0;
+    for (int w = 0; w < kWarps; ++w) own += s_sum[wid][w];
+    if (lane == 0) st[b] = word(b == 0 ? 2u : 1u, own);
+    int before = 0;
+    bool ok = true;
+    for (int j = b - 1; j >= 0 && ok; j -= 32) {
+      const int q = j - lane;
+      unsigned long long v = word(2u, 0);  // before the first block: an inclusive sum of 0
+      int polls = 0;
+      for (;;) {
+        if (q >= 0) v = st[q];
+        const unsigned tag = (unsigned)(v >> 32);
+        const bool ready = (tag >> 2) == (epoch & 0x3fffffffu) && (tag & 3u);
+        if (__all_sync(0xffffffffu, ready)) break;
+        if (++polls > kPassPolls) {
+          ok = false;
+          break;
+        }
+      }
+      const unsigned incl = __ballot_sync(0xffffffffu, ((unsigned)(v >> 32) & 3u) == 2u);
+      const int stop = incl ? __ffs(incl) - 1 : 31;
+      int x = lane <= stop ? (int)(unsigned)v : 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      before += x;
+      if (incl) break;
+    }
+    if (lane == 0) {
+      if (!ok) {
+        atomicOr(err, DERR_TIMEOUT);
+        before = 0;
+      }
+      if (b > 0) st[b] = word(2u, before + own);
+      s_base[wid] = before;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    int off = s_base[k];
+    for (int w = 0; w < wid; ++w) off += s_sum[k][w];
+#pragma unroll
+    for (int it = 0; it < kPassItems; ++it) {
+      const long long g = g0 + 32 * it;
+      const int p = off + __popc(m[k][it] & ((1u << lane) - 1u));
+      if (g <= n) {
+        L.pos[k][g] = p;
+        if ((m[k][it] >> lane) & 1u) L.list[k][p] = (int)g;
+      }
+      off += __popc(m[k][it]);
+    }
+  }
+  if (tid == 0 && atomicAdd(&L.ctl[1], 1u) == (unsigned)nb - 1) {  // every block has taken its ticket and epoch
+    L.ctl[0] = 0;
+    L.ctl[1] = 0;
+    L.ctl[2] = (epoch + 1) & 0x3fffffffu;
+  }
 }
 
 __device__ __forceinline__ bool recon_step(const SysConst &sc, const SysDyn &d) {
@@ -169,51 +275,50 @@ __device__ __forceinline__ void refresh_ghosts(const SysConst &sc, const State &
 
 // ---- pass 1 kernels: marks ----------------------------------------------------------------
 // precon marks: live slot with delta/2 > closestd > epsilon(1.) (reconnection.f90:185).
-__global__ void k_mark_recon(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of,
-                             const double *__restrict__ CD, const int *__restrict__ nxt, int *fa, long long T,
-                             const unsigned *err) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > T) return;
-  int a = 0;
-  if (g < T && !*err) {
+__global__ void __launch_bounds__(kPassThreads) k_mark_recon(const SysConst *__restrict__ scs, SysDyn *dyn,
+                                                            const int *__restrict__ sys_of,
+                                                            const double *__restrict__ CD,
+                                                            const int *__restrict__ nxt, Lists<1> L, long long T,
+                                                            unsigned *err) {
+  const bool run = !*(volatile unsigned *)err;
+  ordered_pass<1>(L, T, err, [&](long long g) -> unsigned {
+    if (g >= T || !run) return 0u;
     const int s = sys_of[g];
     const SysConst &sc = scs[s];
     const int k = (int)(g - sc.base);
-    if (k >= 1 && k <= dyn[s].pcount && recon_step(sc, dyn[s]) && nxt[g] != 0 && !walled(sc)) {
-      const double cd = CD[g];
-      a = (cd < sc.delta / 2.) && (cd > NV_EPS);
-      if (cd > NV_EPS) margin_note(dyn[s], 2, cd, sc.delta / 2.);
-    }
-  }
-  fa[g] = a;
+    if (!(k >= 1 && k <= dyn[s].pcount && recon_step(sc, dyn[s]) && nxt[g] != 0 && !walled(sc))) return 0u;
+    const double cd = CD[g];
+    if (cd > NV_EPS) margin_note(dyn[s], 2, cd, sc.delta / 2.);
+    return (cd < sc.delta / 2.) && (cd > NV_EPS);
+  });
 }
 
 // premove marks: live slot with |x_i - x_{i+2}| < .99 delta (line.f90:113-115).
-__global__ void k_mark_remove(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of,
-                              const double *__restrict__ X, const int *__restrict__ nxt, int *fa, long long T,
-                              const unsigned *err) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > T) return;
-  int a = 0;
-  if (g < T && !*err) {
-    const int s = sys_of[g];
-    const SysConst &sc = scs[s];
-    const int k = (int)(g - sc.base);
-    if (k >= 1 && k <= dyn[s].pcount && recon_step(sc, dyn[s]) && nxt[g] != 0 && !walled(sc)) {
-      double x[3], y[3];
-      load3(X, T, (int)g, x);
-      load3(X, T, nxt[nxt[g]], y);
-      const double dii = dist_gen(x, y);
-      a = dii < e_mul(.99, sc.delta);
-      margin_note(dyn[s], 1, dii, e_mul(.99, sc.delta));
+__global__ void __launch_bounds__(kPassThreads) k_mark_remove(const SysConst *__restrict__ scs, SysDyn *dyn,
+                                                             const int *__restrict__ sys_of,
+                                                             const double *__restrict__ X,
+                                                             const int *__restrict__ nxt, int *fa, Lists<1> L,
+                                                             unsigned *l0, unsigned *l1, long long T, unsigned *err) {
+  const bool run = !*(volatile unsigned *)err;
+  ordered_pass<1>(L, T, err, [&](long long g) -> unsigned {
+    clear_bits(l0, l1, g, T);  // extra visits of the sweep start empty
+    unsigned a = 0;
+    if (g < T && run) {
+      const int s = sys_of[g];
+      const SysConst &sc = scs[s];
+      const int k = (int)(g - sc.base);
+      if (k >= 1 && k <= dyn[s].pcount && recon_step(sc, dyn[s]) && nxt[g] != 0 && !walled(sc)) {
+        double x[3], y[3];
+        load3(X, T, (int)g, x);
+        load3(X, T, nxt[nxt[g]], y);
+        const double dii = dist_gen(x, y);
+        a = dii < e_mul(.99, sc.delta);
+        margin_note(dyn[s], 1, dii, e_mul(.99, sc.delta));
+      }
     }
-  }
-  fa[g] = a;
-}
-
-__global__ void k_scatter(const int *__restrict__ flag, const int *__restrict__ pos, int *__restrict__ list, long long T) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < T && flag[g]) list[pos[g]] = (int)g;
+    fa[g] = (int)a;
+    return a;
+  });
 }
 
 // precon (reconnection.f90:11-61).
@@ -376,6 +481,61 @@ __global__ void k_pclose_brute(const SysConst *__restrict__ scs, const SysDyn *_
 }
 
 
+// The same search with a warp per target, each lane over every 32nd slot in ascending order, the
+// lanes' minima combined by (distance, slot), so that ties keep the lowest slot: for systems
+// of a few thousand slots, whose cell lists cost six launches and a search that few threads
+// make, cell after cell (600 points: 16 us, 78 with the cell list; 4,000: 48, 111; but 8,000
+// points: 155, 112).
+constexpr int kPcloseWarps = 4, kPcloseSlots = 6144;
+__global__ void __launch_bounds__(32 * kPcloseWarps) k_pclose_warps(
+    const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn, const int *__restrict__ sys_of,
+    const double *__restrict__ X, const int *__restrict__ nxt, const int *__restrict__ prv, int *__restrict__ cl,
+    double *__restrict__ CD, long long T, const unsigned *err) {
+  const int lane = threadIdx.x & 31;
+  const long long g = (long long)blockIdx.x * kPcloseWarps + (threadIdx.x >> 5);
+  if (g >= T || *err) return;
+  const int s = sys_of[g];
+  const SysConst &sc = scs[s];
+  if (sc.use_tree || !recon_step(sc, dyn[s])) return;
+  const int pc = dyn[s].pcount;
+  const int k = (int)(g - sc.base);
+  if (k < 1 || k > pc || nxt[g] == 0) return;
+  if (pinned_at(sc, (int)g)) {
+    if (lane == 0) CD[g] = 100.;
+    return;
+  }
+  const int ni = nxt[g], pi = prv[g];
+  double xi[3];
+  load3(X, T, (int)g, xi);
+  double best = 100., best2 = 1e300;
+  int bj = INT_MAX;
+  for (int j = sc.base + 1 + lane; j <= sc.base + pc; j += 32) {
+    double xj[3];
+    load3(X, T, j, xj);
+    const double d2 = e_add(e_add(e_sq(e_sub(xi[0], xj[0])), e_sq(e_sub(xi[1], xj[1]))), e_sq(e_sub(xi[2], xj[2])));
+    if (d2 > best2 || nxt[j] == 0 || j == g || j == ni || j == pi || pinned_at(sc, j)) continue;
+    const double dist = e_sqrt(d2);
+    if (dist < best) {
+      best = dist;
+      best2 = d2;
+      bj = j;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double d = __shfl_xor_sync(0xffffffffu, best, o);
+    const int j = __shfl_xor_sync(0xffffffffu, bj, o);
+    if (d < best || (d == best && j < bj)) {
+      best = d;
+      bj = j;
+    }
+  }
+  if (lane == 0) {
+    if (bj != INT_MAX) cl[g] = bj;
+    CD[g] = best;
+  }
+}
+
 // g as seen from x: the nearest periodic image (get_ghost_p's adjustment)
 __device__ __forceinline__ void ghost_of(const SysConst &sc, const double x[3], const double g[3], double out[3]) {
   for (int c = 0; c < 3; ++c) out[c] = g[c];
@@ -392,77 +552,103 @@ __device__ __forceinline__ void ghost_of(const SysConst &sc, const double x[3], 
 // tested again by the reference and may insert in turn; k_ins_chain resolves those
 // higher-order insertions by a fixed-point iteration over their positions.
 
-// bit0 stale test, bit1 fresh test (ghost of the current infront position); list = either.
-__global__ void k_ins_mark(const SysConst *__restrict__ scs, SysDyn *__restrict__ dyn, const int *__restrict__ sys_of,
-                           const double *__restrict__ X, const double *__restrict__ GI, const int *__restrict__ nxt,
-                           int *fa, int *fb, int *dec, double *len_st, double *len_fr, long long T,
-                           const unsigned *err) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > T) return;
-  int a = 0, b = 0, dv = 0;
-  double lst = 0., lfr = 0.;
-  if (g < T && !*err) {
-    const int s = sys_of[g];
-    const SysConst &sc = scs[s];
-    const int k = (int)(g - sc.base);
-    if (k >= 1 && k <= dyn[s].pcount && !walled(sc)) {
-      if (nxt[g] == 0) {
-        b = 1;
-      } else {
-        double x[3], gi[3], gf[3];
-        load3(X, T, (int)g, x);
-        load3(GI, T, (int)g, gi);
-        load3(X, T, nxt[g], gf);
-        ghost_adjust(sc, x, gf);
-        lst = dist_gen(x, gi);
-        lfr = dist_gen(x, gf);
-        const int st = lst > sc.delta, fr = lfr > sc.delta;
-        dv = st | (fr << 1);
-        a = st | fr;
-        dyn[s].live = 1;
-      }
-    }
-  }
-  fa[g] = a;
-  fb[g] = b;
-  if (g < T) {
-    dec[g] = dv;
-    len_st[g] = lst;
-    len_fr[g] = lfr;
-  }
+struct InsTest {
+  double stale, fresh;  // the two lengths
+  int st, fr;           // the two tests
+};
+__device__ __forceinline__ InsTest ins_test(const SysConst &sc, const double *__restrict__ X,
+                                            const double *__restrict__ GI, const int *__restrict__ nxt, long long T,
+                                            int g) {
+  double x[3], gi[3], gf[3];
+  load3(X, T, g, x);
+  load3(GI, T, g, gi);
+  load3(X, T, nxt[g], gf);
+  ghost_adjust(sc, x, gf);
+  InsTest t;
+  t.stale = dist_gen(x, gi);
+  t.fresh = dist_gen(x, gf);
+  t.st = t.stale > sc.delta;
+  t.fr = t.fresh > sc.delta;
+  return t;
 }
 
-// The length each live slot's test measured (line.f90:38-39): with the ghosts its
-// predecessor's insertion refreshed when that predecessor lies below it and inserts (the
-// same rule as its decision), else with the step-start ghosts; 0 for empty slots.  New points
-// the sweep reaches are written when the insertions are applied.
-__global__ void k_ins_len(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
-                          const int *__restrict__ sys_of, const int *__restrict__ nxt, const int *__restrict__ prv,
-                          const int *__restrict__ dec, const double *__restrict__ len_st,
-                          const double *__restrict__ len_fr, double *__restrict__ seglen, long long T) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= T) return;
-  double v = 0.;
-  const int s = sys_of[g];
-  const int k = (int)(g - scs[s].base);
-  if (k >= 1 && k <= dyn[s].pcount && nxt[g] != 0) {
-    const int p = prv[g];
-    v = (p < g && (dec[p] & 4)) ? len_fr[g] : len_st[g];
+// Whether live slot k (its tests given) inserts.  Where the tests differ the outcome is the
+// fresh one if the predecessor p = behind(k) < k inserts, else the stale one, so it is the
+// stale test flipped by p's outcome; p's in turn may depend on its own predecessor: a chain of
+// such slots, each below the last (the two tests differ only for a length within one step's
+// motion of delta, so chains are one or two slots long).
+__device__ __forceinline__ int ins_outcome(const SysConst &sc, const double *__restrict__ X,
+                                           const double *__restrict__ GI, const int *__restrict__ nxt,
+                                           const int *__restrict__ prv, long long T, int k, InsTest t) {
+  int flip = 0;
+  while (t.st != t.fr) {
+    flip ^= t.st;
+    const int p = prv[k];
+    if (!(p < k)) return flip;
+    k = p;
+    t = ins_test(sc, X, GI, nxt, T, k);
   }
-  seglen[g] = v;
+  return flip ^ t.st;
+}
+
+// Every slot's part of the sweep: dec bit 2 inserts, bit 3 case A (its ghosts were refreshed by
+// its predecessor's insertion); the length its test measured (line.f90:38-39), with the
+// refreshed ghosts where the predecessor lies below it and inserts, else with the step-start
+// ones.  Lists, in slot order: candidates (either test passes), free slots, insertions.  Slot
+// base starts the system's pinsert.
+__global__ void __launch_bounds__(kPassThreads) k_ins_mark(const SysConst *__restrict__ scs, SysDyn *__restrict__ dyn,
+                                                          const int *__restrict__ sys_of,
+                                                          const double *__restrict__ X, const double *__restrict__ GI,
+                                                          const int *__restrict__ nxt, const int *__restrict__ prv,
+                                                          int *dec, double *seglen, Lists<3> L, unsigned *l0,
+                                                          unsigned *l1, long long T, unsigned *err) {
+  const bool run = !*(volatile unsigned *)err;
+  ordered_pass<3>(L, T, err, [&](long long gl) -> unsigned {
+    clear_bits(l0, l1, gl, T);  // extra visits of the serial sweep start empty
+    if (gl >= T) return 0u;
+    const int g = (int)gl, s = sys_of[g];
+    const SysConst &sc = scs[s];
+    const int k = g - sc.base;
+    unsigned f = 0;
+    int dv = 0;
+    double len = 0.;
+    if (k == 0) {
+      SysDyn &d = dyn[s];
+      d.old_pcount = d.pcount;
+      d.ins_fallback = 0;
+      d.ins_conv = d.ins_high = d.ins_high2 = 0;
+    } else if (run && k <= dyn[s].pcount && !walled(sc)) {
+      if (nxt[g] == 0) {
+        f = 2u;
+      } else {
+        const InsTest t = ins_test(sc, X, GI, nxt, T, g);
+        const int p = prv[g];
+        bool fresh = false;  // the predecessor's insertion refreshed this slot's ghosts
+        if (p < g) fresh = ins_outcome(sc, X, GI, nxt, prv, T, p, ins_test(sc, X, GI, nxt, T, p));
+        const int ins = fresh ? t.fr : t.st;
+        dv = t.st | t.fr << 1 | ins << 2 | (ins && fresh) << 3;
+        f = (t.st | t.fr) | (unsigned)ins << 2;
+        len = fresh ? t.fresh : t.stale;
+      }
+    }
+    dec[g] = dv;
+    seglen[g] = len;
+    return f;
+  });
 }
 
 // total_length and avg_sep of the pinsert just made (line.f90:39,95): the measured lengths
 // summed in a fixed order -- block (s, p) sums part p of system s's slots (per thread by
-// stride, then a tree over the block), and k_ins_total adds the parts in order (the reference
-// adds them one after another, which agrees to ~1e-13 relative) -- divided by old_pcount minus
+// stride, then a tree over the block), and the last of a system's blocks adds the parts in
+// order (the reference adds the lengths one after another, which agrees to ~1e-13 relative) --
+// divided by old_pcount minus
 // the empty slots left among the pcount slots.  Many blocks per large system: one block
 // summing a million lengths takes milliseconds.
 constexpr int kTotalThreads = 256;
-__global__ void __launch_bounds__(kTotalThreads) k_ins_part(const SysConst *__restrict__ scs, const SysDyn *dyn,
-                                                            int nsys, int parts, const double *__restrict__ seglen,
-                                                            double *__restrict__ psum, double *__restrict__ pnear,
-                                                            const unsigned *err) {
+__global__ void __launch_bounds__(kTotalThreads) k_ins_total(const SysConst *__restrict__ scs, SysDyn *dyn,
+                                                             int nsys, int parts, const double *__restrict__ seglen,
+                                                             double *psum, double *pnear, int *done,
+                                                             const unsigned *err) {
   __shared__ double sum_[kTotalThreads], near_[kTotalThreads];
   const int s = blockIdx.x / parts, p = blockIdx.x % parts;
   if (s >= nsys || *err) return;
@@ -488,96 +674,28 @@ __global__ void __launch_bounds__(kTotalThreads) k_ins_part(const SysConst *__re
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    psum[blockIdx.x] = sum_[0];
-    pnear[blockIdx.x] = near_[0];
+  if (threadIdx.x != 0) return;
+  double tot = sum_[0];
+  near = near_[0];
+  if (parts > 1) {
+    ((volatile double *)psum)[blockIdx.x] = tot;
+    ((volatile double *)pnear)[blockIdx.x] = near;
+    __threadfence();
+    if (atomicAdd(&done[s], 1) != parts - 1) return;
+    done[s] = 0;
+    __threadfence();
+    tot = 0.;
+    near = 1e300;
+    for (int q = 0; q < parts; ++q) {
+      tot += ((volatile double *)psum)[s * parts + q];
+      near = fmin(near, ((volatile double *)pnear)[s * parts + q]);
+    }
   }
-}
-
-__global__ void k_ins_total(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys, int parts,
-                            const double *__restrict__ psum, const double *__restrict__ pnear, const unsigned *err) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys || *err) return;
-  const SysConst &sc = scs[s];
-  if (walled(sc)) return;
   SysDyn &d = dyn[s];
-  double tot = 0., near = 1e300;
-  for (int p = 0; p < parts; ++p) {
-    tot += psum[s * parts + p];
-    near = fmin(near, pnear[s * parts + p]);
-  }
   d.total_length = tot;
   const int empty = d.pcount - d.nlive;
   d.avg_sep = tot / (double)(d.old_pcount - empty);
   if (d.margin_on && near < 1e300) margin_note_abs(d, 0, near, sc.delta);
-}
-
-// Outcomes: known where the two tests agree (decided here, in parallel); where they differ
-// the outcome is the fresh test if the predecessor p = behind(k) < k inserts, else the stale
-// one -- those "ambiguous" slots are marked for an ordered pass.
-__global__ void k_ins_decide_easy(const int *__restrict__ list_a, const int *__restrict__ n_ptr, int *dec, int *famb,
-                                  const unsigned *err) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= *n_ptr || *err) return;
-  const int k = list_a[e];
-  const int dv = dec[k];
-  const int st = dv & 1, fr = (dv >> 1) & 1;
-  if (st == fr) dec[k] = dv | (st << 2);
-  else famb[k] = 1;
-}
-
-// Ambiguous slots.  The outcome of ambiguous k is its fresh test when p = behind(k) < k
-// inserts, else its stale test; p's outcome is final unless p is ambiguous too.  So the
-// ambiguous slots form chains k -> infront(k) (while infront(k) > k is ambiguous), each
-// starting at a slot whose predecessor is decided or lies above it.  One thread per
-// ambiguous slot; the chain heads walk their chains.
-__global__ void k_ins_decide_amb(const int *__restrict__ list_m, const int *__restrict__ n_ptr,
-                                 const int *__restrict__ nxt, const int *__restrict__ prv,
-                                 const int *__restrict__ famb, int *dec, const unsigned *err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *n_ptr || *err) return;
-  int k = list_m[t];
-  const int p = prv[k];
-  if (p < k && famb[p]) return;  // inside a chain: its head decides it
-  int refreshed = p < k && (dec[p] & 4);
-  for (;;) {
-    const int dv = dec[k];
-    const int d = refreshed ? (dv >> 1) & 1 : dv & 1;
-    dec[k] = dv | (d << 2);
-    const int nx = nxt[k];
-    if (!(nx > k && famb[nx])) break;
-    refreshed = d;
-    k = nx;
-  }
-}
-
-// Per-system state of a pinsert: flags of the fixed-point iteration, live marker.
-__global__ void k_ins_begin(SysDyn *dyn, int nsys) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  dyn[s].live = 0;
-  dyn[s].old_pcount = dyn[s].pcount;
-  dyn[s].ins_fallback = 0;
-  dyn[s].ins_conv = 0;
-  dyn[s].ins_mismatch = 0;
-}
-
-// Case A (ghosts refreshed by the predecessor's insertion) and the insertion flags.
-__global__ void k_ins_decide_case(const int *__restrict__ list_a, const int *__restrict__ n_ptr,
-                                  const int *__restrict__ prv, int *dec, int *fc, const unsigned *err) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= *n_ptr || *err) return;
-  const int k = list_a[e];
-  const int dv = dec[k];
-  const int p = prv[k];
-  const bool caseA = p < k && (dec[p] & 4);
-  if (caseA) dec[k] = dv | 8;
-  fc[k] = (dv >> 2) & 1;
-}
-
-__global__ void k_zero_flags(int *f, long long n) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g <= n) f[g] = 0;
 }
 
 // New points along chains of consecutive insertions, with the insertions of new points the
@@ -592,35 +710,42 @@ __global__ void k_zero_flags(int *f, long long n) {
 // one quantity that couples different chains is the slot of each new point, the free slot
 // of the insertion's rank in sweep order, where the sweep order merges the original
 // insertions (at their slots) with these higher-order ones (at the new points' slots).
-// Given a set H of higher-order positions, pos_c + pos_h give every rank; the walk then
-// yields the higher-order positions H' it implies.  Each event depends only on events at
-// lower positions, so once H' = H every event is the serial sweep's (by induction over the
-// sweep position).  The walk is repeated from H = {} a fixed number of times; a system
-// that has not converged by then runs the serial sweep.
-__global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, State S,
-                            const int *__restrict__ pos_c, const int *__restrict__ list_c,
-                            const int *__restrict__ pos_b, const int *__restrict__ list_b, const int *__restrict__ dec,
-                            const int *__restrict__ pos_h, int *fout, int *newslot, int *segnx, double *xnew,
-                            double *unew, double *dn_new, const int *__restrict__ nev_total, unsigned *err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *nev_total || *err) return;
-  int k = list_c[t];
-  if (dec[k] & 8) return;  // not a chain head
-  const int s = sys_of[k];
-  if (dyn[s].ins_conv || dyn[s].ins_fallback) return;
-  const SysConst &sc = scs[s];
+// Given a set H of higher-order positions, the original insertions (pos_c) and H's elements
+// below a position give its rank; the walk then yields the higher-order positions H' it
+// implies.  Each event depends only on events at lower positions, so once H' = H every event
+// is the serial sweep's (by induction over the sweep position).  The walk from H = {} runs over
+// the whole GPU (k_ins_chain) and nearly always finds H' = {}: a new point lies about half a
+// segment from its neighbours, so it inserts only in a segment of more than twice delta.  Where
+// it finds some, the walk is repeated from H' -- over the whole GPU for large handles, by a block
+// per system for the others (k_ins_rounds).  A system that has not converged after a fixed
+// number of rounds, or whose H outgrows a block's list, runs the serial sweep.
+struct ChainArgs {
+  State S;
+  const int *pos_c, *list_c, *pos_b, *list_b, *dec;
+  int *newslot, *segnx;
+  double *xnew, *unew, *dn_new;
+};
+
+// The chain that starts at inserting slot k.  rank(g): H's elements of the system below g;
+// emit(e): e belongs to H'.
+template <class Rank, class Emit>
+__device__ void ins_chain_walk(const ChainArgs &A, const SysConst &sc, SysDyn &dy, int k, Rank rank, Emit emit) {
+  const State &S = A.S;
+  const int *pos_c = A.pos_c, *list_b = A.list_b, *dec = A.dec;
+  int *newslot = A.newslot, *segnx = A.segnx;
+  double *xnew = A.xnew, *unew = A.unew, *dn_new = A.dn_new;
   const int base = sc.base;
-  const int ev0 = pos_c[base], h0 = pos_h[base];
-  const int fb0 = pos_b[base], nfree = pos_b[base + sc.cap + 1] - fb0;
-  const int pc = dyn[s].pcount;
+  const int ev0 = pos_c[base];
+  const int fb0 = A.pos_b[base], nfree = A.pos_b[base + sc.cap + 1] - fb0;
+  const int pc = dy.pcount;
   const long long T = S.T;
   const int old_last = base + pc;
   // slot of the insertion with sweep rank r: the free slots in ascending order, then pcount+1..
   auto slot_of = [&](int g) -> int {
-    const int r = (pos_c[g] - ev0) + (pos_h[g] - h0);
+    const int r = (pos_c[g] - ev0) + rank(g);
     const int slot = r < nfree ? list_b[fb0 + r] : base + pc + 1 + (r - nfree);
     if (slot > base + sc.cap) {  // possibly an artefact of a not yet consistent H:
-      dyn[s].ins_fallback = 1;    // the serial sweep decides (and reports a real overflow)
+      dy.ins_fallback = 1;        // the serial sweep decides (and reports a real overflow)
       return -1;
     }
     return slot;
@@ -673,7 +798,7 @@ __global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const
       const double dn = dist_gen(xe, gie);
       dn_new[at] = dn;  // the length the new point e measures when the sweep reaches it
       if (!(dn > sc.delta)) break;
-      fout[e] = 1;
+      emit(e);
       const int q = slot_of(e);
       if (q < 0) return;
       ghost_of(sc, xe, xprev, gbe);
@@ -701,50 +826,152 @@ __global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const
   }
 }
 
-// Every system takes the serial sweep (no fixed-point rounds).
-__global__ void k_ins_all_serial(SysDyn *dyn, int nsys) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nsys) dyn[s].ins_fallback = 1;
+// Elements below g of the sorted list h[0 .. n), and whether it holds g.
+__device__ __forceinline__ int rank_in(const int *h, int n, int g) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (h[mid] < g) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+__device__ __forceinline__ bool holds(const int *h, int n, int g) {
+  const int r = rank_in(h, n, g);
+  return r < n && h[r] == g;
 }
 
-// Zero the output flags of the systems still iterating.
-__global__ void k_ins_zero_open(const SysDyn *__restrict__ dyn, const int *__restrict__ sys_of, int *f, long long T) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= T) return;
-  if (!dyn[sys_of[g]].ins_conv) f[g] = 0;
-}
-
-// Count, per system still iterating, the positions where H and H' differ.
-__global__ void k_ins_compare(SysDyn *dyn, const int *__restrict__ sys_of, const int *__restrict__ fin,
-                              const int *__restrict__ fout, long long T) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= T || fin[g] == fout[g]) return;
-  const int s = sys_of[g];
-  if (!dyn[s].ins_conv) atomicAdd(&dyn[s].ins_mismatch, 1);
-}
-
-// A system whose H' equals H has converged (iteration `it`, counted from 1).
-__global__ void k_ins_converge(SysDyn *dyn, int nsys, int it, int last) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
+// One walk: a thread per original insertion, chain heads only, from the system's H (high, sorted,
+// ins_high elements); H' goes to high2.
+__global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, ChainArgs A,
+                            const int *__restrict__ high, int *high2, const int *__restrict__ nev_total,
+                            const unsigned *err) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= *nev_total || *err) return;
+  const int k = A.list_c[t];
+  if (A.dec[k] & 8) return;  // not a chain head
+  const int s = sys_of[k];
+  const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   if (d.ins_conv || d.ins_fallback) return;
-  if (d.ins_mismatch == 0) {
-    d.ins_conv = 1;
-    d.diag[6] = it;
-  } else if (last) {
-    d.ins_fallback = 1;
-    d.diag[6] = it;
+  const int n = d.ins_high;
+  const int *h = high + sc.base;
+  ins_chain_walk(
+      A, sc, d, k, [&](int g) { return n ? rank_in(h, n, g) : 0; },
+      [&](int e) { high2[sc.base + atomicAdd(&d.ins_high2, 1)] = e; });  // (slots of the system: at most cap)
+}
+
+// Slots of a handle from which every walk runs over the whole GPU (two launches a round, whether
+// it is needed or not, 25 us in all) instead of the further ones by a block per system (1M points,
+// 30,000 insertions: 1.7 ms a walk; 32,768 points, 240 insertions: 20 us).
+constexpr long long kAgainSlots = 1 << 18;
+
+constexpr int kHighCap = 2048, kHighThreads = 256;
+
+// v[0 .. m) in ascending order, by a block (bitonic, padded to a power of two with room for it).
+__device__ void sort_block(int *v, int m) {
+  int p = 1;
+  while (p < m) p <<= 1;
+  for (int i = m + threadIdx.x; i < p; i += blockDim.x) v[i] = INT_MAX;
+  __syncthreads();
+  for (int k = 2; k <= p; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = threadIdx.x; i < p; i += blockDim.x) {
+        const int o = i ^ j;
+        if (o > i && ((v[i] > v[o]) == ((i & k) == 0))) {
+          const int x = v[i];
+          v[i] = v[o];
+          v[o] = x;
+        }
+      }
+      __syncthreads();
+    }
+}
+
+// After walk `it` of `iters` over the whole GPU, a block per system: converged where H' equals H,
+// else H' (sorted) takes H's place; the last walk leaves the others to the serial sweep.
+// `rounds`: instead of waiting for the next walk, the block makes the further ones itself.
+__global__ void __launch_bounds__(kHighThreads) k_ins_rounds(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
+                                                             ChainArgs A, int *high, const int *__restrict__ high2,
+                                                             int it, int iters, bool rounds, const unsigned *err) {
+  __shared__ int h[2][kHighCap];
+  __shared__ int s_n;
+  const int s = blockIdx.x, tid = threadIdx.x;
+  if (s >= nsys || *err || walled(scs[s])) return;
+  const SysConst &sc = scs[s];
+  SysDyn &d = dyn[s];
+  int n = d.ins_high;
+  int m = d.ins_high2;
+  const bool gave_up = *(volatile int *)&d.ins_fallback || iters == 0, conv = d.ins_conv;
+  __syncthreads();
+  if (conv) return;
+  if (gave_up || m > kHighCap || (n == 0 && m == 0)) {
+    if (tid == 0) {
+      if (!gave_up) d.diag[6] = it;
+      if (gave_up || m) {
+        d.ins_fallback = 1;
+        d.ins_high = 0;
+      } else {
+        d.ins_conv = 1;
+      }
+    }
+    return;
   }
-  d.ins_mismatch = 0;
+  for (int i = tid; i < n; i += kHighThreads) h[0][i] = high[sc.base + i];
+  for (int i = tid; i < m; i += kHighThreads) h[1][i] = high2[sc.base + i];
+  __syncthreads();
+  const int c0 = A.pos_c[sc.base], c1 = A.pos_c[sc.base + sc.cap + 1];
+  int cur = 0;
+  bool done = false;
+  for (;;) {
+    const int *hc = h[cur];
+    int *hn = h[cur ^ 1];
+    sort_block(hn, m);
+    bool differ = m != n;
+    for (int i = tid; i < min(m, n); i += kHighThreads) differ |= hc[i] != hn[i];
+    done = __syncthreads_or(differ) == 0;
+    if (done || it >= iters) break;
+    cur ^= 1;
+    n = m;
+    if (!rounds) break;
+    ++it;
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    for (int t = c0 + tid; t < c1; t += kHighThreads) {
+      const int k = A.list_c[t];
+      if (A.dec[k] & 8) continue;
+      ins_chain_walk(
+          A, sc, d, k, [&](int g) { return rank_in(h[cur], n, g); },
+          [&](int e) {
+            const int i = atomicAdd(&s_n, 1);
+            if (i < kHighCap) h[cur ^ 1][i] = e;
+          });
+    }
+    __syncthreads();
+    m = s_n;
+    if (m > kHighCap || *(volatile int *)&d.ins_fallback) {
+      it = iters;
+      break;
+    }
+  }
+  __syncthreads();
+  const bool open = !done && it < iters;
+  if (done || open)
+    for (int i = tid; i < n; i += kHighThreads) high[sc.base + i] = h[cur][i];
+  if (tid == 0) {
+    d.diag[6] = it;
+    d.ins_high = done || open ? n : 0;
+    d.ins_high2 = 0;
+    if (done) d.ins_conv = 1;
+    else if (!open) d.ins_fallback = 1;
+  }
 }
 
 // Apply every insertion (links, new point state) and log the events in sweep order: one
 // thread per original insertion, following its sub-chain.
 __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, State S,
                             const int *__restrict__ pos_c, const int *__restrict__ list_c,
-                            const int *__restrict__ pos_h, const int *__restrict__ fh,
-                            const int *__restrict__ newslot, const int *__restrict__ segnx,
+                            const int *__restrict__ high, const int *__restrict__ newslot, const int *__restrict__ segnx,
                             const double *__restrict__ xnew, const double *__restrict__ unew,
                             const double *__restrict__ dn_new, const int *__restrict__ nev_total, DevEvent *ev,
                             int *ev_count, int ev_cap, unsigned *err) {
@@ -755,7 +982,8 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
   if (dyn[s].ins_fallback) return;
   const SysConst &sc = scs[s];
   const long long T = S.T;
-  const int ev0 = pos_c[sc.base], h0 = pos_h[sc.base];
+  const int ev0 = pos_c[sc.base], nh = dyn[s].ins_high;
+  const int *hs = high + sc.base;
   const int seq0 = dyn[s].event_seq, itime = dyn[s].itime;
   const int nx = segnx[k];
   const double zero[3] = {0, 0, 0};
@@ -780,11 +1008,11 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
     S.prv[q] = g;
     S.nxt[g] = q;
     if (dn_new[g] >= 0.) S.seglen[q] = dn_new[g];
-    const int seq = seq0 + (pos_c[g] - ev0) + (pos_h[g] - h0);
+    const int seq = seq0 + (pos_c[g] - ev0) + rank_in(hs, nh, g);
     const int a = atomicAdd(ev_count, 1);
     if (a < ev_cap) ev[a] = DevEvent{s, seq, itime, NV_EV_INSERT, g, q};
     atomicAdd(&dyn[s].ev_hash, event_digest(seq, itime, NV_EV_INSERT, g - sc.base, q - sc.base));
-    if (fh[q]) {  // the sweep reaches q and it inserts
+    if (nh && holds(hs, nh, q)) {  // the sweep reaches q and it inserts
       g = q;
       continue;
     }
@@ -794,18 +1022,40 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
   }
 }
 
-// Ghosts of every slot an insertion touched, from the final links and positions (each
-// touched slot's last refresh in the serial sweep sees exactly this state).
-__global__ void k_ins_ghosts(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
-                             const int *__restrict__ sys_of, State S, const int *__restrict__ list_c,
-                             const int *__restrict__ fh, const int *__restrict__ newslot,
+// Ghosts of every slot an insertion touched, from the final links and positions (each touched
+// slot's last refresh in the serial sweep sees exactly this state); and the systems' counters:
+// pcount grows by the insertions beyond the free slots.
+__global__ void k_ins_ghosts(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, State S,
+                             int nsys, const int *__restrict__ pos_a, const int *__restrict__ pos_b,
+                             const int *__restrict__ pos_c, const int *__restrict__ list_c,
+                             const int *__restrict__ high, const int *__restrict__ newslot,
                              const int *__restrict__ nev_total, unsigned *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *nev_total || *err) return;
+  if (*err) return;
+  if (t < nsys && !walled(scs[t])) {
+    const SysConst &sc = scs[t];
+    SysDyn &d = dyn[t];
+    const int end = sc.base + sc.cap + 1;
+    const int nev = pos_c[end] - pos_c[sc.base] + d.ins_high, nfree = pos_b[end] - pos_b[sc.base];
+    d.diag[0] = pos_a[end] - pos_a[sc.base];
+    d.diag[1] = nev;
+    d.diag[5] = d.ins_high;
+    if (d.nlive == 0) {
+      atomicOr(err, DERR_EMPTY);
+    } else if (!d.ins_fallback) {
+      d.event_seq += nev;
+      d.insert_count += nev;
+      d.nlive += nev;
+      if (nev > nfree) d.pcount += nev - nfree;
+    }
+  }
+  if (t >= *nev_total) return;
   const int k = list_c[t];
   const int s = sys_of[k];
   if (dyn[s].ins_fallback) return;
   const SysConst &sc = scs[s];
+  const int nh = dyn[s].ins_high;
+  const int *hs = high + sc.base;
   refresh_ghosts(sc, S, k);
   int q = newslot[k];
   for (int hops = 0;; ++hops) {
@@ -814,37 +1064,10 @@ __global__ void k_ins_ghosts(const SysConst *__restrict__ scs, const SysDyn *__r
       return;
     }
     refresh_ghosts(sc, S, q);
-    if (!fh[q]) break;
+    if (!(nh && holds(hs, nh, q))) break;
     q = newslot[q];
   }
   refresh_ghosts(sc, S, S.nxt[q]);
-}
-
-// Counters: pcount grows by the insertions beyond the free slots.
-__global__ void k_ins_finish(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys, const int *__restrict__ pos_a,
-                             const int *__restrict__ pos_c, const int *__restrict__ pos_h,
-                             const int *__restrict__ pos_b, unsigned *err) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys || *err) return;
-  const SysConst &sc = scs[s];
-  if (walled(sc)) return;
-  SysDyn &d = dyn[s];
-  if (d.live == 0) {
-    atomicOr(err, DERR_EMPTY);
-    return;
-  }
-  const int end = sc.base + sc.cap + 1;
-  d.diag[0] = pos_a[end] - pos_a[sc.base];
-  const int nhigh = pos_h[end] - pos_h[sc.base];
-  const int nev = pos_c[end] - pos_c[sc.base] + nhigh;
-  d.diag[1] = nev;
-  d.diag[5] = nhigh;
-  if (d.ins_fallback) return;
-  const int nfree = pos_b[end] - pos_b[sc.base];
-  d.event_seq += nev;
-  d.insert_count += nev;
-  d.nlive += nev;
-  if (nev > nfree) d.pcount += nev - nfree;
 }
 
 
@@ -1806,23 +2029,11 @@ State make_state(nv_handle *h) {
                h->topo->seglen};
 }
 
-void compact(nv_handle *h, int *flag, int *pos, int *list) {
+Lists<1> list_a(nv_handle *h) {
   TopoBuffers *tb = h->topo;
-  size_t bytes = tb->cub_bytes;
-  cub::DeviceScan::ExclusiveSum(tb->cub_tmp, bytes, flag, pos, (int)(h->T + 1), h->stream);
-  k_scatter<<<grid_for(h->T, TB), TB, 0, h->stream>>>(flag, pos, list, h->T);
+  return Lists<1>{{tb->pos_a}, {tb->list_a}, tb->pass_state, tb->pass_ctl};
 }
-
-
-// Sweep bitmaps from a flag array.
-Sweep make_sweep(nv_handle *h, const int *flag) {
-  TopoBuffers *tb = h->topo;
-  const long long T = h->T;
-  const long long nw0 = T / 32 + 1;
-  k_bits_l0<<<grid_for(nw0, 256), 256, 0, h->stream>>>(flag, tb->l0, T);
-  k_bits_l1<<<grid_for(nw0 / 32 + 1, 256), 256, 0, h->stream>>>(tb->l0, tb->l1, nw0);
-  return Sweep{tb->l0, tb->l1, T};
-}
+int pass_grid(const nv_handle *h) { return (int)((h->T + kPassSlots) / kPassSlots); }
 
 }  // namespace
 
@@ -1832,10 +2043,8 @@ void topo_alloc(nv_handle *h) {
   cudaMalloc(&tb->flag_a, n * sizeof(int));
   cudaMalloc(&tb->pos_a, n * sizeof(int));
   cudaMalloc(&tb->list_a, n * sizeof(int));
-  cudaMalloc(&tb->flag_b, n * sizeof(int));
   cudaMalloc(&tb->pos_b, n * sizeof(int));
   cudaMalloc(&tb->list_b, n * sizeof(int));
-  cudaMalloc(&tb->flag_c, n * sizeof(int));
   cudaMalloc(&tb->pos_c, n * sizeof(int));
   cudaMalloc(&tb->list_c, n * sizeof(int));
   cudaMalloc(&tb->dec, n * sizeof(int));
@@ -1843,13 +2052,15 @@ void topo_alloc(nv_handle *h) {
   cudaMalloc(&tb->xnew, 3 * n * sizeof(double));
   cudaMalloc(&tb->unew, 3 * n * sizeof(double));
   cudaMalloc(&tb->segnx, n * sizeof(int));
-  cudaMalloc(&tb->fh[0], n * sizeof(int));
-  cudaMalloc(&tb->fh[1], n * sizeof(int));
-  cudaMalloc(&tb->pos_h, n * sizeof(int));
+  cudaMalloc(&tb->high, n * sizeof(int));
+  cudaMalloc(&tb->high2, n * sizeof(int));
+  const size_t pass_words = 3 * ((n + kPassSlots) / kPassSlots);
+  cudaMalloc(&tb->pass_state, pass_words * sizeof(unsigned long long));
+  cudaMemset(tb->pass_state, 0, pass_words * sizeof(unsigned long long));
+  cudaMalloc(&tb->pass_ctl, 3 * sizeof(unsigned));
+  cudaMemset(tb->pass_ctl, 0, 3 * sizeof(unsigned));
   cudaMalloc(&tb->l0, (n / 32 + 2) * sizeof(unsigned));
   cudaMalloc(&tb->l1, (n / 1024 + 2) * sizeof(unsigned));
-  cudaMalloc(&tb->len_st, n * sizeof(double));
-  cudaMalloc(&tb->len_fr, n * sizeof(double));
   cudaMalloc(&tb->seglen, n * sizeof(double));
   cudaMalloc(&tb->dn_new, n * sizeof(double));
   cudaMemset(tb->seglen, 0, n * sizeof(double));
@@ -1859,11 +2070,14 @@ void topo_alloc(nv_handle *h) {
     tb->total_parts = std::min(64, (maxcap + 16383) / 16384);
     cudaMalloc(&tb->psum, (size_t)h->nsys * tb->total_parts * sizeof(double));
     cudaMalloc(&tb->pnear, (size_t)h->nsys * tb->total_parts * sizeof(double));
+    cudaMalloc(&tb->part_done, h->nsys * sizeof(int));
+    cudaMemset(tb->part_done, 0, h->nsys * sizeof(int));
   }
   // cell grids of the systems without a tree: about two slots per cell at full capacity,
   // cells at least as wide as delta/2 and at most 256 per axis
   std::vector<CellGrid> grids(h->nsys);
   long long cells = 0;
+  int most = 0;  // slots of the largest system without a tree
   for (int s = 0; s < h->nsys; ++s) {
     CellGrid &G = grids[s];
     std::memset(&G, 0, sizeof G);
@@ -1881,9 +2095,11 @@ void topo_alloc(nv_handle *h) {
     G.base = cells;
     cells += (long long)G.nc[0] * G.nc[1] * G.nc[2];
   }
+  for (int s = 0; s < h->nsys; ++s)
+    if (!h->sc[s].use_tree) most = std::max(most, h->cap[s]);
+  tb->small_pclose = most <= kPcloseSlots;
   tb->n_cells = cells;
   tb->any_cells = cells > 0 && cells < (1LL << 30);
-  size_t scan_n = n;
   if (tb->any_cells) {
     cudaMalloc(&tb->grid, h->nsys * sizeof(CellGrid));
     cudaMemcpy(tb->grid, grids.data(), h->nsys * sizeof(CellGrid), cudaMemcpyHostToDevice);
@@ -1891,10 +2107,9 @@ void topo_alloc(nv_handle *h) {
     cudaMalloc(&tb->cell_cnt, (cells + 1) * sizeof(int));
     cudaMalloc(&tb->cell_start, (cells + 1) * sizeof(int));
     cudaMalloc(&tb->cell_items, n * sizeof(int));
-    scan_n = std::max(scan_n, (size_t)cells + 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, tb->cub_bytes, tb->cell_cnt, tb->cell_start, (int)(cells + 1));
+    cudaMalloc(&tb->cub_tmp, std::max<size_t>(tb->cub_bytes, 16));
   }
-  cub::DeviceScan::ExclusiveSum(nullptr, tb->cub_bytes, tb->flag_a, tb->pos_a, (int)scan_n);
-  cudaMalloc(&tb->cub_tmp, std::max<size_t>(tb->cub_bytes, 16));
   h->topo = tb;
 }
 
@@ -1902,13 +2117,14 @@ void topo_free(nv_handle *h) {
   TopoBuffers *tb = h->topo;
   if (!tb) return;
   cudaFree(tb->flag_a); cudaFree(tb->pos_a); cudaFree(tb->list_a);
-  cudaFree(tb->flag_b); cudaFree(tb->pos_b); cudaFree(tb->list_b);
-  cudaFree(tb->flag_c); cudaFree(tb->pos_c); cudaFree(tb->list_c);
+  cudaFree(tb->pos_b); cudaFree(tb->list_b);
+  cudaFree(tb->pos_c); cudaFree(tb->list_c);
+  cudaFree(tb->pass_state); cudaFree(tb->pass_ctl);
   cudaFree(tb->dec); cudaFree(tb->newslot); cudaFree(tb->xnew);
-  cudaFree(tb->unew); cudaFree(tb->segnx); cudaFree(tb->fh[0]); cudaFree(tb->fh[1]); cudaFree(tb->pos_h);
+  cudaFree(tb->unew); cudaFree(tb->segnx); cudaFree(tb->high); cudaFree(tb->high2);
   cudaFree(tb->l0); cudaFree(tb->l1);
-  cudaFree(tb->len_st); cudaFree(tb->len_fr); cudaFree(tb->seglen); cudaFree(tb->dn_new);
-  cudaFree(tb->psum); cudaFree(tb->pnear);
+  cudaFree(tb->seglen); cudaFree(tb->dn_new);
+  cudaFree(tb->psum); cudaFree(tb->pnear); cudaFree(tb->part_done);
   cudaFree(tb->grid); cudaFree(tb->cell_of); cudaFree(tb->cell_cnt); cudaFree(tb->cell_start);
   cudaFree(tb->cell_items);
   cudaFree(tb->cub_tmp);
@@ -1920,66 +2136,38 @@ void launch_pinsert(nv_handle *h) {
   ++h->links_epoch;
   TopoBuffers *tb = h->topo;
   const long long T = h->T;
-  k_ins_begin<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(h->d_dyn, h->nsys);
-  k_ins_mark<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->gi, h->nxt,
-                                                         tb->flag_a, tb->flag_b, tb->dec, tb->len_st, tb->len_fr, T,
-                                                         h->d_err);
-  compact(h, tb->flag_a, tb->pos_a, tb->list_a);  // candidates (either test passes)
-  compact(h, tb->flag_b, tb->pos_b, tb->list_b);  // free slots
-  k_zero_flags<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(tb->flag_c, T);
-  const int *ncand = tb->pos_a + T;
-  k_ins_decide_easy<<<grid_for(T, 128), 128, 0, h->stream>>>(tb->list_a, ncand, tb->dec, tb->flag_c, h->d_err);
-  compact(h, tb->flag_c, tb->pos_c, tb->list_c);  // ambiguous slots
-  k_ins_decide_amb<<<grid_for(T, 128), 128, 0, h->stream>>>(tb->list_c, tb->pos_c + T, h->nxt, h->prv, tb->flag_c,
-                                                            tb->dec, h->d_err);
-  k_zero_flags<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(tb->flag_c, T);
-  k_ins_decide_case<<<grid_for(T, 128), 128, 0, h->stream>>>(tb->list_a, ncand, h->prv, tb->dec, tb->flag_c,
-                                                             h->d_err);
-  compact(h, tb->flag_c, tb->pos_c, tb->list_c);  // insertions, in sweep order
-  k_ins_len<<<grid_for(T, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->nxt, h->prv, tb->dec, tb->len_st,
-                                                   tb->len_fr, tb->seglen, T);
+  const Lists<3> lists{{tb->pos_a, tb->pos_b, tb->pos_c}, {tb->list_a, tb->list_b, tb->list_c}, tb->pass_state,
+                       tb->pass_ctl};
+  k_ins_mark<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->gi, h->nxt, h->prv,
+                                                           tb->dec, tb->seglen, lists, tb->l0, tb->l1, T, h->d_err);
   const State S = make_state(h);
+  const ChainArgs A{S,          tb->pos_c, tb->list_c, tb->pos_b, tb->list_b, tb->dec,
+                    tb->newslot, tb->segnx, tb->xnew,  tb->unew,  tb->dn_new};
   // the number of insertions (pos_c[T]) is known only on the device: launch over every
   // slot, threads beyond the count return at once
   const int grid = grid_for(T, 128);
   const int *nev = tb->pos_c + T;
-  const int iters = h->ins_iters;
-  k_zero_flags<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(tb->fh[0], T);
-  if (iters == 0) {
-    k_ins_all_serial<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(h->d_dyn, h->nsys);
-    size_t bytes = tb->cub_bytes;
-    cub::DeviceScan::ExclusiveSum(tb->cub_tmp, bytes, tb->fh[0], tb->pos_h, (int)(T + 1), h->stream);
+  const bool large = T > kAgainSlots;
+  for (int it = 1; it <= (large ? h->ins_iters : std::min(h->ins_iters, 1)); ++it) {
+    k_ins_chain<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, A, tb->high, tb->high2, nev, h->d_err);
+    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, tb->high, tb->high2, it,
+                                                          h->ins_iters, !large, h->d_err);
   }
-  for (int it = 0; it < iters; ++it) {
-    int *fin = tb->fh[it & 1], *fout = tb->fh[(it + 1) & 1];
-    k_ins_zero_open<<<grid_for(T, TB), TB, 0, h->stream>>>(h->d_dyn, h->sys_of, fout, T);
-    size_t bytes = tb->cub_bytes;
-    cub::DeviceScan::ExclusiveSum(tb->cub_tmp, bytes, fin, tb->pos_h, (int)(T + 1), h->stream);
-    k_ins_chain<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->pos_c, tb->list_c, tb->pos_b,
-                                             tb->list_b, tb->dec, tb->pos_h, fout, tb->newslot, tb->segnx, tb->xnew,
-                                             tb->unew, tb->dn_new, nev, h->d_err);
-    k_ins_compare<<<grid_for(T, TB), TB, 0, h->stream>>>(h->d_dyn, h->sys_of, fin, fout, T);
-    k_ins_converge<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(h->d_dyn, h->nsys, it + 1, it + 1 == iters);
-  }
-  const int *fh = tb->fh[iters > 0 ? (iters - 1) & 1 : 0];  // pos_h is its prefix sum
-  k_ins_apply<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->pos_c, tb->list_c, tb->pos_h, fh,
+  if (h->ins_iters == 0)
+    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, tb->high, tb->high2, 0, 0, false,
+                                                          h->d_err);
+  k_ins_apply<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->pos_c, tb->list_c, tb->high,
                                            tb->newslot, tb->segnx, tb->xnew, tb->unew, tb->dn_new, nev, h->d_events,
                                            h->d_event_count, h->event_cap, h->d_err);
-  k_ins_ghosts<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->list_c, fh, tb->newslot, nev,
-                                            h->d_err);
-  k_ins_finish<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, tb->pos_a, tb->pos_c,
-                                                              tb->pos_h, tb->pos_b, h->d_err);
-  // systems with an insertion the parallel form cannot place: the sweep (extra visits start
-  // empty: bitmaps from an all-zero flag array; flag_b is free once the free slots are listed)
-  k_zero_flags<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(tb->flag_b, T);
-  const Sweep sw = make_sweep(h, tb->flag_b);
+  k_ins_ghosts<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, h->nsys, tb->pos_a, tb->pos_b, tb->pos_c,
+                                            tb->list_c, tb->high, tb->newslot, nev, h->d_err);
+  // systems with an insertion the parallel form cannot place
   k_insert_sweep<<<h->nsys, 32, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, S, tb->pos_a, tb->list_a, tb->pos_b,
-                                                tb->list_b, sw, h->d_err, h->d_events, h->d_event_count,
-                                                h->event_cap);
-  k_ins_part<<<h->nsys * tb->total_parts, kTotalThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, tb->total_parts,
-                                                                         tb->seglen, tb->psum, tb->pnear, h->d_err);
-  k_ins_total<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, tb->total_parts, tb->psum,
-                                                             tb->pnear, h->d_err);
+                                                tb->list_b, Sweep{tb->l0, tb->l1, T}, h->d_err, h->d_events,
+                                                h->d_event_count, h->event_cap);
+  k_ins_total<<<h->nsys * tb->total_parts, kTotalThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, tb->total_parts,
+                                                                          tb->seglen, tb->psum, tb->pnear,
+                                                                          tb->part_done, h->d_err);
   launch_solid_pinsert(h);
 }
 
@@ -1990,6 +2178,9 @@ void launch_pclose(nv_handle *h, bool only_brute) {
   if (any_brute && (h->pclose_method == 1 || !tb->any_cells)) {
     k_pclose_brute<<<grid_for(h->T, 128), 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, h->prv,
                                                                h->closest, h->closestd, h->T, h->d_err);
+  } else if (any_brute && tb->small_pclose) {
+    k_pclose_warps<<<grid_for(h->T, kPcloseWarps), 32 * kPcloseWarps, 0, h->stream>>>(
+        h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, h->prv, h->closest, h->closestd, h->T, h->d_err);
   } else if (any_brute) {
     const long long T = h->T;
     cudaMemsetAsync(tb->cell_cnt, 0, (tb->n_cells + 1) * sizeof(int), h->stream);
@@ -2009,9 +2200,8 @@ void launch_pclose(nv_handle *h, bool only_brute) {
 void launch_precon(nv_handle *h) {
   ++h->links_epoch;
   TopoBuffers *tb = h->topo;
-  k_mark_recon<<<grid_for(h->T + 1, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->closestd, h->nxt,
-                                                              tb->flag_a, h->T, h->d_err);
-  compact(h, tb->flag_a, tb->pos_a, tb->list_a);
+  k_mark_recon<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->closestd, h->nxt, list_a(h),
+                                                             h->T, h->d_err);
   k_recon_sweep<<<h->nsys, kReconRound, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, make_state(h), tb->pos_a, tb->list_a,
                                                h->d_err, h->d_events, h->d_event_count, h->event_cap);
   launch_solid_precon(h);
@@ -2020,12 +2210,9 @@ void launch_precon(nv_handle *h) {
 void launch_premove(nv_handle *h) {
   ++h->links_epoch;
   TopoBuffers *tb = h->topo;
-  k_mark_remove<<<grid_for(h->T + 1, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt,
-                                                               tb->flag_a, h->T, h->d_err);
-  compact(h, tb->flag_a, tb->pos_a, tb->list_a);
-  // extra visits start empty: bitmaps from an all-zero flag array
-  k_zero_flags<<<grid_for(h->T + 1, TB), TB, 0, h->stream>>>(tb->flag_b, h->T);
-  const Sweep sw = make_sweep(h, tb->flag_b);
+  k_mark_remove<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, tb->flag_a,
+                                                              list_a(h), tb->l0, tb->l1, h->T, h->d_err);
+  const Sweep sw{tb->l0, tb->l1, h->T};
   k_remove_sweep<<<h->nsys, kRound, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, make_state(h), tb->pos_a, tb->list_a,
                                                 tb->flag_a, sw, h->d_err, h->d_events, h->d_event_count,
                                                 h->event_cap);

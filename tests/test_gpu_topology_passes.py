@@ -1,0 +1,68 @@
+"""Edges of the topology stages' kernels: the ordered one-pass lists (blocks of 1,024 slots, warps
+of 128) at slot counts around whole blocks, pinsert's rounds over the whole GPU (handles above
+262,144 slots) and by a block per system, with too few rounds allowed, and the closest-point
+search by a warp per target and by the cell list on either side of the line between them.
+Everything equal to the oracle's, event for event."""
+import numpy as np
+import pytest
+
+from helpers import config0_params, tangle
+from oracle import Oracle
+from test_gpu_topology import _assert_same, _moved_state, _ring_slots, _run_stage
+
+pytestmark = pytest.mark.gpu
+
+
+def _holed(st, rings):
+    for r in rings:
+        idx = np.asarray(r) - 1
+        for name in ("x", "u", "u1", "u2", "ghosti", "ghostb", "infront", "behind"):
+            getattr(st, name)[idx] = 0
+    return st
+
+
+@pytest.mark.parametrize("slots", [1021, 1022, 1023, 1024, 1151, 2046, 2048])
+def test_lists_around_whole_blocks(slots):
+    # the handle's slots are the capacity and a dummy; live points up to the last slot but 40
+    from nuvort_b200.api import Handle
+    st = tangle(slots, 0.002, n_points=slots - 60)
+    p = config0_params()
+    o = Oracle(p, st)
+    o.step(12)
+    with Handle(p, [slots], states=[st]) as h:
+        h.step(12)
+        assert h.events() == o.events()
+        a, b = h.download(), o.download()
+        assert np.array_equal(a.infront, b.infront) and np.array_equal(a.closest, b.closest)
+
+
+@pytest.mark.parametrize("iters", [1, 2, 6])
+@pytest.mark.parametrize("extra", [16384, 270000])
+def test_pinsert_rounds(iters, extra):
+    st = tangle(31, 0.002, n_rings=12)
+    mv = _moved_state(config0_params(), _holed(st, _ring_slots(st)[2::3]))
+    p_ins = config0_params(delta=0.0009, overide_timestep_check=True)
+    diag = []
+    a, b, ea, eb, ca, cb = _run_stage(p_ins, mv, ["pinsert"], cap_extra=extra, insert_iterations=iters, diag=diag)
+    assert ea == eb and len(eb) > 200
+    _assert_same(a, b)
+    assert ca.insert_count == cb.insert_count and ca.pcount == cb.pcount
+    if iters != 2:  # one round: new points insert again, so the serial sweep takes over
+        assert diag[2] == (1 if iters == 1 else 0)
+
+
+@pytest.mark.parametrize("cap", [6144, 6145])
+def test_closest_points_either_side_of_the_line(cap):
+    from nuvort_b200.api import Handle
+    st = tangle(9, 0.002, n_points=1301)
+    st.x[700] = st.x[17]  # two points in one place: ties, lowest slot first
+    o = Oracle(config0_params(), st, t=0.0, itime=1)
+    o.stage("pclose")
+    b = o.download()
+    for method in (0, 1):
+        with Handle(config0_params(), [cap], states=[st]) as h:
+            h.set_pclose_method(method)
+            h.set_clock(0, 0.0, 1)
+            h.stage("pclose")
+            a = h.download()
+        assert np.array_equal(a.closest, b.closest) and np.array_equal(a.closestd, b.closestd)
