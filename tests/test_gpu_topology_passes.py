@@ -1,5 +1,5 @@
 """Edges of the topology stages' kernels: the ordered one-pass lists (blocks of 1,024 slots, warps
-of 128) at slot counts around whole blocks, pinsert's rounds over the whole GPU (handles above
+of 128) at slot counts around whole blocks, the wall sweeps' chunks of 256 slots, pinsert's rounds over the whole GPU (handles above
 262,144 slots) and by a block per system, with too few rounds allowed, and the closest-point
 search by a warp per target and by the cell list on either side of the line between them.
 Everything equal to the oracle's, event for event."""
@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from helpers import config0_params, tangle
+from nuvort_b200.rings import half_loop
 from oracle import Oracle
 from test_gpu_topology import _assert_same, _moved_state, _ring_slots, _run_stage
 
@@ -66,3 +67,22 @@ def test_closest_points_either_side_of_the_line(cap):
             h.stage("pclose")
             a = h.download()
         assert np.array_equal(a.closest, b.closest) and np.array_equal(a.closestd, b.closestd)
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 300])
+@pytest.mark.parametrize("delta", [0.0003, 0.0008])
+def test_wall_sweeps_around_whole_chunks(n, delta):
+    # segments of 0.75 * 0.0005: at delta 0.0003 every one inserts, at 0.0008 points are removed
+    from nuvort_b200.api import Handle
+    st = half_loop(n, 0.0005)
+    p = config0_params(dt=2e-7, delta=delta, boundary_x="solid", boundary_y="periodic", boundary_z="periodic")
+    o = Oracle(p, st)
+    o.step(4)
+    with Handle(p, [1200], states=[st]) as h:
+        h.step(4)
+        assert len(o.events()) > 50
+        assert h.events() == o.events()
+        a, b = h.download(), o.download()
+        for f in ("infront", "behind", "pinnedi", "pinnedb", "wpinned"):
+            assert np.array_equal(getattr(a, f), getattr(b, f)), f
+        assert np.max(np.abs(a.x - b.x)) < 1e-12
