@@ -22,6 +22,7 @@
 #include <cub/cub.cuh>
 
 #include "handle.cuh"
+#include "lists.cuh"
 
 struct TopoBuffers {
   int *flag_a = nullptr, *pos_a = nullptr, *list_a = nullptr;
@@ -121,121 +122,6 @@ __device__ __forceinline__ void clear_bits(unsigned *l0, unsigned *l1, long long
   }
 }
 
-// ---- ordered lists in one pass ---------------------------------------------------------------
-// flags(g), for 0 <= g <= n in ascending order over the grid, gives K bits per slot; list[k]
-// receives the slots with bit k in ascending order and pos[k][g] the number of such slots below
-// g.  A block takes 1,024 consecutive slots (a ticket, so that the blocks before it have
-// started), counts its bits, and finds the blocks' sum before it by looking back: every block
-// publishes its own sum and, once known, its inclusive sum, each in one 64-bit word with the
-// launch's epoch, so that nothing is cleared between launches (the last block to finish sets up
-// the next).  One launch for what a flag kernel, a two-kernel scan and a scatter did in four
-// (per list): of the 158 launches of a tree system's step, 28 compactions' worth.
-constexpr int kPassThreads = 256, kPassItems = 4, kPassSlots = kPassThreads * kPassItems;
-constexpr int kPassPolls = 1 << 22;  // polls of a predecessor before giving up
-
-template <int K>
-struct Lists {
-  int *pos[K], *list[K];
-  unsigned long long *state;  // [K][blocks]
-  unsigned *ctl;              // ticket, finished blocks, epoch
-};
-
-template <int K, class F>
-__device__ void ordered_pass(const Lists<K> &L, long long n, unsigned *err, F flags) {
-  constexpr int kWarps = kPassThreads / 32;
-  static_assert(K <= kWarps, "a warp looks back for each list");
-  __shared__ int s_block, s_sum[K][kWarps], s_base[K];
-  __shared__ unsigned s_epoch;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) {
-    s_epoch = *(volatile unsigned *)&L.ctl[2];
-    s_block = (int)atomicAdd(&L.ctl[0], 1u);
-  }
-  __syncthreads();
-  const int b = s_block, nb = gridDim.x;
-  const unsigned epoch = s_epoch;
-  const long long g0 = (long long)b * kPassSlots + wid * (32 * kPassItems) + lane;
-  unsigned m[K][kPassItems];
-#pragma unroll
-  for (int it = 0; it < kPassItems; ++it) {
-    const long long g = g0 + 32 * it;
-    const unsigned f = g <= n ? flags(g) : 0u;
-#pragma unroll
-    for (int k = 0; k < K; ++k) m[k][it] = __ballot_sync(0xffffffffu, (f >> k) & 1u);
-  }
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      int v = 0;
-#pragma unroll
-      for (int it = 0; it < kPassItems; ++it) v += __popc(m[k][it]);
-      s_sum[k][wid] = v;
-    }
-  __syncthreads();
-  if (wid < K) {  // warp k: the sum of list k's bits before this block
-    volatile unsigned long long *st = L.state + (long long)wid * nb;
-    auto word = [&](unsigned flag, int v) {
-      return (unsigned long long)((epoch << 2) | flag) << 32 | (unsigned long long)(unsigned)v;
-    };
-    int own = 0;
-    for (int w = 0; w < kWarps; ++w) own += s_sum[wid][w];
-    if (lane == 0) st[b] = word(b == 0 ? 2u : 1u, own);
-    int before = 0;
-    bool ok = true;
-    for (int j = b - 1; j >= 0 && ok; j -= 32) {
-      const int q = j - lane;
-      unsigned long long v = word(2u, 0);  // before the first block: an inclusive sum of 0
-      int polls = 0;
-      for (;;) {
-        if (q >= 0) v = st[q];
-        const unsigned tag = (unsigned)(v >> 32);
-        const bool ready = (tag >> 2) == (epoch & 0x3fffffffu) && (tag & 3u);
-        if (__all_sync(0xffffffffu, ready)) break;
-        if (++polls > kPassPolls) {
-          ok = false;
-          break;
-        }
-      }
-      const unsigned incl = __ballot_sync(0xffffffffu, ((unsigned)(v >> 32) & 3u) == 2u);
-      const int stop = incl ? __ffs(incl) - 1 : 31;
-      int x = lane <= stop ? (int)(unsigned)v : 0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      before += x;
-      if (incl) break;
-    }
-    if (lane == 0) {
-      if (!ok) {
-        atomicOr(err, DERR_TIMEOUT);
-        before = 0;
-      }
-      if (b > 0) st[b] = word(2u, before + own);
-      s_base[wid] = before;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    int off = s_base[k];
-    for (int w = 0; w < wid; ++w) off += s_sum[k][w];
-#pragma unroll
-    for (int it = 0; it < kPassItems; ++it) {
-      const long long g = g0 + 32 * it;
-      const int p = off + __popc(m[k][it] & ((1u << lane) - 1u));
-      if (g <= n) {
-        L.pos[k][g] = p;
-        if ((m[k][it] >> lane) & 1u) L.list[k][p] = (int)g;
-      }
-      off += __popc(m[k][it]);
-    }
-  }
-  if (tid == 0 && atomicAdd(&L.ctl[1], 1u) == (unsigned)nb - 1) {  // every block has taken its ticket and epoch
-    L.ctl[0] = 0;
-    L.ctl[1] = 0;
-    L.ctl[2] = (epoch + 1) & 0x3fffffffu;
-  }
-}
-
 __device__ __forceinline__ bool recon_step(const SysConst &sc, const SysDyn &d) {
   return (d.itime % sc.recon_shots) == 0;
 }
@@ -281,7 +167,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mark_recon(const SysConst *__r
                                                             const int *__restrict__ nxt, Lists<1> L, long long T,
                                                             unsigned *err) {
   const bool run = !*(volatile unsigned *)err;
-  ordered_pass<1>(L, T, err, [&](long long g) -> unsigned {
+  ordered_lists(L, T, err, [&](long long g) -> unsigned {
     if (g >= T || !run) return 0u;
     const int s = sys_of[g];
     const SysConst &sc = scs[s];
@@ -300,7 +186,7 @@ __global__ void __launch_bounds__(kPassThreads) k_mark_remove(const SysConst *__
                                                              const int *__restrict__ nxt, int *fa, Lists<1> L,
                                                              unsigned *l0, unsigned *l1, long long T, unsigned *err) {
   const bool run = !*(volatile unsigned *)err;
-  ordered_pass<1>(L, T, err, [&](long long g) -> unsigned {
+  ordered_lists(L, T, err, [&](long long g) -> unsigned {
     clear_bits(l0, l1, g, T);  // extra visits of the sweep start empty
     unsigned a = 0;
     if (g < T && run) {
@@ -603,7 +489,7 @@ __global__ void __launch_bounds__(kPassThreads) k_ins_mark(const SysConst *__res
                                                           int *dec, double *seglen, Lists<3> L, unsigned *l0,
                                                           unsigned *l1, long long T, unsigned *err) {
   const bool run = !*(volatile unsigned *)err;
-  ordered_pass<3>(L, T, err, [&](long long gl) -> unsigned {
+  ordered_lists(L, T, err, [&](long long gl) -> unsigned {
     clear_bits(l0, l1, gl, T);  // extra visits of the serial sweep start empty
     if (gl >= T) return 0u;
     const int g = (int)gl, s = sys_of[g];
@@ -2031,9 +1917,9 @@ State make_state(nv_handle *h) {
 
 Lists<1> list_a(nv_handle *h) {
   TopoBuffers *tb = h->topo;
-  return Lists<1>{{tb->pos_a}, {tb->list_a}, tb->pass_state, tb->pass_ctl};
+  return Lists<1>{{tb->pos_a}, {tb->list_a}, {tb->pass_state, tb->pass_ctl}};
 }
-int pass_grid(const nv_handle *h) { return (int)((h->T + kPassSlots) / kPassSlots); }
+int pass_grid(const nv_handle *h) { return pass_blocks(h->T); }
 
 }  // namespace
 
@@ -2054,11 +1940,7 @@ void topo_alloc(nv_handle *h) {
   cudaMalloc(&tb->segnx, n * sizeof(int));
   cudaMalloc(&tb->high, n * sizeof(int));
   cudaMalloc(&tb->high2, n * sizeof(int));
-  const size_t pass_words = 3 * ((n + kPassSlots) / kPassSlots);
-  cudaMalloc(&tb->pass_state, pass_words * sizeof(unsigned long long));
-  cudaMemset(tb->pass_state, 0, pass_words * sizeof(unsigned long long));
-  cudaMalloc(&tb->pass_ctl, 3 * sizeof(unsigned));
-  cudaMemset(tb->pass_ctl, 0, 3 * sizeof(unsigned));
+  pass_alloc(&tb->pass_state, &tb->pass_ctl, 3, h->T);
   cudaMalloc(&tb->l0, (n / 32 + 2) * sizeof(unsigned));
   cudaMalloc(&tb->l1, (n / 1024 + 2) * sizeof(unsigned));
   cudaMalloc(&tb->seglen, n * sizeof(double));
@@ -2136,8 +2018,8 @@ void launch_pinsert(nv_handle *h) {
   ++h->links_epoch;
   TopoBuffers *tb = h->topo;
   const long long T = h->T;
-  const Lists<3> lists{{tb->pos_a, tb->pos_b, tb->pos_c}, {tb->list_a, tb->list_b, tb->list_c}, tb->pass_state,
-                       tb->pass_ctl};
+  const Lists<3> lists{{tb->pos_a, tb->pos_b, tb->pos_c}, {tb->list_a, tb->list_b, tb->list_c},
+                       {tb->pass_state, tb->pass_ctl}};
   k_ins_mark<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->gi, h->nxt, h->prv,
                                                            tb->dec, tb->seglen, lists, tb->l0, tb->l1, T, h->d_err);
   const State S = make_state(h);

@@ -18,10 +18,13 @@
 // Walks: one thread per target point, stackless preorder over first_child/skip, with the
 // reference's opening test and arithmetic (tree_walk tree.f90:250-316, closest_tree
 // :206-244) in the same order, so the accumulated velocity is the reference's bit for bit.
+#include <cmath>
+
 #include <cub/cub.cuh>
 
 #include "fp64.cuh"
 #include "handle.cuh"
+#include "lists.cuh"
 #include "mixed.cuh"
 
 constexpr int kMaxLevels = NV_TREE_MAX_DEPTH;
@@ -52,14 +55,14 @@ struct TreeBuffers {
   // roots: a parallel estimate of the centre with a bound on its distance to the exact
   // (sequential) one, so the walks need not wait for the exact sum; (target, image) pairs
   // whose root test the bound cannot settle are listed and redone once the exact sum is in
-  // the roots' split as one stable radix sort of the live slots by (system, octant)
-  unsigned *rkey[2] = {nullptr, nullptr};
-  int *rval[2] = {nullptr, nullptr};
-  int *root_cnt = nullptr;  // per system: members per octant
-  int *root_mb = nullptr;   // per system: first member entry of the children
-  void *rsort_tmp = nullptr;
-  size_t rsort_bytes = 0;
-  int rkey_bits = 0;
+  // the roots' split by an ordered pass over the slots (k_root_lists)
+  unsigned char *rdig = nullptr;  // per slot: its octant, 8 for none
+  int *rrank = nullptr;           // per slot: its rank among its octant's slots
+  int *root_rank = nullptr;       // per system and list: the rank at its first slot
+  int *root_mb = nullptr;         // per system and octant: member entry of rank 0
+  int *root_ok = nullptr;         // per system: the children were made
+  unsigned long long *pass_state = nullptr;
+  unsigned *pass_ctl = nullptr;
   double4 *root_apx = nullptr;  // per system: centre estimate, bound
   double *root_part = nullptr;  // per system and part: partial sums of x, y, z, |x|, |y|, |z|
   int root_parts = 1;
@@ -70,10 +73,8 @@ struct TreeBuffers {
   int *split_blk[3] = {nullptr, nullptr, nullptr};  // nodes of a level split by a block, by level % 3
   int *split_wrp[3] = {nullptr, nullptr, nullptr};  // nodes of a level split by a warp
   int max_blk = 0, max_wrp = 0;
+  int grid_levels = kMaxLevels;  // levels below this one are split by the whole GPU
   int *ctr = nullptr;     // [0] n_nodes [1] n_members [2 + L] first node of level L
-  int *flag = nullptr, *pos = nullptr;
-  void *cub_tmp = nullptr;
-  size_t cub_bytes = 0;
   // walk order: each system's slots sorted along a Hilbert curve (live slots first)
   unsigned long long *okey[2] = {nullptr, nullptr};
   int *oval[2] = {nullptr, nullptr};
@@ -90,59 +91,6 @@ struct TreeBuffers {
 namespace {
 
 constexpr int TB = 256;
-
-__global__ void k_live_flags(const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn,
-                             const int *__restrict__ sys_of, const int *__restrict__ nxt, int *flag, long long T,
-                             int *ctr) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > T) return;
-  int f = 0;
-  if (g < T) {
-    const int s = sys_of[g];
-    const SysConst &sc = scs[s];
-    const int k = (int)(g - sc.base);
-    f = (sc.use_tree || sc.sched_tree) && k >= 1 && k <= dyn[s].pcount && nxt[g] != 0;
-  }
-  flag[g] = f;
-  if (g == 0)
-    for (int b = 0; b < 6; ++b) ctr[kCtrSplit + b] = 0;
-}
-
-__global__ void k_scatter_live(const int *__restrict__ flag, const int *__restrict__ pos, int *__restrict__ members,
-                               long long T) {
-  const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < T && flag[g]) members[pos[g]] = (int)g;
-}
-
-
-// Root of every system (construct_tree, tree.f90:38-59).
-__global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys, const int *__restrict__ nxt,
-                        const int *__restrict__ pos, TreeBuffers tb, long long T) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) {
-    tb.ctr[0] = nsys;
-    tb.ctr[2] = 0;
-    tb.ctr[3] = nsys;
-    tb.ctr[1] = pos[T];
-    tb.ctr[kCtrBig] = 0;
-  }
-  if (s >= nsys) return;
-  const SysConst &sc = scs[s];
-  const int pc = (sc.use_tree || sc.sched_tree) ? dyn[s].pcount : 0;
-  const double h = -sc.bsize / 2.0;
-  tb.nP[s] = make_double4(h, h, h, 0);
-  tb.nA[s] = make_double4(0, 0, 0, sc.bsize);
-  tb.nB[s] = make_double4(0, 0, 0, 0);
-  tb.nI[s] = make_int4(pc, kEnd, kEnd, pc >= 1 ? nxt[sc.base + 1] : 0);
-  tb.nR[s] = make_int2(pos[sc.base], pos[sc.base + sc.cap + 1] - pos[sc.base]);
-  tb.nDepth[s] = 0;
-  tb.nKids[s] = 0;
-  for (int d = 0; d < 8; ++d) tb.root_cnt[8 * s + d] = 0;
-  tb.nLeaf[s] = pc == 1 ? sc.base + 1 : 0;
-  dyn[s].tree_eval = 0;
-  dyn[s].tree_tests = 0;
-  dyn[s].diag[8] = dyn[s].diag[9] = dyn[s].diag[10] = 0;
-}
 
 // Sort keys of the walk order: (system, class, place of the position on a Hilbert curve through a
 // 1024^3 grid of the box); class 0 is the dummy slot, 1 live slots, 2 the rest.  The order only
@@ -245,8 +193,6 @@ __device__ __forceinline__ void load_x(const double *__restrict__ X, long long T
   x[2] = __ldg(X + 2 * T + g);
 }
 
-// Create the non-empty children of node p (counts cnt[0..7]); returns first child id via
-// *id0 and member base via *mb0 (or -1 on overflow).  Called by one thread.
 // What a node's split reserves: child ids, member slots, entries of the next level's block
 // and warp split lists, entries of the block-summed node list.
 struct SplitNeeds {
@@ -309,129 +255,115 @@ __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const S
   return true;
 }
 
+// Create the non-empty children of node p (counts cnt[0..7]); returns first child id via
+// *id0 and member base via *mb0 (or -1 on overflow).  Called by one thread.
 __device__ void make_children(TreeBuffers &tb, int p, const int cnt[8], int *id0_out, int *mb0_out, unsigned *err) {
-  int mask = 0, kept = 0;
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    if (cnt[d]) mask |= 1 << d;
-    kept += cnt[d];
-  }
-  const int nchild = __popc(mask);
-  int4 Ip = tb.nI[p];
-  if (nchild == 0) {
-    *id0_out = -1;
-    *mb0_out = -1;
-    return;
-  }
-  // one reservation per counter for the whole node (node ids, member slots, split-list and
-  // big-node entries), the atomics issued together rather than one per child
-  const int depth = tb.nDepth[p] + 1;
-  const int lb = depth % 3;
-  int nblk = 0, nwrp = 0, nbig = 0;
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    if (cnt[d] >= 2) {
-      if (cnt[d] > kBigNode) ++nblk;
-      else ++nwrp;
-    }
-    if (cnt[d] > kBlockSumNode) ++nbig;
-  }
-  const int id0 = atomicAdd(&tb.ctr[0], nchild);
-  const int mb0 = atomicAdd(&tb.ctr[1], kept);
-  const int qb = nblk ? atomicAdd(&tb.ctr[kCtrSplit + lb], nblk) : 0;
-  const int qw = nwrp ? atomicAdd(&tb.ctr[kCtrSplit + 3 + lb], nwrp) : 0;
-  const int qg = nbig ? atomicAdd(&tb.ctr[kCtrBig], nbig) : 0;
-  if (id0 + nchild > tb.max_nodes || (long long)mb0 + kept > tb.max_members || qb + nblk > tb.max_blk ||
-      qw + nwrp > tb.max_wrp || qg + nbig > tb.max_big) {
-    atomicOr(err, DERR_TREE_NODES);
-    *id0_out = -1;
-    *mb0_out = -1;
-    return;
-  }
-  const double4 P = tb.nP[p];
-  const double h = tb.nA[p].w / 2.0;
-  int off = 0, k = 0, kb = 0, kw = 0, kg = 0;
-#pragma unroll
-  for (int d = 0; d < 8; ++d) {
-    if (!cnt[d]) continue;
-    const int id = id0 + k;
-    const bool last = (k == nchild - 1);
-    const double cx = (d & 1) ? e_add(P.x, h) : P.x;
-    const double cz = (d & 2) ? e_add(P.z, h) : P.z;
-    const double cy = (d & 4) ? e_add(P.y, h) : P.y;
-    tb.nP[id] = make_double4(cx, cy, cz, 0);
-    tb.nA[id] = make_double4(0, 0, 0, h);
-    tb.nI[id] = make_int4(cnt[d], kEnd, last ? Ip.z : id + 1, 0);
-    tb.nR[id] = make_int2(mb0 + off, cnt[d]);
-    tb.nDepth[id] = depth;
-    tb.nKids[id] = 0;
-    if (cnt[d] >= 2) {  // the child's level list of nodes still to split
-      if (cnt[d] > kBigNode) tb.split_blk[lb][qb + kb++] = id;
-      else tb.split_wrp[lb][qw + kw++] = id;
-    }
-    if (cnt[d] > kBlockSumNode) tb.bigl[qg + kg++] = id;
-    off += cnt[d];
-    ++k;
-  }
-  tb.nI[p].y = id0;
-  tb.nKids[p] = nchild;
+  *id0_out = *mb0_out = -1;
+  const SplitNeeds nd = split_needs(cnt);
+  if (nd.nchild == 0) return;
+  // one reservation per counter for the whole node, the atomics issued together
+  const int lb = (tb.nDepth[p] + 1) % 3;
+  const int id0 = atomicAdd(&tb.ctr[0], nd.nchild);
+  const int mb0 = atomicAdd(&tb.ctr[1], nd.kept);
+  const int qb = nd.nblk ? atomicAdd(&tb.ctr[kCtrSplit + lb], nd.nblk) : 0;
+  const int qw = nd.nwrp ? atomicAdd(&tb.ctr[kCtrSplit + 3 + lb], nd.nwrp) : 0;
+  const int qg = nd.nbig ? atomicAdd(&tb.ctr[kCtrBig], nd.nbig) : 0;
+  if (!write_children(tb, p, cnt, nd, id0, mb0, qb, qw, qg, err)) return;
   *id0_out = id0;
   *mb0_out = mb0;
 }
 
-// The roots' split (build_tree at the root, tree.f90:66-94) for every system at once: the
-// live slots, in slot order, are sorted stably by (system, octant digit; 8 for a point in
-// no child), which lists each child's members in slot order, as the warp and block splits
-// do node by node.
-__global__ void k_root_digits(const double *__restrict__ X, long long T, TreeBuffers tb,
-                              const int *__restrict__ sys_of, const int *__restrict__ pos,
-                              const SysConst *__restrict__ scs) {
-  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= T) return;
-  const int n_live = pos[T];
-  if (q >= n_live) {
-    tb.rkey[0][q] = 0xFFFFFFFFu;
-    tb.rval[0][q] = 0;
-    return;
-  }
-  const int g = tb.members[q];
-  const int s = sys_of[g];
-  int d = 8;
-  // a point pinned in front (its segment goes into the wall) counts in the root's centre but
-  // belongs to no child (new_tree, tree.f90:128)
-  if (tb.nI[s].x >= 2 && !(scs[s].pin && pin_i(scs[s].pin[g]))) {
-    double x[3];
-    load_x(X, T, g, x);
-    d = octant(x, tb.nP[s], tb.nA[s].w / 2.0);
-    if (d < 8) {  // one atomic per (system, octant) per warp: 8 counters take all the slots
-      const int key = 8 * s + d;
-      const unsigned peers = __match_any_sync(__activemask(), key);
-      if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&tb.root_cnt[key], __popc(peers));
-    }
-  }
-  tb.rkey[0][q] = ((unsigned)s << 4) | (unsigned)d;
-  tb.rval[0][q] = g;
+// The roots' member lists (the live slots, in slot order) and their split (build_tree at the root,
+// tree.f90:66-94), every system at once, by one ordered pass over the slots: list 0 holds the
+// live slots, list 1 + d those in octant d of their root's cell.  A slot keeps its octant and
+// its rank in that list; the ranks at the systems' first slots (and past the last) tell each
+// root's counts.
+constexpr unsigned kPassFirst = 1u << 31;  // the slot is a system's first (its dummy)
+__global__ void __launch_bounds__(kPassThreads) k_root_lists(const SysConst *__restrict__ scs,
+                                                            const SysDyn *__restrict__ dyn,
+                                                            const int *__restrict__ sys_of,
+                                                            const double *__restrict__ X, const int *__restrict__ nxt,
+                                                            TreeBuffers tb, int nsys, long long T, unsigned *err) {
+  ordered_pass<9>(
+      PassBuffers{tb.pass_state, tb.pass_ctl}, T, err,
+      [&](long long gl) -> unsigned {
+        if (gl == 0) {
+          for (int b = 0; b < 6; ++b) tb.ctr[kCtrSplit + b] = 0;
+          tb.ctr[0] = nsys;
+          tb.ctr[2] = 0;
+          tb.ctr[3] = nsys;
+          tb.ctr[kCtrBig] = 0;
+        }
+        if (gl >= T) return kPassFirst;
+        const int g = (int)gl, s = sys_of[g];
+        const SysConst &sc = scs[s];
+        const int k = g - sc.base;
+        int d = 8;
+        unsigned f = k == 0 ? kPassFirst : 0u;
+        if ((sc.use_tree || sc.sched_tree) && k >= 1 && k <= dyn[s].pcount && nxt[g] != 0) {
+          f |= 1u;
+          // a point pinned in front (its segment goes into the wall) counts in the root's centre
+          // but belongs to no child (new_tree, tree.f90:128)
+          if (dyn[s].pcount >= 2 && !(sc.pin && pin_i(sc.pin[g]))) {
+            double x[3];
+            load_x(X, T, g, x);
+            const double h = -sc.bsize / 2.0;
+            d = octant(x, make_double4(h, h, h, 0), sc.bsize / 2.0);
+            if (d < 8) f |= 2u << d;
+          }
+        }
+        tb.rdig[g] = (unsigned char)d;
+        return f;
+      },
+      [&](long long gl, int k, int p, unsigned word) {
+        if (word & kPassFirst) tb.root_rank[9 * (gl < T ? sys_of[gl] : nsys) + k] = p;
+        if (k == 0) {
+          if (word & 1u) tb.members[p] = (int)gl;
+          if (gl == T) tb.ctr[1] = p;
+        } else if ((word >> k) & 1u) {
+          tb.rrank[gl] = p;
+        }
+      });
 }
 
-__global__ void k_root_children(TreeBuffers tb, int nsys, unsigned *err) {
+// Root of every system (construct_tree, tree.f90:38-59) and its children.
+__global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys, const int *__restrict__ nxt,
+                        TreeBuffers tb, unsigned *err) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys) return;
-  tb.root_mb[s] = -1;
-  if (tb.nI[s].x < 2) return;
-  int cnt[8];
-  for (int d = 0; d < 8; ++d) cnt[d] = tb.root_cnt[8 * s + d];
-  int id0 = -1, mb0 = -1;
-  make_children(tb, s, cnt, &id0, &mb0, err);
-  tb.root_mb[s] = mb0;
+  const SysConst &sc = scs[s];
+  const int pc = (sc.use_tree || sc.sched_tree) ? dyn[s].pcount : 0;
+  const double h = -sc.bsize / 2.0;
+  const int *r0 = tb.root_rank + 9 * s, *r1 = r0 + 9;  // this system's first slot, the next one's
+  tb.nP[s] = make_double4(h, h, h, 0);
+  tb.nA[s] = make_double4(0, 0, 0, sc.bsize);
+  tb.nB[s] = make_double4(0, 0, 0, 0);
+  tb.nI[s] = make_int4(pc, kEnd, kEnd, pc >= 1 ? nxt[sc.base + 1] : 0);
+  tb.nR[s] = make_int2(r0[0], r1[0] - r0[0]);
+  tb.nDepth[s] = 0;
+  tb.nKids[s] = 0;
+  tb.nLeaf[s] = pc == 1 ? sc.base + 1 : 0;
+  dyn[s].tree_eval = 0;
+  dyn[s].tree_tests = 0;
+  dyn[s].diag[8] = dyn[s].diag[9] = dyn[s].diag[10] = 0;
+  int cnt[8], id0 = -1, mb0 = -1;
+  for (int d = 0; d < 8; ++d) cnt[d] = r1[1 + d] - r0[1 + d];
+  if (pc >= 2) make_children(tb, s, cnt, &id0, &mb0, err);
+  tb.root_ok[s] = mb0 >= 0;
+  int off = mb0;
+  for (int d = 0; d < 8; ++d) {  // the slot of rank r in octant d is member entry root_mb + r
+    tb.root_mb[8 * s + d] = off - r0[1 + d];
+    off += cnt[d];
+  }
 }
 
-__global__ void k_root_scatter(TreeBuffers tb, const int *__restrict__ pos, long long T) {
+// The children's member lists; also notes the block-summed nodes listed so far (depth 1).
+__global__ void k_root_scatter(const int *__restrict__ sys_of, TreeBuffers tb, int nsys) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= T || p >= pos[T]) return;
-  const unsigned key = tb.rkey[1][p];
-  const int s = (int)(key >> 4), d = (int)(key & 15u);
-  const int mb = tb.root_mb[s];
-  if (d < 8 && mb >= 0) tb.members[mb + (int)(p - tb.nR[s].x)] = tb.rval[1][p];
+  if (p == 0) tb.ctr[kCtrBigSnap] = min(tb.ctr[kCtrBig], tb.max_big);
+  if (p >= tb.root_rank[9 * nsys]) return;  // the live slots of all systems
+  const int g = tb.members[p], d = tb.rdig[g], s = sys_of[g];
+  if (d < 8 && tb.root_ok[s]) tb.members[tb.root_mb[8 * s + d] + tb.rrank[g]] = g;
 }
 
 // Split node p (at most kBigNode members) with one warp: count the members per octant, make
@@ -669,17 +601,18 @@ __device__ void split_node_block(const double *__restrict__ X, long long T, Tree
 
 // One level of the build: the listed big nodes by blocks, then the other listed nodes by
 // warps.  One block of kSplitThreads per SM, with registers for the loads of several
-// members (or nodes) per lane in flight at once.  The children's lists (level + 1) fill as nodes split; the list of level + 2 is
-// idle during this level (read at level - 1, filled at level + 1) and is emptied here.
-__global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *__restrict__ X, long long T, TreeBuffers tb,
-                                                      int level, unsigned *err) {
+// members (or nodes) per lane in flight at once.  The children's lists (level + 1) fill as nodes
+// split; the list of level + 2 is idle during this level (read at level - 1, filled at
+// level + 1) and is emptied here.
+__device__ void split_level(const double *__restrict__ X, long long T, TreeBuffers &tb, int level, int block, int blocks,
+                            unsigned *err) {
   const int b = level % 3, b2 = (level + 2) % 3;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (block == 0 && threadIdx.x == 0) {
     tb.ctr[kCtrSplit + b2] = 0;
     tb.ctr[kCtrSplit + 3 + b2] = 0;
   }
   const int nbl = min(tb.ctr[kCtrSplit + b], tb.max_blk);
-  for (int bq = blockIdx.x; bq < nbl; bq += gridDim.x) {
+  for (int bq = block; bq < nbl; bq += blocks) {
     const int p = tb.split_blk[b][bq];
     if (tb.nDepth[p] >= kMaxLevels) {
       if (threadIdx.x == 0) atomicOr(err, DERR_TREE_DEPTH);
@@ -693,8 +626,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *
   // lane splits its own when it has at most kLaneNode members, and the warp the larger ones
   // one at a time; elsewhere a warp splits one node at a time.
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int warp = (block * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (blocks * blockDim.x) >> 5;
   const int nwl = min(tb.ctr[kCtrSplit + 3 + b], tb.max_wrp);
   const int lb = (level + 1) % 3;  // the children's level lists
   if (nwl >= 2 * nwarps) {
@@ -722,6 +655,26 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *
       }
       warp_split_one(X, T, tb, p, lane, lb, err);
     }
+  }
+}
+
+__global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *__restrict__ X, long long T, TreeBuffers tb,
+                                                      int level, unsigned *err) {
+  split_level(X, T, tb, level, blockIdx.x, gridDim.x, err);
+}
+
+// The levels from `level` on by one block, until none lists a node: below cells a fraction of a
+// segment wide only pairs of points from different filaments are left together.
+__global__ void __launch_bounds__(kSplitThreads, 1) k_split_rest(const double *__restrict__ X, long long T, TreeBuffers tb,
+                                                     int level, unsigned *err) {
+  for (; level < kMaxLevels; ++level) {
+    volatile int *c = tb.ctr + kCtrSplit + level % 3;
+    const bool none = c[0] == 0 && c[3] == 0;
+    __syncthreads();
+    if (none) return;
+    split_level(X, T, tb, level, 0, 1, err);
+    __threadfence_block();
+    __syncthreads();
   }
 }
 
@@ -1026,9 +979,8 @@ __global__ void __launch_bounds__(kSumThreads) k_root_sums(const double *__restr
 }
 
 // Estimate of each root's centre (the mean over live slots, tree.f90:50-52) by a blocked
-// sum over `parts` blocks per system (k_root_partial, then k_root_approx adding the parts in
-// order), and a bound on its distance to the reference's sequential sum: a sum of N
-// terms in FP64 is within (N-1) u sum|x| of the exact one in either order, so the two means
+// sum over `parts` blocks per system (k_root_partial, then k_root_approx adding the parts), and
+// a bound on its distance to the reference's sequential sum: a sum of N terms in FP64 is within (N-1) u sum|x| of the exact one in either order, so the two means
 // differ by at most 2 u (sum|x| + sum|y| + sum|z|) plus the roundings of the divisions.
 __global__ void __launch_bounds__(256) k_root_partial(const double *__restrict__ X, long long T, TreeBuffers tb,
                                                       int nsys, int parts) {
@@ -1063,11 +1015,14 @@ __global__ void __launch_bounds__(256) k_root_partial(const double *__restrict__
 }
 
 __global__ void k_root_approx(TreeBuffers tb, int nsys, int parts, double band_scale) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= nsys) return;
   double t[6] = {0, 0, 0, 0, 0, 0};
-  for (int q = 0; q < parts; ++q)
+  for (int q = lane; q < parts; q += 32)
     for (int c = 0; c < 6; ++c) t[c] += tb.root_part[((long long)s * parts + q) * 6 + c];
+  for (int c = 0; c < 6; ++c)
+    for (int o = 16; o > 0; o >>= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
+  if (lane) return;
   const int n = tb.nR[s].y;
   const double dn = n > 0 ? (double)n : 1.0;
   const double cx = t[0] / dn, cy = t[1] / dn, cz = t[2] / dn;
@@ -2204,20 +2159,12 @@ void tree_alloc(nv_handle *h) {
   tb->max_big = (int)std::min<long long>((long long)kMaxLevels * (T / (kBlockSumNode + 1) + 1) + 64, 1 << 30);
   cudaMalloc(&tb->bigl, (size_t)tb->max_big * sizeof(int));
   cudaMalloc(&tb->root_apx, (size_t)h->nsys * sizeof(double4));
-  for (int b = 0; b < 2; ++b) {
-    cudaMalloc(&tb->rkey[b], (size_t)T * sizeof(unsigned));
-    cudaMalloc(&tb->rval[b], (size_t)T * sizeof(int));
-  }
-  cudaMalloc(&tb->root_cnt, (size_t)h->nsys * 8 * sizeof(int));
-  cudaMalloc(&tb->root_mb, (size_t)h->nsys * sizeof(int));
-  {
-    int sb = 1;
-    while ((1LL << sb) < h->nsys) ++sb;
-    tb->rkey_bits = std::min(32, 4 + sb);
-    cub::DeviceRadixSort::SortPairs(nullptr, tb->rsort_bytes, tb->rkey[0], tb->rkey[1], tb->rval[0], tb->rval[1],
-                                    (int)T, 0, tb->rkey_bits);
-    cudaMalloc(&tb->rsort_tmp, std::max<size_t>(tb->rsort_bytes, 16));
-  }
+  cudaMalloc(&tb->rdig, (size_t)T);
+  cudaMalloc(&tb->rrank, (size_t)T * sizeof(int));
+  cudaMalloc(&tb->root_rank, ((size_t)h->nsys + 1) * 9 * sizeof(int));
+  cudaMalloc(&tb->root_mb, (size_t)h->nsys * 8 * sizeof(int));
+  cudaMalloc(&tb->root_ok, (size_t)h->nsys * sizeof(int));
+  pass_alloc(&tb->pass_state, &tb->pass_ctl, 9, T);
   tb->root_parts = std::max(1, std::min(64, 4096 / h->nsys));
   cudaMalloc(&tb->root_part, (size_t)h->nsys * tb->root_parts * 6 * sizeof(double));
   cudaMalloc(&tb->defer, (size_t)kDeferCap * sizeof(int));
@@ -2238,10 +2185,6 @@ void tree_alloc(nv_handle *h) {
     cudaMalloc(&tb->split_blk[b], (size_t)tb->max_blk * sizeof(int));
     cudaMalloc(&tb->split_wrp[b], (size_t)tb->max_wrp * sizeof(int));
   }
-  cudaMalloc(&tb->flag, (T + 1) * sizeof(int));
-  cudaMalloc(&tb->pos, (T + 1) * sizeof(int));
-  cub::DeviceScan::ExclusiveSum(nullptr, tb->cub_bytes, tb->flag, tb->pos, (int)(T + 1));
-  cudaMalloc(&tb->cub_tmp, std::max<size_t>(tb->cub_bytes, 16));
   for (int b = 0; b < 2; ++b) {
     cudaMalloc(&tb->okey[b], (size_t)T * sizeof(unsigned long long));
     cudaMalloc(&tb->oval[b], (size_t)T * sizeof(int));
@@ -2255,6 +2198,10 @@ void tree_alloc(nv_handle *h) {
   cub::DeviceRadixSort::SortPairs(nullptr, tb->sort_bytes, tb->okey[0], tb->okey[1], tb->oval[0], tb->oval[1], (int)T,
                                   0, tb->key_bits);
   cudaMalloc(&tb->sort_tmp, std::max<size_t>(tb->sort_bytes, 16));
+  double widest = 1.;  // box over segment length of the systems with a tree
+  for (auto &s : h->sc)
+    if ((s.use_tree || s.sched_tree) && s.delta > 0.) widest = std::max(widest, s.bsize / s.delta);
+  tb->grid_levels = std::min(kMaxLevels, std::max(2, (int)std::ceil(std::log2(std::min(widest, 1e9))) + 3));
   h->tree = tb;
 }
 
@@ -2262,8 +2209,8 @@ void tree_free(nv_handle *h) {
   TreeBuffers *tb = h->tree;
   if (!tb) return;
   void *ptrs[] = {tb->nA, tb->nB, tb->nP, tb->nI, tb->nR, tb->nDepth, tb->nLeaf, tb->nKids, tb->members, tb->bigl, tb->root_apx, tb->root_part, tb->defer, tb->defer_n,
-                  tb->rkey[0], tb->rkey[1], tb->rval[0], tb->rval[1], tb->root_cnt, tb->root_mb, tb->rsort_tmp, tb->ctr,
-                  tb->flag, tb->pos, tb->cub_tmp, tb->mx.C, tb->mx.W, tb->mx.G, tb->okey[0], tb->okey[1],
+                  tb->rdig, tb->rrank, tb->root_rank, tb->root_mb, tb->root_ok, tb->pass_state, tb->pass_ctl, tb->ctr,
+                  tb->mx.C, tb->mx.W, tb->mx.G, tb->okey[0], tb->okey[1],
                   tb->oval[0], tb->oval[1], tb->iperm, tb->sort_tmp, tb->split_blk[0], tb->split_blk[1],
                   tb->split_blk[2], tb->split_wrp[0], tb->split_wrp[1], tb->split_wrp[2]};
   for (void *p : ptrs)
@@ -2276,17 +2223,16 @@ void launch_tree_build(nv_handle *h) {
   TreeBuffers *tb = h->tree;
   if (!tb) return;
   const long long T = h->T;
-  k_live_flags<<<grid_for(T + 1, TB), TB, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->nxt, tb->flag, T,
-                                                         tb->ctr);
-  size_t bytes = tb->cub_bytes;
-  cub::DeviceScan::ExclusiveSum(tb->cub_tmp, bytes, tb->flag, tb->pos, (int)(T + 1), h->stream);
-  k_scatter_live<<<grid_for(T, TB), TB, 0, h->stream>>>(tb->flag, tb->pos, tb->members, T);
-  k_roots<<<grid_for(h->nsys, 64), 64, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, h->nxt, tb->pos, *tb, T);
-  // the walk order and the roots' exact sums (one long sequential chain per system) run
-  // on the side stream; the walks wait for the order, the fix-up of deferred root tests
+  k_root_lists<<<pass_blocks(T), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, *tb, h->nsys,
+                                                               T, h->d_err);
+  k_roots<<<grid_for(h->nsys, 64), 64, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, h->nxt, *tb, h->d_err);
+  // the roots' estimates, the walk order and the roots' exact sums (one long sequential chain per
+  // system) run on the side stream; the walks wait for the first two, the fix-up of deferred root tests
   // and the closest-point walk for the sums
   cudaEventRecord(h->fork_ev, h->stream);
   cudaStreamWaitEvent(h->side, h->fork_ev, 0);
+  k_root_partial<<<h->nsys * tb->root_parts, 256, 0, h->side>>>(h->x, T, *tb, h->nsys, tb->root_parts);
+  k_root_approx<<<grid_for(32LL * h->nsys, 128), 128, 0, h->side>>>(*tb, h->nsys, tb->root_parts, h->root_band_scale);
   k_order_keys<<<grid_for(T, TB), TB, 0, h->side>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->nxt, tb->okey[0],
                                                     tb->oval[0], T);
   {
@@ -2299,28 +2245,21 @@ void launch_tree_build(nv_handle *h) {
   k_root_sums<<<h->nsys, kSumThreads, kSumSmem, h->side>>>(h->x, T, *tb, h->nsys, h->nxt, h->d_err);
   cudaEventRecord(h->join_ev, h->side);
   const int sms = n_sms();
-  k_root_digits<<<grid_for(T, TB), TB, 0, h->stream>>>(h->x, T, *tb, h->sys_of, tb->pos, h->d_sc);
-  {
-    size_t sb = tb->rsort_bytes;
-    cub::DeviceRadixSort::SortPairs(tb->rsort_tmp, sb, tb->rkey[0], tb->rkey[1], tb->rval[0], tb->rval[1], (int)T, 0,
-                                    tb->rkey_bits, h->stream);
-  }
-  k_root_children<<<grid_for(h->nsys, 64), 64, 0, h->stream>>>(*tb, h->nsys, h->d_err);
-  k_root_scatter<<<grid_for(T, TB), TB, 0, h->stream>>>(*tb, tb->pos, T);
+  k_root_scatter<<<grid_for(T, TB), TB, 0, h->stream>>>(h->sys_of, *tb, h->nsys);
   // the big depth-1 nodes' sums (the longest sequential chains after the roots') start as soon
   // as the roots' split has listed them and written their member lists, beside the levels
-  k_big_snapshot<<<1, 32, 0, h->stream>>>(*tb);
   cudaEventRecord(h->fork2_ev, h->stream);
   cudaStreamWaitEvent(h->side2, h->fork2_ev, 0);
   k_node_sums_block<<<sms, kSumThreads, kSumSmem, h->side2>>>(h->x, h->gi, h->nxt, T, *tb, 0, h->d_err);
   cudaEventRecord(h->join2_ev, h->side2);
-  for (int L = 1; L < kMaxLevels; ++L)
+  // A launch per level down to cells of about an eighth of delta, the rest by one block (32,768 points,
+  // 41 launches 172 us, now 9 in 122 us and the block in 1.4; 1,048,576 points, 10 and 35 us)
+  for (int L = 1; L < tb->grid_levels; ++L)
     k_split_level<<<sms, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, L, h->d_err);
+  k_split_rest<<<1, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, tb->grid_levels, h->d_err);
   k_node_sums_block<<<sms, kSumThreads, kSumSmem, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, 1, h->d_err);
   k_node_sums_big<<<sms * 8, 128, 0, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, h->nsys, h->d_err);
   k_node_sums_small<<<sms * 8, 128, 0, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, h->nsys, h->d_err);
-  k_root_partial<<<h->nsys * tb->root_parts, 256, 0, h->stream>>>(h->x, T, *tb, h->nsys, tb->root_parts);
-  k_root_approx<<<grid_for(h->nsys, 128), 128, 0, h->stream>>>(*tb, h->nsys, tb->root_parts, h->root_band_scale);
   cudaStreamWaitEvent(h->stream, h->sort_ev, 0);
   cudaStreamWaitEvent(h->stream, h->join2_ev, 0);
   if (h->precision == NV_PREC_MIXED) {

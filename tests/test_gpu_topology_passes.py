@@ -1,12 +1,13 @@
-"""Edges of the topology stages' kernels: the ordered one-pass lists (blocks of 1,024 slots, warps
-of 128) at slot counts around whole blocks, the wall sweeps' chunks of 256 slots, pinsert's rounds over the whole GPU (handles above
-262,144 slots) and by a block per system, with too few rounds allowed, and the closest-point
-search by a warp per target and by the cell list on either side of the line between them.
-Everything equal to the oracle's, event for event."""
+"""Edges of the topology stages' kernels and of the tree build: the ordered one-pass lists (blocks
+of 1,024 slots, warps of 128) at slot counts around whole blocks, the wall sweeps' chunks of 256
+slots, pinsert's rounds over the whole GPU (handles above 262,144 slots) and by a block per
+system, with too few rounds allowed, the closest-point search by a warp per target and by the
+cell list on either side of the line between them, the octrees of systems of unlike sizes and the
+levels of the octree that one block splits.  Everything equal to the oracle's, event for event."""
 import numpy as np
 import pytest
 
-from helpers import config0_params, tangle
+from helpers import config0_params, config1_params, tangle
 from nuvort_b200.rings import half_loop
 from oracle import Oracle
 from test_gpu_topology import _assert_same, _moved_state, _ring_slots, _run_stage
@@ -86,3 +87,28 @@ def test_wall_sweeps_around_whole_chunks(n, delta):
         for f in ("infront", "behind", "pinnedi", "pinnedb", "wpinned"):
             assert np.array_equal(getattr(a, f), getattr(b, f)), f
         assert np.max(np.abs(a.x - b.x)) < 1e-12
+
+
+@pytest.mark.parametrize("pairs", [0, 3, 60])
+@pytest.mark.parametrize("sizes", [(1021,), (700, 1, 1300, 90), (2046, 1025)])
+def test_octrees_and_their_deep_levels(sizes, pairs):
+    # pairs of points 1e-10 apart: some 25 levels below the cells of a segment's width
+    from nuvort_b200.api import Handle
+    p = config1_params("Tree")
+    states = []
+    for i, n in enumerate(sizes):
+        st = tangle(20 + i, 0.001, n_points=max(n - 40, 20))
+        m = min(pairs, st.pcount // 3)
+        st.x[st.pcount - m:st.pcount] = st.x[:m] + 1e-10
+        states.append(st)
+    with Handle([p] * len(sizes), [max(n, s.pcount) for n, s in zip(sizes, states)], states=states) as h:
+        h.stage("ghostp")
+        h.stage("construct_tree")
+        for i, st in enumerate(states):
+            o = Oracle(p, st)
+            o.stage("ghostp")
+            o.stage("construct_tree")
+            a, b = h.tree_dump(i), o.tree_dump()
+            assert len(a) == len(b)
+            for f in ("pos", "width", "cent", "circ", "pcount", "depth", "leaf", "first_next"):
+                assert np.array_equal(a[f], b[f]), f
