@@ -112,3 +112,20 @@ def test_octrees_and_their_deep_levels(sizes, pairs):
             assert len(a) == len(b)
             for f in ("pos", "width", "cent", "circ", "pcount", "depth", "leaf", "first_next"):
                 assert np.array_equal(a[f], b[f]), f
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_octree_out_of_nodes_is_an_error(precision):
+    # 320 pairs 1e-10 apart need some 7,000 nodes below the segments' cells; 981 slots have 4,000
+    from nuvort_b200.api import Handle, NuvortError
+    p = config1_params("Tree", precision=precision)
+    st = tangle(21, 0.001, n_points=940)
+    good = st.copy()
+    st.x[-320:] = st.x[:320] + 1e-10
+    with Handle(p, [980], states=[st]) as h:
+        with pytest.raises(NuvortError, match="octree node buffer exhausted"):
+            h.calc_velocity()
+        h.upload(0, good)
+        u = h.calc_velocity()
+    with Handle(p, [980], states=[good]) as h:
+        assert np.array_equal(u, h.calc_velocity())
