@@ -315,6 +315,15 @@ int cleared() {
   return NV_OK;
 }
 
+// A host block to the device before anything else on the handle's stream: a plain cudaMemcpy runs
+// on the null stream, returns once its pageable source is staged, and a kernel of the
+// (non-blocking) stream launched next could still read the old bytes.
+int put_bytes(nv_handle *h, void *dst, const void *src, size_t n) {
+  NV_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, h->stream));
+  NV_CUDA(cudaStreamSynchronize(h->stream));
+  return NV_OK;
+}
+
 void build_worklist(nv_handle *h, int which, std::vector<int2> &w, int tb) {
   w.clear();
   for (int s = 0; s < h->nsys; ++s) {
@@ -530,8 +539,7 @@ int set_restart_counters(nv_handle *h, int sys, double t, int itime, int recon_c
   h->h_dyn[sys].t = t;
   h->h_dyn[sys].itime = itime;
   h->h_dyn[sys].recon_count = recon_count;
-  NV_CUDA(cudaMemcpy(h->d_dyn + sys, &h->h_dyn[sys], sizeof(SysDyn), cudaMemcpyHostToDevice));
-  return NV_OK;
+  return put_bytes(h, h->d_dyn + sys, &h->h_dyn[sys], sizeof(SysDyn));
 }
 
 int sys_capacity(nv_handle *h, int sys) { return (h && sys >= 0 && sys < h->nsys) ? h->cap[sys] : -1; }
@@ -846,10 +854,8 @@ int nv_upload(nv_handle *h, int32_t sys, const nv_host_state *st) {
   if (rc) return rc;
   d.pcount = n;
   d.nlive = check[1];
-  NV_CUDA(cudaMemcpy(h->d_dyn + sys, &d, sizeof(SysDyn), cudaMemcpyHostToDevice));
-  unsigned zero = 0;
-  NV_CUDA(cudaMemcpy(h->d_err, &zero, sizeof zero, cudaMemcpyHostToDevice));
-  return NV_OK;
+  NV_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), sm));
+  return put_bytes(h, h->d_dyn + sys, &d, sizeof(SysDyn));
 }
 
 int nv_download(nv_handle *h, int32_t sys, nv_host_state *st, int32_t cap) {
@@ -1278,8 +1284,7 @@ int nv_set_clock(nv_handle *h, int32_t sys, double t, int32_t itime) {
   if (rc || (rc = pull_dyn_one(h, sys))) return rc;
   h->h_dyn[sys].t = t;
   h->h_dyn[sys].itime = itime;
-  NV_CUDA(cudaMemcpy(h->d_dyn + sys, &h->h_dyn[sys], sizeof(SysDyn), cudaMemcpyHostToDevice));
-  return NV_OK;
+  return put_bytes(h, h->d_dyn + sys, &h->h_dyn[sys], sizeof(SysDyn));
 }
 
 int nv_counters_get(nv_handle *h, int32_t sys, nv_counters *c) {
@@ -1466,8 +1471,7 @@ int nv_set_walk_range(nv_handle *h, int32_t sys, int32_t lo, int32_t hi) {
   if (rc) return rc;
   c.walk_lo = lo;
   c.walk_hi = hi;
-  NV_CUDA(cudaMemcpy(h->d_sc + sys, &c, sizeof(SysConst), cudaMemcpyHostToDevice));
-  return NV_OK;
+  return put_bytes(h, h->d_sc + sys, &c, sizeof(SysConst));
 }
 
 int nv_velocity_pack(nv_handle *h, int32_t sys, int32_t lo, int32_t count, double *d_buf) {
@@ -1539,7 +1543,7 @@ int nv_set_event_margins(nv_handle *h, int32_t on) {
     SysDyn &d = h->h_dyn[s];
     d.margin_on = on ? 1 : 0;
     for (double &v : d.margin) v = 1e300;
-    NV_CUDA(cudaMemcpy(h->d_dyn + s, &d, sizeof(SysDyn), cudaMemcpyHostToDevice));
+    if ((rc = put_bytes(h, h->d_dyn + s, &d, sizeof(SysDyn)))) return rc;
   }
   return NV_OK;
 }
@@ -1578,14 +1582,14 @@ int nf_upload(nv_handle *h, const double *src, size_t n, const double **dst) {
   void *p = nullptr;
   NV_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(double)));
   h->nf_buffers.push_back(p);
-  NV_CUDA(cudaMemcpy(p, src, n * sizeof(double), cudaMemcpyHostToDevice));
+  const int rc = put_bytes(h, p, src, n * sizeof(double));
+  if (rc) return rc;
   *dst = static_cast<const double *>(p);
   return NV_OK;
 }
 int sc_refresh(nv_handle *h, int sys) {
-  NV_CUDA(cudaMemcpy(h->d_sc + sys, &h->sc[sys], sizeof(SysConst), cudaMemcpyHostToDevice));
   h->graph_valid = false;
-  return NV_OK;
+  return put_bytes(h, h->d_sc + sys, &h->sc[sys], sizeof(SysConst));
 }
 }  // namespace
 
@@ -1710,7 +1714,7 @@ int nv_calc_velocity_direct_at(nv_handle *h, int32_t sys, const int32_t *targets
   double *du = nullptr;
   NV_CUDA(cudaMalloc(&dt, std::max(n, 1) * sizeof(int)));
   NV_CUDA(cudaMalloc(&du, std::max(n, 1) * 3 * sizeof(double)));
-  cudaMemcpy(dt, g.data(), n * sizeof(int), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(dt, g.data(), n * sizeof(int), cudaMemcpyHostToDevice, h->stream);
   cudaMemsetAsync(du, 0, std::max(n, 1) * 3 * sizeof(double), h->stream);
   launch_ghost(h);
   launch_direct_targets(h, sys, dt, n, du);
