@@ -37,6 +37,7 @@ constexpr int kSnapLevel = 1;  // the early block sums: the big nodes of depth 1
 // ctr[kCtrSplit + b]: entries of the level lists of nodes to split, by level % 3 = b:
 // [+0..+2] nodes above kBigNode members (split by a block), [+3..+5] the others with >= 2
 constexpr int kCtrSplit = kMaxLevels + 8;
+constexpr int kCtrFail = kMaxLevels + 14;  // lowest level at which a split ran out of room, or INT_MAX
 constexpr int kCtrSize = kMaxLevels + 16;
 constexpr int kDeferCap = 1 << 20;  // targets with a deferred root test listed per velocity pass
 
@@ -193,6 +194,12 @@ __device__ __forceinline__ void load_x(const double *__restrict__ X, long long T
   x[2] = __ldg(X + 2 * T + g);
 }
 
+// Whether a split at a level above this one ran out of room (the same answer to every thread of
+// this level's kernel, which may itself lower the level noted).
+__device__ __forceinline__ bool failed_above(const TreeBuffers &tb, int level) {
+  return *(const volatile int *)&tb.ctr[kCtrFail] < level;
+}
+
 // What a node's split reserves: child ids, member slots, entries of the next level's block
 // and warp split lists, entries of the block-summed node list.
 struct SplitNeeds {
@@ -214,23 +221,15 @@ __device__ SplitNeeds split_needs(const int cnt[8]) {
 }
 
 // The children of node p at reserved offsets (id0, mb0, qb, qw, qg); false when they do not
-// fit the buffers (error set): what was reserved of them is then marked unused (the counters
-// have moved on, and later readers go up to them).
+// fit the buffers (error set).  The counters have then moved past entries never written, which
+// the levels below, the sums and the walks must not read: they return (failed_above).  (Marking
+// the entries unused here instead cost the levels' kernel 36 of 157 us at 32,768 points.)
 __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const SplitNeeds &n, int id0, int mb0,
                                int qb, int qw, int qg, unsigned *err) {
   if (id0 + n.nchild > tb.max_nodes || (long long)mb0 + n.kept > tb.max_members || qb + n.nblk > tb.max_blk ||
       qw + n.nwrp > tb.max_wrp || qg + n.nbig > tb.max_big) {
     atomicOr(err, DERR_TREE_NODES);
-    for (int id = id0; id < id0 + n.nchild && id < tb.max_nodes; ++id) {
-      tb.nI[id] = make_int4(0, kEnd, kEnd, 0);
-      tb.nR[id] = make_int2(0, 0);
-      tb.nDepth[id] = 0;
-      tb.nKids[id] = 0;
-    }
-    const int lb = (tb.nDepth[p] + 1) % 3;
-    for (int q = qb; q < qb + n.nblk && q < tb.max_blk; ++q) tb.split_blk[lb][q] = kEnd;
-    for (int q = qw; q < qw + n.nwrp && q < tb.max_wrp; ++q) tb.split_wrp[lb][q] = kEnd;
-    for (int q = qg; q < qg + n.nbig && q < tb.max_big; ++q) tb.bigl[q] = kEnd;
+    atomicMin(&tb.ctr[kCtrFail], tb.nDepth[p]);
     return false;
   }
   const int4 Ip = tb.nI[p];
@@ -304,6 +303,7 @@ __global__ void __launch_bounds__(kPassThreads) k_root_lists(const SysConst *__r
           tb.ctr[2] = 0;
           tb.ctr[3] = nsys;
           tb.ctr[kCtrBig] = 0;
+          tb.ctr[kCtrFail] = INT_MAX;
         }
         if (gl >= T) return kPassFirst;
         const int g = (int)gl, s = sys_of[g];
@@ -617,6 +617,7 @@ __device__ void split_node_block(const double *__restrict__ X, long long T, Tree
 // level + 1) and is emptied here.
 __device__ void split_level(const double *__restrict__ X, long long T, TreeBuffers &tb, int level, int block, int blocks,
                             unsigned *err) {
+  if (failed_above(tb, level)) return;
   const int b = level % 3, b2 = (level + 2) % 3;
   if (block == 0 && threadIdx.x == 0) {
     tb.ctr[kCtrSplit + b2] = 0;
@@ -625,7 +626,6 @@ __device__ void split_level(const double *__restrict__ X, long long T, TreeBuffe
   const int nbl = min(tb.ctr[kCtrSplit + b], tb.max_blk);
   for (int bq = block; bq < nbl; bq += blocks) {
     const int p = tb.split_blk[b][bq];
-    if (p == kEnd) continue;
     if (tb.nDepth[p] >= kMaxLevels) {
       if (threadIdx.x == 0) atomicOr(err, DERR_TREE_DEPTH);
       continue;
@@ -661,8 +661,7 @@ __device__ void split_level(const double *__restrict__ X, long long T, TreeBuffe
   } else {
     for (int wq = warp; wq < nwl; wq += nwarps) {
       const int p = tb.split_wrp[b][wq];
-      if (p == kEnd) continue;
-      if (tb.nDepth[p] >= kMaxLevels) {
+        if (tb.nDepth[p] >= kMaxLevels) {
         if (lane == 0) atomicOr(err, DERR_TREE_DEPTH);
         continue;
       }
@@ -730,7 +729,8 @@ __device__ __forceinline__ void finish_node(TreeBuffers &tb, int id, bool root, 
 // Nodes with at most kSmallNode members (most of them leaves): one thread each.
 __global__ void k_node_sums_small(const double *__restrict__ X, const double *__restrict__ GI,
                                   const int *__restrict__ nxt, long long T, TreeBuffers tb, int nsys, unsigned *err) {
-  const int n = min(tb.ctr[0], tb.max_nodes);
+  if (failed_above(tb, INT_MAX)) return;
+  const int n = tb.ctr[0];
   for (int id = nsys + blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const int2 R = tb.nR[id];
     if (R.y > kSmallNode) continue;
@@ -829,7 +829,8 @@ __global__ void __launch_bounds__(128) k_node_sums_big(const double *__restrict_
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int n = min(tb.ctr[0], tb.max_nodes);
+  if (failed_above(tb, INT_MAX)) return;
+  const int n = tb.ctr[0];
   // The warp's nodes are ids nsys + warp + j nwarps (consecutive ids, often one level's
   // nodes of similar size, go to different warps); their records are read 32 at a time and
   // the ones in this kernel's size range summed in turn.
@@ -953,11 +954,11 @@ __global__ void __launch_bounds__(kSumThreads) k_node_sums_block(const double *_
   // summed beside the level splits (which read their width and write their first child,
   // fields the sums leave alone); part 1, after the levels: every other big node
   extern __shared__ double sm_dyn[];
+  if (failed_above(tb, part == 0 ? 1 : INT_MAX)) return;
   const int snap = tb.ctr[kCtrBigSnap];
   const int nbig = part == 0 ? snap : min(tb.ctr[kCtrBig], tb.max_big);
   for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
     const int id = tb.bigl[b];
-    if (id == kEnd) continue;  // (the build ran out of nodes)
     const bool early = b < snap && tb.nDepth[id] <= kSnapLevel;
     if (early != (part == 0)) continue;  // block-uniform
     const int2 R = tb.nR[id];
@@ -969,10 +970,6 @@ __global__ void __launch_bounds__(kSumThreads) k_node_sums_block(const double *_
     if (threadIdx.x == 0) finish_node(tb, id, false, cx, cy, cz, qx, qy, qz, nxt, err);
     __syncthreads();
   }
-}
-
-__global__ void k_big_snapshot(TreeBuffers tb) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) tb.ctr[kCtrBigSnap] = min(tb.ctr[kCtrBig], tb.max_big);
 }
 
 // Roots: the masked mean over live slots (tree.f90:50-54), circulation zero.  One block per
@@ -1627,7 +1624,8 @@ __global__ void k_closest_tree(const SysConst *__restrict__ scs, const SysDyn *_
 constexpr float kTestBand = 1e-5f;
 
 __global__ void k_node_prep(TreeBuffers tb, int nsys, double theta0, int corr, const int *__restrict__ prv) {
-  const int n = min(tb.ctr[0], tb.max_nodes);
+  if (failed_above(tb, INT_MAX)) return;
+  const int n = tb.ctr[0];
   for (int id = nsys + blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const double4 A = tb.nA[id], B = tb.nB[id];
     const double t0 = A.w / theta0;
@@ -1650,7 +1648,8 @@ __global__ void k_node_prep(TreeBuffers tb, int nsys, double theta0, int corr, c
 // A leaf's record holds prv of its member, the start of the leaf's segment, for the walk's
 // own-segment test; this refreshes it when points were relinked after the build.
 __global__ void k_leaf_links(TreeBuffers tb, int nsys, const int *__restrict__ prv) {
-  const int n = min(tb.ctr[0], tb.max_nodes);
+  if (failed_above(tb, INT_MAX)) return;
+  const int n = tb.ctr[0];
   for (int id = nsys + blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const int4 I = tb.nI[id];
     if (I.x == 1) tb.mx.W[id].d.w = prv[I.w];
