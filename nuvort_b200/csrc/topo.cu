@@ -970,10 +970,18 @@ __global__ void k_ins_ghosts(const SysConst *__restrict__ scs, SysDyn *dyn, cons
 struct ReconIn {
   int i, pari, parb, j, nj, parjb;
   int yes;  // 1: reconnect, 0: no, -1: skip (reconnection.f90:181-190)
-  double dot_val, l_before, l_after;
+  double dot_val, l_before, l_bridge;  // l_bridge: l_after without its last distance
 };
 
-__device__ ReconIn recon_decide(const State &S, int i, double half_delta, int cl_i) {
+// reconnection.f90:199-203 from the two sums that links do not enter and the two slots they name
+__device__ __forceinline__ bool recon_shortens(const State &S, double l_before, double l_bridge, int pari, int parjb) {
+  double xpi[3], xpj[3];
+  load3(S.X, S.T, pari, xpi);
+  load3(S.X, S.T, parjb, xpj);
+  return e_add(l_bridge, dist_gen(xpi, xpj)) <= l_before;
+}
+
+__device__ ReconIn recon_decide(const State &S, int i, int cl_i) {
   ReconIn r;
   r.i = i;
   r.pari = S.nxt[i];
@@ -982,7 +990,7 @@ __device__ ReconIn recon_decide(const State &S, int i, double half_delta, int cl
   r.nj = 0;
   r.parjb = 0;
   r.yes = -1;
-  r.dot_val = r.l_before = r.l_after = 0;
+  r.dot_val = r.l_before = r.l_bridge = 0;
   if (r.pari == 0) return r;
   const int j = r.j;
   if (j == r.pari || j == r.parb || j == 0) return r;
@@ -998,19 +1006,16 @@ __device__ ReconIn recon_decide(const State &S, int i, double half_delta, int cl
     return r;
   }
   const long long T = S.T;
-  double xi[3], gii[3], gbi[3], xj[3], gij[3], gbj[3], xpi[3], xpj[3];
+  double xi[3], gii[3], gbi[3], xj[3], gij[3], gbj[3];
   load3(S.X, T, i, xi);
   load3(S.GI, T, i, gii);
   load3(S.GB, T, i, gbi);
   load3(S.X, T, j, xj);
   load3(S.GI, T, j, gij);
   load3(S.GB, T, j, gbj);
-  load3(S.X, T, r.pari, xpi);
-  load3(S.X, T, r.parjb, xpj);
   r.l_before = e_add(e_add(e_add(dist_gen(xi, gii), dist_gen(xi, gbi)), dist_gen(xj, gij)), dist_gen(xj, gbj));
-  r.l_after = e_add(e_add(e_add(dist_gen(xi, gbi), dist_gen(xi, xj)), dist_gen(xj, gij)), dist_gen(xpi, xpj));
-  r.yes = r.l_after <= r.l_before ? 1 : 0;
-  (void)half_delta;
+  r.l_bridge = e_add(e_add(dist_gen(xi, gbi), dist_gen(xi, xj)), dist_gen(xj, gij));
+  r.yes = recon_shortens(S, r.l_before, r.l_bridge, r.pari, r.parjb) ? 1 : 0;
   return r;
 }
 
@@ -1192,9 +1197,20 @@ __device__ int loop_count(const State &S, int particle, int pcount, const int (&
 // A block of kRound threads loads kRound candidates at once and decides each on the state at
 // the start of the round; warp 0 then walks them in ascending order, lane 0 applying the
 // events.  Lane 0 stops only at candidates whose prefetched test passes or whose inputs an
-// earlier event of the round wrote (the "need" bits, recomputed by the whole warp against
-// the shared-memory touched set after every event, for the candidates the sweep has not
-// reached yet); every other candidate's test fails in the serial sweep too.
+// earlier event of the round wrote (the "need" bits, set through the round's map after every
+// event, for the candidates the sweep has not reached yet); every other candidate's test fails
+// in the serial sweep too.
+//
+// What bounds a sweep is lane 0: some 600 instructions an event, one after the other.  So an
+// event that no other candidate of the round comes near is applied by its own thread, together
+// with the others of its kind up to the next candidate (or extra slot) that lane 0 has to stop
+// at.  "Near" is decided in the map: the event's neighbourhood -- every slot whose links its
+// test, its writes and its loop_killer walk read or write -- is recorded in it, and must be free
+// of every other candidate's.  Such an event meets the links it was decided on, changes none
+// that another one reads, and gets its number from its rank; an event of lane 0 that comes near
+// it after all marks it as needed, and lane 0 then takes it at its place.
+// 1,048,576 points: removals 8.74 ms (3,620 events of 3,896 candidates), now 2.60;
+// reconnections 4.12 ms (1,214 events of 41,193 candidates), now 2.76.
 constexpr int kRound = 256;
 // precon's rounds are larger: its candidates are many (every close pair), its events few, and
 // a round's fixed cost (the prefetch's chain of dependent loads) is paid once per round
@@ -1204,11 +1220,11 @@ constexpr int kExtraHeap = 1024;  // pending extra slots of the premove sweep he
 constexpr int kRoundWords = kRound / 32;
 using RoundTouched = SlotSet<11, 1024>;
 
-// first candidate above pos whose bit is set in a | b (words of 32), or n
-__device__ __forceinline__ int next_marked(const unsigned *a, const unsigned *b, int pos, int n) {
+// first candidate above pos whose bit is set in (a and not lone) | b (words of 32), or n
+__device__ __forceinline__ int next_marked(const unsigned *a, const unsigned *lone, const unsigned *b, int pos, int n) {
   for (int l = pos + 1; l < n;) {
     const int wd = l >> 5;
-    const unsigned bits = (a[wd] | b[wd]) & (~0u << (l & 31));
+    const unsigned bits = ((a[wd] & ~lone[wd]) | b[wd]) & (~0u << (l & 31));
     if (bits) {
       const int r = (wd << 5) + __ffs(bits) - 1;
       return r < n ? r : n;
@@ -1218,11 +1234,31 @@ __device__ __forceinline__ int next_marked(const unsigned *a, const unsigned *b,
   return n;
 }
 
+// Events due together: the lone candidates lo .. hi - 1 without a need bit (words of 32 of the
+// lone and the need bits), with consecutive numbers and places in the event list.
+struct Due {
+  int lo, hi, n, seq, at;
+};
+// lone candidates lo .. hi - 1 without a need bit
+__device__ __forceinline__ int due_below(const unsigned *lone, const unsigned *need, int lo, int hi) {
+  int c = 0;
+  for (int w = lo >> 5; w <= (hi - 1) >> 5 && lo < hi; ++w) {
+    unsigned b = lone[w] & ~need[w];
+    if (w == lo >> 5) b &= ~0u << (lo & 31);
+    if (w == (hi - 1) >> 5) b &= ~0u >> (31 - ((hi - 1) & 31));
+    c += __popc(b);
+  }
+  return c;
+}
+__device__ __forceinline__ bool is_due(const Due &due, const unsigned *lone, const unsigned *need, int q) {
+  return q >= due.lo && q < due.hi && ((lone[q >> 5] & ~need[q >> 5]) >> (q & 31) & 1u);
+}
+
 // Slot -> index of a candidate of the current round that reads that slot's links (one
 // entry per slot a candidate reads; duplicates allowed), so that an event can mark exactly
 // the candidates it affects.  Built by the whole block at the start of a round.
 constexpr int kMapBits = 11;
-constexpr int kMapCap = 1 << kMapBits;  // up to 4 entries per candidate at half load
+constexpr int kMapCap = 1 << kMapBits;  // three quarters full at most
 struct CandMap {
   int *key;
   int *idx;
@@ -1234,6 +1270,24 @@ struct CandMap {
         idx[h] = q;
         return;
       }
+    }
+  }
+  // calls f on every candidate recorded under slot g
+  template <class F>
+  __device__ void each(int g, F f) const {
+    for (int h = home(g);; h = (h + 1) & (kMapCap - 1)) {
+      const int k = key[h];
+      if (k == 0) return;
+      if (k == g) f(idx[h]);
+    }
+  }
+  // the candidate at slot j with closest point i, or -1
+  template <class Rec>
+  __device__ int pair_of(int i, int j, const Rec *rec) const {
+    for (int h = home(j);; h = (h + 1) & (kMapCap - 1)) {
+      const int k = key[h];
+      if (k == 0) return -1;
+      if (k == j && rec[idx[h]].i == j && rec[idx[h]].j == i) return idx[h];
     }
   }
   // set the need bit of every candidate q > bound recorded under slot g
@@ -1253,6 +1307,11 @@ struct CandMap {
 struct ReconRec {
   int i, yes, pari, j, parjb, nj, a1, a2, a3, b2;
 };
+// slots of a reconnection's neighbourhood (those past the second are recorded for events only),
+// and the most events a round may have for them to fit the map
+constexpr size_t kReconSmem = kReconRound * sizeof(double2);
+constexpr int kReconHood = 7;
+constexpr int kReconLone = (kMapCap * 3 / 4 - 2 * kReconRound) / (kReconHood - 2);
 
 __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
                                                         State S, const int *__restrict__ pos_a,
@@ -1262,7 +1321,10 @@ __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__r
   __shared__ int mkey[kMapCap], midx[kMapCap];
   __shared__ DevEvent ebuf[kEventStage];
   __shared__ ReconRec rec[kReconRound];
-  __shared__ unsigned ymask[kReconWords], nmask[kReconWords];
+  extern __shared__ double2 len[];  // l_before and l_bridge of the round's candidates
+  __shared__ unsigned ymask[kReconWords], nmask[kReconWords], lone[kReconWords];
+  __shared__ unsigned long long s_hash;
+  __shared__ Due s_due;
   __shared__ int s_used;
   const int s = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1277,14 +1339,16 @@ __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__r
   EventStage es{ebuf, 0, ev, ev_count, ev_cap};
   const int li = pos_a[base], le = pos_a[base + sc.cap + 1];
   Tally d = Tally::of(dyn[s], base);  // thread 0 applies the events
-  const double half_delta = sc.delta / 2.;
+  if (tid == 0) s_hash = 0;
   __syncthreads();
   for (int c0 = li; c0 < le; c0 += kReconRound) {
     const int n = min(kReconRound, le - c0);
     ReconRec r{0, -1, 0, 0, 0, 0, 0, 0, 0, 0};
+    int parb = 0;
+    bool never = true;
     if (tid < n) {
       const int i = list_a[c0 + tid];
-      const ReconIn in = recon_decide(S, i, half_delta, S.cl[i]);
+      const ReconIn in = recon_decide(S, i, S.cl[i]);
       if (in.yes >= 0) margin_note(dyn[s], 3, in.dot_val, 0.9);
       r.i = i;
       r.yes = in.yes;
@@ -1292,15 +1356,20 @@ __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__r
       r.j = in.j;
       r.parjb = in.parjb;
       r.nj = in.nj;
+      parb = in.parb;
       if (in.yes == 1) {  // the links the two loop_killer walks follow
         r.a1 = S.nxt[in.pari];
         r.b2 = S.nxt[in.nj];
         r.a2 = S.nxt[r.a1];
         r.a3 = S.nxt[r.a2];
       }
-      // the decision reads the links of i and j
-      map.insert(i, tid);
-      if (in.j != i) map.insert(in.j, tid);
+      // the decision reads the links of i and j; of near parallel lines it is no whatever they are
+      never = in.yes == 0 && in.dot_val > 0.9;
+      if (!never) {
+        map.insert(i, tid);
+        if (in.j != i) map.insert(in.j, tid);
+      }
+      len[tid] = make_double2(in.l_before, in.l_bridge);
     }
     rec[tid] = r;
     const unsigned yb = __ballot_sync(0xffffffffu, r.yes == 1);
@@ -1308,61 +1377,150 @@ __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__r
       ymask[wid] = yb;
       nmask[wid] = 0;
     }
+    // the rest of an event's neighbourhood, where the round's events fit the map
+    const bool alone_ok = __syncthreads_count(r.yes == 1) <= kReconLone;
+    const int hood[kReconHood] = {r.i, r.j, r.pari, r.parjb, r.nj, r.a1, r.a2};
+    if (alone_ok && r.yes == 1) {
+#pragma unroll
+      for (int q = 2; q < kReconHood; ++q) map.insert(hood[q], tid);
+    }
     __syncthreads();
-    if (tid == 0) {
-      int bound = -1;
-      auto on_clear = [&](int g) { map.mark(g, bound, nmask); };
-      for (int pos = -1;;) {
-        const int l = next_marked(ymask, nmask, pos, n);
-        if (l >= n) break;
-        bound = l;
-        const ReconRec &c = rec[l];
-        int i = c.i, j = c.j, yes = c.yes, pari = c.pari, parjb = c.parjb;
-        bool live = (nmask[l >> 5] >> (l & 31)) & 1u;
-        if (live) {  // an earlier event of the round wrote the links of i or j
-          if (S.nxt[i] == 0) {
-            yes = -1;
+    // The candidate at j whose closest point is i, usually there, is no neighbour to avoid: past
+    // an event at i < j it is left out (i is its behind then), and it comes first if j < i.
+    int mate = -1;
+    bool alone = alone_ok && r.yes == 1;
+    if (alone) {
+      mate = map.pair_of(r.i, r.j, rec);
+      alone = !(mate >= 0 && mate < tid && rec[mate].yes == 1);
+#pragma unroll
+      for (int q = 0; q < kReconHood; ++q)
+        map.each(hood[q], [&](int o) { alone = alone && (o == tid || o == mate || rec[o].yes != 1); });
+      const int key[7] = {r.parjb, r.i, r.pari, r.a1, r.a2, r.j, r.nj};
+      const int val[7] = {r.pari, r.j, r.a1, r.a2, r.a3, r.nj, r.b2};
+      alone = alone && loop_count(S, r.pari, dyn[s].pcount, key, val) >= 4 &&
+              loop_count(S, r.i, dyn[s].pcount, key, val) >= 4;
+    }
+    const unsigned ab = __ballot_sync(0xffffffffu, alone);
+    if (lane == 0) lone[wid] = ab;
+    __syncthreads();
+    // A candidate without an event whose links one lone event before it writes: decided on them
+    // (i's own pair is left out, as above); with more of them, or now an event, at its place.
+    if (!never && r.yes != 1) {
+      int by = -1, n_by = 0;
+      auto written = [&](int o) {
+        if (o < tid && (lone[o >> 5] >> (o & 31) & 1u) && o != by) {
+          by = o;
+          ++n_by;
+        }
+      };
+      map.each(r.i, written);
+      map.each(r.j, written);
+      if (n_by > 0) {
+        const ReconRec &e = rec[by];
+        auto ahead = [&](int g, int nx) { return g == e.parjb ? e.pari : g == e.i ? e.j : nx; };
+        auto behind = [&](int g, int pv) { return g == e.pari ? e.parjb : g == e.j ? e.i : pv; };
+        bool visit = n_by > 1;
+        if (!visit && !(e.i == r.j && e.j == r.i)) {
+          if (r.yes < 0) {
+            visit = r.pari != 0;
           } else {
-            const ReconIn q = recon_decide(S, i, half_delta, S.cl[i]);
-            if (q.yes >= 0) margin_note(dyn[s], 3, q.dot_val, 0.9);
-            yes = q.yes;
-            pari = q.pari;
-            parjb = q.parjb;
+            const int pi = ahead(r.i, r.pari), pb = behind(r.i, parb), pj = behind(r.j, r.parjb);
+            visit = r.j != pi && r.j != pb && recon_shortens(S, len[tid].x, len[tid].y, pi, pj);
           }
         }
-        if (yes == 1) {
-          live = live || tc.has(pari) || tc.has(c.a1) || tc.has(c.a2) || tc.has(c.nj);
-          d.recon++;
-          es.add(d, s, NV_EV_RECON, i, j);
-          S.nxt[parjb] = pari;
-          S.prv[pari] = parjb;
-          S.nxt[i] = j;
-          S.prv[j] = i;
-          tc.add(i);
-          tc.add(j);
-          tc.add(pari);
-          tc.add(parjb);
-          map.mark(i, l, nmask);
-          map.mark(j, l, nmask);
-          map.mark(pari, l, nmask);
-          map.mark(parjb, l, nmask);
-          if (live) {
-            loop_killer_stage(S, d, s, pari, d.pcount, es, tc, on_clear);
-            loop_killer_stage(S, d, s, i, d.pcount, es, tc, on_clear);
-          } else {
-            const int key[7] = {parjb, i, pari, c.a1, c.a2, j, c.nj};
-            const int val[7] = {pari, j, c.a1, c.a2, c.a3, c.nj, c.b2};
-            bool killed = false;
-            if (loop_count(S, pari, d.pcount, key, val) < 4) {
-              loop_killer_stage(S, d, s, pari, d.pcount, es, tc, on_clear);
-              killed = true;
-            }
-            if (killed || loop_count(S, i, d.pcount, key, val) < 4)
-              loop_killer_stage(S, d, s, i, d.pcount, es, tc, on_clear);
-          }
-        }
-        pos = l;
+        if (visit) atomicOr(&nmask[tid >> 5], 1u << (tid & 31));
       }
+    }
+    __syncthreads();
+    int pos = -1;
+    for (;;) {
+      if (tid == 0) {
+        int bound = -1;
+        auto on_clear = [&](int g) { map.mark(g, bound, nmask); };
+        for (;;) {
+          const int l = next_marked(ymask, lone, nmask, pos, n);
+          const int due = due_below(lone, nmask, pos + 1, l);
+          if (due) {
+            s_due = Due{pos + 1, l, due, d.seq, atomicAdd(ev_count, due)};
+            d.seq += due;
+            d.recon += due;
+            pos = l - 1;
+            break;
+          }
+          s_due.n = 0;
+          if (l >= n) break;
+          bound = l;
+          const ReconRec &c = rec[l];
+          int i = c.i, j = c.j, yes = c.yes, pari = c.pari, parjb = c.parjb;
+          bool live = (nmask[l >> 5] >> (l & 31)) & 1u;
+          if (live) {  // an earlier event of the round wrote the links of i or j
+            if (S.nxt[i] == 0) {
+              yes = -1;
+            } else if (c.yes >= 0) {  // all but the links as at the start of the round
+              pari = S.nxt[i];
+              const int parb = S.prv[i], nj = S.nxt[j];
+              parjb = S.prv[j];
+              yes = j == pari || j == parb || nj == 0                               ? -1
+                    : recon_shortens(S, len[l].x, len[l].y, pari, parjb) ? 1 : 0;
+            } else {
+              const ReconIn q = recon_decide(S, i, S.cl[i]);
+              if (q.yes >= 0) margin_note(dyn[s], 3, q.dot_val, 0.9);
+              yes = q.yes;
+              pari = q.pari;
+              parjb = q.parjb;
+            }
+          }
+          if (yes == 1) {
+            live = live || tc.has(pari) || tc.has(c.a1) || tc.has(c.a2) || tc.has(c.nj);
+            d.recon++;
+            es.add(d, s, NV_EV_RECON, i, j);
+            S.nxt[parjb] = pari;
+            S.prv[pari] = parjb;
+            S.nxt[i] = j;
+            S.prv[j] = i;
+            tc.add(i);
+            tc.add(j);
+            tc.add(pari);
+            tc.add(parjb);
+            map.mark(i, l, nmask);
+            map.mark(j, l, nmask);
+            map.mark(pari, l, nmask);
+            map.mark(parjb, l, nmask);
+            if (live) {
+              loop_killer_stage(S, d, s, pari, d.pcount, es, tc, on_clear);
+              loop_killer_stage(S, d, s, i, d.pcount, es, tc, on_clear);
+            } else {
+              const int key[7] = {parjb, i, pari, c.a1, c.a2, j, c.nj};
+              const int val[7] = {pari, j, c.a1, c.a2, c.a3, c.nj, c.b2};
+              bool killed = false;
+              if (loop_count(S, pari, d.pcount, key, val) < 4) {
+                loop_killer_stage(S, d, s, pari, d.pcount, es, tc, on_clear);
+                killed = true;
+              }
+              if (killed || loop_count(S, i, d.pcount, key, val) < 4)
+                loop_killer_stage(S, d, s, i, d.pcount, es, tc, on_clear);
+            }
+          }
+          pos = l;
+        }
+      }
+      __syncthreads();
+      const Due due = s_due;
+      if (due.n == 0) break;
+      if (is_due(due, lone, nmask, tid)) {
+        const int rank = due_below(lone, nmask, due.lo, tid), at = due.at + rank;
+        S.nxt[r.parjb] = r.pari;
+        S.prv[r.pari] = r.parjb;
+        S.nxt[r.i] = r.j;
+        S.prv[r.j] = r.i;
+        if (mate > tid) atomicAnd(&ymask[mate >> 5], ~(1u << (mate & 31)));
+        atomicAdd(&s_hash, event_digest(due.seq + rank, d.itime, NV_EV_RECON, r.i - base, r.j - base));
+        if (at < ev_cap) ev[at] = DevEvent{s, due.seq + rank, d.itime, NV_EV_RECON, r.i, r.j};
+      }
+      __threadfence_block();
+      __syncthreads();
+    }
+    if (tid == 0) {
       if (es.n) es.spill();
       s_used = tc.n | tc.full;
       tc.n = 0;
@@ -1376,6 +1534,7 @@ __global__ void __launch_bounds__(kReconRound) k_recon_sweep(const SysConst *__r
     __syncthreads();
   }
   if (tid == 0) {
+    d.hash += s_hash;
     d.store(dyn[s]);
     dyn[s].diag[3] = le - li;
   }
@@ -1403,9 +1562,11 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
   __shared__ int mkey[kMapCap], midx[kMapCap];
   __shared__ DevEvent ebuf[kEventStage];
   __shared__ RemoveRec rec[kRound];
-  __shared__ unsigned ymask[kRoundWords], nmask[kRoundWords];
+  __shared__ unsigned ymask[kRoundWords], nmask[kRoundWords], lone[kRoundWords];
   __shared__ int heap[kExtraHeap];  // pending extra slots (a min-heap); the bitmap past it
-  __shared__ int s_used;
+  __shared__ unsigned long long s_hash;
+  __shared__ Due s_due;
+  __shared__ int s_used, s_extra;
   const int s = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (s >= nsys || *err) return;
@@ -1423,6 +1584,7 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
   const int lastslot = base + d.pcount;
   const double thr = e_mul(.99, sc.delta);
   const long long T = S.T;
+  const bool margins = dyn[s].margin_on;
   int last = base;               // thread 0: last slot visited
   int bound = -1;                // thread 0: candidates above this index are not reached yet
   long long n_live = 0, n_extra = 0;  // visits on the live state: candidates, extra slots
@@ -1499,6 +1661,7 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
     tc.add(tinfront, 2u);
     map.mark(i, bound, nmask);
     map.mark(infront, bound, nmask);
+    map.mark(tinfront, bound, nmask);
     clear_particle(S, infront);
     es.add(d, s, NV_EV_REMOVE, i, infront);
     loop_killer_stage(S, d, s, i, d.pcount, es, tc, on_clear);
@@ -1521,6 +1684,7 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
     tc.add(tinfront, 2u);
     map.mark(i, bound, nmask);
     map.mark(infront, bound, nmask);
+    map.mark(tinfront, bound, nmask);
     clear_particle(S, infront);
     es.add(d, s, NV_EV_REMOVE, i, infront);
     const int key[4] = {i, infront, tinfront, c.c1};  // infront is cleared: no infront link
@@ -1533,10 +1697,15 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
     d.remove++;
     if (p > i && p <= lastslot && !pc) push_extra(p);
   };
+  if (tid == 0) {
+    s_hash = 0;
+    s_extra = 0;
+  }
   __syncthreads();
   for (int c0 = li; c0 < le; c0 += kRound) {
     const int n = min(kRound, le - c0);
     RemoveRec r{0, 0, 0, 0, 0, 0, 0, 1};
+    bool alone = false, extra = false;  // extra: p = behind(i) is visited later, and passes
     if (tid < n) {
       r.i = list_a[c0 + tid];
       r.inf = S.nxt[r.i];
@@ -1551,13 +1720,28 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
         if (r.yes) {
           r.pv = S.prv[r.i];
           r.c1 = S.nxt[r.tinf];
-          if (r.pv > r.i && r.pv <= lastslot) r.pcand = cand[r.pv];
+          alone = !margins && r.c1 && r.pv;  // (the margins note the tests in the sweep's order)
+          if (r.pv > r.i && r.pv <= lastslot) {
+            r.pcand = cand[r.pv];
+            if (!r.pcand) {
+              double xp[3];
+              load3(S.X, T, r.pv, xp);
+              extra = true;
+              alone = alone && !(dist_gen(xp, xt) < thr);
+            }
+          }
           r.c2 = S.nxt[r.c1];
         }
       }
-      // the test reads the infront links of i and infront(i)
+      // the test reads the infront links of i and infront(i); an event also those behind and ahead
       map.insert(r.i, tid);
       if (r.inf != r.i) map.insert(r.inf, tid);
+      if (r.yes) {
+        map.insert(r.pv, tid);
+        map.insert(r.tinf, tid);
+        map.insert(r.c1, tid);
+        map.insert(r.c2, tid);
+      }
     }
     rec[tid] = r;
     const unsigned yb = __ballot_sync(0xffffffffu, r.yes != 0);
@@ -1566,31 +1750,82 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
       nmask[wid] = 0;
     }
     __syncthreads();
-    if (tid == 0) {
-      for (int pos = -1;;) {
-        const int l = next_marked(ymask, nmask, pos, n);
-        // the sweep position of the next candidate; past the round: the next round's first
-        const int kl = l < n ? rec[l].i : c0 + n < le ? list_a[c0 + n] : lastslot + 1;
-        const int e = hsize > 0 || bm_extras > 0 ? take_extra(min(kl - 1, lastslot)) : INT_MAX;
-        if (e != INT_MAX) {  // an extra slot below the next candidate
-          last = e;
-          bound = pos;
-          ++n_extra;
-          visit(e);
-          continue;
-        }
-        if (l >= n) break;
-        last = kl;
-        bound = l;
-        const RemoveRec &c = rec[l];
-        if (((nmask[l >> 5] >> (l & 31)) & 1u) || tc.has(c.tinf, 1u) || tc.has(c.c1, 1u)) {
-          ++n_live;  // an earlier event wrote links the test or the loop_killer walk reads
-          visit(kl);
-        } else {
-          remove_fast(c);
-        }
-        pos = l;
+    if (alone) {
+      const int hood[6] = {r.pv, r.i, r.inf, r.tinf, r.c1, r.c2};
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        map.each(hood[q], [&](int o) { alone = alone && o == tid; });
+#pragma unroll
+        for (int p = 0; p < q; ++p) alone = alone && hood[p] != hood[q];  // (a loop of five or fewer)
       }
+    }
+    const unsigned ab = __ballot_sync(0xffffffffu, alone);
+    if (lane == 0) lone[wid] = ab;
+    __syncthreads();
+    int pos = -1, held = INT_MAX;  // thread 0: the last candidate reached, an extra slot taken
+    for (;;) {
+      if (tid == 0) {
+        for (;;) {
+          const int l = next_marked(ymask, lone, nmask, pos, n);
+          // the sweep position of the next candidate; past the round: the next round's first
+          const int kl = l < n ? rec[l].i : c0 + n < le ? list_a[c0 + n] : lastslot + 1;
+          if (held == INT_MAX && (hsize > 0 || bm_extras > 0)) held = take_extra(min(kl - 1, lastslot));
+          int hi = l;  // the candidates up to the next stop
+          if (held != INT_MAX) {
+            int lo = pos + 1;
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              if (rec[mid].i < held) lo = mid + 1;
+              else hi = mid;
+            }
+          }
+          const int due = due_below(lone, nmask, pos + 1, hi);
+          if (due) {
+            s_due = Due{pos + 1, hi, due, d.seq, atomicAdd(ev_count, due)};
+            d.seq += due;
+            d.remove += due;
+            pos = hi - 1;
+            last = max(last, rec[pos].i);
+            break;
+          }
+          s_due.n = 0;
+          if (held != INT_MAX) {  // an extra slot below the next candidate
+            last = held;
+            pos = bound = hi - 1;
+            ++n_extra;
+            visit(held);
+            held = INT_MAX;
+            continue;
+          }
+          if (l >= n) break;
+          last = kl;
+          bound = l;
+          const RemoveRec &c = rec[l];
+          if (((nmask[l >> 5] >> (l & 31)) & 1u) || tc.has(c.tinf, 1u) || tc.has(c.c1, 1u)) {
+            ++n_live;  // an earlier event wrote links the test or the loop_killer walk reads
+            visit(kl);
+          } else {
+            remove_fast(c);
+          }
+          pos = l;
+        }
+      }
+      __syncthreads();
+      const Due due = s_due;
+      if (due.n == 0) break;
+      if (is_due(due, lone, nmask, tid)) {
+        const int rank = due_below(lone, nmask, due.lo, tid), at = due.at + rank;
+        S.prv[r.tinf] = r.i;
+        S.nxt[r.i] = r.tinf;
+        clear_particle(S, r.inf);
+        atomicAdd(&s_hash, event_digest(due.seq + rank, d.itime, NV_EV_REMOVE, r.i - base, r.inf - base));
+        if (at < ev_cap) ev[at] = DevEvent{s, due.seq + rank, d.itime, NV_EV_REMOVE, r.i, r.inf};
+        if (extra) atomicAdd(&s_extra, 1);
+      }
+      __threadfence_block();
+      __syncthreads();
+    }
+    if (tid == 0) {
       if (es.n) es.spill();
       s_used = tc.n | tc.full;
       tc.n = 0;
@@ -1614,6 +1849,8 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
       visit(e);
     }
     if (es.n) es.spill();
+    d.hash += s_hash;
+    n_extra += s_extra;
     d.store(dyn[s]);
     dyn[s].diag[4] = le - li;
     dyn[s].diag[7] = (n_extra << 32) | n_live;
@@ -1941,6 +2178,7 @@ void topo_alloc(nv_handle *h) {
   cudaMalloc(&tb->high, n * sizeof(int));
   cudaMalloc(&tb->high2, n * sizeof(int));
   pass_alloc(&tb->pass_state, &tb->pass_ctl, 3, h->T);
+  cudaFuncSetAttribute(k_recon_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReconSmem);
   cudaMalloc(&tb->l0, (n / 32 + 2) * sizeof(unsigned));
   cudaMalloc(&tb->l1, (n / 1024 + 2) * sizeof(unsigned));
   cudaMalloc(&tb->seglen, n * sizeof(double));
@@ -2084,7 +2322,7 @@ void launch_precon(nv_handle *h) {
   TopoBuffers *tb = h->topo;
   k_mark_recon<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->closestd, h->nxt, list_a(h),
                                                              h->T, h->d_err);
-  k_recon_sweep<<<h->nsys, kReconRound, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, make_state(h), tb->pos_a, tb->list_a,
+  k_recon_sweep<<<h->nsys, kReconRound, kReconSmem, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, make_state(h), tb->pos_a, tb->list_a,
                                                h->d_err, h->d_events, h->d_event_count, h->event_cap);
   launch_solid_precon(h);
 }

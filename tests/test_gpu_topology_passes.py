@@ -1,13 +1,15 @@
 """Edges of the topology stages' kernels and of the tree build: the ordered one-pass lists (blocks
 of 1,024 slots, warps of 128) at slot counts around whole blocks, the wall sweeps' chunks of 256
 slots, pinsert's rounds over the whole GPU (handles above 262,144 slots) and by a block per
-system, with too few rounds allowed, the closest-point search by a warp per target and by the
+system, with too few rounds allowed, the removal and reconnection sweeps with events few and far
+between, in clusters and everywhere, the closest-point search by a warp per target and by the
 cell list on either side of the line between them, the octrees of systems of unlike sizes and the
 levels of the octree that one block splits.  Everything equal to the oracle's, event for event."""
 import numpy as np
 import pytest
 
 from helpers import config0_params, config1_params, tangle
+from nuvort_b200.abi import event_digest
 from nuvort_b200.rings import half_loop
 from oracle import Oracle
 from test_gpu_topology import _assert_same, _moved_state, _ring_slots, _run_stage
@@ -129,3 +131,48 @@ def test_octree_out_of_nodes_is_an_error(precision):
         u = h.calc_velocity()
     with Handle(p, [980], states=[good]) as h:
         assert np.array_equal(u, h.calc_velocity())
+
+
+def _shuffled(st, seed):
+    """The same lines with their points in random slots."""
+    to = np.random.default_rng(seed).permutation(st.pcount)
+    out = st.copy()
+    for name in ("x", "u", "u1", "u2", "ghosti", "ghostb"):
+        getattr(out, name)[to] = getattr(st, name)
+    for name in ("infront", "behind"):
+        link = getattr(st, name)
+        getattr(out, name)[to] = np.where(link > 0, to[link - 1] + 1, 0)
+    return out
+
+
+def _crowded(seed, shuffle, n_rings, jitter):
+    st = _moved_state(config0_params(), tangle(seed, 0.002, n_rings=n_rings))
+    st.x[:st.pcount] += np.random.default_rng(seed).normal(0.0, jitter, (st.pcount, 3))
+    return _shuffled(st, seed) if shuffle else st
+
+
+@pytest.mark.parametrize("shuffle", [False, True])
+@pytest.mark.parametrize("share", [0.003, 0.05, 0.3, 0.8])
+def test_removals_apart_and_in_clusters(share, shuffle):
+    st = _crowded(31, shuffle, 40, 4e-4)
+    live = st.infront[:st.pcount] > 0
+    ahead = st.infront[np.maximum(st.infront[:st.pcount], 1) - 1] - 1
+    gap = np.linalg.norm(st.x[:st.pcount] - st.x[ahead], axis=1)[live]
+    p = config0_params(delta=float(np.quantile(gap, share)) / 0.99, overide_timestep_check=True)
+    a, b, ea, eb, ca, cb = _run_stage(p, st, ["premove"])
+    assert len(eb) > 5
+    assert ea == eb
+    _assert_same(a, b)
+    assert (ca.remove_count, ca.loop_kills, ca.event_hash) == (cb.remove_count, cb.loop_kills, event_digest(eb))
+
+
+@pytest.mark.parametrize("shuffle", [False, True])
+@pytest.mark.parametrize("n_rings,delta", [(12, 0.002), (60, 0.002), (60, 0.006), (150, 0.01)])
+def test_reconnections_apart_and_in_clusters(n_rings, delta, shuffle):
+    st = _crowded(32, shuffle, n_rings, 2e-4)
+    p = config0_params(delta=delta, overide_timestep_check=True)
+    a, b, ea, eb, ca, cb = _run_stage(p, st, ["pclose", "precon", "premove"])
+    assert len(eb) > 0
+    assert ea == eb
+    _assert_same(a, b)
+    assert (ca.recon_count, ca.loop_kills, ca.event_hash) == (cb.recon_count, cb.loop_kills, event_digest(eb))
