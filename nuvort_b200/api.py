@@ -352,9 +352,9 @@ class Handle:
         _check(lib().nv_step(self.h, int(n)))
 
     def calc_velocity(self, sys: int = 0) -> np.ndarray:
-        u = np.zeros((self.capacity[sys], 3), np.float64)
+        u = np.empty((self.counters(sys).pcount, 3), np.float64)  # written whole; the call adds no slots
         _check(lib().nv_calc_velocity(self.h, int(sys), u.ctypes.data_as(C.POINTER(C.c_double))))
-        return u[: self.counters(sys).pcount].copy()
+        return u
 
     def calc_velocity_direct_at(self, sys: int, targets) -> np.ndarray:
         """FP64 direct-sum (BS) velocity at the listed 1-based slots of system sys."""

@@ -4,7 +4,7 @@ slots, pinsert's rounds over the whole GPU (handles above 262,144 slots) and by 
 system, with too few rounds allowed, the removal and reconnection sweeps with events few and far
 between, in clusters and everywhere, the closest-point search by a warp per target and by the
 cell list on either side of the line between them, the octrees of systems of unlike sizes and the
-levels of the octree that one block splits.  Everything equal to the oracle's, event for event."""
+levels of the octree that one block splits, and the rows of a velocity call.  Everything equal to the oracle's, event for event."""
 import numpy as np
 import pytest
 
@@ -176,3 +176,20 @@ def test_reconnections_apart_and_in_clusters(n_rings, delta, shuffle):
     assert ea == eb
     _assert_same(a, b)
     assert (ca.recon_count, ca.loop_kills, ca.event_hash) == (cb.recon_count, cb.loop_kills, event_digest(eb))
+
+
+@pytest.mark.parametrize("velocity,precision", [("BS", "fp64"), ("Tree", "fp64"), ("Tree", "mixed")])
+@pytest.mark.parametrize("extra", [0, 1, 300])
+def test_velocity_rows(velocity, precision, extra):
+    # as many rows as points, those of empty slots zero, the others the handle's u
+    from nuvort_b200.api import Handle
+    p = config1_params(velocity, precision=precision)
+    states = [tangle(60 + i, 0.001, n_points=n) for i, n in enumerate((700, 255, 1024))]
+    _holed(states[1], _ring_slots(states[1])[:1])
+    with Handle([p] * 3, [s.pcount + extra for s in states], states=states) as h:
+        for i, st in enumerate(states):
+            u = h.calc_velocity(i)
+            live = st.infront[:st.pcount] > 0
+            assert u.shape == (st.pcount, 3) and u.flags.c_contiguous and u.flags.owndata
+            assert np.array_equal(u[live], h.download(i).u[:st.pcount][live])
+            assert not u[~live].any() and u[live].any(axis=1).all()
