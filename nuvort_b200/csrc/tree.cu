@@ -661,7 +661,7 @@ __device__ void split_level(const double *__restrict__ X, long long T, TreeBuffe
   } else {
     for (int wq = warp; wq < nwl; wq += nwarps) {
       const int p = tb.split_wrp[b][wq];
-        if (tb.nDepth[p] >= kMaxLevels) {
+      if (tb.nDepth[p] >= kMaxLevels) {
         if (lane == 0) atomicOr(err, DERR_TREE_DEPTH);
         continue;
       }
