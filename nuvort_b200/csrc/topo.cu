@@ -1584,7 +1584,6 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
   const int lastslot = base + d.pcount;
   const double thr = e_mul(.99, sc.delta);
   const long long T = S.T;
-  const bool margins = dyn[s].margin_on;
   int last = base;               // thread 0: last slot visited
   int bound = -1;                // thread 0: candidates above this index are not reached yet
   long long n_live = 0, n_extra = 0;  // visits on the live state: candidates, extra slots
@@ -1706,6 +1705,7 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
     const int n = min(kRound, le - c0);
     RemoveRec r{0, 0, 0, 0, 0, 0, 0, 1};
     bool alone = false, extra = false;  // extra: p = behind(i) is visited later, and passes
+    double gap = 0.;                    // what its test measures
     if (tid < n) {
       r.i = list_a[c0 + tid];
       r.inf = S.nxt[r.i];
@@ -1720,14 +1720,15 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
         if (r.yes) {
           r.pv = S.prv[r.i];
           r.c1 = S.nxt[r.tinf];
-          alone = !margins && r.c1 && r.pv;  // (the margins note the tests in the sweep's order)
+          alone = r.c1 && r.pv;
           if (r.pv > r.i && r.pv <= lastslot) {
             r.pcand = cand[r.pv];
             if (!r.pcand) {
               double xp[3];
               load3(S.X, T, r.pv, xp);
               extra = true;
-              alone = alone && !(dist_gen(xp, xt) < thr);
+              gap = dist_gen(xp, xt);
+              alone = alone && !(gap < thr);
             }
           }
           r.c2 = S.nxt[r.c1];
@@ -1820,7 +1821,10 @@ __global__ void __launch_bounds__(kRound) k_remove_sweep(const SysConst *__restr
         clear_particle(S, r.inf);
         atomicAdd(&s_hash, event_digest(due.seq + rank, d.itime, NV_EV_REMOVE, r.i - base, r.inf - base));
         if (at < ev_cap) ev[at] = DevEvent{s, due.seq + rank, d.itime, NV_EV_REMOVE, r.i, r.inf};
-        if (extra) atomicAdd(&s_extra, 1);
+        if (extra) {
+          atomicAdd(&s_extra, 1);
+          margin_note(dyn[s], 1, gap, thr);
+        }
       }
       __threadfence_block();
       __syncthreads();
