@@ -110,7 +110,7 @@ struct SysDyn {
   int old_pcount;
   int ins_fallback;  // pinsert needs the serial sweep this step
   int ins_conv;      // pinsert's fixed-point iteration has converged
-  int ins_high, ins_high2;  // elements of its H, of the last walk's H'
+  int ins_high, ins_high2;  // elements of its H; whether the last walk's H' has one
   int noise_counter; // noisey_xflow: 1-based sample in use (xflow_noise_counter)
   int wall_recon_count;  // wall_recon cuts (reconnection.f90:91)
   long long diag[12];  // see nv_diagnostics

@@ -35,7 +35,8 @@ struct TopoBuffers {
   double *xnew = nullptr;   // per insertion position: new point position [3][T]
   double *unew = nullptr;   // per insertion position: new point velocity [3][T]
   int *segnx = nullptr;     // per insertion position: infront of the original slot
-  int *high = nullptr, *high2 = nullptr;  // per system, from its first slot: higher-order insertion positions
+  unsigned *high = nullptr, *high2 = nullptr;  // bit sets of higher-order insertion positions, H and H'
+  int *high_before = nullptr;                  // per word of H: its elements before the word
   unsigned *l0 = nullptr, *l1 = nullptr;  // sweep bitmaps
   // pinsert's measured segment lengths (total_length, line.f90:39): per slot the distance the
   // sweep used, and per inserting slot the distance its new point measured when the sweep
@@ -438,6 +439,33 @@ __device__ __forceinline__ void ghost_of(const SysConst &sc, const double x[3], 
 // tested again by the reference and may insert in turn; k_ins_chain resolves those
 // higher-order insertions by a fixed-point iteration over their positions.
 
+// The higher-order positions, a bit per slot: system s's words start at high_word(sc, s), bit k of
+// them is its slot k; `before` is known of H once it is not empty.
+struct HighSets {
+  unsigned *h, *h2;  // H, H'
+  int *before;
+  int nsys;
+  // slot g's share of emptying both (a pass over 0 <= g <= T clears their (T >> 5) + nsys + 1 words)
+  __device__ __forceinline__ void clear(long long g, long long T) const {
+    if ((g & 31) == 0) h[g >> 5] = h2[g >> 5] = 0;
+    if (g < nsys) h[(T >> 5) + 1 + g] = h2[(T >> 5) + 1 + g] = 0;
+  }
+};
+__host__ __device__ __forceinline__ long long high_word(long long base, int s) { return (base >> 5) + s; }
+struct HighRef {
+  unsigned *h, *h2;
+  int *before, base;
+  __device__ HighRef(const HighSets &H, const SysConst &sc, int s)
+      : h(H.h + high_word(sc.base, s)), h2(H.h2 + high_word(sc.base, s)), before(H.before + high_word(sc.base, s)),
+        base(sc.base) {}
+  __device__ int rank(int g) const {  // elements of H below g
+    const int k = g - base;
+    return before[k >> 5] + __popc(h[k >> 5] & ((1u << (k & 31)) - 1u));
+  }
+  __device__ bool has(int g) const { return h[(g - base) >> 5] >> ((g - base) & 31) & 1u; }
+  __device__ void put(int e) const { atomicOr(&h2[(e - base) >> 5], 1u << ((e - base) & 31)); }
+};
+
 struct InsTest {
   double stale, fresh;  // the two lengths
   int st, fr;           // the two tests
@@ -487,10 +515,11 @@ __global__ void __launch_bounds__(kPassThreads) k_ins_mark(const SysConst *__res
                                                           const double *__restrict__ X, const double *__restrict__ GI,
                                                           const int *__restrict__ nxt, const int *__restrict__ prv,
                                                           int *dec, double *seglen, Lists<3> L, unsigned *l0,
-                                                          unsigned *l1, long long T, unsigned *err) {
+                                                          unsigned *l1, HighSets H, long long T, unsigned *err) {
   const bool run = !*(volatile unsigned *)err;
   ordered_lists(L, T, err, [&](long long gl) -> unsigned {
     clear_bits(l0, l1, gl, T);  // extra visits of the serial sweep start empty
+    H.clear(gl, T);
     if (gl >= T) return 0u;
     const int g = (int)gl, s = sys_of[g];
     const SysConst &sc = scs[s];
@@ -604,7 +633,11 @@ __global__ void __launch_bounds__(kTotalThreads) k_ins_total(const SysConst *__r
 // segment from its neighbours, so it inserts only in a segment of more than twice delta.  Where
 // it finds some, the walk is repeated from H' -- over the whole GPU for large handles, by a block
 // per system for the others (k_ins_rounds).  A system that has not converged after a fixed
-// number of rounds, or whose H outgrows a block's list, runs the serial sweep.
+// number of rounds runs the serial sweep.
+//
+// H and H' are sets: while H is not yet consistent, sub-chains of different chains can run
+// through the same slot (a new point's rank is then that of the original insertion after it) and
+// each puts it into H'.  So they are bits, one per slot, not lists of what the chains found.
 struct ChainArgs {
   State S;
   const int *pos_c, *list_c, *pos_b, *list_b, *dec;
@@ -712,26 +745,10 @@ __device__ void ins_chain_walk(const ChainArgs &A, const SysConst &sc, SysDyn &d
   }
 }
 
-// Elements below g of the sorted list h[0 .. n), and whether it holds g.
-__device__ __forceinline__ int rank_in(const int *h, int n, int g) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (h[mid] < g) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-__device__ __forceinline__ bool holds(const int *h, int n, int g) {
-  const int r = rank_in(h, n, g);
-  return r < n && h[r] == g;
-}
-
-// One walk: a thread per original insertion, chain heads only, from the system's H (high, sorted,
-// ins_high elements); H' goes to high2.
+// One walk: a thread per original insertion, chain heads only, from the system's H (ins_high
+// elements); H' is built in h2 (ins_high2: it has an element).
 __global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, ChainArgs A,
-                            const int *__restrict__ high, int *high2, const int *__restrict__ nev_total,
-                            const unsigned *err) {
+                            HighSets H, const int *__restrict__ nev_total, const unsigned *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= *nev_total || *err) return;
   const int k = A.list_c[t];
@@ -740,11 +757,14 @@ __global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   if (d.ins_conv || d.ins_fallback) return;
-  const int n = d.ins_high;
-  const int *h = high + sc.base;
+  const bool any = d.ins_high > 0;
+  const HighRef R(H, sc, s);
   ins_chain_walk(
-      A, sc, d, k, [&](int g) { return n ? rank_in(h, n, g) : 0; },
-      [&](int e) { high2[sc.base + atomicAdd(&d.ins_high2, 1)] = e; });  // (slots of the system: at most cap)
+      A, sc, d, k, [&](int g) { return any ? R.rank(g) : 0; },
+      [&](int e) {
+        R.put(e);
+        *(volatile int *)&d.ins_high2 = 1;
+      });
 }
 
 // Slots of a handle from which every walk runs over the whole GPU (two launches a round, whether
@@ -752,49 +772,73 @@ __global__ void k_ins_chain(const SysConst *__restrict__ scs, SysDyn *dyn, const
 // 30,000 insertions: 1.7 ms a walk; 32,768 points, 240 insertions: 20 us).
 constexpr long long kAgainSlots = 1 << 18;
 
-constexpr int kHighCap = 2048, kHighThreads = 256;
+constexpr int kHighThreads = 512;
 
-// v[0 .. m) in ascending order, by a block (bitonic, padded to a power of two with room for it).
-__device__ void sort_block(int *v, int m) {
-  int p = 1;
-  while (p < m) p <<= 1;
-  for (int i = m + threadIdx.x; i < p; i += blockDim.x) v[i] = INT_MAX;
-  __syncthreads();
-  for (int k = 2; k <= p; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < p; i += blockDim.x) {
-        const int o = i ^ j;
-        if (o > i && ((v[i] > v[o]) == ((i & k) == 0))) {
-          const int x = v[i];
-          v[i] = v[o];
-          v[o] = x;
-        }
-      }
-      __syncthreads();
+// H' takes H's place and is emptied; the elements before each word of it; by a block, a strip of
+// words per thread, eight loads in flight.  Returns the number of elements.
+__device__ int take_high(const HighRef &R, int words) {
+  __shared__ int s_part[kHighThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int strip = (words + kHighThreads - 1) / kHighThreads;
+  const int w0 = min(words, tid * strip), w1 = min(words, w0 + strip);
+  constexpr int kU = 8;
+  unsigned v[kU];
+  auto strip_of = [&](const unsigned *p, auto f) {
+    for (int w = w0; w < w1; w += kU) {
+#pragma unroll
+      for (int u = 0; u < kU; ++u) v[u] = w + u < w1 ? p[w + u] : 0u;
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (w + u < w1) f(w + u, v[u]);
     }
+  };
+  int c = 0;
+  strip_of(R.h2, [&](int w, unsigned b) {
+    R.h[w] = b;
+    R.h2[w] = 0;
+    c += __popc(b);
+  });
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) s_part[wid] = incl;
+  __syncthreads();
+  int at = incl - c, total = 0;
+  for (int q = 0; q < kHighThreads / 32; ++q) {
+    if (q < wid) at += s_part[q];
+    total += s_part[q];
+  }
+  strip_of(R.h, [&](int w, unsigned b) {
+    R.before[w] = at;
+    at += __popc(b);
+  });
+  __syncthreads();
+  return total;
 }
 
 // After walk `it` of `iters` over the whole GPU, a block per system: converged where H' equals H,
-// else H' (sorted) takes H's place; the last walk leaves the others to the serial sweep.
+// else H' takes H's place; the last walk leaves the others to the serial sweep.
 // `rounds`: instead of waiting for the next walk, the block makes the further ones itself.
 __global__ void __launch_bounds__(kHighThreads) k_ins_rounds(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
-                                                             ChainArgs A, int *high, const int *__restrict__ high2,
-                                                             int it, int iters, bool rounds, const unsigned *err) {
-  __shared__ int h[2][kHighCap];
-  __shared__ int s_n;
+                                                             ChainArgs A, HighSets H, int it, int iters, bool rounds,
+                                                             const unsigned *err) {
+  __shared__ int s_any;
   const int s = blockIdx.x, tid = threadIdx.x;
   if (s >= nsys || *err || walled(scs[s])) return;
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   int n = d.ins_high;
-  int m = d.ins_high2;
+  const bool any = d.ins_high2;
   const bool gave_up = *(volatile int *)&d.ins_fallback || iters == 0, conv = d.ins_conv;
   __syncthreads();
   if (conv) return;
-  if (gave_up || m > kHighCap || (n == 0 && m == 0)) {
+  if (gave_up || (n == 0 && !any)) {
     if (tid == 0) {
       if (!gave_up) d.diag[6] = it;
-      if (gave_up || m) {
+      if (gave_up) {
         d.ins_fallback = 1;
         d.ins_high = 0;
       } else {
@@ -803,47 +847,31 @@ __global__ void __launch_bounds__(kHighThreads) k_ins_rounds(const SysConst *__r
     }
     return;
   }
-  for (int i = tid; i < n; i += kHighThreads) h[0][i] = high[sc.base + i];
-  for (int i = tid; i < m; i += kHighThreads) h[1][i] = high2[sc.base + i];
-  __syncthreads();
+  const HighRef R(H, sc, s);
+  const int words = (d.pcount >> 5) + 1;  // the sweep reaches slots up to pcount
   const int c0 = A.pos_c[sc.base], c1 = A.pos_c[sc.base + sc.cap + 1];
-  int cur = 0;
-  bool done = false;
+  bool done = false, open = false;
   for (;;) {
-    const int *hc = h[cur];
-    int *hn = h[cur ^ 1];
-    sort_block(hn, m);
-    bool differ = m != n;
-    for (int i = tid; i < min(m, n); i += kHighThreads) differ |= hc[i] != hn[i];
-    done = __syncthreads_or(differ) == 0;
+    unsigned differ = 0;
+#pragma unroll 8
+    for (int w = tid; w < words; w += kHighThreads) differ |= R.h[w] ^ R.h2[w];
+    done = __syncthreads_or(differ != 0) == 0;
     if (done || it >= iters) break;
-    cur ^= 1;
-    n = m;
-    if (!rounds) break;
+    n = take_high(R, words);
+    open = !rounds;
+    if (open) break;
     ++it;
-    if (tid == 0) s_n = 0;
-    __syncthreads();
     for (int t = c0 + tid; t < c1; t += kHighThreads) {
       const int k = A.list_c[t];
       if (A.dec[k] & 8) continue;
-      ins_chain_walk(
-          A, sc, d, k, [&](int g) { return rank_in(h[cur], n, g); },
-          [&](int e) {
-            const int i = atomicAdd(&s_n, 1);
-            if (i < kHighCap) h[cur ^ 1][i] = e;
-          });
+      ins_chain_walk(A, sc, d, k, [&](int g) { return n ? R.rank(g) : 0; }, [&](int e) { R.put(e); });
     }
+    if (tid == 0) s_any = 0;
     __syncthreads();
-    m = s_n;
-    if (m > kHighCap || *(volatile int *)&d.ins_fallback) {
-      it = iters;
-      break;
-    }
+    if (*(volatile int *)&d.ins_fallback) s_any = 1;
+    __syncthreads();
+    if (s_any) break;  // out of slots
   }
-  __syncthreads();
-  const bool open = !done && it < iters;
-  if (done || open)
-    for (int i = tid; i < n; i += kHighThreads) high[sc.base + i] = h[cur][i];
   if (tid == 0) {
     d.diag[6] = it;
     d.ins_high = done || open ? n : 0;
@@ -857,7 +885,7 @@ __global__ void __launch_bounds__(kHighThreads) k_ins_rounds(const SysConst *__r
 // thread per original insertion, following its sub-chain.
 __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, State S,
                             const int *__restrict__ pos_c, const int *__restrict__ list_c,
-                            const int *__restrict__ high, const int *__restrict__ newslot, const int *__restrict__ segnx,
+                            HighSets H, const int *__restrict__ newslot, const int *__restrict__ segnx,
                             const double *__restrict__ xnew, const double *__restrict__ unew,
                             const double *__restrict__ dn_new, const int *__restrict__ nev_total, DevEvent *ev,
                             int *ev_count, int ev_cap, unsigned *err) {
@@ -868,8 +896,9 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
   if (dyn[s].ins_fallback) return;
   const SysConst &sc = scs[s];
   const long long T = S.T;
-  const int ev0 = pos_c[sc.base], nh = dyn[s].ins_high;
-  const int *hs = high + sc.base;
+  const int ev0 = pos_c[sc.base];
+  const bool nh = dyn[s].ins_high > 0;
+  const HighRef R(H, sc, s);
   const int seq0 = dyn[s].event_seq, itime = dyn[s].itime;
   const int nx = segnx[k];
   const double zero[3] = {0, 0, 0};
@@ -894,11 +923,11 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
     S.prv[q] = g;
     S.nxt[g] = q;
     if (dn_new[g] >= 0.) S.seglen[q] = dn_new[g];
-    const int seq = seq0 + (pos_c[g] - ev0) + rank_in(hs, nh, g);
+    const int seq = seq0 + (pos_c[g] - ev0) + (nh ? R.rank(g) : 0);
     const int a = atomicAdd(ev_count, 1);
     if (a < ev_cap) ev[a] = DevEvent{s, seq, itime, NV_EV_INSERT, g, q};
     atomicAdd(&dyn[s].ev_hash, event_digest(seq, itime, NV_EV_INSERT, g - sc.base, q - sc.base));
-    if (nh && holds(hs, nh, q)) {  // the sweep reaches q and it inserts
+    if (nh && R.has(q)) {  // the sweep reaches q and it inserts
       g = q;
       continue;
     }
@@ -914,7 +943,7 @@ __global__ void k_ins_apply(const SysConst *__restrict__ scs, SysDyn *dyn, const
 __global__ void k_ins_ghosts(const SysConst *__restrict__ scs, SysDyn *dyn, const int *__restrict__ sys_of, State S,
                              int nsys, const int *__restrict__ pos_a, const int *__restrict__ pos_b,
                              const int *__restrict__ pos_c, const int *__restrict__ list_c,
-                             const int *__restrict__ high, const int *__restrict__ newslot,
+                             HighSets H, const int *__restrict__ newslot,
                              const int *__restrict__ nev_total, unsigned *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (*err) return;
@@ -940,8 +969,8 @@ __global__ void k_ins_ghosts(const SysConst *__restrict__ scs, SysDyn *dyn, cons
   const int s = sys_of[k];
   if (dyn[s].ins_fallback) return;
   const SysConst &sc = scs[s];
-  const int nh = dyn[s].ins_high;
-  const int *hs = high + sc.base;
+  const bool nh = dyn[s].ins_high > 0;
+  const HighRef R(H, sc, s);
   refresh_ghosts(sc, S, k);
   int q = newslot[k];
   for (int hops = 0;; ++hops) {
@@ -950,7 +979,7 @@ __global__ void k_ins_ghosts(const SysConst *__restrict__ scs, SysDyn *dyn, cons
       return;
     }
     refresh_ghosts(sc, S, q);
-    if (!(nh && holds(hs, nh, q))) break;
+    if (!(nh && R.has(q))) break;
     q = newslot[q];
   }
   refresh_ghosts(sc, S, S.nxt[q]);
@@ -2179,8 +2208,10 @@ void topo_alloc(nv_handle *h) {
   cudaMalloc(&tb->xnew, 3 * n * sizeof(double));
   cudaMalloc(&tb->unew, 3 * n * sizeof(double));
   cudaMalloc(&tb->segnx, n * sizeof(int));
-  cudaMalloc(&tb->high, n * sizeof(int));
-  cudaMalloc(&tb->high2, n * sizeof(int));
+  const size_t hw = high_word(h->T, h->nsys) + 1;
+  cudaMalloc(&tb->high, hw * sizeof(unsigned));
+  cudaMalloc(&tb->high2, hw * sizeof(unsigned));
+  cudaMalloc(&tb->high_before, hw * sizeof(int));
   pass_alloc(&tb->pass_state, &tb->pass_ctl, 3, h->T);
   cudaFuncSetAttribute(k_recon_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReconSmem);
   cudaMalloc(&tb->l0, (n / 32 + 2) * sizeof(unsigned));
@@ -2245,7 +2276,7 @@ void topo_free(nv_handle *h) {
   cudaFree(tb->pos_c); cudaFree(tb->list_c);
   cudaFree(tb->pass_state); cudaFree(tb->pass_ctl);
   cudaFree(tb->dec); cudaFree(tb->newslot); cudaFree(tb->xnew);
-  cudaFree(tb->unew); cudaFree(tb->segnx); cudaFree(tb->high); cudaFree(tb->high2);
+  cudaFree(tb->unew); cudaFree(tb->segnx); cudaFree(tb->high); cudaFree(tb->high2); cudaFree(tb->high_before);
   cudaFree(tb->l0); cudaFree(tb->l1);
   cudaFree(tb->seglen); cudaFree(tb->dn_new);
   cudaFree(tb->psum); cudaFree(tb->pnear); cudaFree(tb->part_done);
@@ -2262,8 +2293,9 @@ void launch_pinsert(nv_handle *h) {
   const long long T = h->T;
   const Lists<3> lists{{tb->pos_a, tb->pos_b, tb->pos_c}, {tb->list_a, tb->list_b, tb->list_c},
                        {tb->pass_state, tb->pass_ctl}};
+  const HighSets H{tb->high, tb->high2, tb->high_before, h->nsys};
   k_ins_mark<<<pass_grid(h), kPassThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, h->x, h->gi, h->nxt, h->prv,
-                                                           tb->dec, tb->seglen, lists, tb->l0, tb->l1, T, h->d_err);
+                                                           tb->dec, tb->seglen, lists, tb->l0, tb->l1, H, T, h->d_err);
   const State S = make_state(h);
   const ChainArgs A{S,          tb->pos_c, tb->list_c, tb->pos_b, tb->list_b, tb->dec,
                     tb->newslot, tb->segnx, tb->xnew,  tb->unew,  tb->dn_new};
@@ -2273,18 +2305,18 @@ void launch_pinsert(nv_handle *h) {
   const int *nev = tb->pos_c + T;
   const bool large = T > kAgainSlots;
   for (int it = 1; it <= (large ? h->ins_iters : std::min(h->ins_iters, 1)); ++it) {
-    k_ins_chain<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, A, tb->high, tb->high2, nev, h->d_err);
-    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, tb->high, tb->high2, it,
+    k_ins_chain<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, A, H, nev, h->d_err);
+    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, H, it,
                                                           h->ins_iters, !large, h->d_err);
   }
   if (h->ins_iters == 0)
-    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, tb->high, tb->high2, 0, 0, false,
+    k_ins_rounds<<<h->nsys, kHighThreads, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, A, H, 0, 0, false,
                                                           h->d_err);
-  k_ins_apply<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->pos_c, tb->list_c, tb->high,
+  k_ins_apply<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, tb->pos_c, tb->list_c, H,
                                            tb->newslot, tb->segnx, tb->xnew, tb->unew, tb->dn_new, nev, h->d_events,
                                            h->d_event_count, h->event_cap, h->d_err);
   k_ins_ghosts<<<grid, 128, 0, h->stream>>>(h->d_sc, h->d_dyn, h->sys_of, S, h->nsys, tb->pos_a, tb->pos_b, tb->pos_c,
-                                            tb->list_c, tb->high, tb->newslot, nev, h->d_err);
+                                            tb->list_c, H, tb->newslot, nev, h->d_err);
   // systems with an insertion the parallel form cannot place
   k_insert_sweep<<<h->nsys, 32, 0, h->stream>>>(h->d_sc, h->d_dyn, h->nsys, S, tb->pos_a, tb->list_a, tb->pos_b,
                                                 tb->list_b, Sweep{tb->l0, tb->l1, T}, h->d_err, h->d_events,
