@@ -1728,6 +1728,7 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_tree_walk_mixed(
     TreeBuffers tb, double near_factor, Fp32Guards gd, unsigned *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WalkShared<W> &S = *reinterpret_cast<WalkShared<W> *>(smem_raw);
+  __shared__ int s_abort;  // one thread reads the error word: blocks of this launch may set it meanwhile
   constexpr unsigned kAll = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int2 w = work[blockIdx.x];  // system, first position
@@ -1737,7 +1738,8 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_tree_walk_mixed(
   const int k = g - sc.base;
   // A walk range's ends fall on group boundaries (nv_set_walk_range): a group walks all its
   // targets or none, so its rounds and partial sums are the same as without a range.
-  const bool valid = !*err && k >= 1 && k <= dyn[w.x].pcount && nxt[g] != 0 && q >= sc.walk_lo && q < sc.walk_hi;
+  const bool valid = k >= 1 && k <= dyn[w.x].pcount && nxt[g] != 0 && q >= sc.walk_lo && q < sc.walk_hi;
+  if (tid == 0) s_abort = (*err != 0);
   unsigned evals = 0, tests = 0, n64 = 0, nband = 0;
   double xi[3] = {0, 0, 0};
   int pi_ = 0;
@@ -1757,6 +1759,7 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_tree_walk_mixed(
   }
   for (int i = tid; i < 3 * n_img; i += 32 * W) S.shift[i / 3][i % 3] = i < 3 ? 0.0 : sc.shift[i / 3 - 1][i % 3];
   __syncthreads();
+  if (s_abort) return;
   // the root's test in every image from the centre estimate: accepted (nothing to add), opened
   // (the walk starts at its children) or undecided: the target is redone whole once the exact
   // centre is known
