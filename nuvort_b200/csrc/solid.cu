@@ -88,6 +88,16 @@ __device__ void loop_killer(const SolidState &S, SysDyn &d, int s, int base, int
 // precon 296 -> 5 (before: one thread per system).
 constexpr int kSweep = 256;
 
+// Whether an earlier launch failed.  One thread reads the error word for the block: other
+// systems' blocks of this launch may set it meanwhile (pinsert's), and a block whose threads
+// disagreed would part at the sweep's barriers.
+__device__ bool failed_before(const unsigned *err) {
+  __shared__ unsigned s_err;
+  if (threadIdx.x == 0) s_err = *err;
+  __syncthreads();
+  return s_err != 0;
+}
+
 template <class Test, class Passed, class After, class Act>
 __device__ void ordered_sweep(int base, int n, Test test, Passed passed, After after, Act act) {
   __shared__ int s_first;
@@ -133,7 +143,7 @@ __global__ void __launch_bounds__(kSweep) k_solid_pinsert(const SysConst *__rest
                                                           SolidState S, unsigned *err) {
   __shared__ double s_len[kSweep];
   const int s = blockIdx.x, tid = threadIdx.x;
-  if (s >= nsys || *err || !solid_system(scs[s])) return;
+  if (s >= nsys || !solid_system(scs[s]) || failed_before(err)) return;
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   const int base = sc.base;
@@ -241,7 +251,7 @@ __device__ bool clear_wall_pair(const SolidState &S, SysDyn &d, int s, int base,
 __global__ void __launch_bounds__(kSweep) k_solid_precon(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
                                                          SolidState S, const unsigned *err) {
   const int s = blockIdx.x;
-  if (s >= nsys || *err || !solid_system(scs[s])) return;
+  if (s >= nsys || !solid_system(scs[s]) || failed_before(err)) return;
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   if ((d.itime % sc.recon_shots) != 0) return;
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(kSweep) k_solid_precon(const SysConst *__restr
 __global__ void __launch_bounds__(kSweep) k_solid_wall_recon(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
                                                              SolidState S, const unsigned *err) {
   const int s = blockIdx.x;
-  if (s >= nsys || *err || !solid_system(scs[s])) return;
+  if (s >= nsys || !solid_system(scs[s]) || failed_before(err)) return;
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   if ((d.itime % sc.recon_shots) != 0) return;
@@ -373,7 +383,7 @@ __global__ void __launch_bounds__(kSweep) k_solid_wall_recon(const SysConst *__r
 __global__ void __launch_bounds__(kSweep) k_solid_premove(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
                                                           SolidState S, const unsigned *err) {
   const int s = blockIdx.x;
-  if (s >= nsys || *err || !solid_system(scs[s])) return;
+  if (s >= nsys || !solid_system(scs[s]) || failed_before(err)) return;
   const SysConst &sc = scs[s];
   SysDyn &d = dyn[s];
   if ((d.itime % sc.recon_shots) != 0) return;

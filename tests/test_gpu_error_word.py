@@ -4,7 +4,7 @@ then takes good states and gives what a new handle gives."""
 import numpy as np
 import pytest
 
-from helpers import config1_params, tangle
+from helpers import config0_params, config1_params, tangle
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +34,34 @@ def test_singular_pair_in_one_system(precision, parts):
             h.upload(5, good[5])
             for s in (0, 5, 12):
                 assert np.array_equal(h.calc_velocity(s), want[s])
+
+
+@pytest.mark.parametrize("what", ["capacity", "empty"])
+def test_walled_system_that_cannot_insert(what):
+    # 40 walled systems, each with hundreds of insertions; one has no room for its own, or no line
+    from nuvort_b200.api import Handle, NuvortError
+    from nuvort_b200.rings import half_loop
+    p = config0_params(dt=2e-7, delta=0.0003, boundary_x="solid", boundary_y="periodic", boundary_z="periodic")
+    good = [half_loop(250 + 3 * i, 0.0005) for i in range(40)]
+    good[7] = half_loop(200, 0.0003)  # inserts nothing
+    caps = [1200] * 40
+    caps[7] = 300
+    bad = half_loop(271, 0.0005)
+    if what == "empty":
+        bad.infront[:] = bad.behind[:] = bad.pinnedi[:] = bad.pinnedb[:] = 0
+    with Handle([p] * 40, caps, states=good) as h:
+        h.step(2)
+        want = [h.download(s) for s in range(40)]
+        for _ in range(REPEATS):
+            for s in range(40):
+                h.upload(s, bad if s == 7 else good[s])
+                h.set_clock(s, 0.0, 0)
+            with pytest.raises(NuvortError, match="capacity" if what == "capacity" else "length is 0"):
+                h.step(2)
+        for s in range(40):
+            h.upload(s, good[s])
+            h.set_clock(s, 0.0, 0)
+        h.step(2)
+        for s in range(40):
+            a = h.download(s)
+            assert np.array_equal(a.x, want[s].x) and np.array_equal(a.infront, want[s].infront)
