@@ -43,6 +43,7 @@ __device__ __noinline__ double3 direct_term64(const double4 *__restrict__ rec, d
 struct MixedTarget : LaneTarget {
   double x[3], s[3];  // position, image shift
   int behind, own;    // segments (from 0) that are skipped
+  int n;              // segments of the system: the last pair's second half may lie past them
   bool active;
 };
 
@@ -74,7 +75,7 @@ __device__ __forceinline__ void pair_guarded(const PairVec &r, const PairSeg &d,
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
       const int j = 2 * p + h;
-      if (!(h ? bad[1] : bad[0]) || j == t.behind || j == t.own) continue;
+      if (!(h ? bad[1] : bad[0]) || j >= t.n || j == t.behind || j == t.own) continue;
       const double3 v = direct_term64(seg64 + 2 * (long long)j, t.s[0], t.s[1], t.s[2], t.x[0], t.x[1], t.x[2], gq64);
       n[0] += v.x;
       n[1] += v.y;
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
   // without one is far from everything.  The behind segment is skipped in every image, the
   // target's own in the central one (their pairs take the guarded path, which skips them).
   t.behind = t.own = -1;
+  t.n = pc;
   for (int c = 0; c < 3; ++c) {
     t.s[c] = m > 0 ? sc.shift[m - 1][c] : 0.0;
     t.x[c] = -1e9;
