@@ -702,6 +702,9 @@ int nv_create(const nv_params *params, int32_t nsys, const int32_t *capacity, in
       cudaEventCreateWithFlags(&h->fork2_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->join2_ev, cudaEventDisableTiming) != cudaSuccess)
     return bail(set_error(NV_ERR_CUDA, "stream creation failed"));
+  if (direct_kernels_setup() != cudaSuccess || mixed_kernels_setup() != cudaSuccess ||
+      tree_kernels_setup() != cudaSuccess)
+    return bail(set_error(NV_ERR_CUDA, "shared-memory limit of a kernel"));
   const long long T = h->T;
   if ((rc = dalloc(&h->d_sc, nsys)) || (rc = dalloc(&h->d_dyn, nsys)) || (rc = dalloc(&h->x, 3 * T)) ||
       (rc = dalloc(&h->u, 3 * T)) || (rc = dalloc(&h->u1, 3 * T)) || (rc = dalloc(&h->u2, 3 * T)) ||

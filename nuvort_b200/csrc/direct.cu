@@ -399,9 +399,6 @@ __global__ void __launch_bounds__(kSplitThreads, G == 8 ? 2 : 3) k_direct_fp64_s
 template <int G>
 void launch_split(cudaStream_t st, const nv_handle *h, const int2 *work, int nwork, const int *targets, int ntargets,
                   double *Uout) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_direct_fp64_split<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem(G));
-  (void)attr;
   k_direct_fp64_split<G><<<nwork, kSplitThreads, split_smem(G), st>>>(h->d_sc, h->d_dyn, work, h->x, h->gi, h->gb, h->nxt, h->prv,
                                                    h->seg, h->u, h->T, h->d_err, targets, ntargets, Uout);
 }
@@ -416,7 +413,18 @@ void launch_split_g(int G, cudaStream_t st, const nv_handle *h, const int2 *work
   }
 }
 
+template <int G>
+cudaError_t allow_split() {
+  return cudaFuncSetAttribute(k_direct_fp64_split<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem(G));
+}
+
 }  // namespace
+
+cudaError_t direct_kernels_setup() {
+  for (cudaError_t e : {allow_split<1>(), allow_split<2>(), allow_split<4>(), allow_split<8>()})
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
 
 // Direct-sum targets per block in use for this many target slots (direct_split, set by
 // nv_set_direct_split, overrides the choice): 8 per block of the split kernel, except

@@ -118,6 +118,11 @@ const int *tree_iperm(nv_handle *h);  // slot -> walk position of the last tree 
 const int *tree_perm(nv_handle *h);   // walk position (global: base + q) -> slot
 // tree (tree.cu)
 constexpr int kMaxWalkParts = 8;
+// The kernels that need more shared memory than a launch gets unasked, on the current device (the
+// limit is the device's, not the process's): by every handle at its creation.
+cudaError_t direct_kernels_setup();
+cudaError_t mixed_kernels_setup();
+cudaError_t tree_kernels_setup();
 int n_sms_host();                  // SMs of the current device
 void tree_alloc(nv_handle *h);
 void tree_free(nv_handle *h);

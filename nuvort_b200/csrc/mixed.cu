@@ -252,11 +252,12 @@ __global__ void k_mixed_combine(const SysConst *__restrict__ scs, const SysDyn *
 
 }  // namespace
 
+cudaError_t mixed_kernels_setup() {
+  return cudaFuncSetAttribute(k_direct_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMixedSmem);
+}
+
 void launch_direct_mixed(nv_handle *h) {
   if (h->n_work_img == 0) return;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(k_direct_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMixedSmem);
-  (void)attr;
   k_direct_mixed<<<h->n_work_img, kTB, kMixedSmem, h->stream>>>(
       h->d_sc, h->d_dyn, h->d_work_img, h->x, h->nxt, h->prv, h->seg32, h->seg, h->partial, h->T, h->near_factor, h->guards,
       h->d_err);

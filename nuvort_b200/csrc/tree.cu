@@ -2319,14 +2319,21 @@ void launch_tree_walk(nv_handle *h) {
 namespace {
 template <int W>
 void launch_walk(nv_handle *h) {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_tree_walk_mixed<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared<W>));
-  (void)attr;
   k_tree_walk_mixed<W><<<h->n_work_grp, 32 * W, sizeof(WalkShared<W>), h->stream>>>(
       h->d_sc, h->d_dyn, h->d_work_grp, h->x, h->nxt, h->prv, h->partial, h->T, *h->tree, h->near_factor, h->guards,
       h->d_err);
 }
+template <int W>
+cudaError_t allow_walk() {
+  return cudaFuncSetAttribute(k_tree_walk_mixed<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WalkShared<W>));
+}
 }  // namespace
+
+cudaError_t tree_kernels_setup() {
+  for (cudaError_t e : {allow_walk<1>(), allow_walk<2>(), allow_walk<4>(), allow_walk<8>()})
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
 
 void launch_tree_walk_mixed(nv_handle *h) {
   TreeBuffers *tb = h->tree;
