@@ -47,6 +47,21 @@ struct MixedTarget : LaneTarget {
   bool active;
 };
 
+// The halves of pair p that this lane's guards send to FP64, into n.
+__device__ __forceinline__ void add_exact(const bool bad[2], const MixedTarget &t, int p,
+                                          const double4 *__restrict__ seg64, double gq64, double n[3]) {
+  if (!(t.active && (bad[0] || bad[1]))) return;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int j = 2 * p + h;
+    if (!(h ? bad[1] : bad[0]) || j >= t.n || j == t.behind || j == t.own) continue;
+    const double3 v = direct_term64(seg64 + 2 * (long long)j, t.s[0], t.s[1], t.s[2], t.x[0], t.x[1], t.x[2], gq64);
+    n[0] += v.x;
+    n[1] += v.y;
+    n[2] += v.z;
+  }
+}
+
 // A pair that some lane of the warp is not far from: every lane's own guards decide between
 // FP32 and FP64 (into n).
 __device__ __forceinline__ void pair_guarded(const PairVec &r, const PairSeg &d, const MixedTarget &t, int p,
@@ -71,27 +86,51 @@ __device__ __forceinline__ void pair_guarded(const PairVec &r, const PairSeg &d,
   u[0] = fma2(ff, g.cx, u[0]);
   u[1] = fma2(ff, g.cy, u[1]);
   u[2] = fma2(ff, g.cz, u[2]);
-  if (t.active && (bad[0] || bad[1])) {
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      const int j = 2 * p + h;
-      if (!(h ? bad[1] : bad[0]) || j >= t.n || j == t.behind || j == t.own) continue;
-      const double3 v = direct_term64(seg64 + 2 * (long long)j, t.s[0], t.s[1], t.s[2], t.x[0], t.x[1], t.x[2], gq64);
-      n[0] += v.x;
-      n[1] += v.y;
-      n[2] += v.z;
-    }
+  add_exact(bad, t, p, seg64, gq64, n);
+}
+
+// floats as integers in the same order, and back
+__device__ __forceinline__ int ordered(float x) {
+  const int i = __float_as_int(x);
+  return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float float_of(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+
+// The pairs of a sub-sum (bit p: pair p) with a segment whose line guard may act on a target of the
+// warp: all targets lie within a ball around the point that `c` holds as a target, of radius R, so
+// |r x d| of each is at least |rc x d| - R |d| and |r| at most |rc| + R, and the guard cannot act
+// where |rc x d| exceeds |d| (R + sqrt(line) (|rc| + R)).  A lane takes one pair for all targets.
+struct WarpBall {
+  LaneTarget c;
+  float radius, slope;  // R (1 + sqrt(line)) and sqrt(line), widened for the FP32 rounding
+};
+__device__ __forceinline__ unsigned line_mask(const ulonglong2 *pairs, int np, const WarpBall &ball) {
+  const int lane = threadIdx.x & 31;
+  static_assert(kWarpPairs <= 32, "a lane per pair");
+  bool may = false;
+  if (lane < np) {
+    const PairVec r = pair_vec(pairs + 6 * lane, ball.c);
+    const PairSeg d = pair_seg(pairs + 6 * lane);
+    const f32x2 kMinus = pack2(-1.f, -1.f), radius = pack2(ball.radius, ball.radius), slope = pack2(ball.slope, ball.slope);
+    const f32x2 cx = fma2(r.ry, d.dz, mul2(r.rz, d.ndy)), cy = fma2(r.rz, d.dx, mul2(mul2(r.rx, kMinus), d.dz)),
+                cz = fma2(r.rx, d.dy, mul2(r.ry, d.ndx));
+    const f32x2 reach = fma2(slope, pack2(sqrt_fast(lo2(r.a)), sqrt_fast(hi2(r.a))), radius);
+    const f32x2 cr2 = square2(cx, cy, cz), lim = mul2(square2(d.dx, d.dy, d.dz), mul2(reach, reach));
+    may = lo2(cr2) < lo2(lim) || hi2(cr2) < hi2(lim);
   }
+  return __ballot_sync(0xffffffffu, may);
 }
 
 // Bound: the FP32 pipe (about 35 lane operations a far term, the adds, multiplies and FMAs of
 // two segments packed into one instruction).  A pair of segments that every lane's target is
-// far from needs none of the conditioning guards, nearly all pairs of a tangle; the other
-// pairs take them lane by lane.  The tiles pass through a ring of kStages buffers with an
-// mbarrier for full and one for empty each, so that no warp waits for the block's others.
-// 30,011 points: 39.4 ms; 1,500 points: 147 us (a lane per target and image with scalar
+// far from needs none of the conditioning guards but the line guard, and that only where
+// line_mask, once per sub-sum, finds that it may act; the other pairs take the guards lane by
+// lane.  The tiles pass through a ring of kStages buffers with an mbarrier for full and one
+// for empty each, so that no warp waits for the block's others.
+// 30,011 points: 42.0 ms; 1,501 points: 151 us (a lane per target and image with scalar
 // arithmetic and all guards, 113 issue slots a term: 74.1 ms and 409 us; packed, but all guards
-// and a barrier per tile: 55.4 ms and 236 us).
+// and a barrier per tile: 55.4 ms and 236 us).  The line guard left out beyond 4|d|: 38.8 ms and
+// 136 us; its exact test on every far pair: 44.8 ms and 153 us.
 __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restrict__ scs,
                                                          const SysDyn *__restrict__ dyn,
                                                          const int4 *__restrict__ work, const double *__restrict__ X,
@@ -147,6 +186,27 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
     t.l[c] = pack2(l, l);
   }
   const int behind_p = t.behind >= 0 ? t.behind >> 1 : -1;
+  const bool any = __any_sync(0xffffffffu, t.active);
+  WarpBall ball;
+  {
+    const float sin_line = sqrtf(gd.line);
+    float half2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {  // the ball around the box of the targets, by FP32 positions
+      const float x = (float)t.x[c];
+      const float lo = float_of(__reduce_min_sync(0xffffffffu, t.active ? ordered(x) : INT_MAX)),
+                  hi = float_of(__reduce_max_sync(0xffffffffu, t.active ? ordered(x) : INT_MIN));
+      const float mid = any ? 0.5f * lo + 0.5f * hi : 0.f;
+      const double v = t.s[c] - (double)mid;
+      const float h = (float)v, l = (float)(v - (double)h);
+      const float half = any ? fmaxf(hi - mid, mid - lo) + 1e-6f * fmaxf(fabsf(lo), fabsf(hi)) : 0.f;
+      ball.c.h[c] = pack2(h, h);
+      ball.c.l[c] = pack2(l, l);
+      half2 = fmaf(half, half, half2);
+    }
+    ball.slope = sin_line * 1.00001f + 1e-6f;
+    ball.radius = sqrtf(half2) * (1.00001f + ball.slope);
+  }
   const double gq64 = sc.quant_circ / (4.0 * NV_PI);
   const double nr = near_factor * sc.delta;
   const float near2 = (float)(nr * nr);
@@ -180,19 +240,35 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
     const int p0 = wid * kWarpPairs, p1 = min(min(kPairs, np - k * kPairs), p0 + kWarpPairs);
     if (p0 < p1) {
       const int bp = behind_p - k * kPairs;
+      // the pairs that not every target may take without guards however far it is: a line guard
+      // may act, or the pair holds some target's behind segment
+      unsigned special = line_mask(tile + 6 * p0, p1 - p0, ball) |
+                         __reduce_or_sync(0xffffffffu, bp >= p0 && bp < p1 ? 1u << (bp - p0) : 0u);
       f32x2 u[3] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
 #pragma unroll 2
       for (int p = p0; p < p1; ++p) {
         const ulonglong2 *q = tile + 6 * p;
         const PairVec r = pair_vec(q, t);
         const PairSeg d = pair_seg(q);
-        if (__all_sync(0xffffffffu, lo2(r.a) > lo2(d.far) && hi2(r.a) > hi2(d.far) && p != bp)) {
+        const bool plain = !(special & 1u), far = lo2(r.a) > lo2(d.far) && hi2(r.a) > hi2(d.far);
+        special >>= 1;
+        if (__all_sync(0xffffffffu, far && plain)) {
           const PairGeo g2 = pair_geo(r, d);
           const f32x2 sum = add2(g2.pp, g2.re);
           const f32x2 f = mul2(g2.num, pack2(rcp_fast(lo2(sum)), rcp_fast(hi2(sum))));
           u[0] = fma2(f, g2.cx, u[0]);
           u[1] = fma2(f, g2.cy, u[1]);
           u[2] = fma2(f, g2.cz, u[2]);
+        } else if (__all_sync(0xffffffffu, far && p != bp)) {  // the line guard alone, target by target
+          const PairGeo g2 = pair_geo(r, d);
+          const f32x2 sum = add2(g2.pp, g2.re), c = square2(d.dx, d.dy, d.dz), cr2 = square2(g2.cx, g2.cy, g2.cz);
+          const bool bad[2] = {lo2(cr2) < gd.line * lo2(c) * fminf(lo2(r.a), lo2(g2.ee)),
+                               hi2(cr2) < gd.line * hi2(c) * fminf(hi2(r.a), hi2(g2.ee))};
+          const f32x2 f = mul2(g2.num, pack2(bad[0] ? 0.f : rcp_fast(lo2(sum)), bad[1] ? 0.f : rcp_fast(hi2(sum))));
+          u[0] = fma2(f, g2.cx, u[0]);
+          u[1] = fma2(f, g2.cy, u[1]);
+          u[2] = fma2(f, g2.cz, u[2]);
+          add_exact(bad, t, k * kPairs + p, rec64, gq64, n);
         } else {
           pair_guarded(r, d, t, k * kPairs + p, near2, gd, rec64, gq64, u, n);
         }

@@ -118,6 +118,11 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float rcp_fast(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -133,13 +138,11 @@ __host__ __device__ __forceinline__ long long seg32_at(long long base, int k) {
   return 12 * (base + 1) + 24 * (long long)((k - 1) >> 1);
 }
 
-// Terms beyond far_ratio |d|^2 are taken without the guards: there, beyond 4|d|, the segment
-// subtends less than 30 degrees, r.e > 0 and |e| > 3/4 |r|, so that nothing cancels in FP32 but
-// r x d for a target near the segment's line, whose error stays 2^-24 |r||d|, that of a term
-// off the line.  Guards that a caller widened past these bounds apply to every term.
-inline float far_ratio(const Fp32Guards &g) {
-  return g.angle <= 1.9f && g.end <= 0.5f && g.line <= 1e-3f ? 16.f : 3e38f;
-}
+// Terms beyond far_ratio |d|^2 are taken without the angle and end guards: there, beyond 4|d|,
+// the segment subtends less than 30 degrees, r.e > 0 and |e| > 3/4 |r|, so that neither acts.
+// (The line guard does: r x d cancels for a target near the line however far it is.)  Guards
+// that a caller widened past these bounds apply to every term.
+inline float far_ratio(const Fp32Guards &g) { return g.angle <= 1.9f && g.end <= 0.5f ? 16.f : 3e38f; }
 
 // What a lane holds of its target for the packed terms, and a pair of segments (or accepted
 // tree nodes) as a 24-float record q (see seg32_at): r from the target, its square, the term's
