@@ -55,7 +55,7 @@ struct TopoBuffers {
   int *cell_start = nullptr;        // per cell: first entry in cell_items (exclusive sum, n_cells + 1)
   int *cell_items = nullptr;        // slots grouped by cell
   bool any_cells = false;
-  bool small_pclose = false;  // the tree-less systems' slots are few: a warp per target scans them
+  bool small_pclose = false;  // the tree-less systems' pairs of slots are few: a warp per target scans them
 };
 
 // A system's cell grid over its box [-L/2, L/2)^3 (points outside are clamped to the edge
@@ -369,11 +369,15 @@ __global__ void k_pclose_brute(const SysConst *__restrict__ scs, const SysDyn *_
 
 
 // The same search with a warp per target, each lane over every 32nd slot in ascending order, the
-// lanes' minima combined by (distance, slot), so that ties keep the lowest slot: for systems
-// of a few thousand slots, whose cell lists cost six launches and a search that few threads
-// make, cell after cell (600 points: 16 us, 78 with the cell list; 4,000: 48, 111; but 8,000
-// points: 155, 112).
+// lanes' minima combined by (distance, slot), so that ties keep the lowest slot: for a few
+// systems of a few thousand slots, whose cell lists cost six launches and a search that few
+// threads make, cell after cell (600 points: 16 us, 78 with the cell list; 4,000: 48, 111; but
+// 8,000 points: 155, 112).  Several systems share the GPU, so what counts is their pairs of slots
+// together (8 systems of 2,000 points, 3.9e7 pairs: 60 us, 139; 64 of 600, 4.1e7: 58, 101; but 8
+// of 4,000, 1.4e8: 192, 151; 512 of 300, 1.3e8: 145, 136; 512 of 4,000: 12.2 ms, 1.3), and a
+// warp is launched for every slot of the handle, also of the systems that search the tree.
 constexpr int kPcloseWarps = 4, kPcloseSlots = 6144;
+constexpr long long kPclosePairs = 60'000'000, kPcloseAllSlots = 1 << 17;
 __global__ void __launch_bounds__(32 * kPcloseWarps) k_pclose_warps(
     const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn, const int *__restrict__ sys_of,
     const double *__restrict__ X, const int *__restrict__ nxt, const int *__restrict__ prv, int *__restrict__ cl,
@@ -2250,9 +2254,13 @@ void topo_alloc(nv_handle *h) {
     G.base = cells;
     cells += (long long)G.nc[0] * G.nc[1] * G.nc[2];
   }
+  long long pairs = 0;
   for (int s = 0; s < h->nsys; ++s)
-    if (!h->sc[s].use_tree) most = std::max(most, h->cap[s]);
-  tb->small_pclose = most <= kPcloseSlots;
+    if (!h->sc[s].use_tree) {
+      most = std::max(most, h->cap[s]);
+      pairs += (long long)h->cap[s] * h->cap[s];
+    }
+  tb->small_pclose = most <= kPcloseSlots && pairs <= kPclosePairs && h->T <= kPcloseAllSlots;
   tb->n_cells = cells;
   tb->any_cells = cells > 0 && cells < (1LL << 30);
   if (tb->any_cells) {
