@@ -201,17 +201,18 @@ __device__ __forceinline__ bool failed_above(const TreeBuffers &tb, int level) {
 }
 
 // What a node's split reserves: child ids, member slots, entries of the next level's block
-// and warp split lists, entries of the block-summed node list.
+// and warp split lists (kList), entries of the block-summed node list.
 struct SplitNeeds {
   int nchild, kept, nblk, nwrp, nbig;
 };
+template <bool kList = true>
 __device__ SplitNeeds split_needs(const int cnt[8]) {
   SplitNeeds n{0, 0, 0, 0, 0};
 #pragma unroll
   for (int d = 0; d < 8; ++d) {
     n.nchild += cnt[d] != 0;
     n.kept += cnt[d];
-    if (cnt[d] >= 2) {
+    if (kList && cnt[d] >= 2) {
       if (cnt[d] > kBigNode) ++n.nblk;
       else ++n.nwrp;
     }
@@ -224,6 +225,7 @@ __device__ SplitNeeds split_needs(const int cnt[8]) {
 // fit the buffers (error set).  The counters have then moved past entries never written, which
 // the levels below, the sums and the walks must not read: they return (failed_above).  (Marking
 // the entries unused here instead cost the levels' kernel 36 of 157 us at 32,768 points.)
+template <bool kList = true>
 __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const SplitNeeds &n, int id0, int mb0,
                                int qb, int qw, int qg, unsigned *err) {
   if (id0 + n.nchild > tb.max_nodes || (long long)mb0 + n.kept > tb.max_members || qb + n.nblk > tb.max_blk ||
@@ -252,7 +254,7 @@ __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const S
     tb.nR[id] = make_int2(mb0 + off, cnt[d]);
     tb.nDepth[id] = depth;
     tb.nKids[id] = 0;
-    if (cnt[d] >= 2) {  // the child's level list of nodes still to split
+    if (kList && cnt[d] >= 2) {  // the child's level list of nodes still to split
       if (cnt[d] > kBigNode) tb.split_blk[lb][qb + kb++] = id;
       else tb.split_wrp[lb][qw + kw++] = id;
     }
@@ -267,9 +269,10 @@ __device__ bool write_children(TreeBuffers &tb, int p, const int cnt[8], const S
 
 // Create the non-empty children of node p (counts cnt[0..7]); returns first child id via
 // *id0 and member base via *mb0 (or -1 on overflow).  Called by one thread.
+template <bool kList = true>
 __device__ void make_children(TreeBuffers &tb, int p, const int cnt[8], int *id0_out, int *mb0_out, unsigned *err) {
   *id0_out = *mb0_out = -1;
-  const SplitNeeds nd = split_needs(cnt);
+  const SplitNeeds nd = split_needs<kList>(cnt);
   if (nd.nchild == 0) return;
   // one reservation per counter for the whole node, the atomics issued together
   const int lb = (tb.nDepth[p] + 1) % 3;
@@ -278,7 +281,7 @@ __device__ void make_children(TreeBuffers &tb, int p, const int cnt[8], int *id0
   const int qb = nd.nblk ? atomicAdd(&tb.ctr[kCtrSplit + lb], nd.nblk) : 0;
   const int qw = nd.nwrp ? atomicAdd(&tb.ctr[kCtrSplit + 3 + lb], nd.nwrp) : 0;
   const int qg = nd.nbig ? atomicAdd(&tb.ctr[kCtrBig], nd.nbig) : 0;
-  if (!write_children(tb, p, cnt, nd, id0, mb0, qb, qw, qg, err)) return;
+  if (!write_children<kList>(tb, p, cnt, nd, id0, mb0, qb, qw, qg, err)) return;
   *id0_out = id0;
   *mb0_out = mb0;
 }
@@ -467,18 +470,19 @@ __device__ __forceinline__ int *split_ctr(TreeBuffers &tb, int c, int lb) {
 }
 
 // Node p split by the whole warp: count, lane 0 reserves and writes the children, scatter.
+template <bool kList = true>
 __device__ void warp_split_one(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int lane, int lb,
                                unsigned *err) {
   int cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   warp_count(X, T, tb, p, lane, cnt);
-  const SplitNeeds nd = split_needs(cnt);
+  const SplitNeeds nd = split_needs<kList>(cnt);
   int mb0 = -1;
   if (lane == 0 && nd.nchild > 0) {
     const int v[5] = {nd.nchild, nd.kept, nd.nblk, nd.nwrp, nd.nbig};
     int base[5];
 #pragma unroll
     for (int c = 0; c < 5; ++c) base[c] = v[c] ? atomicAdd(split_ctr(tb, c, lb), v[c]) : 0;
-    if (write_children(tb, p, cnt, nd, base[0], base[1], base[2], base[3], base[4], err)) mb0 = base[1];
+    if (write_children<kList>(tb, p, cnt, nd, base[0], base[1], base[2], base[3], base[4], err)) mb0 = base[1];
   }
   mb0 = __shfl_sync(0xffffffffu, mb0, 0);
   if (mb0 >= 0) warp_scatter(X, T, tb, p, lane, cnt, mb0);
@@ -490,6 +494,7 @@ __device__ void warp_split_one(const double *__restrict__ X, long long T, TreeBu
 // writes its children and scatters its members in member order.
 constexpr int kLaneNode = 16;
 
+template <bool kList = true>
 __device__ void lane_split(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int2 R, int lane,
                            int lb, unsigned *err) {
   const bool mine = p >= 0;
@@ -509,7 +514,7 @@ __device__ void lane_split(const double *__restrict__ X, long long T, TreeBuffer
 #pragma unroll
     for (int dd = 0; dd < 8; ++dd) cnt[dd] = (int)((cp >> (5 * dd)) & 31u);
   }
-  const SplitNeeds nd = mine ? split_needs(cnt) : SplitNeeds{0, 0, 0, 0, 0};
+  const SplitNeeds nd = mine ? split_needs<kList>(cnt) : SplitNeeds{0, 0, 0, 0, 0};
   const int v[5] = {nd.nchild, nd.kept, nd.nblk, nd.nwrp, nd.nbig};
   int off[5], base[5];
 #pragma unroll
@@ -527,7 +532,7 @@ __device__ void lane_split(const double *__restrict__ X, long long T, TreeBuffer
   }
   if (!mine || nd.nchild == 0) return;
   const int mb0 = base[1] + off[1];
-  if (!write_children(tb, p, cnt, nd, base[0] + off[0], mb0, base[2] + off[2], base[3] + off[3], base[4] + off[4],
+  if (!write_children<kList>(tb, p, cnt, nd, base[0] + off[0], mb0, base[2] + off[2], base[3] + off[3], base[4] + off[4],
                       err))
     return;
   unsigned long long op = 0, run = 0;  // children's list offsets and fill, 5 bits each
@@ -550,6 +555,7 @@ __device__ void lane_split(const double *__restrict__ X, long long T, TreeBuffer
 // Split node p (more than kBigNode members) with a whole block: each warp takes a contiguous
 // slice of the member list and the slices' counts are prefix-summed, so the partition stays
 // stable.
+template <bool kList = true>
 __device__ void split_node_block(const double *__restrict__ X, long long T, TreeBuffers &tb, int p,
                                  unsigned *err) {
   __shared__ int wcnt[32][8];
@@ -587,7 +593,7 @@ __device__ void split_node_block(const double *__restrict__ X, long long T, Tree
     int c[8];
     for (int dd = 0; dd < 8; ++dd) c[dd] = s_cnt[dd];
     int id0, mb0;
-    make_children(tb, p, c, &id0, &mb0, err);
+    make_children<kList>(tb, p, c, &id0, &mb0, err);
     s_id0 = id0;
     s_mb0 = mb0;
   }
@@ -615,9 +621,10 @@ __device__ void split_node_block(const double *__restrict__ X, long long T, Tree
 // members (or nodes) per lane in flight at once.  The children's lists (level + 1) fill as nodes
 // split; the list of level + 2 is idle during this level (read at level - 1, filled at
 // level + 1) and is emptied here.
-__device__ void split_level(const double *__restrict__ X, long long T, TreeBuffers &tb, int level, int block, int blocks,
-                            unsigned *err) {
+__global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *__restrict__ X, long long T, TreeBuffers tb,
+                                                      int level, unsigned *err) {
   if (failed_above(tb, level)) return;
+  const int block = blockIdx.x, blocks = gridDim.x;
   const int b = level % 3, b2 = (level + 2) % 3;
   if (block == 0 && threadIdx.x == 0) {
     tb.ctr[kCtrSplit + b2] = 0;
@@ -670,23 +677,142 @@ __device__ void split_level(const double *__restrict__ X, long long T, TreeBuffe
   }
 }
 
-__global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *__restrict__ X, long long T, TreeBuffers tb,
-                                                      int level, unsigned *err) {
-  split_level(X, T, tb, level, blockIdx.x, gridDim.x, err);
+// Below cells a fraction of a segment wide only pairs of points from different filaments are left
+// together, as a rule: a few nodes a level.  There a node listed at `level` is split with all that
+// lies below it by whoever takes it -- a lane up to kLaneNode members, a warp or a block above
+// that -- without a barrier or a list between the levels, over the whole GPU: a state whose points
+// lie closer than its delta lists as many nodes here as on the levels before.
+
+// The subtrees of the nodes that next() gives the lanes (-1: no more), at most kLaneNode members each.
+// A lane's nodes still to split share no member and have two at least.
+template <class Next>
+__device__ void small_subtrees(const double *__restrict__ X, long long T, TreeBuffers &tb, Next next, int lane,
+                               unsigned *err) {
+  int stack[kLaneNode / 2];
+  int top = 0;
+  for (;;) {
+    int p = top > 0 ? stack[--top] : next();
+    if (!__any_sync(0xffffffffu, p >= 0)) return;
+    if (p >= 0 && tb.nDepth[p] >= kMaxLevels) {
+      atomicOr(err, DERR_TREE_DEPTH);
+      p = -1;
+    }
+    lane_split<false>(X, T, tb, p, p >= 0 ? tb.nR[p] : make_int2(0, 0), lane, 0, err);
+    if (p < 0) continue;
+    const int n = tb.nKids[p], id = tb.nI[p].y;
+    for (int c = 0; c < n; ++c)
+      if (tb.nR[id + c].y >= 2) stack[top++] = id + c;
+  }
 }
 
-// The levels from `level` on by one block, until none lists a node: below cells a fraction of a
-// segment wide only pairs of points from different filaments are left together.
+// The subtree of node p (kLaneNode < members <= kBigNode) by a warp.
+constexpr int kWarpStack = kBigNode / (kLaneNode + 1) + 1;
+__device__ void warp_subtree(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int *stack, int lane,
+                             unsigned *err) {
+  for (int top = 0;;) {
+    if (tb.nDepth[p] >= kMaxLevels) {
+      if (lane == 0) atomicOr(err, DERR_TREE_DEPTH);
+    } else {
+      warp_split_one<false>(X, T, tb, p, lane, 0, err);
+      __syncwarp();
+      const int n = tb.nKids[p], id = tb.nI[p].y;
+      const int m = lane < n ? tb.nR[id + lane].y : 0;
+      const unsigned large = __ballot_sync(0xffffffffu, m > kLaneNode);
+      if (m > kLaneNode) stack[top + __popc(large & ((1u << lane) - 1u))] = id + lane;
+      top += __popc(large);
+      __syncwarp();
+      bool todo = m >= 2 && m <= kLaneNode;
+      small_subtrees(
+          X, T, tb,
+          [&]() {
+            const int q = todo ? id + lane : -1;
+            todo = false;
+            return q;
+          },
+          lane, err);
+    }
+    if (top == 0) return;
+    p = stack[--top];
+    __syncwarp();
+  }
+}
+
+// The subtree of node p (more than kBigNode members) by a block: its own splits one after the
+// other, their smaller children a warp each.
+constexpr int kBlockStack = 7 * kMaxLevels + 8;
+__device__ void block_subtree(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int *block_stack,
+                              int *warp_stack, unsigned *err) {
+  __shared__ int s_top;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __syncthreads();  // (the last node's stack has been left by all)
+  if (threadIdx.x == 0) {
+    s_top = 1;
+    block_stack[0] = p;
+  }
+  __syncthreads();
+  for (;;) {
+    const int top = s_top;
+    if (top == 0) return;
+    p = block_stack[top - 1];
+    __syncthreads();
+    if (threadIdx.x == 0) s_top = top - 1;
+    if (tb.nDepth[p] >= kMaxLevels) {
+      if (threadIdx.x == 0) atomicOr(err, DERR_TREE_DEPTH);
+      __syncthreads();
+      continue;
+    }
+    split_node_block<false>(X, T, tb, p, err);
+    __syncthreads();
+    const int n = tb.nKids[p], id = tb.nI[p].y;
+    if (wid < n) {
+      const int c = id + wid, m = tb.nR[c].y;
+      if (m > kBigNode) {
+        if (lane == 0) block_stack[atomicAdd(&s_top, 1)] = c;
+      } else if (m > kLaneNode) {
+        warp_subtree(X, T, tb, c, warp_stack, lane, err);
+      } else if (m >= 2) {
+        bool todo = lane == 0;
+        small_subtrees(
+            X, T, tb,
+            [&]() {
+              const int q = todo ? c : -1;
+              todo = false;
+              return q;
+            },
+            lane, err);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The subtrees of the nodes listed at `level`: 32,768 points 2.6 us, 1,048,576 points 24 us (by one
+// block, level after level, 1.5 and 36 us; but with 1,048,576 points at a delta of 40 segments the
+// tree stage took 15.2 ms so, 5.6 now and with a launch for every level).
 __global__ void __launch_bounds__(kSplitThreads, 1) k_split_rest(const double *__restrict__ X, long long T, TreeBuffers tb,
                                                      int level, unsigned *err) {
-  for (; level < kMaxLevels; ++level) {
-    volatile int *c = tb.ctr + kCtrSplit + level % 3;
-    const bool none = c[0] == 0 && c[3] == 0;
-    __syncthreads();
-    if (none) return;
-    split_level(X, T, tb, level, 0, 1, err);
-    __threadfence_block();
-    __syncthreads();
+  __shared__ int s_block[kBlockStack], s_warp[kSplitThreads / 32][kWarpStack];
+  if (failed_above(tb, level)) return;
+  const int b = level % 3, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int nbl = min(tb.ctr[kCtrSplit + b], tb.max_blk), nwl = min(tb.ctr[kCtrSplit + 3 + b], tb.max_wrp);
+  for (int bq = blockIdx.x; bq < nbl; bq += gridDim.x)
+    block_subtree(X, T, tb, tb.split_blk[b][bq], s_block, s_warp[wid], err);
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int per = min(32, (nwl + nwarps - 1) / nwarps);
+  for (int wq0 = warp * per; wq0 < nwl; wq0 += nwarps * per) {
+    const int p = lane < per && wq0 + lane < nwl ? tb.split_wrp[b][wq0 + lane] : -1;
+    const int m = p >= 0 ? tb.nR[p].y : 0;
+    for (unsigned large = __ballot_sync(0xffffffffu, m > kLaneNode); large; large &= large - 1)
+      warp_subtree(X, T, tb, __shfl_sync(0xffffffffu, p, __ffs(large) - 1), s_warp[wid], lane, err);
+    bool todo = p >= 0 && m <= kLaneNode;
+    small_subtrees(
+        X, T, tb,
+        [&]() {
+          const int q = todo ? p : -1;
+          todo = false;
+          return q;
+        },
+        lane, err);
   }
 }
 
@@ -2268,11 +2394,11 @@ void launch_tree_build(nv_handle *h) {
   cudaStreamWaitEvent(h->side2, h->fork2_ev, 0);
   k_node_sums_block<<<sms, kSumThreads, kSumSmem, h->side2>>>(h->x, h->gi, h->nxt, T, *tb, 0, h->d_err);
   cudaEventRecord(h->join2_ev, h->side2);
-  // A launch per level down to cells of about an eighth of delta, the rest by one block (32,768 points,
-  // 41 launches 172 us, now 9 in 122 us and the block in 1.4; 1,048,576 points, 10 and 35 us)
+  // A launch per level down to cells of about an eighth of delta, one for the rest (32,768 points,
+  // 41 launches 172 us, now 9 in 122 us and the one in 2.6; 1,048,576 points, 10 and 24 us)
   for (int L = 1; L < tb->grid_levels; ++L)
     k_split_level<<<sms, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, L, h->d_err);
-  k_split_rest<<<1, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, tb->grid_levels, h->d_err);
+  k_split_rest<<<sms, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, tb->grid_levels, h->d_err);
   k_node_sums_block<<<sms, kSumThreads, kSumSmem, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, 1, h->d_err);
   k_node_sums_big<<<sms * 8, 128, 0, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, h->nsys, h->d_err);
   k_node_sums_small<<<sms * 8, 128, 0, h->stream>>>(h->x, h->gi, h->nxt, T, *tb, h->nsys, h->d_err);
