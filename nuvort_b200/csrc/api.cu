@@ -376,11 +376,14 @@ void build_image_worklist(nv_handle *h, int tb, std::vector<int4> &w) {
   }
 }
 
-// Warps per group of 32 targets of the mixed tree walk: 8 while the groups' blocks are all
-// resident at once (three of 256 threads to an SM), where a group's own time counts (8,000
-// points: 164 us, 217 with 4), 4 up to 40 groups an SM (100,000 points: 1.41 ms; 1.67 with 8,
-// 1.54 with 2), and 2 beyond, where the groups fill the GPU anyway and a round's barriers
-// cost more than its parallelism gives (1M points: 9.8 ms, 10.3 with 4, 10.2 with 1).
+// Warps per group of 32 targets of the mixed tree walk: 8 while the groups with targets are all
+// resident at once, two blocks of 256 threads to an SM (their shared memory, 79 KB each, allows
+// no third), where a group's own time counts (8,000 points: 160 us, 214 with 4; but 12,000, 2.5
+// groups an SM: 254, 241).  The groups counted are those of the slots, of which the usual
+// capacity, 1.6 times the points, fills two thirds, so the line is at three an SM.  4 up to 40 an
+// SM (100,000 points: 1.39 ms; 1.58 with 8, 1.56 with 2), and 2 beyond, where the groups fill the
+// GPU anyway and a round's barriers cost more than its parallelism gives (1,048,576 points of
+// undisturbed rings: 9.9 ms, 10.2 with 4, 10.3 with 1).
 int auto_walk_parts(const nv_handle *h) {
   long long groups = 0;
   for (int s = 0; s < h->nsys; ++s)
