@@ -5,9 +5,9 @@
 // (cp.async.bulk + mbarrier, double-buffered).  The summation order is the reference's:
 //   u_bs = sum_j ascending (unshifted)                   timestep.f90:83-85
 //   u_bs' = sum_images (in periodic_loop_array order) sum_j ascending   :88-92
-// with every operation rounded once (no FMA), so the result is bit-identical to the
-// reference arithmetic except for the ulp-level difference of the device log() in the
-// local term.  The image loop is outside the tile loop for that reason: each image
+// with every operation rounded once (the quotients as fp64.cuh says), so the result is
+// bit-identical to the reference arithmetic except for the ulp-level difference of the device
+// log() in the local term.  The image loop is outside the tile loop for that reason: each image
 // re-streams the tiles (from L2; the kernel is FP64-pipe bound, not memory bound).
 #include <vector>
 

@@ -1,10 +1,12 @@
-// fp64.cuh -- correctly rounded FP64 quotients and square roots that share their seeds.
+// fp64.cuh -- FP64 quotients and square roots, rounded as the IEEE operations round them, that share
+// their seeds.
 //
 // A Biot-Savart term in the reference's arithmetic (timestep.f90:162-170) takes two square
 // roots and five quotients, three of them by one divisor and two by the square roots.  Taken
 // one by one they are most of the term's FP64 instructions (166 of them a term were counted,
-// against 81 with the forms below).  Here a square root hands its reciprocal on to the
-// quotient by it, and the three quotients by one divisor share one reciprocal.
+// against 84 with the forms below, the sums' three additions among them).  Here a square root
+// hands its reciprocal on to the quotient by it, and the three quotients by one divisor share
+// one reciprocal.
 //
 // Method: the hardware approximations (relative error measured at most 2^-19) are taken to the
 // FP64 rounding level by one third-order Newton step (the error cubed).  A quotient q = n y,
@@ -12,10 +14,15 @@
 // (one FMA): q + r y, as P. Markstein (IBM J. Res. Dev. 34, 1990) describes; the square root
 // likewise from g = x y and its residual x - g^2.  Before the last rounding the value is off
 // by about 2^-52 units of its last place, so it rounds as the exact value does unless that
-// lies as close to the middle of two doubles.  Against the IEEE operations on 2^32 random
-// operands no square root differed, and quotients only where n and x both lie within a few
-// units of the last place of a power of two (their quotient is such a middle but for 2^-52).
-// Operands outside the ranges stated take the IEEE operations instead.
+// lies as close to the middle of two doubles.  That happens where n and x both lie a few units
+// below a power of two (their quotient is such a middle but for 2^-52 of a unit): there a
+// quotient can be a unit of its last place off.  Random operands meet it about once in 2^50
+// quotients, and none did in 2^32; no square root differed.
+// Divisors and radicands outside the ranges stated take the IEEE operations instead.  Numerators
+// are not looked at: one of zero gives zero (+0.0 also for -0.0, the same in the sums), and one
+// below 2^-969, whose residual is subnormal, a quotient up to two units off.  They are r x d
+// times the circulation, 2 r.d and 2 |d|^2 + 2 r.d, products of two differences of positions:
+// so small only where those are below 1e-146 cm.
 #pragma once
 
 #include "common.cuh"
@@ -47,7 +54,7 @@ __device__ __forceinline__ double near_rcp(double x) {
   return fma(y, fma(e, e, e), y);
 }
 
-// n / x, correctly rounded, given y = near_rcp(x) (or the reciprocal near_sqrt gives).
+// n / x, rounded as said above, given y = near_rcp(x) (or the reciprocal near_sqrt gives).
 __device__ __forceinline__ double quot(double n, double x, double y) {
   const double q = n * y;
   return fma(fma(-q, x, n), y, q);
