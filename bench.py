@@ -215,13 +215,20 @@ def measured_peaks():
 
 def profile_traffic(kernel: str, workload: str):
     """DRAM bytes per launch of `kernel` on `workload` from its committed ncu summary
-    (profiles/traffic.json), or None where no capture of that workload exists."""
+    (profiles/traffic.json), or None where no capture of that workload exists.  (The file also
+    keeps the figures of the mixed walk node by node, "k_tree_walk_mixed", which has given way to
+    the one by groups of targets, "k_tree_walk_mixed<W>".)"""
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
             entry = json.load(f).get(kernel, {}).get(workload)
         return dict(entry, workload=workload) if entry else None
     except Exception:
         return None
+
+
+def present_traffic(kernel: str, workload: str):
+    """profile_traffic of the kernel as it is now launched under this name."""
+    return profile_traffic({"k_tree_walk_mixed": "k_tree_walk_mixed<W>"}.get(kernel, kernel), workload)
 
 
 def rms_rel(a, b):
@@ -419,7 +426,7 @@ def roofline_of(params, states, m, steps, precision, local, workload):
                   "direct_pair_images": pairs, "ms": m["vel_ms"] / steps}
     achieved = flops / (m["vel_ms"] / steps * 1e-3) / 1e12
     return {"bound": "fp32" if mixed else "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": achieved / peak if peak else None, "traffic": profile_traffic(kernel, workload), "kernel": kernel,
+            "frac": achieved / peak if peak else None, "traffic": present_traffic(kernel, workload), "kernel": kernel,
             "peak_source": ("FP32" if mixed else "FP64") + " FMA rate measured on this GPU by nv_measure_fp"
                            + ("32" if mixed else "64") + "_peak (MEASURED_PEAKS.json covers HBM and bf16 tensor "
                            "only); algorithmic flops = 43 per interaction or pair-image + 12 per opening test; "

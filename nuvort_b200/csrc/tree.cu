@@ -1810,11 +1810,12 @@ __global__ void k_leaf_links(TreeBuffers tb, int nsys, const int *__restrict__ p
 // leaves within the near radius and ill-conditioned terms are evaluated in FP64.  Writes the
 // target's sum over all images.
 //
-// Bound: instruction issue, three quarters of it in the terms (61 issue slots a term of two
-// packed ones, of which the conditioning guards that the long summed circulations need take
-// about 20), with 58 % of the lanes in an average term's mask; a fifth of the nodes need the
-// target-by-target test.  100,000 points: 1.41 ms; 1M: 9.8 ms (2.27 and 14.1 ms for a warp
-// stepping through the union of its targets' walks node by node, 148 issue slots a node).
+// Bound: latencies that 16 to 20 warps an SM, all that their shared memory lets reside, do not
+// cover.  32,768 points: 16 warps active, 2.24 instructions a cycle of 4, 7.1 cycles between two
+// of a warp, of them 1.8 fixed latencies, 1.0 at barriers and 1.2 for loads; ALU, FMA and XU at 38, 36
+// and 27 % of their rates, DRAM at 0.2 %.  100,003 points: 1.39 ms; 1,048,576: 9.9 ms, 11.0 after
+// some steps (2.27 and 14.1 ms for a warp stepping through the union of its targets' walks node
+// by node).
 // FP64 terms where they occur instead of from the queue: 1.59 ms at 100,000 points in place of
 // 1.54 (both on the Morton order).
 constexpr int walk_cap(int W) { return W == 8 ? 4096 : W == 4 ? 2048 : 1024; }  // work-list entries

@@ -23,3 +23,12 @@ print([k for k in ("pclose_warps", "pclose_cells") if any(k in n for n in names)
 ])
 def test_closest_points_of_systems_without_a_tree(tmp_path, caps, tree, kernel):
     assert f"['pclose_{kernel}']" in run(tmp_path, PCLOSE % (caps, tree))
+
+
+def test_traffic_of_the_present_walk():
+    # the walk by groups writes one sum a target, not 27: under 0.5 KB of DRAM a target, both ways
+    import bench
+    for workload, targets in (("tangle32k", 32768), ("tangle1m", 1048576), ("ensemble512", 2670000)):
+        t = bench.present_traffic("k_tree_walk_mixed", workload)
+        assert t["bytes_per_launch"] < 512 * targets and t["source"].endswith("k_tree_walk_mixed_groups.md")
+    assert bench.present_traffic("k_tree_walk_fp64", "tangle32k") == bench.profile_traffic("k_tree_walk_fp64", "tangle32k")
