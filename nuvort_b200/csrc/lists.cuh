@@ -18,6 +18,9 @@ struct PassBuffers {
   unsigned long long *state;  // [K][blocks]
   unsigned *ctl;              // ticket, finished blocks, epoch
 };
+// The launch's epoch (below 2^30), the same to all its threads until they have called flags for
+// their last slot.
+__device__ __forceinline__ unsigned pass_epoch(const PassBuffers &L) { return *(const volatile unsigned *)&L.ctl[2]; }
 inline int pass_blocks(long long n) { return (int)((n + kPassSlots) / kPassSlots); }  // slots 0..n
 inline void pass_alloc(unsigned long long **state, unsigned **ctl, int K, long long n) {
   const size_t words = (size_t)K * pass_blocks(n);
