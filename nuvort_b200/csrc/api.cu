@@ -365,15 +365,33 @@ int upload_worklist4(int4 **dptr, int *n, const std::vector<int4> &w) {
   return NV_OK;
 }
 
-// (system, image, first slot) items over every image of every direct-sum system.
-void build_image_worklist(nv_handle *h, int tb, std::vector<int4> &w) {
-  w.clear();
+// (system, image, first slot) items over every image of every direct-sum system: those of systems
+// up to `small` slots in w1, the others' in w8.
+void build_image_worklists(nv_handle *h, int small, std::vector<int4> &w8, std::vector<int4> &w1) {
+  w8.clear();
+  w1.clear();
   for (int s = 0; s < h->nsys; ++s) {
     const SysConst &sc = h->sc[s];
     if (sc.velocity == NV_VEL_LIA || sc.sched_tree) continue;
+    std::vector<int4> &w = h->cap[s] <= small ? w1 : w8;
     for (int m = 0; m <= sc.n_shift; ++m)
-      for (int k = 1; k <= h->cap[s]; k += tb) w.push_back(make_int4(s, m, sc.base + k, 0));
+      for (int k = 1; k <= h->cap[s]; k += 32) w.push_back(make_int4(s, m, sc.base + k, 0));
   }
+}
+
+// Slots up to which a system's items of the mixed direct sum go to a warp each instead of a block of
+// eight, whose warps share out a tile of 256 segments and whose setup costs eight times as much:
+// 1,000, where the items of such systems are 20 an SM at least, fewer than half of what can be
+// resident (velocity stage, us, a warp and a block: 2,000 systems of 30 points 397, 1,571; 512 of
+// 100 606, 1,351; 16 of 100, 3,024 items, 68, 80; 100 of 500 1,612, 1,782; but 64 of 1,000,
+// 1,640 slots each, 3,781, 3,702; and 4 of 100, 756 items, 62, 49; 4 of 300, 1,836 items, 100, 70).
+int mixed_small_slots(const nv_handle *h) {
+  constexpr int kSmall = 1000;
+  long long items = 0;
+  for (int s = 0; s < h->nsys; ++s)
+    if (h->sc[s].velocity != NV_VEL_LIA && !h->sc[s].sched_tree && h->cap[s] <= kSmall)
+      items += (long long)(1 + h->sc[s].n_shift) * ((h->cap[s] + 31) / 32);
+  return items >= 20LL * n_sms_host() ? kSmall : 0;
 }
 
 // Warps per group of 32 targets of the mixed tree walk: 8 while the groups with targets are all
@@ -395,9 +413,11 @@ int rebuild_worklists(nv_handle *h) {
   std::vector<int2> w;
   int rc;
   if (h->precision == NV_PREC_MIXED) {
-    std::vector<int4> w4;
-    build_image_worklist(h, 32, w4);
-    if ((rc = upload_worklist4(&h->d_work_img, &h->n_work_img, w4)) != NV_OK) return rc;
+    std::vector<int4> w8, w1;
+    build_image_worklists(h, mixed_small_slots(h), w8, w1);
+    if ((rc = upload_worklist4(&h->d_work_img, &h->n_work_img, w8)) != NV_OK ||
+        (rc = upload_worklist4(&h->d_work_img1, &h->n_work_img1, w1)) != NV_OK)
+      return rc;
     h->walk_parts_used = h->walk_parts > 0 ? h->walk_parts : auto_walk_parts(h);
     build_worklist(h, 2, w, 32);
     if ((rc = upload_worklist(&h->d_work_grp, &h->n_work_grp, w)) != NV_OK) return rc;
@@ -780,7 +800,7 @@ int nv_destroy(nv_handle *h) {
   for (void *p : h->nf_buffers) cudaFree(p);
   void *ptrs[] = {h->bstage, h->d_btab, h->d_bcheck, h->pin, h->umir, h->usm, h->cs, h->d_drec, h->partial, h->stage, h->d_upck, h->d_sc, h->d_dyn, h->x, h->u, h->u1, h->u2, h->gi, h->gb, h->closestd, h->nxt, h->prv,
                   h->closest, h->sys_of, h->seg, h->seg32, h->d_err, h->d_events, h->d_event_count,
-                  h->d_work_direct, h->d_work_tree, h->d_work_lia, h->d_work_img, h->d_work_grp, h->d_work_split};
+                  h->d_work_direct, h->d_work_tree, h->d_work_lia, h->d_work_img, h->d_work_img1, h->d_work_grp, h->d_work_split};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (auto &e : h->ev)

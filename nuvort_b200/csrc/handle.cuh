@@ -48,8 +48,10 @@ struct nv_handle {
   int4 *d_btab = nullptr;    // their per-system table (base, rows, n, offset), nsys entries
   int *d_bcheck = nullptr;   // their link checks, two ints per system
   int *d_upck = nullptr;     // nv_upload checks: [0] link errors (1 out of range, 2 empty-slot mismatch), [1] live slots
-  int4 *d_work_img = nullptr;  // (system, image, first slot) items of 32 slots of the mixed direct sum
-  int n_work_img = 0;
+  // (system, image, first slot) items of 32 slots of the mixed direct sum: by a block of eight warps,
+  // by a warp
+  int4 *d_work_img = nullptr, *d_work_img1 = nullptr;
+  int n_work_img = 0, n_work_img1 = 0;
   int2 *d_work_grp = nullptr;  // (system, first walk position) items of 32 targets of the mixed tree walk
   int n_work_grp = 0;
   double near_factor = 2.0;    // near field: pairs closer than near_factor*delta run in FP64

@@ -1,7 +1,8 @@
 // mixed.cu -- mixed-precision direct sum and the FP64 epilogue shared with the mixed tree walk.
 //
-// k_direct_mixed: a block per 32 targets and periodic image, each of its eight warps (a lane per
-// target) over an eighth of every tile of the target system's segments.  The tiles stream
+// k_direct_mixed<W>: a block of W warps per 32 targets and periodic image, each warp (a lane per
+// target) over its share of every tile of the target system's segments (W = 8; 1 for ensembles of
+// small systems).  The tiles stream
 // through shared memory by 1-D bulk copies (pairs of segments side by side, 96 bytes a pair:
 // position hi, position lo, segment vector).  r = x_j - x_i is formed from the hi/lo split, so
 // it is exact to ~1e-16 before rounding to FP32.  Every 32 terms are summed in FP32 and those
@@ -16,12 +17,14 @@
 
 namespace {
 
-constexpr int kPairs = 128;                // segment pairs per staged tile (96 B each)
-constexpr int kWarps = 8;                  // warps of a block, sharing its 32 targets
-constexpr int kTB = 32 * kWarps;
-constexpr int kWarpPairs = kPairs / kWarps;  // pairs of a tile per warp: one FP32 sub-sum
-constexpr int kStages = 4;
-constexpr size_t kMixedSmem = kStages * kPairs * 96;
+constexpr int kWarpPairs = 16;  // segment pairs (96 B each) of an FP32 sub-sum
+// A block of W warps that share 32 targets (8, or 1 for many small systems): pairs per staged tile,
+// tiles in flight
+template <int W>
+struct MixedShape {
+  static constexpr int kPairs = W == 8 ? 128 : 32, kStages = W == 8 ? 4 : 3;
+  static constexpr size_t kSmem = (size_t)kStages * kPairs * 96;
+};
 
 // One term in FP64 from the FP64 segment records, for near and ill-conditioned pairs: the
 // reference's skip decision (4ac - b^2 == 0, timestep.f90:166,192) in its own arithmetic, the
@@ -131,17 +134,16 @@ __device__ __forceinline__ unsigned line_mask(const ulonglong2 *pairs, int np, c
 // arithmetic and all guards, 113 issue slots a term: 74.1 ms and 409 us; packed, but all guards
 // and a barrier per tile: 55.4 ms and 236 us).  The line guard left out beyond 4|d|: 38.8 ms and
 // 136 us; its exact test on every far pair: 44.8 ms and 153 us.
-__global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restrict__ scs,
-                                                         const SysDyn *__restrict__ dyn,
-                                                         const int4 *__restrict__ work, const double *__restrict__ X,
-                                                         const int *__restrict__ nxt, const int *__restrict__ prv,
-                                                         const float *__restrict__ seg32,
-                                                         const double4 *__restrict__ seg64,
-                                                         double *__restrict__ partial, long long T,
-                                                         double near_factor, Fp32Guards gd, unsigned *err) {
+template <int W>
+__global__ void __launch_bounds__(32 * W, 24 / W) k_direct_mixed(
+    const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn, const int4 *__restrict__ work,
+    const double *__restrict__ X, const int *__restrict__ nxt, const int *__restrict__ prv,
+    const float *__restrict__ seg32, const double4 *__restrict__ seg64, double *__restrict__ partial, long long T,
+    double near_factor, Fp32Guards gd, unsigned *err) {
+  constexpr int kPairs = MixedShape<W>::kPairs, kStages = MixedShape<W>::kStages;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   ulonglong2 *tiles = reinterpret_cast<ulonglong2 *>(smem_raw);  // [kStages][6 * kPairs]
-  __shared__ double s_red[3][kWarps][32];
+  __shared__ double s_red[3][W][32];
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages];
   __shared__ int s_abort;
 
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
     s_abort = (*err != 0);
     for (int k = 0; k < kStages; ++k) {
       mbar_init(&full[k], 1);
-      mbar_init(&empty[k], kWarps);
+      mbar_init(&empty[k], W);
     }
     mbar_fence_init();
   }
@@ -237,8 +239,9 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
       break;
     }
     const ulonglong2 *tile = tiles + (k % kStages) * 6 * kPairs;
-    const int p0 = wid * kWarpPairs, p1 = min(min(kPairs, np - k * kPairs), p0 + kWarpPairs);
-    if (p0 < p1) {
+    const int in_tile = min(kPairs, np - k * kPairs);
+    for (int p0 = wid * kWarpPairs; p0 < in_tile; p0 += W * kWarpPairs) {
+      const int p1 = min(in_tile, p0 + kWarpPairs);
       const int bp = behind_p - k * kPairs;
       // the pairs that not every target may take without guards however far it is: a line guard
       // may act, or the pair holds some target's behind segment
@@ -285,11 +288,12 @@ __global__ void __launch_bounds__(kTB, 3) k_direct_mixed(const SysConst *__restr
   // A give-up leaves copies in flight: wait for them (bounded) before shared memory is released.
   if (tid == 0)
     for (int k = max(0, issued - kStages); k < issued; ++k) mbar_wait(&full[k % kStages], (unsigned)((k / kStages) & 1));
-  if (wid < 3 && t.active) {
+  if (!t.active) return;
+  for (int c = wid; c < 3; c += W) {
     double v = 0.;
 #pragma unroll
-    for (int k = 0; k < kWarps; ++k) v += s_red[wid][k][lane];
-    partial[((long long)m * 3 + wid) * T + g] = v;
+    for (int k = 0; k < W; ++k) v += s_red[c][k][lane];
+    partial[((long long)m * 3 + c) * T + g] = v;
   }
 }
 
@@ -329,17 +333,20 @@ __global__ void k_mixed_combine(const SysConst *__restrict__ scs, const SysDyn *
 }  // namespace
 
 cudaError_t mixed_kernels_setup() {
-  return cudaFuncSetAttribute(k_direct_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMixedSmem);
+  return cudaFuncSetAttribute(k_direct_mixed<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)MixedShape<8>::kSmem);
 }
 
 void launch_direct_mixed(nv_handle *h) {
-  if (h->n_work_img == 0) return;
-  k_direct_mixed<<<h->n_work_img, kTB, kMixedSmem, h->stream>>>(
-      h->d_sc, h->d_dyn, h->d_work_img, h->x, h->nxt, h->prv, h->seg32, h->seg, h->partial, h->T, h->near_factor, h->guards,
-      h->d_err);
+  auto launch = [&](auto kernel, int w, size_t smem, const int4 *work, int n) {
+    if (n > 0)
+      kernel<<<n, 32 * w, smem, h->stream>>>(h->d_sc, h->d_dyn, work, h->x, h->nxt, h->prv, h->seg32, h->seg, h->partial,
+                                             h->T, h->near_factor, h->guards, h->d_err);
+  };
+  launch(k_direct_mixed<8>, 8, MixedShape<8>::kSmem, h->d_work_img, h->n_work_img);
+  launch(k_direct_mixed<1>, 1, MixedShape<1>::kSmem, h->d_work_img1, h->n_work_img1);
 }
 
-// which: 1 = direct-sum systems, 2 = tree systems
 void launch_mixed_combine(nv_handle *h, int which) {
   const int2 *wl = which == 1 ? h->d_work_direct : h->d_work_tree;
   const int n = which == 1 ? h->n_work_direct : h->n_work_tree;

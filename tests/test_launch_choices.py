@@ -32,3 +32,24 @@ def test_traffic_of_the_present_walk():
         t = bench.present_traffic("k_tree_walk_mixed", workload)
         assert t["bytes_per_launch"] < 512 * targets and t["source"].endswith("k_tree_walk_mixed_groups.md")
     assert bench.present_traffic("k_tree_walk_fp64", "tangle32k") == bench.profile_traffic("k_tree_walk_fp64", "tangle32k")
+
+
+MIXED = """
+from helpers import config0_params
+from nuvort_b200.api import Handle
+caps = %r
+with Handle([config0_params(precision="mixed")] * len(caps), caps) as h:
+    launched()
+    h.calc_velocity()
+    names = launched()
+print([w for w in (1, 8) if any("k_direct_mixedILi%%dE" %% w in n for n in names)])
+"""
+
+
+@pytest.mark.parametrize("caps,warps", [
+    ([1000], [8]), ([88] * 2000, [1]), ([1000] * 4, [1]), ([1001] * 4, [8]), ([200] * 4, [8]),
+    ([96] * 36, [8]), ([96] * 37, [1]),  # 2,916 and 2,997 items of 32 slots in 27 images, 20 an SM: 2,960
+    ([88] * 2000 + [5000], [1, 8]),
+])
+def test_warps_of_the_mixed_direct_sum(tmp_path, caps, warps):
+    assert str(warps) in run(tmp_path, MIXED % (caps,))
