@@ -678,141 +678,137 @@ __global__ void __launch_bounds__(kSplitThreads, 1) k_split_level(const double *
 }
 
 // Below cells a fraction of a segment wide only pairs of points from different filaments are left
-// together, as a rule: a few nodes a level.  There a node listed at `level` is split with all that
-// lies below it by whoever takes it -- a lane up to kLaneNode members, a warp or a block above
-// that -- without a barrier or a list between the levels, over the whole GPU: a state whose points
-// lie closer than its delta lists as many nodes here as on the levels before.
+// together, as a rule: a few nodes a level.  There the nodes listed at `level` are shared out over
+// the blocks, and a block splits its share with all that lies below, level after level by lists in
+// shared memory: nothing is waited for outside the block, and a state whose points lie closer
+// than its delta, with as many nodes here as on the levels before, still has the whole GPU.
+constexpr int kRestMembers = 8192;  // of the nodes that a block takes at once
+struct RestShared {
+  int list[2][kRestMembers / 2];  // nodes of this level and of the next (two members at least each)
+  int n, warp_sum[kSplitThreads / 32], big[7 * kMaxLevels + 8], n_big;
+};
 
-// The subtrees of the nodes that next() gives the lanes (-1: no more), at most kLaneNode members each.
-// A lane's nodes still to split share no member and have two at least.
-template <class Next>
-__device__ void small_subtrees(const double *__restrict__ X, long long T, TreeBuffers &tb, Next next, int lane,
-                               unsigned *err) {
-  int stack[kLaneNode / 2];
-  int top = 0;
-  for (;;) {
-    int p = top > 0 ? stack[--top] : next();
-    if (!__any_sync(0xffffffffu, p >= 0)) return;
-    if (p >= 0 && tb.nDepth[p] >= kMaxLevels) {
-      atomicOr(err, DERR_TREE_DEPTH);
-      p = -1;
-    }
-    lane_split<false>(X, T, tb, p, p >= 0 ? tb.nR[p] : make_int2(0, 0), lane, 0, err);
-    if (p < 0) continue;
-    const int n = tb.nKids[p], id = tb.nI[p].y;
-    for (int c = 0; c < n; ++c)
-      if (tb.nR[id + c].y >= 2) stack[top++] = id + c;
-  }
-}
-
-// The subtree of node p (kLaneNode < members <= kBigNode) by a warp.
-constexpr int kWarpStack = kBigNode / (kLaneNode + 1) + 1;
-__device__ void warp_subtree(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int *stack, int lane,
-                             unsigned *err) {
-  for (int top = 0;;) {
-    if (tb.nDepth[p] >= kMaxLevels) {
-      if (lane == 0) atomicOr(err, DERR_TREE_DEPTH);
-    } else {
-      warp_split_one<false>(X, T, tb, p, lane, 0, err);
-      __syncwarp();
-      const int n = tb.nKids[p], id = tb.nI[p].y;
-      const int m = lane < n ? tb.nR[id + lane].y : 0;
-      const unsigned large = __ballot_sync(0xffffffffu, m > kLaneNode);
-      if (m > kLaneNode) stack[top + __popc(large & ((1u << lane) - 1u))] = id + lane;
-      top += __popc(large);
-      __syncwarp();
-      bool todo = m >= 2 && m <= kLaneNode;
-      small_subtrees(
-          X, T, tb,
-          [&]() {
-            const int q = todo ? id + lane : -1;
-            todo = false;
-            return q;
-          },
-          lane, err);
-    }
-    if (top == 0) return;
-    p = stack[--top];
-    __syncwarp();
-  }
-}
-
-// The subtree of node p (more than kBigNode members) by a block: its own splits one after the
-// other, their smaller children a warp each.
-constexpr int kBlockStack = 7 * kMaxLevels + 8;
-__device__ void block_subtree(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, int *block_stack,
-                              int *warp_stack, unsigned *err) {
-  __shared__ int s_top;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();  // (the last node's stack has been left by all)
-  if (threadIdx.x == 0) {
-    s_top = 1;
-    block_stack[0] = p;
-  }
-  __syncthreads();
-  for (;;) {
-    const int top = s_top;
-    if (top == 0) return;
-    p = block_stack[top - 1];
+// The subtrees of the n nodes in S.list[0] (kRestMembers members together at most, kBigNode each), by the
+// block: a lane per node up to kLaneNode members, a warp above that.
+__device__ void split_below(const double *__restrict__ X, long long T, TreeBuffers &tb, int n, RestShared &S,
+                            unsigned *err) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  for (int cur = 0; n > 0; cur ^= 1) {
+    if (threadIdx.x == 0) S.n = 0;
     __syncthreads();
-    if (threadIdx.x == 0) s_top = top - 1;
-    if (tb.nDepth[p] >= kMaxLevels) {
-      if (threadIdx.x == 0) atomicOr(err, DERR_TREE_DEPTH);
-      __syncthreads();
-      continue;
-    }
-    split_node_block<false>(X, T, tb, p, err);
-    __syncthreads();
-    const int n = tb.nKids[p], id = tb.nI[p].y;
-    if (wid < n) {
-      const int c = id + wid, m = tb.nR[c].y;
-      if (m > kBigNode) {
-        if (lane == 0) block_stack[atomicAdd(&s_top, 1)] = c;
-      } else if (m > kLaneNode) {
-        warp_subtree(X, T, tb, c, warp_stack, lane, err);
-      } else if (m >= 2) {
-        bool todo = lane == 0;
-        small_subtrees(
-            X, T, tb,
-            [&]() {
-              const int q = todo ? c : -1;
-              todo = false;
-              return q;
-            },
-            lane, err);
+    const int per = min(32, (n + nwarps - 1) / nwarps);
+    for (int q0 = wid * per; q0 < n; q0 += nwarps * per) {
+      int p = lane < per && q0 + lane < n ? S.list[cur][q0 + lane] : -1;
+      if (p >= 0 && tb.nDepth[p] >= kMaxLevels) {
+        atomicOr(err, DERR_TREE_DEPTH);
+        p = -1;
+      }
+      const int2 R = p >= 0 ? tb.nR[p] : make_int2(0, 0);
+      lane_split<false>(X, T, tb, R.y <= kLaneNode ? p : -1, R, lane, 0, err);
+      for (unsigned large = __ballot_sync(0xffffffffu, R.y > kLaneNode); large; large &= large - 1)
+        warp_split_one<false>(X, T, tb, __shfl_sync(0xffffffffu, p, __ffs(large) - 1), lane, 0, err);
+      __syncwarp();
+      if (p >= 0) {
+        const int kids = tb.nKids[p], id = tb.nI[p].y;
+        for (int c = 0; c < kids; ++c)
+          if (tb.nR[id + c].y >= 2) S.list[cur ^ 1][atomicAdd(&S.n, 1)] = id + c;
       }
     }
     __syncthreads();
+    n = S.n;
+    __syncthreads();
   }
 }
 
-// The subtrees of the nodes listed at `level`: 32,768 points 2.6 us, 1,048,576 points 24 us (by one
+// Up to blockDim.x nodes behind the n in S.list[0], as many as keep their members below kRestMembers
+// (the first in any case, when the list is empty); returns how many, and adds to n and members.
+__device__ int take_nodes(const TreeBuffers &tb, const int *nodes, int count, int &n, int &members, RestShared &S) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int p = tid < count ? nodes[tid] : -1, m = p >= 0 ? tb.nR[p].y : 0;
+  int incl = m;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) S.warp_sum[wid] = incl;
+  __syncthreads();
+  for (int w = 0; w < wid; ++w) incl += S.warp_sum[w];
+  const bool fits = p >= 0 && members + incl <= kRestMembers;
+  if (fits) S.list[0][n + tid] = p;
+  const int took = __syncthreads_count(fits);
+  if (tid == took - 1) S.n = incl;
+  __syncthreads();
+  n += took;
+  if (took) members += S.n;
+  __syncthreads();
+  return took;
+}
+
+// The subtree of node p (more than kBigNode members) by the block: its own splits one after the other,
+// and below the other children.
+__device__ void split_below_big(const double *__restrict__ X, long long T, TreeBuffers &tb, int p, RestShared &S,
+                                unsigned *err) {
+  __syncthreads();  // (every thread has left the last node's loop)
+  if (threadIdx.x == 0) {
+    S.big[0] = p;
+    S.n_big = 1;
+  }
+  __syncthreads();
+  while (S.n_big > 0) {
+    p = S.big[S.n_big - 1];
+    __syncthreads();
+    if (threadIdx.x == 0) --S.n_big;
+    int kids = 0, id = 0;
+    if (tb.nDepth[p] >= kMaxLevels) {
+      if (threadIdx.x == 0) atomicOr(err, DERR_TREE_DEPTH);
+    } else {
+      split_node_block<false>(X, T, tb, p, err);
+      __syncthreads();
+      kids = tb.nKids[p];
+      id = tb.nI[p].y;
+    }
+    for (int c0 = 0; c0 < kids; c0 += kRestMembers / kBigNode) {
+      if (threadIdx.x == 0) {
+        S.n = 0;
+        for (int c = c0; c < min(kids, c0 + kRestMembers / kBigNode); ++c) {
+          const int m = tb.nR[id + c].y;
+          if (m > kBigNode) S.big[S.n_big++] = id + c;
+          else if (m >= 2) S.list[0][S.n++] = id + c;
+        }
+      }
+      __syncthreads();
+      const int n = S.n;
+      __syncthreads();
+      split_below(X, T, tb, n, S, err);
+    }
+    __syncthreads();
+  }
+}
+
+// The nodes listed at `level` with all below them: 32,768 points 2.8 us, 1,048,576 points 22 us (by one
 // block, level after level, 1.5 and 36 us; but with 1,048,576 points at a delta of 40 segments the
-// tree stage took 15.2 ms so, 5.6 now and with a launch for every level).
+// tree stage took 15.2 ms so, 5.6 now and with a launch for every level; one ring of 300,000
+// points, a segment's width 1,600 times theirs: 1.35 ms, 1.52 with a launch for every level, 2.10
+// with each subtree by the warp that takes its root).
 __global__ void __launch_bounds__(kSplitThreads, 1) k_split_rest(const double *__restrict__ X, long long T, TreeBuffers tb,
                                                      int level, unsigned *err) {
-  __shared__ int s_block[kBlockStack], s_warp[kSplitThreads / 32][kWarpStack];
+  __shared__ RestShared S;
   if (failed_above(tb, level)) return;
-  const int b = level % 3, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int b = level % 3;
   const int nbl = min(tb.ctr[kCtrSplit + b], tb.max_blk), nwl = min(tb.ctr[kCtrSplit + 3 + b], tb.max_wrp);
-  for (int bq = blockIdx.x; bq < nbl; bq += gridDim.x)
-    block_subtree(X, T, tb, tb.split_blk[b][bq], s_block, s_warp[wid], err);
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int per = min(32, (nwl + nwarps - 1) / nwarps);
-  for (int wq0 = warp * per; wq0 < nwl; wq0 += nwarps * per) {
-    const int p = lane < per && wq0 + lane < nwl ? tb.split_wrp[b][wq0 + lane] : -1;
-    const int m = p >= 0 ? tb.nR[p].y : 0;
-    for (unsigned large = __ballot_sync(0xffffffffu, m > kLaneNode); large; large &= large - 1)
-      warp_subtree(X, T, tb, __shfl_sync(0xffffffffu, p, __ffs(large) - 1), s_warp[wid], lane, err);
-    bool todo = p >= 0 && m <= kLaneNode;
-    small_subtrees(
-        X, T, tb,
-        [&]() {
-          const int q = todo ? p : -1;
-          todo = false;
-          return q;
-        },
-        lane, err);
+  for (int bq = blockIdx.x; bq < nbl; bq += gridDim.x) split_below_big(X, T, tb, tb.split_blk[b][bq], S, err);
+  int i = (int)((long long)nwl * blockIdx.x / gridDim.x);
+  const int end = (int)((long long)nwl * (blockIdx.x + 1) / gridDim.x);
+  while (i < end) {
+    int n = 0, members = 0;
+    for (;;) {
+      const int count = min((int)blockDim.x, end - i);
+      const int took = take_nodes(tb, tb.split_wrp[b] + i, count, n, members, S);
+      i += took;
+      if (took < count || i == end) break;
+    }
+    split_below(X, T, tb, n, S, err);
   }
 }
 
@@ -2398,7 +2394,7 @@ void launch_tree_build(nv_handle *h) {
   k_node_sums_block<<<sms, kSumThreads, kSumSmem, h->side2>>>(h->x, h->gi, h->nxt, T, *tb, 0, h->d_err);
   cudaEventRecord(h->join2_ev, h->side2);
   // A launch per level down to cells of about an eighth of delta, one for the rest (32,768 points,
-  // 41 launches 172 us, now 9 in 122 us and the one in 2.6; 1,048,576 points, 10 and 24 us)
+  // 41 launches 172 us, now 9 in 122 us and the one in 2.8; 1,048,576 points, 10 and 22 us)
   for (int L = 1; L < tb->grid_levels; ++L)
     k_split_level<<<sms, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, L, h->d_err);
   k_split_rest<<<sms, kSplitThreads, 0, h->stream>>>(h->x, T, *tb, tb->grid_levels, h->d_err);

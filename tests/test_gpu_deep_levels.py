@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from helpers import config1_params, tangle
+from nuvort_b200.rings import single_ring
 from oracle import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -40,6 +41,12 @@ def _compare(params, states, extra=0):
 @pytest.mark.parametrize("n,delta", [(3000, 0.02), (3000, 0.2), (20000, 0.05)])
 def test_points_closer_than_delta(n, delta):
     _compare([config1_params("Tree", delta=delta, overide_timestep_check=True)], [tangle(5, 0.001, n_points=n)])
+
+
+@pytest.mark.parametrize("n", [700, 40000])
+def test_one_ring_of_points_far_closer_than_delta(n):
+    # cells of an eighth of delta hold some hundred points each
+    _compare([config1_params("Tree")], [single_ring(0.03 if n > 1000 else 0.003, n)], extra=3000)
 
 
 @pytest.mark.parametrize("radius", [1e-6, 1e-8])
