@@ -53,11 +53,12 @@ __device__ void log_event(const SolidState &S, SysDyn &d, int s, int base, int k
   if (a < S.ev_cap) S.ev[a] = DevEvent{s, seq, d.itime, kind, i, j};
 }
 
-// loop_killer (reconnection.f90:155-182): a loop that meets a pinned point is left alone.
+// loop_killer (reconnection.f90:155-182): a loop that meets a pinned point is left alone.  Only
+// fewer than four points matter, so the count stops after three hops.
 __device__ void loop_killer(const SolidState &S, SysDyn &d, int s, int base, int particle) {
   const int pc = d.pcount;
   int counter = 1, next = particle;
-  for (int it = 1; it <= pc; ++it) {
+  for (int it = 1; it <= min(pc, 3); ++it) {
     if (pin_i(S.pin[next]) || pin_b(S.pin[next])) return;
     next = S.nxt[next];
     if (next == particle) break;
@@ -85,8 +86,12 @@ __device__ void loop_killer(const SolidState &S, SysDyn &d, int s, int base, int
 // been.  So events happen one by one and in
 // order, and everything between them costs a chunk of tests instead of a chain of loads per
 // slot: 1,273 points, in us a step, premove 590 -> 8, pinsert 500 -> 17, wall_recon 370 -> 7,
-// precon 296 -> 5 (before: one thread per system).
-constexpr int kSweep = 256;
+// precon 296 -> 5 (before: one thread per system).  Where events crowd, the chunks and barriers
+// would cost more than they save: after two events within kNear slots thread 0 goes on alone, by
+// serial(g), the reference's statements whatever slot g does, until kNear slots pass without an
+// event; it says whether g had one (24,297 points that all insert: 84 ms; 121 with a chunk for
+// every event, 78 by one thread).  Not for the cuts, of which the time goes into the events.
+constexpr int kSweep = 256, kCrowd = 3;
 
 // Whether an earlier launch failed.  One thread reads the error word for the block: other
 // systems' blocks of this launch may set it meanwhile (pinsert's), and a block whose threads
@@ -98,10 +103,11 @@ __device__ bool failed_before(const unsigned *err) {
   return s_err != 0;
 }
 
-template <class Test, class Passed, class After, class Act>
-__device__ void ordered_sweep(int base, int n, Test test, Passed passed, After after, Act act) {
-  __shared__ int s_first;
+template <int kNear, class Test, class Passed, class After, class Act, class Serial>
+__device__ void ordered_sweep(int base, int n, Test test, Passed passed, After after, Act act, Serial serial) {
+  __shared__ int s_first, s_next, s_last;
   const int tid = threadIdx.x;
+  int last = -kNear;  // the last event's slot
   for (int i0 = 1; i0 <= n;) {
     const int i = i0 + tid;
     if (tid == 0) s_first = INT_MAX;
@@ -114,9 +120,21 @@ __device__ void ordered_sweep(int base, int n, Test test, Passed passed, After a
     after(min(first, min(n + 1, i0 + kSweep)) - i0);
     if (first == INT_MAX) {
       i0 += kSweep;
-    } else {
+    } else if (kNear == 0 || first - last > kNear) {
       act(base + first);  // every thread: thread 0 applies, the others may help
+      last = first;
       i0 = first + 1;
+    } else {
+      if (tid == 0) {
+        int k = first, l = first;
+        for (; k <= n && k - l <= kNear; ++k)
+          if (serial(base + k)) l = k;
+        s_next = k;
+        s_last = l;
+      }
+      __syncthreads();
+      last = s_last;
+      i0 = s_next;
     }
     __syncthreads();
   }
@@ -157,8 +175,13 @@ __global__ void __launch_bounds__(kSweep) k_solid_pinsert(const SysConst *__rest
   }
   if (tid == 0) d.old_pcount = old_pcount;
   double total_length = 0.0;  // thread 0: in slot order, as the reference adds
-  int free_at = 1;            // no slot below the first empty one empties during the sweep
-  bool full = false;
+  __shared__ int s_free_at;   // no slot below it is empty, nor empties during the sweep
+  __shared__ bool s_full;
+  if (tid == 0) {
+    s_free_at = 1;
+    s_full = false;
+  }
+  __syncthreads();
   auto length = [&](int g) {
     double x[3], gi[3];
     load3(S.X, T, g, x);
@@ -166,8 +189,53 @@ __global__ void __launch_bounds__(kSweep) k_solid_pinsert(const SysConst *__rest
     return dist_gen(x, gi);
   };
   auto tested = [&](int g) { return S.nxt[g] != 0 && !pin_i(S.pin[g]); };
-  ordered_sweep(
-      base, old_pcount, [&](int g) { return !full && tested(g) && length(g) > sc.delta; },
+  // The insertion at slot g, its length measured: into slot s_free_at (by thread 0).  False: out of slots.
+  auto insert = [&](int g, double disti, int pc) {
+    if (s_free_at > pc && pc + 1 > sc.cap) {
+      s_full = true;
+      atomicOr(err, DERR_CAPACITY);
+      return false;
+    }
+    double x[3], gi[3], gb[3];
+    load3(S.X, T, g, x);
+    load3(S.GI, T, g, gi);
+    load3(S.GB, T, g, gb);
+    const int pn = base + s_free_at;
+    if (s_free_at > pc) {
+      d.pcount = pc + 1;
+      clear_slot(S, pn);
+    }
+    // the new point (line.f90:62-84)
+    double xn[3];
+    new_point(x, gi, gb, disti, xn);
+    const int nx = S.nxt[g];
+    for (int c = 0; c < 3; ++c) {
+      S.X[c * T + pn] = xn[c];
+      S.U[c * T + pn] = e_mul(0.5, e_add(S.U[c * T + g], S.U[c * T + nx]));
+      S.U1[c * T + pn] = 0.0;
+      S.U2[c * T + pn] = 0.0;
+    }
+    S.pin[pn] = 0;  // the pinned conditions zeroed (line.f90:82-84)
+    S.prv[pn] = g;
+    S.nxt[pn] = nx;
+    refresh(sc, S, pn);
+    S.prv[nx] = pn;
+    refresh(sc, S, nx);
+    S.nxt[g] = pn;
+    refresh(sc, S, g);
+    log_event(S, d, s, base, NV_EV_INSERT, g, pn);
+    d.insert_count += 1;
+    d.nlive += 1;
+    return true;
+  };
+  auto measure = [&](int g) {  // by thread 0, in slot order
+    const double disti = length(g);
+    total_length = e_add(total_length, disti);
+    margin_note(d, 0, disti, sc.delta);
+    return disti;
+  };
+  ordered_sweep<kCrowd>(
+      base, old_pcount, [&](int g) { return !s_full && tested(g) && length(g) > sc.delta; },
       [&](int g, int k) {
         const bool t = tested(g);
         s_len[k] = t ? length(g) : 0.0;
@@ -180,47 +248,22 @@ __global__ void __launch_bounds__(kSweep) k_solid_pinsert(const SysConst *__rest
       [&](int g) {
         // the first empty slot (minloc(f(:)%infront)), else the array grows by one
         const int pc = *(volatile int *)&d.pcount;
-        free_at = first_free(S, base, free_at, pc);
-        if (free_at > pc && pc + 1 > sc.cap) {
-          full = true;
-          if (tid == 0) atomicOr(err, DERR_CAPACITY);
-          return;
-        }
+        const int f = first_free(S, base, s_free_at, pc);
         if (tid != 0) return;
-        double x[3], gi[3], gb[3];
-        load3(S.X, T, g, x);
-        load3(S.GI, T, g, gi);
-        load3(S.GB, T, g, gb);
-        const double disti = dist_gen(x, gi);
-        total_length = e_add(total_length, disti);
-        margin_note(d, 0, disti, sc.delta);
-        const int pn = base + free_at;
-        if (free_at > pc) {
-          d.pcount = pc + 1;
-          clear_slot(S, pn);
-        }
-        // the new point (line.f90:62-84)
-        double xn[3];
-        new_point(x, gi, gb, disti, xn);
-        const int nx = S.nxt[g];
-        for (int c = 0; c < 3; ++c) {
-          S.X[c * T + pn] = xn[c];
-          S.U[c * T + pn] = e_mul(0.5, e_add(S.U[c * T + g], S.U[c * T + nx]));
-          S.U1[c * T + pn] = 0.0;
-          S.U2[c * T + pn] = 0.0;
-        }
-        S.pin[pn] = 0;  // the pinned conditions zeroed (line.f90:82-84)
-        S.prv[pn] = g;
-        S.nxt[pn] = nx;
-        refresh(sc, S, pn);
-        S.prv[nx] = pn;
-        refresh(sc, S, nx);
-        S.nxt[g] = pn;
-        refresh(sc, S, g);
-        log_event(S, d, s, base, NV_EV_INSERT, g, pn);
-        d.insert_count += 1;
-        d.nlive += 1;
+        s_free_at = f;
+        insert(g, measure(g), pc);
+      },
+      [&](int g) {
+        if (s_full || !tested(g)) return false;
+        const double disti = measure(g);
+        if (!(disti > sc.delta)) return false;
+        const int pc = d.pcount;
+        int f = s_free_at;
+        while (f <= pc && S.nxt[base + f] != 0) ++f;
+        s_free_at = f;
+        return insert(g, disti, pc);
       });
+  const bool full = s_full;
   if (full) return;
   int empty = 0;
   const int pc = *(volatile int *)&d.pcount;
@@ -257,7 +300,56 @@ __global__ void __launch_bounds__(kSweep) k_solid_precon(const SysConst *__restr
   if ((d.itime % sc.recon_shots) != 0) return;
   const int base = sc.base;
   const long long T = S.T;
-  ordered_sweep(
+  // The reference's statements for slot g (by thread 0); whether its closest point was near enough.
+  auto slot = [&](int g) {
+    if (S.nxt[g] == 0) return false;
+    const int pari = S.nxt[g], parb = S.prv[g];
+    const double cd = S.CD[g];
+    if (cd > NV_EPS) margin_note(d, 2, cd, sc.delta / 2.);
+    if (!((cd < sc.delta / 2.) && (cd > NV_EPS))) return false;
+    const int j = S.cl[g];
+    if (j == pari || j == parb || j == 0) return true;
+    if (S.nxt[j] == 0) return true;
+    const int parjb = S.prv[j];
+    double t1[3], t2[3], x[3], gi_[3], gb_[3];
+    for (int q = 0; q < 2; ++q) {  // norm_tanf (general.f90:106-117)
+      double *t = q ? t2 : t1;
+      const int p = q ? j : g;
+      load3(S.X, T, p, x);
+      load3(S.GI, T, p, gi_);
+      load3(S.GB, T, p, gb_);
+      deriv1(x, gi_, gb_, t);
+      const double len = e_sqrt(e_add(e_add(e_sq(t[0]), e_sq(t[1])), e_sq(t[2])));
+      for (int c = 0; c < 3; ++c) t[c] = e_div(t[c], len);
+    }
+    const double dot_val = dot3(t1, t2);
+    margin_note(d, 3, dot_val, 0.9);
+    if (dot_val > 0.9) return true;
+    double xi[3], gii[3], gbi[3], xj[3], gij[3], gbj[3], xpi[3], xpj[3];
+    load3(S.X, T, g, xi);
+    load3(S.GI, T, g, gii);
+    load3(S.GB, T, g, gbi);
+    load3(S.X, T, j, xj);
+    load3(S.GI, T, j, gij);
+    load3(S.GB, T, j, gbj);
+    load3(S.X, T, pari, xpi);
+    load3(S.X, T, parjb, xpj);
+    const double l_before =
+        e_add(e_add(e_add(dist_gen(xi, gii), dist_gen(xi, gbi)), dist_gen(xj, gij)), dist_gen(xj, gbj));
+    const double l_after =
+        e_add(e_add(e_add(dist_gen(xi, gbi), dist_gen(xi, xj)), dist_gen(xj, gij)), dist_gen(xpi, xpj));
+    if (!(l_after <= l_before)) return true;
+    d.recon_count += 1;
+    log_event(S, d, s, base, NV_EV_RECON, g, j);
+    S.nxt[parjb] = pari;
+    S.prv[pari] = parjb;
+    S.nxt[g] = j;
+    S.prv[j] = g;
+    loop_killer(S, d, s, base, pari);
+    loop_killer(S, d, s, base, g);
+    return true;
+  };
+  ordered_sweep<0>(
       base, d.pcount,
       [&](int g) {
         const double cd = S.CD[g];
@@ -268,53 +360,9 @@ __global__ void __launch_bounds__(kSweep) k_solid_precon(const SysConst *__restr
       },
       [](int) {},
       [&](int g) {
-        if (threadIdx.x != 0) return;
-        if (S.nxt[g] == 0) return;
-        const int pari = S.nxt[g], parb = S.prv[g];
-        const double cd = S.CD[g];
-        if (cd > NV_EPS) margin_note(d, 2, cd, sc.delta / 2.);
-        if (!((cd < sc.delta / 2.) && (cd > NV_EPS))) return;
-        const int j = S.cl[g];
-        if (j == pari || j == parb || j == 0) return;
-        if (S.nxt[j] == 0) return;
-        const int parjb = S.prv[j];
-        double t1[3], t2[3], x[3], gi_[3], gb_[3];
-        for (int q = 0; q < 2; ++q) {  // norm_tanf (general.f90:106-117)
-          double *t = q ? t2 : t1;
-          const int p = q ? j : g;
-          load3(S.X, T, p, x);
-          load3(S.GI, T, p, gi_);
-          load3(S.GB, T, p, gb_);
-          deriv1(x, gi_, gb_, t);
-          const double len = e_sqrt(e_add(e_add(e_sq(t[0]), e_sq(t[1])), e_sq(t[2])));
-          for (int c = 0; c < 3; ++c) t[c] = e_div(t[c], len);
-        }
-        const double dot_val = dot3(t1, t2);
-        margin_note(d, 3, dot_val, 0.9);
-        if (dot_val > 0.9) return;
-        double xi[3], gii[3], gbi[3], xj[3], gij[3], gbj[3], xpi[3], xpj[3];
-        load3(S.X, T, g, xi);
-        load3(S.GI, T, g, gii);
-        load3(S.GB, T, g, gbi);
-        load3(S.X, T, j, xj);
-        load3(S.GI, T, j, gij);
-        load3(S.GB, T, j, gbj);
-        load3(S.X, T, pari, xpi);
-        load3(S.X, T, parjb, xpj);
-        const double l_before =
-            e_add(e_add(e_add(dist_gen(xi, gii), dist_gen(xi, gbi)), dist_gen(xj, gij)), dist_gen(xj, gbj));
-        const double l_after =
-            e_add(e_add(e_add(dist_gen(xi, gbi), dist_gen(xi, xj)), dist_gen(xj, gij)), dist_gen(xpi, xpj));
-        if (!(l_after <= l_before)) return;
-        d.recon_count += 1;
-        log_event(S, d, s, base, NV_EV_RECON, g, j);
-        S.nxt[parjb] = pari;
-        S.prv[pari] = parjb;
-        S.nxt[g] = j;
-        S.prv[j] = g;
-        loop_killer(S, d, s, base, pari);
-        loop_killer(S, d, s, base, g);
-      });
+        if (threadIdx.x == 0) slot(g);
+      },
+      slot);
 }
 
 // wall_recon (reconnection.f90:66-150) for one system: a point within delta/2 of a solid
@@ -328,7 +376,47 @@ __global__ void __launch_bounds__(kSweep) k_solid_wall_recon(const SysConst *__r
   if ((d.itime % sc.recon_shots) != 0) return;
   const int base = sc.base;
   const long long T = S.T;
-  ordered_sweep(
+  // The reference's statements for slot g (by thread 0); whether they did anything.
+  auto slot = [&](int g) {
+    if (S.nxt[g] == 0) return false;
+    // a cleared pair: the reference goes on to test the cleared i at x = 0, inside every
+    // wall while delta < box, so nothing more happens to it
+    if (clear_wall_pair(S, d, s, base, g)) return true;
+    if (pin_i(S.pin[g]) || pin_b(S.pin[g])) return false;
+    bool cut = false;
+    for (int a = 0; a < 3; ++a) {  // x, y, z walls in turn, each on the state the last left
+      if (!sc.solid[a]) continue;
+      const double xa = S.X[a * T + g];
+      const double lim = e_mul(0.5, e_sub(sc.box[a], sc.delta));
+      int side = 0;
+      if (xa > lim) side = 1;
+      else if (xa < -lim) side = -1;
+      if (side == 0) continue;
+      cut = true;
+      const int pari = S.nxt[g], parb = S.prv[g];
+      int w[3] = {0, 0, 0};
+      w[a] = side;
+      S.pin[pari] = pin_encode(pin_i(S.pin[pari]), 1, w);
+      S.prv[pari] = pari;
+      S.pin[parb] = pin_encode(1, pin_b(S.pin[parb]), w);
+      S.nxt[parb] = parb;
+      clear_slot(S, g);
+      int cleared = 1;
+      if (pin_i(S.pin[pari]) && pin_b(S.pin[pari])) {
+        clear_slot(S, pari);
+        ++cleared;
+      }
+      if (pin_i(S.pin[parb]) && pin_b(S.pin[parb])) {
+        clear_slot(S, parb);
+        ++cleared;
+      }
+      log_event(S, d, s, base, NV_EV_WALL, g, cleared);
+      d.wall_recon_count += 1;
+      d.nlive -= cleared;
+    }
+    return cut;
+  };
+  ordered_sweep<0>(
       base, d.pcount,
       [&](int g) {
         if (S.nxt[g] == 0) return false;
@@ -341,42 +429,9 @@ __global__ void __launch_bounds__(kSweep) k_solid_wall_recon(const SysConst *__r
       },
       [](int, int) {}, [](int) {},
       [&](int g) {
-        if (threadIdx.x != 0) return;
-        if (S.nxt[g] == 0) return;
-        // a cleared pair: the reference goes on to test the cleared i at x = 0, inside every
-        // wall while delta < box, so nothing more happens to it
-        if (clear_wall_pair(S, d, s, base, g)) return;
-        if (pin_i(S.pin[g]) || pin_b(S.pin[g])) return;
-        for (int a = 0; a < 3; ++a) {  // x, y, z walls in turn, each on the state the last left
-          if (!sc.solid[a]) continue;
-          const double xa = S.X[a * T + g];
-          const double lim = e_mul(0.5, e_sub(sc.box[a], sc.delta));
-          int side = 0;
-          if (xa > lim) side = 1;
-          else if (xa < -lim) side = -1;
-          if (side == 0) continue;
-          const int pari = S.nxt[g], parb = S.prv[g];
-          int w[3] = {0, 0, 0};
-          w[a] = side;
-          S.pin[pari] = pin_encode(pin_i(S.pin[pari]), 1, w);
-          S.prv[pari] = pari;
-          S.pin[parb] = pin_encode(1, pin_b(S.pin[parb]), w);
-          S.nxt[parb] = parb;
-          clear_slot(S, g);
-          int cleared = 1;
-          if (pin_i(S.pin[pari]) && pin_b(S.pin[pari])) {
-            clear_slot(S, pari);
-            ++cleared;
-          }
-          if (pin_i(S.pin[parb]) && pin_b(S.pin[parb])) {
-            clear_slot(S, parb);
-            ++cleared;
-          }
-          log_event(S, d, s, base, NV_EV_WALL, g, cleared);
-          d.wall_recon_count += 1;
-          d.nlive -= cleared;
-        }
-      });
+        if (threadIdx.x == 0) slot(g);
+      },
+      slot);
 }
 
 // premove (line.f90:103-129) for one system.
@@ -397,35 +452,40 @@ __global__ void __launch_bounds__(kSweep) k_solid_premove(const SysConst *__rest
     load3(S.X, T, S.nxt[S.nxt[g]], y);
     return dist_gen(x, y);
   };
-  ordered_sweep(
+  // The reference's statements for slot g (by thread 0); whether its test passed.
+  auto slot = [&](int g) {
+    if (S.nxt[g] == 0) return false;
+    if (pin_i(S.pin[g])) return false;
+    const int infront = S.nxt[g];
+    if (pin_i(S.pin[infront])) return false;
+    const int tinfront = S.nxt[infront];
+    double xi[3], xt[3];
+    load3(S.X, T, g, xi);
+    load3(S.X, T, tinfront, xt);
+    const double dii = dist_gen(xi, xt);
+    margin_note(d, 1, dii, thr);
+    if (dii < thr) {
+      S.prv[tinfront] = g;
+      S.nxt[g] = tinfront;
+      clear_slot(S, infront);
+      log_event(S, d, s, base, NV_EV_REMOVE, g, infront);
+      d.nlive -= 1;
+      loop_killer(S, d, s, base, g);
+      d.remove_count += 1;
+    }
+    clear_wall_pair(S, d, s, base, g);
+    return dii < thr;
+  };
+  ordered_sweep<kCrowd>(
       base, d.pcount, [&](int g) { return looked_at(g) && distance(g) < thr; },
       [&](int g, int) {
         if (looked_at(g)) margin_note(d, 1, distance(g), thr);
       },
       [](int) {},
       [&](int g) {
-        if (threadIdx.x != 0) return;
-        if (S.nxt[g] == 0) return;
-        if (pin_i(S.pin[g])) return;
-        const int infront = S.nxt[g];
-        if (pin_i(S.pin[infront])) return;
-        const int tinfront = S.nxt[infront];
-        double xi[3], xt[3];
-        load3(S.X, T, g, xi);
-        load3(S.X, T, tinfront, xt);
-        const double dii = dist_gen(xi, xt);
-        margin_note(d, 1, dii, thr);
-        if (dii < thr) {
-          S.prv[tinfront] = g;
-          S.nxt[g] = tinfront;
-          clear_slot(S, infront);
-          log_event(S, d, s, base, NV_EV_REMOVE, g, infront);
-          d.nlive -= 1;
-          loop_killer(S, d, s, base, g);
-          d.remove_count += 1;
-        }
-        clear_wall_pair(S, d, s, base, g);
-      });
+        if (threadIdx.x == 0) slot(g);
+      },
+      slot);
 }
 
 }  // namespace
