@@ -430,8 +430,10 @@ cudaError_t direct_kernels_setup() {
 // nv_set_direct_split, overrides the choice): 8 per block of the split kernel, except
 //   * 2 while the blocks of 2 (three to an SM) about fit the GPU at once, counting two thirds
 //     of the slots as live: the summing chain sets the time then, and it is the shorter the
-//     fewer terms an SM computes beside it (600 points: 183 us, 206 with 8; but 1000 points,
-//     a second wave of blocks: 452 us, 327 with 8; 4 per block is nowhere ahead by 3 %);
+//     fewer terms an SM computes beside it (600 points: 181 us, 203 with 8; but 1000 points,
+//     a second wave of blocks: 450 us, 322 with 8; 4 per block is nowhere ahead by 3 %).  Handles
+//     allocated to their points lose by it from 889 to 1,332 slots, where the share of live
+//     slots, known only at upload, would decide for 8 (714 us at 1000 points before either);
 //   * one thread per target (64 to a block) from 80,000 slots on, four warps to each
 //     scheduler, which need no exchange (50,000 points: 623 ms, 488 with 8; 80,000: 1.22 s,
 //     1.23 s).

@@ -346,14 +346,15 @@ __global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys) return;
   const SysConst &sc = scs[s];
-  const int pc = (sc.use_tree || sc.sched_tree) ? dyn[s].pcount : 0;
+  const bool lost = *err & DERR_TIMEOUT;  // the pass before gave up: its ranks say nothing
+  const int pc = (sc.use_tree || sc.sched_tree) && !lost ? dyn[s].pcount : 0;
   const double h = -sc.bsize / 2.0;
   const int *r0 = tb.root_rank + 9 * s, *r1 = r0 + 9;  // this system's first slot, the next one's
   tb.nP[s] = make_double4(h, h, h, 0);
   tb.nA[s] = make_double4(0, 0, 0, sc.bsize);
   tb.nB[s] = make_double4(0, 0, 0, 0);
   tb.nI[s] = make_int4(pc, kEnd, kEnd, pc >= 1 ? nxt[sc.base + 1] : 0);
-  tb.nR[s] = make_int2(r0[0], r1[0] - r0[0]);
+  tb.nR[s] = lost ? make_int2(0, 0) : make_int2(r0[0], r1[0] - r0[0]);
   tb.nDepth[s] = 0;
   tb.nKids[s] = 0;
   tb.nLeaf[s] = pc == 1 ? sc.base + 1 : 0;
@@ -372,10 +373,10 @@ __global__ void k_roots(const SysConst *__restrict__ scs, SysDyn *dyn, int nsys,
 }
 
 // The children's member lists; also notes the block-summed nodes listed so far (depth 1).
-__global__ void k_root_scatter(const int *__restrict__ sys_of, TreeBuffers tb, int nsys) {
+__global__ void k_root_scatter(const int *__restrict__ sys_of, TreeBuffers tb, int nsys, const unsigned *err) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p == 0) tb.ctr[kCtrBigSnap] = min(tb.ctr[kCtrBig], tb.max_big);
-  if (p >= tb.root_rank[9 * nsys]) return;  // the live slots of all systems
+  if (*err & DERR_TIMEOUT || p >= tb.root_rank[9 * nsys]) return;  // (the live slots of all systems)
   const int g = tb.members[p], d = tb.rdig[g], s = sys_of[g];
   if (d < 8 && tb.root_ok[s]) tb.members[tb.root_mb[8 * s + d] + tb.rrank[g]] = g;
 }
@@ -2386,7 +2387,7 @@ void launch_tree_build(nv_handle *h) {
   k_root_sums<<<h->nsys, kSumThreads, kSumSmem, h->side>>>(h->x, T, *tb, h->nsys, h->nxt, h->d_err);
   cudaEventRecord(h->join_ev, h->side);
   const int sms = n_sms();
-  k_root_scatter<<<grid_for(T, TB), TB, 0, h->stream>>>(h->sys_of, *tb, h->nsys);
+  k_root_scatter<<<grid_for(T, TB), TB, 0, h->stream>>>(h->sys_of, *tb, h->nsys, h->d_err);
   // the big depth-1 nodes' sums (the longest sequential chains after the roots') start as soon
   // as the roots' split has listed them and written their member lists, beside the levels
   cudaEventRecord(h->fork2_ev, h->stream);
