@@ -382,9 +382,10 @@ void build_image_worklists(nv_handle *h, int small, std::vector<int4> &w8, std::
 // Slots up to which a system's items of the mixed direct sum go to a warp each instead of a block of
 // eight, whose warps share out a tile of 256 segments and whose setup costs eight times as much:
 // 1,000, where the items of such systems are 20 an SM at least, fewer than half of what can be
-// resident (velocity stage, us, a warp and a block: 2,000 systems of 30 points 397, 1,571; 512 of
-// 100 606, 1,351; 16 of 100, 3,024 items, 68, 80; 100 of 500 1,612, 1,782; but 64 of 1,000,
-// 1,640 slots each, 3,781, 3,702; and 4 of 100, 756 items, 62, 49; 4 of 300, 1,836 items, 100, 70).
+// resident (velocity stage, us, a warp and a block: 2,000 systems of 30 points 370, 1,506; 512 of
+// 100 519, 1,285; 16 of 100, 3,024 items, 65, 78; 100 of 500, 840 slots each, 1,316, 1,658; less
+// above that, 16 of 3,000 6,499, 6,591; but 4 of 100, 756 items, 61, 49; 4 of 300, 1,836 items,
+// 92, 69; one of 1,000 169, 85).
 int mixed_small_slots(const nv_handle *h) {
   constexpr int kSmall = 1000;
   long long items = 0;

@@ -2,9 +2,8 @@
 //
 // k_direct_mixed<W>: a block of W warps per 32 targets and periodic image, each warp (a lane per
 // target) over its share of every tile of the target system's segments (W = 8; 1 for ensembles of
-// small systems).  The tiles stream
-// through shared memory by 1-D bulk copies (pairs of segments side by side, 96 bytes a pair:
-// position hi, position lo, segment vector).  r = x_j - x_i is formed from the hi/lo split, so
+// small systems).  The tiles stream through shared memory by 1-D bulk copies (pairs of segments
+// side by side, 96 bytes a pair: position hi, position lo, segment vector).  r = x_j - x_i is formed from the hi/lo split, so
 // it is exact to ~1e-16 before rounding to FP32.  Every 32 terms are summed in FP32 and those
 // sums are added with Kahan compensation; pairs closer than near_radius are evaluated in FP64
 // with the reference expression from the FP64 segment records.  The warps' sums are added in
@@ -99,41 +98,46 @@ __device__ __forceinline__ int ordered(float x) {
 }
 __device__ __forceinline__ float float_of(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
 
-// The pairs of a sub-sum (bit p: pair p) with a segment whose line guard may act on a target of the
-// warp: all targets lie within a ball around the point that `c` holds as a target, of radius R, so
-// |r x d| of each is at least |rc x d| - R |d| and |r| at most |rc| + R, and the guard cannot act
-// where |rc x d| exceeds |d| (R + sqrt(line) (|rc| + R)).  A lane takes one pair for all targets.
+// The pairs of a sub-sum (bit p: pair p) that need no guard for any of the warp's targets: all targets
+// lie within a ball around the point that `c` holds as a target, of radius R, so |r| of each lies
+// between |rc| - R and |rc| + R and |r x d| is at least |rc x d| - R |d|.  A pair is beyond every
+// target's far bound where (|rc| - R)^2 exceeds it, and the line guard cannot act where |rc x d|
+// exceeds |d| (R + sqrt(line) (|rc| + R)).  A lane takes one pair for all targets.
 struct WarpBall {
   LaneTarget c;
-  float radius, slope;  // R (1 + sqrt(line)) and sqrt(line), widened for the FP32 rounding
+  float radius, reach, slope;  // R, R (1 + sqrt(line)) and sqrt(line), widened for the FP32 rounding
 };
-__device__ __forceinline__ unsigned line_mask(const ulonglong2 *pairs, int np, const WarpBall &ball) {
+__device__ __forceinline__ unsigned clean_mask(const ulonglong2 *pairs, int np, const WarpBall &ball) {
   const int lane = threadIdx.x & 31;
   static_assert(kWarpPairs <= 32, "a lane per pair");
-  bool may = false;
+  bool clean = false;
   if (lane < np) {
     const PairVec r = pair_vec(pairs + 6 * lane, ball.c);
     const PairSeg d = pair_seg(pairs + 6 * lane);
-    const f32x2 kMinus = pack2(-1.f, -1.f), radius = pack2(ball.radius, ball.radius), slope = pack2(ball.slope, ball.slope);
+    const f32x2 kMinus = pack2(-1.f, -1.f), reach = pack2(ball.reach, ball.reach), slope = pack2(ball.slope, ball.slope),
+                radius = pack2(-ball.radius, -ball.radius), shrink = pack2(0.99999f, 0.99999f);
     const f32x2 cx = fma2(r.ry, d.dz, mul2(r.rz, d.ndy)), cy = fma2(r.rz, d.dx, mul2(mul2(r.rx, kMinus), d.dz)),
                 cz = fma2(r.rx, d.dy, mul2(r.ry, d.ndx));
-    const f32x2 reach = fma2(slope, pack2(sqrt_fast(lo2(r.a)), sqrt_fast(hi2(r.a))), radius);
-    const f32x2 cr2 = square2(cx, cy, cz), lim = mul2(square2(d.dx, d.dy, d.dz), mul2(reach, reach));
-    may = lo2(cr2) < lo2(lim) || hi2(cr2) < hi2(lim);
+    const f32x2 rl = pack2(sqrt_fast(lo2(r.a)), sqrt_fast(hi2(r.a)));
+    const f32x2 over = fma2(slope, rl, reach), gap = fma2(shrink, rl, radius), gap2 = mul2(gap, gap);
+    const f32x2 cr2 = square2(cx, cy, cz), lim = mul2(square2(d.dx, d.dy, d.dz), mul2(over, over));
+    clean = lo2(gap) > 0.f && hi2(gap) > 0.f && lo2(gap2) > lo2(d.far) && hi2(gap2) > hi2(d.far) &&
+            lo2(cr2) >= lo2(lim) && hi2(cr2) >= hi2(lim);
   }
-  return __ballot_sync(0xffffffffu, may);
+  return __ballot_sync(0xffffffffu, clean);
 }
 
 // Bound: the FP32 pipe (about 35 lane operations a far term, the adds, multiplies and FMAs of
-// two segments packed into one instruction).  A pair of segments that every lane's target is
-// far from needs none of the conditioning guards but the line guard, and that only where
-// line_mask, once per sub-sum, finds that it may act; the other pairs take the guards lane by
-// lane.  The tiles pass through a ring of kStages buffers with an mbarrier for full and one
-// for empty each, so that no warp waits for the block's others.
-// 30,011 points: 42.0 ms; 1,501 points: 151 us (a lane per target and image with scalar
+// two segments packed into one instruction) and the special-function unit.  Nearly all pairs of a
+// tangle need no guard for any target of the warp; clean_mask finds them, once per sub-sum, and
+// they are taken four at a time without a test or a vote.  Of the others, those that every
+// target is far from take the line guard alone, target by target, the rest all guards.  The tiles
+// pass through a ring of kStages buffers with an mbarrier for full and one for empty each, so
+// that no warp waits for the block's others.
+// 30,011 points: 36.6 ms; 1,501 points: 138 us (a lane per target and image with scalar
 // arithmetic and all guards, 113 issue slots a term: 74.1 ms and 409 us; packed, but all guards
-// and a barrier per tile: 55.4 ms and 236 us).  The line guard left out beyond 4|d|: 38.8 ms and
-// 136 us; its exact test on every far pair: 44.8 ms and 153 us.
+// and a barrier per tile: 55.4 ms and 236 us; a vote per pair on the far bound, the line guard's
+// exact test on every far pair: 44.8 ms and 153 us, without that guard 38.8 ms and 136 us).
 template <int W>
 __global__ void __launch_bounds__(32 * W, 24 / W) k_direct_mixed(
     const SysConst *__restrict__ scs, const SysDyn *__restrict__ dyn, const int4 *__restrict__ work,
@@ -207,7 +211,8 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_direct_mixed(
       half2 = fmaf(half, half, half2);
     }
     ball.slope = sin_line * 1.00001f + 1e-6f;
-    ball.radius = sqrtf(half2) * (1.00001f + ball.slope);
+    ball.radius = sqrtf(half2) * 1.00001f;
+    ball.reach = ball.radius * (1.f + ball.slope);
   }
   const double gq64 = sc.quant_circ / (4.0 * NV_PI);
   const double nr = near_factor * sc.delta;
@@ -243,26 +248,42 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_direct_mixed(
     for (int p0 = wid * kWarpPairs; p0 < in_tile; p0 += W * kWarpPairs) {
       const int p1 = min(in_tile, p0 + kWarpPairs);
       const int bp = behind_p - k * kPairs;
-      // the pairs that not every target may take without guards however far it is: a line guard
-      // may act, or the pair holds some target's behind segment
-      unsigned special = line_mask(tile + 6 * p0, p1 - p0, ball) |
-                         __reduce_or_sync(0xffffffffu, bp >= p0 && bp < p1 ? 1u << (bp - p0) : 0u);
+      // (a pair that holds some target's behind segment is never clean)
+      unsigned clean = clean_mask(tile + 6 * p0, p1 - p0, ball) &
+                       ~__reduce_or_sync(0xffffffffu, bp >= p0 && bp < p1 ? 1u << (bp - p0) : 0u);
       f32x2 u[3] = {pack2(0.f, 0.f), pack2(0.f, 0.f), pack2(0.f, 0.f)};
-#pragma unroll 2
+      auto fast = [&](int p) {
+        const ulonglong2 *q = tile + 6 * p;
+        const PairVec r = pair_vec(q, t);
+        const PairGeo g2 = pair_geo(r, pair_seg(q));
+        const f32x2 sum = add2(g2.pp, g2.re);
+        const f32x2 f = mul2(g2.num, pack2(rcp_fast(lo2(sum)), rcp_fast(hi2(sum))));
+        u[0] = fma2(f, g2.cx, u[0]);
+        u[1] = fma2(f, g2.cy, u[1]);
+        u[2] = fma2(f, g2.cz, u[2]);
+      };
+#pragma unroll 1
       for (int p = p0; p < p1; ++p) {
+        if ((clean & 15u) == 15u) {  // (no bits past p1)
+          fast(p);
+          fast(p + 1);
+          fast(p + 2);
+          fast(p + 3);
+          clean >>= 4;
+          p += 3;
+          continue;
+        }
+        const bool plain = clean & 1u;
+        clean >>= 1;
+        if (plain) {
+          fast(p);
+          continue;
+        }
         const ulonglong2 *q = tile + 6 * p;
         const PairVec r = pair_vec(q, t);
         const PairSeg d = pair_seg(q);
-        const bool plain = !(special & 1u), far = lo2(r.a) > lo2(d.far) && hi2(r.a) > hi2(d.far);
-        special >>= 1;
-        if (__all_sync(0xffffffffu, far && plain)) {
-          const PairGeo g2 = pair_geo(r, d);
-          const f32x2 sum = add2(g2.pp, g2.re);
-          const f32x2 f = mul2(g2.num, pack2(rcp_fast(lo2(sum)), rcp_fast(hi2(sum))));
-          u[0] = fma2(f, g2.cx, u[0]);
-          u[1] = fma2(f, g2.cy, u[1]);
-          u[2] = fma2(f, g2.cz, u[2]);
-        } else if (__all_sync(0xffffffffu, far && p != bp)) {  // the line guard alone, target by target
+        if (__all_sync(0xffffffffu, lo2(r.a) > lo2(d.far) && hi2(r.a) > hi2(d.far) && p != bp)) {
+          // the line guard alone, target by target
           const PairGeo g2 = pair_geo(r, d);
           const f32x2 sum = add2(g2.pp, g2.re), c = square2(d.dx, d.dy, d.dz), cr2 = square2(g2.cx, g2.cy, g2.cz);
           const bool bad[2] = {lo2(cr2) < gd.line * lo2(c) * fminf(lo2(r.a), lo2(g2.ee)),
