@@ -65,22 +65,27 @@ def test_crowded_lines(share):
 
 
 def test_a_line_that_loses_most_of_its_points():
-    # in slot order: no event is alone (32,768 points, 95 % pass: 68 ms when every round looked for
-    # such events with the neighbourhoods in its map, 37 ms one after the other)
+    # in slot order: no event is alone.  32,768 points, 95 % pass: 38 ms, 17 times as long as where 5 %
+    # pass and most events are alone (68 ms, 31 times, when every round looked for such events with
+    # the neighbourhoods in its map)
     from nuvort_b200.api import Handle
     st = tangle(3, 0.001, n_points=32768)
     st.x = st.x + np.random.default_rng(1).normal(0.0, 1.5e-4, st.x.shape)
     ahead = st.infront[st.infront - 1] - 1
     two = np.linalg.norm(st.x - st.x[ahead], axis=1)
-    p = config0_params(delta=float(np.quantile(two, 0.95)) / 0.99, overide_timestep_check=True)
-    with Handle(p, [st.pcount + 8], states=[st]) as h:
-        best = 1e9
-        for _ in range(4):
-            h.upload(0, st)
-            h.set_clock(0, 0.0, 1)
-            h.counters()
-            t = time.perf_counter()
-            h.stage("premove")
-            best = min(best, time.perf_counter() - t)
-        assert h.counters().remove_count > 12000
-    assert best < 0.052
+    took = []
+    for share in (0.05, 0.95):
+        p = config0_params(delta=float(np.quantile(two, share)) / 0.99, overide_timestep_check=True)
+        with Handle(p, [st.pcount + 8], states=[st]) as h:
+            best = 1e9
+            for _ in range(4):
+                h.upload(0, st)
+                h.set_clock(0, 0.0, 1)
+                h.counters()
+                t = time.perf_counter()
+                h.stage("premove")
+                best = min(best, time.perf_counter() - t)
+            took.append(best)
+            removed = h.counters().remove_count
+    assert removed > 12000
+    assert took[1] < 24 * took[0]
